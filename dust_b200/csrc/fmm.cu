@@ -192,6 +192,8 @@ extern "C" int dust_octree_create(const dust_fmm_params *prm, dust_octree **out)
   }
   for (int e = 0; e < 12; ++e) cudaEventCreate(&o->ev[e]);
   st = build_tables(o);
+  if (st == DUST_OK) st = grow(o->small, 64 * 8);
+  if (st == DUST_OK && cudaMemset(o->small.p, 0, 64 * 8) != cudaSuccess) st = DUST_ERR_CUDA;
   if (st == DUST_OK) st = build_shift_tables(o);
   if (st == DUST_OK) st = m2l_batch_tables(o);
   if (st != DUST_OK) {
@@ -207,13 +209,13 @@ extern "C" int dust_octree_destroy(dust_octree *o) {
   cudaStreamSynchronize(o->stream);
   for (int l = 0; l <= DUST_MAXLEV; ++l) {
     devbuf_free(o->dtab[l]);
-    devbuf_free(o->dtab32[l]);
     devbuf_free(o->dtabs[l]);
   }
   devbuf_free(o->m2l_buf);
   devbuf_free(o->ahat);
   devbuf_free(o->m2l_bat);
   devbuf_free(o->jsum);
+  devbuf_free(o->srcix);
   devbuf_free(o->shift);
   devbuf_free(o->ffbuf);
   devbuf_free(o->elem_work);
@@ -373,15 +375,23 @@ __global__ void k_indicators(uint32_t ntot, const uint8_t *__restrict__ flags,
 
 __global__ void k_compact(TreeGeom G, uint32_t ntot, const uint8_t *__restrict__ flags,
                           const uint32_t *__restrict__ cidx,
-                          const uint32_t *__restrict__ lidx, uint32_t *__restrict__ act_key,
-                          uint8_t *__restrict__ act_lev, uint32_t *__restrict__ leaf_ci) {
+                          const uint32_t *__restrict__ lidx,
+                          const uint32_t *__restrict__ cstart, uint32_t *__restrict__ act_key,
+                          uint8_t *__restrict__ act_lev, uint32_t *__restrict__ leaf_ci,
+                          uint32_t *__restrict__ srcix) {
   uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ntot) return;
   uint8_t f = flags[c];
-  if (!(f & FL_ACTIVE)) return;
+  if (!(f & FL_ACTIVE)) {
+    srcix[c] = ~0u;
+    return;
+  }
   int l = 1;
   while (l < G.ll && c >= G.lev_off[l + 1]) ++l;
   uint32_t ci = cidx[c];
+  const uint32_t key = c - G.lev_off[l];
+  // M2L sources: an empty active cell has a = 0
+  srcix[c] = cell_hi(G, cstart, l, key) > cell_lo(G, cstart, l, key) ? ci : ~0u;
   act_key[ci] = c - G.lev_off[l];
   act_lev[ci] = (uint8_t)l;
   if (f & FL_LEAF) leaf_ci[lidx[c]] = ci;
@@ -1365,7 +1375,7 @@ int fmm_prepare_device(dust_octree *o, int n, const double *cen, const double *d
   DUST_TRY(grow(o->ind, (size_t)(ntot + 1) * 8));
   DUST_TRY(grow(o->cidx, (size_t)(ntot + 1) * 4));
   DUST_TRY(grow(o->lidx, (size_t)(ntot + 1) * 4));
-  DUST_TRY(grow(o->small, 64 * 8));
+  DUST_TRY(grow(o->srcix, (size_t)(ntot + 1) * 4));
   DUST_TRY(grow(o->outs, N * 9 * 8));
   uint32_t *keys = (uint32_t *)o->keys.p, *keys_s = (uint32_t *)o->keys_s.p;
   uint32_t *vals = (uint32_t *)o->vals.p, *perm = (uint32_t *)o->perm.p;
@@ -1410,13 +1420,17 @@ int fmm_prepare_device(dust_octree *o, int n, const double *cen, const double *d
   DUST_CUDA(cub::DeviceScan::ExclusiveSum(o->cub_tmp.p, tb, ia, cidx, (int)ntot + 1, st));
   DUST_CUDA(cub::DeviceScan::ExclusiveSum(o->cub_tmp.p, tb, il, lidx, (int)ntot + 1, st));
   k_level_counts<<<1, 32, 0, st>>>(G, cidx, lidx, small);
-  int64_t hsmall[DUST_MAXLEV + 3];
-  int herr = 0, hperr = 0;
-  DUST_CUDA(cudaMemcpyAsync(hsmall, small, sizeof(int64_t) * (ll + 2), cudaMemcpyDeviceToHost,
-                            st));
-  DUST_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  DUST_CUDA(cudaMemcpyAsync(&hperr, perr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  int64_t hsmall[64];
+  DUST_CUDA(cudaMemcpyAsync(hsmall, small, sizeof(hsmall), cudaMemcpyDeviceToHost, st));
   DUST_CUDA(cudaStreamSynchronize(st));
+  int herr, hperr;
+  memcpy(&herr, &hsmall[40], sizeof(int));
+  memcpy(&hperr, &hsmall[41], sizeof(int));
+  if (hsmall[50]) {  // of the previous evaluation: a bounded wait of its M2L gave up
+    DUST_CUDA(cudaMemsetAsync(small + 48, 0, 4 * sizeof(int64_t), st));
+    dust_set_last_error("a wait in the previous M2L gave up", __FILE__, __LINE__);
+    return DUST_ERR_TIMEOUT;
+  }
   if (herr != 0x7fffffff) {
     o->bad_particle = herr;
     return DUST_ERR_OUT_OF_BOX;
@@ -1434,9 +1448,9 @@ int fmm_prepare_device(dust_octree *o, int n, const double *cen, const double *d
   DUST_TRY(grow(o->leaf_ci, (size_t)std::max<int64_t>(o->n_leaves, 1) * 4));
   size_t nmp = (size_t)3 * (2 * o->nm + o->nm1);
   DUST_TRY(grow(o->mp, (size_t)std::max<int64_t>(nact, 1) * nmp * 8));
-  k_compact<<<nblk(ntot, 256), 256, 0, st>>>(G, ntot, flags, cidx, lidx,
+  k_compact<<<nblk(ntot, 256), 256, 0, st>>>(G, ntot, flags, cidx, lidx, cstart,
                                              (uint32_t *)o->act_key.p, (uint8_t *)o->act_lev.p,
-                                             (uint32_t *)o->leaf_ci.p);
+                                             (uint32_t *)o->leaf_ci.p, (uint32_t *)o->srcix.p);
   FmmDev d;
   fill_dev(o, d, n);
   d.cstart = cstart;
@@ -1681,7 +1695,7 @@ int fmm_collect_stats(dust_octree *o, int n, int64_t n_elem) {
     cudaMemcpy(c, o->dev.counters, sizeof(c), cudaMemcpyDeviceToHost);
     s.n_m2l_pairs = c[0];
     s.n_p2p_pairs = c[1];
-    if (c[2]) status = DUST_ERR_TIMEOUT;  // a bounded wait of the tensor-core M2L gave up
+    if (c[2]) status = DUST_ERR_TIMEOUT;  // a bounded wait of the M2L gave up
   }
   s.n_particles = n;
   s.n_leaves = o->n_leaves;

@@ -69,9 +69,9 @@ struct dust_octree {
   DevBuf elem_work;                    // FP32C element sums: far sums, near-pair list
   size_t near_cap = 0;                 // capacity of the near-pair list
   DevBuf dtabs[DUST_MAXLEV + 1];       // dimensionless scalar M2L tables (FP64)
-  DevBuf dtab32[DUST_MAXLEV + 1];      // dimensionless scalar M2L tables (FP32)
-  DevBuf jsum;                         // scalar M2L index table [n][slot][lane]
-  int m2l_nJ = 0, m2l_SL = 0, m2l_P = 0;  // L indices, 32-lane slots, table stride
+  DevBuf jsum;                         // M2L index table, then the classes' offsets
+  DevBuf srcix;                        // per cell: active index if non-empty, else ~0
+  int m2l_nJ = 0, m2l_P = 0;           // L indices, table stride
   DevBuf m2l_buf;                      // class-sorted M2L target lists
   DevBuf m2l_bat;                      // M2L batch descriptors
   uint32_t *m2l_list = nullptr;

@@ -58,10 +58,9 @@ extern "C" {
 #define DUST_PREC_FP64   0     /* plain: FP64 everywhere                      */
 #define DUST_PREC_FP32C  1     /* FP32 pair arithmetic on tile-relative
                                   coordinates, partial sums per tile in FP32
-                                  and across tiles in FP64; M2L of levels >= 2
-                                  in FP32 (SIMT, FP64 accumulation across
-                                  offsets); tables, level-1 M2L, P2M, M2M,
-                                  L2L, L2P and near element pairs stay FP64   */
+                                  and across tiles in FP64; tables, M2L, P2M,
+                                  M2M, L2L, L2P and near element pairs stay
+                                  FP64                                        */
 
 /* Octree / FMM parameters.  One field per DUST input key
  * (src/general/mod_sim_param.f90:376-452, read at :772-804). */

@@ -301,3 +301,19 @@ def test_fmm_points_uvort_errors():
     oc.prepare(cen, dir_, mag, rv, np.array([[0.1, 0.2, 0.3]]))  # the handle stays usable
     u = oc.points_uvort()
     assert u.shape == (1, 3) and np.all(np.isfinite(u))
+
+
+@pytest.mark.parametrize("p,vs,n", [(0, True, 900), (1, True, 900), (3, True, 1500),
+                                    (3, False, 1500), (4, False, 9000), (5, True, 1500),
+                                    (7, True, 900), (8, False, 900)])
+def test_fmm_every_degree_matches_oracle(p, vs, n):
+    """Every instance of the tensor-core M2L: j-tile and source-row remainders
+    of each degree, with and without the gradient's extra degree, offsets
+    shared among CTAs."""
+    cen, dir_, mag, rv = ring(n, seed=20 + p)
+    prm = prm_ring(multipole_degree=p, n_octree_levels=5, min_octree_part=5, vortstretch=vs)
+    ov, os_, orr, _ = O.fmm_apply(prm, cen, dir_, mag, rv)
+    v, s, r = octree.initialize_octree(prm).apply_multipole(cen, dir_, mag, rv)
+    assert rel(v, ov) < TOL64 and rel(s, os_) < TOL64
+    if vs:
+        assert rel(r, orr) < TOL64
