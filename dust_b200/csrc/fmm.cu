@@ -216,6 +216,7 @@ extern "C" int dust_octree_destroy(dust_octree *o) {
   devbuf_free(o->m2l_bat);
   devbuf_free(o->jsum);
   devbuf_free(o->srcix);
+  devbuf_free(o->p2p_work);
   devbuf_free(o->shift);
   devbuf_free(o->ffbuf);
   devbuf_free(o->elem_work);
@@ -1027,40 +1028,131 @@ __device__ __forceinline__ void p2p_pair_f(const float *tp, const float *ta, flo
   }
 }
 
-// L2P + P2P, one warp per leaf.  Leaves hold a few particles (6 on average
-// in the 2M-particle full step), so a CTA per leaf would leave most lanes
-// idle.  The warp lists the leaf's near field as particle ranges (the 26
-// active same-level neighbours, the coarser leaf neighbours of every level
-// above -- leaf_neigh, mod_octree.f90:964-988 -- and the leaf itself, at most
-// 26 * DUST_MAXLEV + 1 ranges), then takes its targets 32 at a time: lanes
-// are split into G = 32 / cnt groups of cnt lanes (one lane per target),
-// lane (tl, grp) accumulates target tl over the sources u = grp mod G of
-// each 32-source tile staged in the warp's own shared memory, and group 0
-// adds the other groups' sums from shared memory.  A source is found from
-// its position in the concatenated ranges by a binary search over the
-// range prefix sums (walked forward tile by tile).
+// L2P + P2P, one warp per leaf or, where a leaf's near field is large, per
+// share of it.  Leaves hold a few particles (6 on average in the 2M-particle
+// full step), so a CTA per leaf would leave most lanes idle.  The warp lists
+// the leaf's near field as particle ranges (the 26 active same-level
+// neighbours, the coarser leaf neighbours of every level above -- leaf_neigh,
+// mod_octree.f90:964-988 -- and the leaf itself, at most 26 * DUST_MAXLEV + 1
+// ranges), then takes its targets 32 at a time: lanes are split into
+// G = 32 / cnt groups of cnt lanes (one lane per target), lane (tl, grp)
+// accumulates target tl over the sources u = grp mod G of each 32-source tile
+// staged in the warp's own shared memory, and group 0 adds the other groups'
+// sums from shared memory.  A source is found from its position in the
+// concatenated ranges by a search over the range prefix sums (walked forward
+// tile by tile).
 //   FP64: pairs by p2p_pair on absolute coordinates, summed in FP64.
 //   FP32C (F32): pairs by p2p_pair_f on coordinates relative to the leaf
 //   centre (differences formed in FP64, rounded once), FP32 partial sums of
 //   up to 128 sources folded into FP64.
 // L2P (mod_octree.f90:1171-1212) is FP64 in both.
-#define P2W_WARPS 1  // one warp per CTA: leaves finish independently
+//
+// A coarse leaf beside a fine cluster has the whole cluster as its near field
+// (its same-level neighbours are branches): tens of thousands of sources for
+// one warp, a chain that outlasted the rest of the grid (110k ring particles,
+// FP64: 11.0 ms for 120M pairs, 1.3 ms cut; 1.1M FP32C: SMs idle for 44 % of
+// 9.2 ms, 4.6 ms cut).  So k_p2p_split first counts every leaf's sources and cuts the leaves of more
+// than `it` pair iterations per 32 targets into items of (32 targets, at most
+// it * G sources), which the grid's first CTAs work off; items add to
+// the outputs atomically, the first one of a target also its L2P.
 #define P2W_TILE 32
 #define P2W_MAXR (26 * DUST_MAXLEV + 4)
 #define P2W_NV 8  // staged per source: x y z, alpha x y z, r_v^2, 1 / r_v^2
 #define P2W_LQ 4  // levels whose near-field loads are issued together
+#define P2W_XB (148 * 16)  // CTAs for the items: the resident ones
+#define P2W_CAP (1u << 18) // items (4 MB)
+
+struct P2PItems {
+  uint8_t *split;    // per leaf: its work is in the items
+  uint4 *item;       // leaf, first target, sources [z, w) of the concatenated ranges
+  unsigned long long *count;  // [0] items, [1] next item
+  uint32_t cap;
+  int it;            // pair iterations of an item
+};
+
+// the near-field ranges of P2W_LQ levels from lev0 up for this lane's
+// neighbour: flags and ranges are loaded without branches (predicated on the
+// neighbour lying in the box), so the loads of all levels are in flight
+// together rather than one dependent chain per level
+__device__ __forceinline__ void p2p_ranges(const FmmDev &d, int l, int ci, int cj, int ck,
+                                           int lev0, int lane, uint32_t (&a0)[P2W_LQ],
+                                           uint32_t (&len)[P2W_LQ]) {
+  uint32_t a1[P2W_LQ];
+  bool ok[P2W_LQ], want[P2W_LQ];
+  const int di = lane % 3 - 1, dj = (lane / 3) % 3 - 1, dk = lane / 9 - 1;
+#pragma unroll
+  for (int q = 0; q < P2W_LQ; ++q) {
+    const int lev = lev0 - q, sh = l - lev;
+    const int ai = (ci >> sh) + di, aj = (cj >> sh) + dj, ak = (ck >> sh) + dk;
+    ok[q] = lev >= 1 && lane < 27 && lane != 13 && cart_in(d.G, lev, ai, aj, ak);
+    const uint32_t nk = ok[q] ? key_of(d.G, lev, ai, aj, ak) : 0u;
+    const uint8_t f = ok[q] ? d.flags[d.G.lev_off[lev] + nk] : (uint8_t)0;
+    a0[q] = ok[q] ? cell_lo(d.G, d.cstart, lev, nk) : 0u;
+    a1[q] = ok[q] ? cell_hi(d.G, d.cstart, lev, nk) : 0u;
+    want[q] = (lev == l) ? (f & FL_ACTIVE) != 0 : (f & FL_LEAF) != 0;
+  }
+#pragma unroll
+  for (int q = 0; q < P2W_LQ; ++q) len[q] = ok[q] && want[q] ? a1[q] - a0[q] : 0u;
+}
+
+// one warp per leaf: the number of its sources; cuts a large leaf into items
+// (a leaf that no longer fits the list stays whole) and zeroes its outputs
+__global__ void __launch_bounds__(256) k_p2p_split(FmmDev d, P2PItems w) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t leaf = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (leaf >= d.n_leaves) return;
+  const uint32_t ci = d.leaf_ci[leaf];
+  const int l = d.act_lev[ci];
+  const uint32_t key = d.act_key[ci];
+  int i, j, k;
+  cart_of_key(d.G, l, key, i, j, k);
+  const uint32_t lo = cell_lo(d.G, d.cstart, l, key), hi = cell_hi(d.G, d.cstart, l, key);
+  const uint32_t nt = hi - lo;
+  uint32_t S = 0;
+  if (nt > 0)
+    for (int lev0 = l; lev0 >= 1; lev0 -= P2W_LQ) {
+      uint32_t a0[P2W_LQ], len[P2W_LQ];
+      p2p_ranges(d, l, i, j, k, lev0, lane, a0, len);
+      for (int q = 0; q < P2W_LQ; ++q) S += len[q];
+    }
+  S = __reduce_add_sync(0xffffffffu, S) + nt;
+  if (lane == 0 && nt > 0 && d.counters)
+    atomicAdd((unsigned long long *)d.counters + 1, (unsigned long long)nt * (S - 1));
+  // sources per item of a full block of 32 targets and of the last block
+  const uint32_t nb = nt / 32, rem = nt % 32;
+  const uint32_t seg_r = rem ? (uint32_t)w.it * (32u / rem) : 1u;
+  const uint32_t ni_b = (S + w.it - 1) / w.it, ni_r = rem ? (S + seg_r - 1) / seg_r : 0u;
+  const uint32_t ni = nb * ni_b + ni_r;
+  bool split = ni > 1;
+  unsigned long long at = 0;
+  if (split) {
+    if (lane == 0) at = atomicAdd(w.count, (unsigned long long)ni);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at + ni > w.cap) split = false;
+    for (uint32_t e = lane; e < ni; e += 32) {
+      const uint32_t b = min(e / ni_b, nb), s = e - b * ni_b, seg = b < nb ? (uint32_t)w.it : seg_r;
+      // (an item past the list's end is never read: the count is clamped)
+      if (at + e < w.cap)
+        w.item[at + e] = split ? make_uint4(leaf, 32 * b, s * seg, min(S, (s + 1) * seg))
+                               : make_uint4(leaf, 0, 0, 0);
+    }
+    if (split)
+      for (uint32_t t = lane; t < nt; t += 32)
+        for (int e = 0; e < 9; ++e) d.out[(size_t)e * d.n + lo + t] = 0.0;
+  }
+  if (lane == 0) w.split[leaf] = split;
+}
 
 template <bool VS, bool DF, bool VD, bool TV, bool F32>
-__global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
+__device__ __forceinline__ void p2p_share(const FmmDev &d, uint32_t leaf, int tb, int te,
+                                          uint32_t s_lo, uint32_t s_hi, bool split) {
   using R = typename std::conditional<F32, float, double>::type;
-  __shared__ R s_src[P2W_WARPS][P2W_NV][P2W_TILE];
-  __shared__ uint32_t s_sid[P2W_WARPS][P2W_TILE];
-  __shared__ uint32_t s_rlo[P2W_WARPS][P2W_MAXR];
-  __shared__ uint32_t s_rcum[P2W_WARPS][P2W_MAXR + 1];
-  __shared__ double s_acc[P2W_WARPS][12][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t leaf = blockIdx.x * P2W_WARPS + w;
-  if (leaf >= d.n_leaves) return;  // warp-uniform: no CTA-wide barriers below
+  __shared__ __align__(16) R s_src[P2W_NV][P2W_TILE];
+  __shared__ uint32_t s_sid[P2W_TILE];
+  __shared__ uint32_t rlo[P2W_MAXR];
+  __shared__ uint32_t rcum[P2W_MAXR + 1];
+  __shared__ double s_acc[12][32];
+  const int lane = threadIdx.x & 31;
   const uint32_t ci = d.leaf_ci[leaf];
   const int l = d.act_lev[ci];
   const uint32_t key = d.act_key[ci];
@@ -1070,62 +1162,44 @@ __global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
   cell_center(d.G, l, ci_, cj, ck, cc);
   const uint32_t lo = cell_lo(d.G, d.cstart, l, key), hi = cell_hi(d.G, d.cstart, l, key);
   if (hi == lo) return;
-  uint32_t *rlo = s_rlo[w], *rcum = s_rcum[w];
-  // near-field source ranges: same level first, then coarser levels.  The
-  // flags and particle ranges of P2W_LQ levels are loaded without branches
-  // (predicated on the neighbour lying in the box), so those loads are in
-  // flight together rather than one dependent chain per level.
+  // near-field source ranges: same level first, then coarser levels, the leaf
+  // itself last; rcum their positions in the concatenation
   int nr = 0;
+  uint32_t S = 0;
   for (int lev0 = l; lev0 >= 1; lev0 -= P2W_LQ) {
-    bool predq[P2W_LQ];
-    uint32_t a0q[P2W_LQ], a1q[P2W_LQ];
+    uint32_t a0q[P2W_LQ], len[P2W_LQ];
+    p2p_ranges(d, l, ci_, cj, ck, lev0, lane, a0q, len);
 #pragma unroll
     for (int q = 0; q < P2W_LQ; ++q) {
-      const int lev = lev0 - q;
-      const int sh = l - lev;
-      const int ai = ci_ >> sh, aj = cj >> sh, ak = ck >> sh;
-      const int di = lane % 3 - 1, dj = (lane / 3) % 3 - 1, dk = lane / 9 - 1;
-      const bool ok = lev >= 1 && lane < 27 && lane != 13 &&
-                      cart_in(d.G, lev, ai + di, aj + dj, ak + dk);
-      const uint32_t nk = ok ? key_of(d.G, lev, ai + di, aj + dj, ak + dk) : 0u;
-      const uint8_t f = ok ? d.flags[d.G.lev_off[lev] + nk] : (uint8_t)0;
-      a0q[q] = ok ? cell_lo(d.G, d.cstart, lev, nk) : 0u;
-      a1q[q] = ok ? cell_hi(d.G, d.cstart, lev, nk) : 0u;
-      const bool want = (lev == l) ? (f & FL_ACTIVE) != 0 : (f & FL_LEAF) != 0;
-      predq[q] = ok && want && a1q[q] > a0q[q];
-    }
+      const unsigned msk = __ballot_sync(0xffffffffu, len[q] > 0);
+      if (!msk) continue;
+      uint32_t run = len[q];  // inclusive scan over the lanes
 #pragma unroll
-    for (int q = 0; q < P2W_LQ; ++q) {
-      const unsigned msk = __ballot_sync(0xffffffffu, predq[q]);
-      // 26 per level and l <= DUST_MAXLEV levels: the list cannot overflow
-      if (predq[q] && nr + __popc(msk) < P2W_MAXR) {
-        const int pos = nr + __popc(msk & ((1u << lane) - 1u));
-        rlo[pos] = a0q[q];
-        rcum[pos] = a1q[q] - a0q[q];
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += v;
       }
+      const int pos = nr + __popc(msk & ((1u << lane) - 1u));
+      // 26 per level and l <= DUST_MAXLEV levels: the list cannot overflow
+      if (len[q] > 0 && pos < P2W_MAXR - 1) {
+        rlo[pos] = a0q[q];
+        rcum[pos] = S + run - len[q];
+      }
+      S += __shfl_sync(0xffffffffu, run, 31);
       nr = min(nr + __popc(msk), P2W_MAXR - 1);
     }
   }
-  __syncwarp();
   if (lane == 0) {
     rlo[nr] = lo;
-    rcum[nr] = hi - lo;
-    ++nr;
-    uint32_t run = 0;
-    for (int r = 0; r < nr; ++r) {
-      const uint32_t len = rcum[r];
-      rcum[r] = run;
-      run += len;
-    }
-    rcum[nr] = run;
+    rcum[nr] = S;
+    rcum[nr + 1] = S + (hi - lo);
   }
-  nr = __shfl_sync(0xffffffffu, nr, 0);  // lane 0 appended the own leaf
+  ++nr;
+  S += hi - lo;
   __syncwarp();
-  const uint32_t S = rcum[nr];
+  s_hi = min(s_hi, S);
   const size_t n = d.n;
   const int nt = (int)(hi - lo), nm = d.nm, nm1 = d.nm1;
-  if (lane == 0 && d.counters)
-    atomicAdd((unsigned long long *)d.counters + 1, (unsigned long long)nt * (S - 1));
   const double k4pi = 1.0 / (4.0 * DUST_PI);
   const double *bl = d.B + (size_t)ci * 3 * nm, *gl = d.Gx + (size_t)ci * 3 * nm1;
   // L2P of one target (FP64): velocity and the gradient of the local field
@@ -1175,9 +1249,9 @@ __global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     ave_ros = part / (double)nt;
   }
-  R *fs = &s_src[w][0][0];
-  double *acc = &s_acc[w][0][lane];  // this lane's 12 FP64 sums, stride 32
-  for (int t0 = 0; t0 < nt; t0 += 32) {
+  R *fs = &s_src[0][0];
+  double *acc = &s_acc[0][lane];  // this lane's 12 FP64 sums, stride 32
+  for (int t0 = tb; t0 < min(nt, te); t0 += 32) {
     // G groups of cnt lanes (one lane per target) split the sources; lanes
     // beyond G * cnt idle
     const int cnt = min(32, nt - t0);
@@ -1208,7 +1282,7 @@ __global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
     uint32_t psid = 0;
     bool pv = false;
     auto fetch = [&](uint32_t v) {
-      pv = v < S;
+      pv = v < s_hi;
       if (pv) {
         while (ra + 1 < nr && rcum[ra + 1] <= v) ++ra;  // last r with rcum[r] <= v
         psid = rlo[ra] + (v - rcum[ra]);
@@ -1216,11 +1290,11 @@ __global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
         for (int q = 0; q < 7; ++q) pf[q] = d.P[(size_t)q * n + psid];
       }
     };
-    fetch(lane);
-    for (uint32_t s0 = 0; s0 < S; s0 += P2W_TILE) {
+    fetch(s_lo + lane);
+    for (uint32_t s0 = s_lo; s0 < s_hi; s0 += P2W_TILE) {
       __syncwarp();
       if (pv) {
-        s_sid[w][lane] = psid;
+        s_sid[lane] = psid;
         for (int q = 0; q < 3; ++q)
           fs[q * P2W_TILE + lane] = F32 ? (R)(pf[q] - cc[q]) : (R)pf[q];
         for (int q = 3; q < 6; ++q) fs[q * P2W_TILE + lane] = (R)pf[q];
@@ -1237,10 +1311,10 @@ __global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
       }
       __syncwarp();
       fetch(s0 + P2W_TILE + lane);
-      const int m = (int)min((uint32_t)P2W_TILE, S - s0);
+      const int m = (int)min((uint32_t)P2W_TILE, s_hi - s0);
       if (act)
         for (int u = grp; u < m; u += G) {
-          if (s_sid[w][u] == ti) continue;
+          if (s_sid[u] == ti) continue;
           if constexpr (F32)
             p2p_pair_f<VS, DF, VD>(tp, ta, fs[u], fs[P2W_TILE + u], fs[2 * P2W_TILE + u],
                                    fs[3 * P2W_TILE + u], fs[4 * P2W_TILE + u],
@@ -1252,7 +1326,7 @@ __global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
                                  fs[5 * P2W_TILE + u], fs[6 * P2W_TILE + u],
                                  fs[7 * P2W_TILE + u], A);
         }
-      if (F32 && (++since == 4 || s0 + P2W_TILE >= S)) {
+      if (F32 && (++since == 4 || s0 + P2W_TILE >= s_hi)) {
         // FP32 partial sums of up to 128 sources folded into FP64
         since = 0;
         for (int e = 0; e < 3; ++e) {
@@ -1283,15 +1357,16 @@ __global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
     __syncwarp();
     // L2P (FP64) split over the groups: lane (tl, grp) sums the monomials
     // grp, grp + G, ... of its target; group 0 adds the other groups' parts
-    double lv[3], g[9];
-    if (act) {
+    // (with the first sources of the target only)
+    double lv[3] = {0, 0, 0}, g[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (act && s_lo == 0) {
       l2p(ti, grp, G, lv, g);
       for (int e = 0; e < 3; ++e) acc[32 * e] = lv[e];
       for (int e = 0; e < 9; ++e) acc[32 * (3 + e)] = g[e];
     }
     __syncwarp();
     if (act && grp == 0) {
-      for (int q = 1; q < G; ++q) {
+      for (int q = 1; q < G && s_lo == 0; ++q) {
         for (int e = 0; e < 3; ++e) lv[e] += acc[32 * e + q * TPR];
         for (int e = 0; e < 9; ++e) g[e] += acc[32 * (3 + e) + q * TPR];
       }
@@ -1311,13 +1386,45 @@ __global__ void __launch_bounds__(P2W_WARPS * 32, 16) k_p2p_w(FmmDev d) {
         nu += (0.11 * rv) * (0.11 * rv) * sqrt(2.0 * ave_ros);
       }
       for (int e = 0; e < 3; ++e) {
-        d.out[(size_t)e * n + ti] = lv[e] + Q[e] * k4pi;
-        d.out[(size_t)(3 + e) * n + ti] = ls[e] + Q[3 + e] * k4pi + (VD ? Q[9 + e] * nu : 0.0);
-        d.out[(size_t)(6 + e) * n + ti] = lr[e] + Q[6 + e] * k4pi;
+        const double o0 = lv[e] + Q[e] * k4pi, o2 = lr[e] + Q[6 + e] * k4pi,
+                     o1 = ls[e] + Q[3 + e] * k4pi + (VD ? Q[9 + e] * nu : 0.0);
+        double *o = d.out + ti;
+        if (split) {
+          atomicAdd(o + (size_t)e * n, o0);
+          if (VS || VD) atomicAdd(o + (size_t)(3 + e) * n, o1);
+          if (DF) atomicAdd(o + (size_t)(6 + e) * n, o2);
+        } else {
+          o[(size_t)e * n] = o0;
+          o[(size_t)(3 + e) * n] = o1;
+          o[(size_t)(6 + e) * n] = o2;
+        }
       }
     }
     __syncwarp();  // acc is reused by the next 32 targets
   }
+}
+
+template <bool VS, bool DF, bool VD, bool TV, bool F32>
+__global__ void __launch_bounds__(32, 16) k_p2p_w(FmmDev d, P2PItems w) {
+  uint32_t leaf, tb = 0, te = 0xffffffffu >> 1, s_lo = 0, s_hi = 0xffffffffu;
+  const bool items = blockIdx.x < P2W_XB;
+  if (!items) {
+    leaf = blockIdx.x - P2W_XB;
+    if (w.split[leaf]) return;
+  }
+  do {
+    if (items) {
+      unsigned long long i = 0;
+      if (threadIdx.x == 0) i = atomicAdd(w.count + 1, 1ull);
+      i = __shfl_sync(0xffffffffu, i, 0);
+      if (i >= min(w.count[0], (unsigned long long)w.cap)) return;
+      const uint4 it = w.item[i];
+      leaf = it.x, tb = it.y, te = it.y + 1, s_lo = it.z, s_hi = it.w;
+      if (s_hi == 0) continue;  // of a leaf that did not fit the list
+      __syncwarp();
+    }
+    p2p_share<VS, DF, VD, TV, F32>(d, leaf, (int)tb, (int)te, s_lo, s_hi, items);
+  } while (items);
 }
 
 // ======================================================== host orchestration
@@ -1536,13 +1643,28 @@ int fmm_near_device(dust_octree *o, cudaStream_t st) {
   if (o->n_leaves > 0) {
     bool vs = d.use_vs, df = d.use_df, vd = d.use_vd, tv = o->prm.turbulent_viscosity != 0;
     const bool f32 = o->prm.precision == DUST_PREC_FP32C;
-    const unsigned grid = (unsigned)((o->n_leaves + P2W_WARPS - 1) / P2W_WARPS);
+    // an item's iterations: short ones where the leaves alone would not fill
+    // the resident warps twice, since then the longest item is the time
+    // (3,000 particles: 57 us with 64, 90 with 128, 139 with 256); else long
+    // enough that listing the ranges again for every item costs little (110k:
+    // 1.28 ms with 256, 1.36 with 512, 1.47 with 1024)
+    const bool small = o->n_leaves < 2 * P2W_XB;
+    P2PItems w;
+    w.it = small ? 64 : 256;
+    w.cap = P2W_CAP;
+    DUST_TRY(grow(o->p2p_work, 256 + (size_t)P2W_CAP * sizeof(uint4) + (size_t)o->n_leaves));
+    w.count = (unsigned long long *)o->p2p_work.p;
+    w.item = (uint4 *)((char *)o->p2p_work.p + 256);
+    w.split = (uint8_t *)(w.item + P2W_CAP);
+    DUST_CUDA(cudaMemsetAsync(w.count, 0, 16, st));
+    k_p2p_split<<<nblk(o->n_leaves, 8), 256, 0, st>>>(d, w);
+    const unsigned grid = (unsigned)(P2W_XB + o->n_leaves);
 #define LAUNCH_P2P(A, B, C, D)                                                   \
   do {                                                                         \
     if (f32)                                                                   \
-      k_p2p_w<A, B, C, D, true><<<grid, P2W_WARPS * 32, 0, st>>>(d);           \
+      k_p2p_w<A, B, C, D, true><<<grid, 32, 0, st>>>(d, w);                    \
     else                                                                       \
-      k_p2p_w<A, B, C, D, false><<<grid, P2W_WARPS * 32, 0, st>>>(d);          \
+      k_p2p_w<A, B, C, D, false><<<grid, 32, 0, st>>>(d, w);                   \
   } while (0)
     if (vs && df && vd && !tv) LAUNCH_P2P(true, true, true, false);
     else if (vs && df && vd && tv) LAUNCH_P2P(true, true, true, true);

@@ -70,6 +70,7 @@ struct dust_octree {
   size_t near_cap = 0;                 // capacity of the near-pair list
   DevBuf dtabs[DUST_MAXLEV + 1];       // dimensionless scalar M2L tables (FP64)
   DevBuf jsum;                         // M2L index table, then the classes' offsets
+  DevBuf p2p_work;                     // near-field items and per-leaf split flags
   DevBuf srcix;                        // per cell: active index if non-empty, else ~0
   int m2l_nJ = 0, m2l_P = 0;           // L indices, table stride
   DevBuf m2l_buf;                      // class-sorted M2L target lists

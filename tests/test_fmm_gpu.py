@@ -317,3 +317,24 @@ def test_fmm_every_degree_matches_oracle(p, vs, n):
     assert rel(v, ov) < TOL64 and rel(s, os_) < TOL64
     if vs:
         assert rel(r, orr) < TOL64
+
+
+@pytest.mark.parametrize("n_far", [5, 31, 32, 33, 70])
+@pytest.mark.parametrize("prec", [abi.DUST_PREC_FP64, abi.DUST_PREC_FP32C])
+def test_fmm_split_near_field_matches_oracle(n_far, prec):
+    """A coarse leaf of n_far particles beside a fine cluster: its near field
+    is cut into items (blocks of 32 targets, part blocks, several source
+    segments each)."""
+    rng = np.random.default_rng(n_far)
+    cen = np.concatenate([rng.uniform(0.1, 1.9, (n_far, 3)),
+                          [-0.2, -0.3, -0.1] + 0.1 * rng.standard_normal((3000, 3))])
+    dir_ = rng.standard_normal(cen.shape)
+    dir_ /= np.linalg.norm(dir_, axis=1)[:, None]
+    mag = np.abs(1e-3 + 1e-4 * rng.standard_normal(len(cen)))
+    rv = np.full(len(cen), 0.05)
+    prm = prm_ring(n_octree_levels=6, min_octree_part=5, precision=prec, rankine_rad=0.05)
+    ov, os_, orr, _ = O.fmm_apply(prm, cen, dir_, mag, rv)
+    v, s, r = octree.initialize_octree(prm).apply_multipole(cen, dir_, mag, rv)
+    tol = TOL64 if prec == abi.DUST_PREC_FP64 else TOL32
+    assert rel(v, ov) < tol and rel(s, os_) < tol and rel(r, orr) < tol
+    assert rel(v[:n_far], ov[:n_far]) < tol and rel(r[:n_far], orr[:n_far]) < tol
