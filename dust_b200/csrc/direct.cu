@@ -105,6 +105,15 @@ __device__ __forceinline__ double rsqrt_hh(double x) {
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+// x^-3/2 for a normal FP32-range x > 0: with the FP32 approximation y0 and
+// e = 1 - x y0^2, x^-3/2 = y0^3 (1 + 3e/2 + 15e^2/8 + O(e^3)); y0^2 is exact
+// in FP64.  One operation less than the cube of rsqrt_hh.
+__device__ __forceinline__ double rcube_hh(double x) {
+  const double y = (double)rsqrt_approx((float)x);
+  const double t = y * y, e = fma(-x, t, 1.0), y3 = t * y;
+  return fma(y3 * e, fma(1.875, e, 1.5), y3);
+}
+
 __global__ void __launch_bounds__(EO_T) k_elem_out(FmmDev d, ElemDev e, const FFRec *ff,
                                                    double *vel, double *str, double *rot) {
   __shared__ __align__(16) double s_pk[EO_LOAD][EO_PK];
@@ -458,7 +467,7 @@ __global__ void __launch_bounds__(EF2_T) k_elem_far(FmmDev d, ElemDev e, const F
         float acc[EF2_PPT][3];
 #pragma unroll
         for (int i = 0; i < EF2_PPT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = 0.f;
-#pragma unroll 2
+#pragma unroll 4
         for (int q = 0; q < EF2_TILE; ++q) {
           const int ql = sb * EF2_TILE + q;
           const float *pk = &s_pk[ql >> 1][ql & 1];
@@ -684,8 +693,37 @@ int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
 // particles for 128 points and adds its partial sums atomically.
 #define UV2_T 128
 #define UV2_TILE 128
+// resident CTAs per SM of the four kernels
+#define UVD_OCC 6
+#define UVDP_OCC 5
+#define UV2_OCC 4
+#define UV2P_OCC 3
 
-// FP64 uvort (plain mode): particles in the caller's order, UVD_PPT points
+// Particles per CTA for pb point blocks: whole waves of the resident CTAs.
+// The time is that of ceil(CTAs / resident) chunks one after the other (plus
+// the staging and the atomic additions of each, about 32 particles' worth),
+// so a grid that spills a little over a wave pays for a whole one (13,920
+// points x 2M particles, packed FP32: 2.7 waves 21.0 ms, 4.0 waves 19.0 ms;
+// 18.8 ms with the inner loop unrolled by 4).  Small sums take chunks down to
+// 32 particles to reach every SM (400 points x 12,800: 35 -> 18 us).
+static int uvort_chunk(int pb, int n, int occ) {
+  const int slots = 148 * occ;
+  int best = n;
+  double cost = 1e30;
+  for (int w = 1; w <= 8; ++w) {
+    const int nch = std::max(1, (int)((int64_t)w * slots / pb));
+    const int c = std::max(32, ((n + nch - 1) / nch + 31) / 32 * 32);
+    const int64_t ctas = (int64_t)pb * ((n + c - 1) / c);
+    const double t = (double)((ctas + slots - 1) / slots) * (c + 32);
+    if (t < cost) cost = t, best = c;
+  }
+  return best;
+}
+
+// FP64 uvort (plain mode): FP64-pipe and latency bound (18 FP64 operations and
+// two conversions a pair; 7,001 points x 50,021 particles 576 -> 502 us, 0.66
+// of the operations' rate; 2 points per thread and 6 CTAs per SM, 4 and 4:
+// 508 us).  Particles in the caller's order, UVD_PPT points
 // per thread (consecutive CTA slices of UV2_T points) against a shared tile
 // of (x, y, z, r_v^2, alpha, w = x x alpha) records; the reciprocal square
 // root as in k_elem_out (FP32 seed, one Householder step in FP64).  With
@@ -694,8 +732,8 @@ int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
 // two 3-vector FMA accumulations per pair instead of a cross product and its
 // accumulation; in FP64 the difference of the two sums costs at most about
 // 1e-13 relative for a point very close to a particle.
-#define UVD_PPT 4
-__global__ void __launch_bounds__(UV2_T) k_uvort(int npts, const double *pts, int n,
+#define UVD_PPT 2
+__global__ void __launch_bounds__(UV2_T, UVD_OCC) k_uvort(int npts, const double *pts, int n,
                                                  const double *cen, const double *dir,
                                                  const double *mag, const double *rv,
                                                  int chunk, double *uv) {
@@ -730,7 +768,7 @@ __global__ void __launch_bounds__(UV2_T) k_uvort(int npts, const double *pts, in
 #pragma unroll
     for (int i = 0; i < UVD_PPT; ++i)
       for (int c = 0; c < 3; ++c) A[i][c] = W[i][c] = 0.0;
-#pragma unroll 2
+#pragma unroll 4
     for (int u = 0; u < m; ++u) {
       const double2 *w = (const double2 *)s_q[u];
       const double2 X = w[0], Y = w[1], Z = w[2], P = w[3], Q = w[4];
@@ -739,8 +777,7 @@ __global__ void __launch_bounds__(UV2_T) k_uvort(int npts, const double *pts, in
       for (int i = 0; i < UVD_PPT; ++i) {
         const double dx = pos[i][0] - X.x, dy = pos[i][1] - X.y, dz = pos[i][2] - Y.x;
         const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, Y.y)));
-        const double ir = rsqrt_hh(r2);
-        const double c = ir * ir * ir;
+        const double c = rcube_hh(r2);
         A[i][0] = fma(c, Z.x, A[i][0]);
         A[i][1] = fma(c, Z.y, A[i][1]);
         A[i][2] = fma(c, P.x, A[i][2]);
@@ -772,7 +809,7 @@ __global__ void __launch_bounds__(UV2_T) k_uvort(int npts, const double *pts, in
 // difference, rho^2 and rho^-3, so the pressure term adds four FMAs per pair
 // to k_uvort's nineteen FP64 operations instead of a second pass over the
 // particles.  pt[i] = sum_q (x_q - p_i) . (dir_q x vel_q) mag_q rho^-3.
-__global__ void __launch_bounds__(UV2_T) k_uvort_pres(int npts, const double *pts, int n,
+__global__ void __launch_bounds__(UV2_T, UVDP_OCC) k_uvort_pres(int npts, const double *pts, int n,
                                                       const double *cen, const double *dir,
                                                       const double *mag, const double *rv,
                                                       const double *vel, int chunk, double *uv,
@@ -819,7 +856,7 @@ __global__ void __launch_bounds__(UV2_T) k_uvort_pres(int npts, const double *pt
       for (int c = 0; c < 3; ++c) A[i][c] = W[i][c] = 0.0;
       Pq[i] = 0.0;
     }
-#pragma unroll 2
+#pragma unroll 4
     for (int u = 0; u < m; ++u) {
       const double2 *w = (const double2 *)s_q[u];
       const double2 X = w[0], Y = w[1], Z = w[2], P = w[3], Q = w[4], R = w[5], S = w[6];
@@ -829,8 +866,7 @@ __global__ void __launch_bounds__(UV2_T) k_uvort_pres(int npts, const double *pt
       for (int i = 0; i < UVD_PPT; ++i) {
         const double dx = pos[i][0] - X.x, dy = pos[i][1] - X.y, dz = pos[i][2] - Y.x;
         const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, Y.y)));
-        const double ir = rsqrt_hh(r2);
-        const double c = ir * ir * ir;
+        const double c = rcube_hh(r2);
         A[i][0] = fma(c, Z.x, A[i][0]);
         A[i][1] = fma(c, Z.y, A[i][1]);
         A[i][2] = fma(c, P.x, A[i][2]);
@@ -894,7 +930,7 @@ __global__ void k_uv_gather(int n, const uint32_t *perm, const double *cen, cons
 #ifndef UV2_PPT
 #define UV2_PPT 4
 #endif
-__global__ void __launch_bounds__(UV2_T) k_uvort_sorted(int npts, const double *pts, int n,
+__global__ void __launch_bounds__(UV2_T, UV2_OCC) k_uvort_sorted(int npts, const double *pts, int n,
                                                         const double *X, const float *F,
                                                         int chunk, double *uv) {
   // one tile of particles per pass, coordinates relative to the tile's first
@@ -949,7 +985,7 @@ __global__ void __launch_bounds__(UV2_T) k_uvort_sorted(int npts, const double *
       for (int c = 0; c < 3; ++c) V[i][c] = make_float2(0.f, 0.f);
     }
     const int mp = (m + 1) >> 1;
-#pragma unroll 2
+#pragma unroll 4
     for (int u = 0; u < mp; ++u) {
       const float4 P0 = *(const float4 *)&s_pk[u][0], P1 = *(const float4 *)&s_pk[u][4],
                    P2 = *(const float4 *)&s_pk[u][8], P3 = *(const float4 *)&s_pk[u][12],
@@ -1012,7 +1048,7 @@ __global__ void k_uvp_gather(int n, const uint32_t *perm, const double *cen, con
 // the difference, rho^-3 and the cross product of uvort, and d . (-w) rho^-3
 // for the pressure term; 13 values per particle, interleaved in pairs
 // as in k_uvort_sorted (value k of particle q at [q / 2][2 k + q % 2]).
-__global__ void __launch_bounds__(UV2_T) k_uvort_pres_sorted(int npts, const double *pts, int n,
+__global__ void __launch_bounds__(UV2_T, UV2P_OCC) k_uvort_pres_sorted(int npts, const double *pts, int n,
                                                              const double *X, const float *F,
                                                              int chunk, double *uv, double *pt) {
   __shared__ __align__(16) float s_pk[UV2_TILE / 2][28];
@@ -1064,7 +1100,7 @@ __global__ void __launch_bounds__(UV2_T) k_uvort_pres_sorted(int npts, const dou
       W[i] = make_float2(0.f, 0.f);
     }
     const int mp = (m + 1) >> 1;
-#pragma unroll 2
+#pragma unroll 4
     for (int u = 0; u < mp; ++u) {
       const float4 P0 = *(const float4 *)&s_pk[u][0], P1 = *(const float4 *)&s_pk[u][4],
                    P2 = *(const float4 *)&s_pk[u][8], P3 = *(const float4 *)&s_pk[u][12],
@@ -1110,12 +1146,17 @@ __global__ void __launch_bounds__(UV2_T) k_uvort_pres_sorted(int npts, const dou
     }
 }
 
+// UL_LINES lines per thread and point: one line is a chain of square roots and
+// quotients, so a thread that walked all of them was latency bound (7,001
+// points, 64 lines: 47 us, 8 us in shares of 8)
+#define UL_LINES 8
 __global__ void k_uvort_lines(int npts, const double *pts, ElemDev e, double *uv) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npts) return;
   double pos[3] = {pts[3 * (size_t)t], pts[3 * (size_t)t + 1], pts[3 * (size_t)t + 2]};
   double v[3] = {0, 0, 0};
-  for (int q = 0; q < e.nline; ++q) {
+  const int q1 = min(e.nline, ((int)blockIdx.y + 1) * UL_LINES);
+  for (int q = blockIdx.y * UL_LINES; q < q1; ++q) {
     double u[3];
     vel_line(e.rp, e.lines[q], pos, u);
     for (int c = 0; c < 3; ++c) v[c] += u[c];
@@ -1124,10 +1165,23 @@ __global__ void k_uvort_lines(int npts, const double *pts, ElemDev e, double *uv
   for (int c = 0; c < 3; ++c) atomicAdd(uv + 3 * (size_t)t + c, v[c] * k4pi);
 }
 
+static void launch_lines(int npts, const double *pts, const ElemDev &e, double *uv,
+                         cudaStream_t st) {
+  // (a grid has at most 65,535 rows)
+  const int step = 65535 * UL_LINES;
+  for (int q = 0; q < e.nline; q += step) {
+    ElemDev part = e;
+    part.lines = e.lines + q;
+    part.nline = std::min(step, e.nline - q);
+    k_uvort_lines<<<dim3(nblk(npts, 128), nblk(part.nline, UL_LINES)), 128, 0, st>>>(npts, pts,
+                                                                                    part, uv);
+  }
+}
+
 void points_lines_add(int npts, const double *pts, const ElemDev &lines, double *uv,
                       cudaStream_t st) {
   if (npts > 0 && lines.nline > 0)
-    k_uvort_lines<<<nblk(npts, 128), 128, 0, st>>>(npts, pts, lines, uv);
+    launch_lines(npts, pts, lines, uv, st);
 }
 
 // Morton order of n particles over the octree box of prm (keys of 10 bits
@@ -1173,10 +1227,7 @@ int points_uvort_run(const dust_fmm_params *prm, int n_pts, const double *pts, i
     // point blocks: UV2_T points (UV2_T * UV2_PPT for the sorted FP32 kernel)
     const bool srt = prm->precision == DUST_PREC_FP32C;
     int pb = (int)nblk(n_pts, UV2_T * (srt ? UV2_PPT : UVD_PPT));
-    // enough CTAs for every SM several times over; chunks of whole tiles
-    int want = std::max(1, (148 * 8 + pb - 1) / pb);
-    int chunk = (n + want - 1) / want;
-    chunk = std::max(UV2_TILE, (chunk + UV2_TILE - 1) / UV2_TILE * UV2_TILE);
+    const int chunk = uvort_chunk(pb, n, srt ? UV2_OCC : UVD_OCC);
     int nch = (n + chunk - 1) / chunk;
     dim3 grd(pb, nch);
     if (prm->precision == DUST_PREC_FP32C) {
@@ -1205,7 +1256,7 @@ int points_uvort_run(const dust_fmm_params *prm, int n_pts, const double *pts, i
       k_uvort<<<grd, UV2_T, 0, st>>>(n_pts, pts, n, cen, dir, mag, rv, chunk, uv);
     }
   }
-  if (lines.nline > 0) k_uvort_lines<<<nblk(n_pts, 128), 128, 0, st>>>(n_pts, pts, lines, uv);
+  if (lines.nline > 0) launch_lines(n_pts, pts, lines, uv, st);
   DUST_CUDA(cudaGetLastError());
   return DUST_OK;
 }
@@ -1276,9 +1327,7 @@ extern "C" int dust_points_uvort_device_noalloc(const dust_fmm_params *prm, int 
   DUST_CUDA(cudaMemsetAsync(uvort, 0, (size_t)n_pts * 24, st));
   if (n > 0) {
     int pb = (int)nblk(n_pts, UV2_T * (f32 ? UV2_PPT : UVD_PPT));
-    int want = std::max(1, (148 * 8 + pb - 1) / pb);
-    int chunk = (n + want - 1) / want;
-    chunk = std::max(UV2_TILE, (chunk + UV2_TILE - 1) / UV2_TILE * UV2_TILE);
+    const int chunk = uvort_chunk(pb, n, f32 ? UV2_OCC : UVD_OCC);
     int nch = (n + chunk - 1) / chunk;
     dim3 grd(pb, nch);
     if (f32) {
@@ -1298,7 +1347,7 @@ extern "C" int dust_points_uvort_device_noalloc(const dust_fmm_params *prm, int 
       k_uvort<<<grd, UV2_T, 0, st>>>(n_pts, pts, n, cen, dir, mag, r_vortex, chunk, uvort);
     }
   }
-  if (nl > 0) k_uvort_lines<<<nblk(n_pts, 128), 128, 0, st>>>(n_pts, pts, e, uvort);
+  if (nl > 0) launch_lines(n_pts, pts, e, uvort, st);
   DUST_CUDA(cudaGetLastError());
   return DUST_OK;
 }
@@ -1340,17 +1389,13 @@ static int uvort_pressure_run(const dust_fmm_params *prm, int n_pts, const doubl
                                               st));
     k_uvp_gather<<<nblk(n, 256), 256, 0, st>>>(n, v_out, cen, dir, mag, r_vortex, vel, X, F);
     const int pb = (int)nblk(n_pts, UV2_T * UV2_PPT);
-    const int want = std::max(1, (148 * 8 + pb - 1) / pb);
-    int chunk = (n + want - 1) / want;
-    chunk = std::max(UV2_TILE, (chunk + UV2_TILE - 1) / UV2_TILE * UV2_TILE);
+    const int chunk = uvort_chunk(pb, n, UV2P_OCC);
     const int nch = (n + chunk - 1) / chunk;
     k_uvort_pres_sorted<<<dim3(pb, nch), UV2_T, 0, st>>>(n_pts, pts, n, X, F, chunk, uvort,
                                                          pterm);
   } else if (n > 0) {
     const int pb = (int)nblk(n_pts, UV2_T * UVD_PPT);
-    const int want = std::max(1, (148 * 8 + pb - 1) / pb);
-    int chunk = (n + want - 1) / want;
-    chunk = std::max(UV2_TILE, (chunk + UV2_TILE - 1) / UV2_TILE * UV2_TILE);
+    const int chunk = uvort_chunk(pb, n, UVDP_OCC);
     const int nch = (n + chunk - 1) / chunk;
     k_uvort_pres<<<dim3(pb, nch), UV2_T, 0, st>>>(n_pts, pts, n, cen, dir, mag, r_vortex, vel,
                                                   chunk, uvort, pterm);

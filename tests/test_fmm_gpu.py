@@ -338,3 +338,20 @@ def test_fmm_split_near_field_matches_oracle(n_far, prec):
     tol = TOL64 if prec == abi.DUST_PREC_FP64 else TOL32
     assert rel(v, ov) < tol and rel(s, os_) < tol and rel(r, orr) < tol
     assert rel(v[:n_far], ov[:n_far]) < tol and rel(r[:n_far], orr[:n_far]) < tol
+
+
+@pytest.mark.parametrize("npts,n,nl", [(1, 1, 0), (129, 31, 1), (257, 33, 8), (511, 4097, 9),
+                                       (1025, 700, 17)])
+@pytest.mark.parametrize("prec", [abi.DUST_PREC_FP64, abi.DUST_PREC_FP32C])
+def test_uvort_chunks_match_oracle(npts, n, nl, prec):
+    """Point blocks, particle chunks and line shares at their remainders."""
+    rng = np.random.default_rng(npts)
+    pts = rng.uniform(-1.5, 1.5, (npts, 3))
+    cen, dir_, mag = synth.ring_particles(n, 0, seed=n)
+    rv = np.full(n, 0.05)
+    prm = prm_ring(precision=prec)
+    v0 = rng.uniform(1.6, 2.0, (nl, 3))
+    ev = abi.LineSet(np.stack([v0, v0 + 0.3], axis=1), rng.standard_normal(nl))
+    uo = O.points_uvort(prm, pts, cen, dir_, mag, rv, ev)
+    ug = octree.points_uvort(prm, pts, cen, dir_, mag, rv, ev)
+    assert rel(ug, uo) < (TOL64 if prec == abi.DUST_PREC_FP64 else TOL32)
