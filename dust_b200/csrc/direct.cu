@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "dust_common.cuh"
 #include "elements.cuh"
@@ -59,28 +60,22 @@ __global__ void k_ffrec(const PanelGeo *pg, int n, double ff_dou, FFRec *out) {
   out[j] = r;
 }
 
-// exact reference evaluation of one panel (x 4 pi)
-__device__ inline void near_pan(const RegParams &rp, const PanelGeo *pg, int j,
-                                const double *pos, double *v) {
-  vel_pan_near(rp, pg[j], pos, v);
-}
-
-// FP64 element sums (plain mode): far field by the closed form above, near
-// pairs by the reference's formulas; then end vortices, wind and the scatter
-// of all outputs to the caller's order.
+// FP64 element sums (plain mode): far field by the closed form above in
+// k_elem_far64, near pairs listed for k_elem_near (the reference's formulas),
+// then end vortices, wind and the scatter of all outputs to the caller's
+// order in k_elem_fin.
 //
 // EO_PPT particles per thread against shared-memory tiles of EO_LOAD panels
-// (far-field records, FP64).  The loader threads test each panel against the
-// bounding box of the CTA's particles: a sub-tile of EO_TILE panels that
-// lies beyond the far-field radius of the whole box runs the far formula
-// without a per-pair test (the box distance is formed with the per-pair
-// test's own operation order, so rounding, being monotone, cannot make the
-// box call far a pair the per-pair test calls near).  In the other sub-tiles
-// each pair is tested; the near pairs of a particle are marked in a bit mask
-// and evaluated after the sub-tile's far loop, in panel order, so the sums
-// are deterministic.  The reciprocal square root of the far formula is the
-// FP32 approximation refined by one second-order Newton-Raphson
-// (Householder) step in FP64: with y0 = x^-1/2 (1 + d) and e = 1 - x y0^2,
+// (far-field records, FP64); blockIdx.y takes a chunk of the panels.  The
+// loader threads test each panel against the bounding box of the CTA's
+// particles: a sub-tile of EO_TILE panels that lies beyond the far-field
+// radius of the whole box runs the far formula without a per-pair test (the
+// box distance is formed with the per-pair test's own operation order, so
+// rounding, being monotone, cannot make the box call far a pair the per-pair
+// test calls near).  In the other sub-tiles each pair is tested and a near
+// pair queued.  The reciprocal square root of the far formula is the FP32
+// approximation refined by one second-order Newton-Raphson (Householder) step
+// in FP64: with y0 = x^-1/2 (1 + d) and e = 1 - x y0^2,
 // y = y0 (1 + e/2 + 3 e^2/8) has relative error O(d^3), below the FP64
 // rounding for |d| < 2^-21.
 #define EO_PPT 2
@@ -90,6 +85,7 @@ __device__ inline void near_pan(const RegParams &rp, const PanelGeo *pg, int j,
 #define EO_SUB 4
 #define EO_LOAD (EO_TILE * EO_SUB)
 #define EO_PK 12  // nm x/y/z, mn x/y/z, -c x/y/z, as, ff2, pad
+#define EO_QCAP (EO_NP * EO_TILE)  // one sub-tile's worst case
 static_assert(EO_LOAD <= EO_T && EO_LOAD % 32 == 0 && EO_TILE <= 32, "staging layout");
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
@@ -114,14 +110,43 @@ __device__ __forceinline__ double rcube_hh(double x) {
   return fma(y3 * e, fma(1.875, e, 1.5), y3);
 }
 
-__global__ void __launch_bounds__(EO_T) k_elem_out(FmmDev d, ElemDev e, const FFRec *ff,
-                                                   double *vel, double *str, double *rot) {
+struct NearPair {
+  uint32_t t, j;  // particle (sorted order), panel
+};
+
+// appends the CTA's queue (panel relative to p_lo << 10 | local particle) to
+// the list of near pairs; pairs beyond its capacity are only counted
+template <int T>
+__device__ __forceinline__ void near_flush(const uint32_t *s_q, int qn, uint32_t t0, uint32_t p_lo,
+                                           unsigned long long *count, NearPair *list,
+                                           unsigned long long cap, unsigned long long *s_base) {
+  if (qn == 0) return;  // (the same in every thread)
+  if (threadIdx.x == 0) *s_base = atomicAdd(count, (unsigned long long)qn);
+  __syncthreads();
+  const unsigned long long base = *s_base;
+  for (int k = threadIdx.x; k < qn; k += T) {
+    const unsigned long long at = base + (unsigned long long)k;
+    if (at < cap) {
+      const uint32_t en = s_q[k];
+      list[at] = NearPair{t0 + (en & 0x3ffu), p_lo + (en >> 10)};
+    }
+  }
+}
+
+__global__ void __launch_bounds__(EO_T) k_elem_far64(FmmDev d, ElemDev e, const FFRec *ff,
+                                                     int chunk, double *farv,
+                                                     unsigned long long *count, NearPair *list,
+                                                     unsigned long long cap) {
   __shared__ __align__(16) double s_pk[EO_LOAD][EO_PK];
   __shared__ unsigned s_nearw[EO_LOAD / 32];
   __shared__ double s_box[EO_T / 32][6];
+  __shared__ uint32_t s_q[EO_QCAP];
+  __shared__ int s_qn;
+  __shared__ unsigned long long s_base;
   const size_t n = d.n;
   const uint32_t t0 = blockIdx.x * EO_NP;
   const int tid = threadIdx.x;
+  const int p_lo = blockIdx.y * chunk, p_hi = min(e.nbody + e.nwake, p_lo + chunk);
   double pos[EO_PPT][3], v[EO_PPT][3];
   bool act[EO_PPT];
   double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -146,16 +171,16 @@ __global__ void __launch_bounds__(EO_T) k_elem_out(FmmDev d, ElemDev e, const FF
     }
   if ((tid & 31) == 0)
     for (int c = 0; c < 3; ++c) s_box[tid >> 5][c] = lo[c], s_box[tid >> 5][3 + c] = hi[c];
+  if (tid == 0) s_qn = 0;
   __syncthreads();
   for (int w = 0; w < EO_T / 32; ++w)
     for (int c = 0; c < 3; ++c) lo[c] = fmin(lo[c], s_box[w][c]), hi[c] = fmax(hi[c], s_box[w][3 + c]);
-  const int ntot = e.nbody + e.nwake;
-  for (int p0 = 0; p0 < ntot; p0 += EO_LOAD) {
+  for (int p0 = p_lo; p0 < p_hi; p0 += EO_LOAD) {
     __syncthreads();
     bool near_box = false;
     if (tid < EO_LOAD) {
       double *pk = s_pk[tid];
-      if (p0 + tid < ntot) {
+      if (p0 + tid < p_hi) {
         const FFRec &r = ff[p0 + tid];
         for (int c = 0; c < 3; ++c) {
           pk[c] = 3.0 * r.amu * r.n[c];
@@ -176,19 +201,29 @@ __global__ void __launch_bounds__(EO_T) k_elem_out(FmmDev d, ElemDev e, const FF
         // padding: no strength, far away
         for (int c = 0; c < 11; ++c) pk[c] = 0.0;
         pk[6] = -1.0e6;
+        pk[10] = -1.0;
       }
       pk[11] = 0.0;
     }
     const unsigned nb = __ballot_sync(0xffffffffu, near_box);
     if ((tid & 31) == 0 && tid < EO_LOAD) s_nearw[tid >> 5] = nb;
     __syncthreads();
-    const int nsub = min(EO_SUB, (ntot - p0 + EO_TILE - 1) / EO_TILE);
+    const int nsub = min(EO_SUB, (p_hi - p0 + EO_TILE - 1) / EO_TILE);
     for (int sb = 0; sb < nsub; ++sb) {
       const int qs = sb * EO_TILE;
       const bool near_sub = (s_nearw[qs >> 5] >> (qs & 31)) & ((1u << EO_TILE) - 1u);
-      unsigned nmask[EO_PPT];
-#pragma unroll
-      for (int i = 0; i < EO_PPT; ++i) nmask[i] = 0u;
+      if (near_sub) {
+        // the queue must hold one sub-tile's worst case: flush first if not
+        // (near_sub is the same in every thread, so are these barriers)
+        __syncthreads();
+        const int qn = s_qn;
+        if (qn > EO_QCAP - EO_NP * EO_TILE) {
+          near_flush<EO_T>(s_q, qn, t0, (uint32_t)p_lo, count, list, cap, &s_base);
+          __syncthreads();
+          if (tid == 0) s_qn = 0;
+        }
+        __syncthreads();
+      }
 #pragma unroll 4
       for (int q = 0; q < EO_TILE; ++q) {
         const double2 *pk = (const double2 *)s_pk[qs + q];
@@ -208,43 +243,24 @@ __global__ void __launch_bounds__(EO_T) k_elem_out(FmmDev d, ElemDev e, const FF
             v[i][0] = fma(k3, fma(coef, rx, B.y), v[i][0]);
             v[i][1] = fma(k3, fma(coef, ry, C.x), v[i][1]);
             v[i][2] = fma(k3, fma(coef, rz, C.y), v[i][2]);
-          } else {
-            nmask[i] |= 1u << q;
-          }
-        }
-      }
-      if (near_sub) {
-#pragma unroll
-        for (int i = 0; i < EO_PPT; ++i) {
-          unsigned m = act[i] ? nmask[i] : 0u;
-          while (m) {
-            const int q = __ffs(m) - 1;
-            m &= m - 1u;
-            const int j = p0 + qs + q;
-            const PanelGeo *pg = j < e.nbody ? e.body + j : e.wake + (j - e.nbody);
-            double u[3];
-            vel_pan_near(e.rp, *pg, pos[i], u);
-            for (int c = 0; c < 3; ++c) v[i][c] += u[c];
+          } else if (act[i]) {
+            s_q[atomicAdd(&s_qn, 1)] =
+                ((uint32_t)(p0 - p_lo + qs + q) << 10) | (uint32_t)(tid + i * EO_T);
           }
         }
       }
     }
   }
-  const double k4pi = 1.0 / (4.0 * DUST_PI);
+  __syncthreads();
+  near_flush<EO_T>(s_q, s_qn, t0, (uint32_t)p_lo, count, list, cap, &s_base);
 #pragma unroll
   for (int i = 0; i < EO_PPT; ++i) {
     if (!act[i]) continue;
-    for (int q = 0; q < e.nline; ++q) {
-      double u[3];
-      vel_line(e.rp, e.lines[q], pos[i], u);
-      for (int c = 0; c < 3; ++c) v[i][c] += u[c];
-    }
     const uint32_t t = t0 + tid + i * EO_T;
-    const uint32_t ip = d.perm[t];
     for (int c = 0; c < 3; ++c) {
-      vel[3 * (size_t)ip + c] = d.out[(size_t)c * n + t] + v[i][c] * k4pi + d.u_inf[c];
-      if (str) str[3 * (size_t)ip + c] = (d.use_vs || d.use_vd) ? d.out[(size_t)(3 + c) * n + t] : 0.0;
-      if (rot) rot[3 * (size_t)ip + c] = (d.use_vs && d.use_df) ? d.out[(size_t)(6 + c) * n + t] : 0.0;
+      double *o = farv + (size_t)c * n + t;
+      if (gridDim.y == 1) *o = v[i][c];
+      else atomicAdd(o, v[i][c]);
     }
   }
 }
@@ -252,15 +268,20 @@ __global__ void __launch_bounds__(EO_T) k_elem_out(FmmDev d, ElemDev e, const FF
 // FP32C element sums, far and near pairs in separate kernels.
 //
 // k_elem_far runs the far-field test and formula in FP32 for EF2_PPT
-// particles per thread against a shared-memory tile of EF2_TILE panels; the
-// tile's partial sums are FP32, added into FP64 per tile.  A pair that is
-// not clearly far (threshold widened by 1e-4 so a pair far in FP32 is far in
-// FP64) is queued in shared memory and the queue is appended to a global list
-// of near pairs.  k_elem_near evaluates that list with the reference's exact
-// FP64 formulas (vel_pan_near), one pair per thread, and k_elem_fin adds the end
-// vortices and writes the outputs in the caller's order.  Keeping the heavy
-// FP64 formulas out of the FP32 kernel keeps its register count, and so its
-// occupancy, at the level of the far-field arithmetic.
+// particles per thread against a shared-memory tile of EF2_TILE panels, two
+// panels at a time in packed arithmetic; the tile's partial sums are FP32,
+// added into FP64 per tile; blockIdx.y takes a chunk of the panels.  A pair
+// that is not clearly far (threshold widened by 1e-4 so a pair far in FP32 is
+// far in FP64) is queued in shared memory and the queue is appended to a
+// global list of near pairs.  k_elem_near evaluates that list with the
+// reference's exact FP64 formulas (vel_pan_near), one pair per thread, and
+// k_elem_fin adds the end vortices and writes the outputs in the caller's
+// order.  Keeping the heavy FP64 formulas out of the far kernels keeps their
+// register count, and so their occupancy, at the level of the far-field
+// arithmetic, and spreads the near pairs over all threads: the FP64 form
+// evaluated them inside k_elem_out's divergent branches by a thread per two
+// particles (12,800 particles x 440 panels 887 us, 60,000 x 3,270 8.3 ms; now
+// 76 us and 1.0 ms with k_elem_fin).
 //
 // Most tiles lie beyond the far-field radius of every particle of the CTA:
 // the loader threads test each panel against the bounding box of the CTA's
@@ -268,62 +289,38 @@ __global__ void __launch_bounds__(EO_T) k_elem_out(FmmDev d, ElemDev e, const FF
 // pair the per-pair test would queue) and such tiles run a loop without the
 // per-pair test.  A tile shorter than EF2_TILE is padded with null panels
 // (no strength, 1e6 away) so both loops are fully unrolled.
-#ifndef EF2_PPT
+//
+// Bound: the FP32 pipe, 18 packed operations per two pairs (2M particles x
+// 14,596 panels: 20.4 ms with a scalar per-pair test in the tiles near the
+// box and 64-panel loads, 19.8 ms now, 0.73 of the operations' rate).
 #define EF2_PPT 2
-#endif
 #define EF2_T 128
 #define EF2_NP (EF2_T * EF2_PPT)
 #define EF2_TILE 16  // panels per FP32 partial sum and per near-queue check
-#ifndef EF2_SUB
-#define EF2_SUB 4  // sub-tiles staged per barrier pair
-#endif
+#define EF2_SUB 8  // sub-tiles staged per barrier pair: every thread loads a panel
 #define EF2_LOAD (EF2_TILE * EF2_SUB)
 #define EF2_QCAP (EF2_NP * EF2_TILE)  // one tile's worst case
 static_assert(EF2_LOAD % 32 == 0 && EF2_LOAD <= EF2_T && EF2_SUB <= 32, "staging layout");
 static_assert(EF2_NP <= 1024, "local particle index is packed in 10 bits");
 
-struct NearPair {
-  uint32_t t, j;  // particle (sorted order), panel
-};
-
-__device__ __forceinline__ void ef2_flush(const uint32_t *s_q, int qn, uint32_t t0,
-                                          unsigned long long *count, NearPair *list,
-                                          unsigned long long cap, unsigned long long *s_base) {
-  if (threadIdx.x == 0) *s_base = atomicAdd(count, (unsigned long long)qn);
-  __syncthreads();
-  const unsigned long long base = *s_base;
-  for (int k = threadIdx.x; k < qn; k += EF2_T) {
-    const unsigned long long at = base + (unsigned long long)k;
-    if (at < cap) {
-      const uint32_t en = s_q[k];
-      list[at] = NearPair{t0 + (en & 0x3ffu), en >> 10};
-    }
-  }
-}
-
-// far-field term of a panel at r = p - c, added to acc:
+// far-field terms of two panels at r = p - c in packed FP32 (f32x2), added to
+// acc:
 //   nm = 3 A mu n, mn = -A mu n, as = A sigma:
 //   acc += (1/r^3) (r (r.nm / r^2 + as) + mn)
-__device__ __forceinline__ void ef2_term(float rx, float ry, float rz, float r2, float nmx,
-                                         float nmy, float nmz, float mnx, float mny, float mnz,
-                                         float as, float *acc) {
-  const float ir = rsqrt_approx(r2);
-  const float ir2 = ir * ir;
-  const float k3 = ir2 * ir;
-  const float rn = fmaf(rx, nmx, fmaf(ry, nmy, rz * nmz));
-  const float coef = fmaf(rn, ir2, as);
-  acc[0] = fmaf(k3, fmaf(coef, rx, mnx), acc[0]);
-  acc[1] = fmaf(k3, fmaf(coef, ry, mny), acc[1]);
-  acc[2] = fmaf(k3, fmaf(coef, rz, mnz), acc[2]);
-}
-
-// The same term for two panels at once in packed FP32 (f32x2) arithmetic.
-__device__ __forceinline__ void ef2_term2(float2 px, float2 py, float2 pz, float2 ncx, float2 ncy,
-                                          float2 ncz, float2 nmx, float2 nmy, float2 nmz,
-                                          float2 mnx, float2 mny, float2 mnz, float2 as,
-                                          float2 *acc) {
+// With NEAR, a panel not beyond its widened far-field radius (r^2 <= ff) is
+// reported in the returned bits and its term vanishes (1 / r^3 underflows).
+template <bool NEAR>
+__device__ __forceinline__ unsigned ef2_term2(float2 px, float2 py, float2 pz, float2 ncx,
+                                              float2 ncy, float2 ncz, float2 nmx, float2 nmy,
+                                              float2 nmz, float2 mnx, float2 mny, float2 mnz,
+                                              float2 as, float2 ff, float2 *acc) {
   const float2 rx = __fadd2_rn(px, ncx), ry = __fadd2_rn(py, ncy), rz = __fadd2_rn(pz, ncz);
-  const float2 r2 = __ffma2_rn(rx, rx, __ffma2_rn(ry, ry, __fmul2_rn(rz, rz)));
+  float2 r2 = __ffma2_rn(rx, rx, __ffma2_rn(ry, ry, __fmul2_rn(rz, rz)));
+  unsigned near = 0;
+  if (NEAR) {
+    if (!(r2.x > ff.x)) near |= 1u, r2.x = 3.0e38f;
+    if (!(r2.y > ff.y)) near |= 2u, r2.y = 3.0e38f;
+  }
   const float2 ir = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
   const float2 ir2 = __fmul2_rn(ir, ir);
   const float2 k3 = __fmul2_rn(ir2, ir);
@@ -332,6 +329,7 @@ __device__ __forceinline__ void ef2_term2(float2 px, float2 py, float2 pz, float
   acc[0] = __ffma2_rn(k3, __ffma2_rn(coef, rx, mnx), acc[0]);
   acc[1] = __ffma2_rn(k3, __ffma2_rn(coef, ry, mny), acc[1]);
   acc[2] = __ffma2_rn(k3, __ffma2_rn(coef, rz, mnz), acc[2]);
+  return near;
 }
 
 // Shared-memory tile: panels in pairs (q, q+1); the ten values of a pair
@@ -340,11 +338,12 @@ __device__ __forceinline__ void ef2_term2(float2 px, float2 py, float2 pz, float
 // operands of ef2_term2.
 #define EF2_PK 20
 
-__global__ void __launch_bounds__(EF2_T) k_elem_far(FmmDev d, ElemDev e, const FFRec *ff,
-                                                    double *farv, unsigned long long *count,
-                                                    NearPair *list, unsigned long long cap) {
+__global__ void __launch_bounds__(EF2_T, 8) k_elem_far(FmmDev d, ElemDev e, const FFRec *ff,
+                                                    int chunk, double *farv,
+                                                    unsigned long long *count, NearPair *list,
+                                                    unsigned long long cap) {
   __shared__ __align__(16) float s_pk[EF2_LOAD / 2][EF2_PK];
-  __shared__ float s_ff[EF2_LOAD];  // widened ff2
+  __shared__ __align__(8) float s_ff[EF2_LOAD];  // widened ff2
   __shared__ unsigned s_nearw[EF2_LOAD / 32];
   __shared__ uint32_t s_q[EF2_QCAP];  // (panel << 10) | local particle
   __shared__ float s_box[EF2_T / 32][6];
@@ -353,6 +352,7 @@ __global__ void __launch_bounds__(EF2_T) k_elem_far(FmmDev d, ElemDev e, const F
   const size_t n = d.n;
   const uint32_t t0 = blockIdx.x * EF2_NP;
   const int tid = threadIdx.x;
+  const int p_lo = blockIdx.y * chunk, p_hi = min(e.nbody + e.nwake, p_lo + chunk);
   const double ref[3] = {d.P[t0], d.P[n + t0], d.P[2 * n + t0]};
   float px[EF2_PPT], py[EF2_PPT], pz[EF2_PPT];
   bool act[EF2_PPT];
@@ -389,15 +389,14 @@ __global__ void __launch_bounds__(EF2_T) k_elem_far(FmmDev d, ElemDev e, const F
   for (int w = 0; w < EF2_T / 32; ++w)
     for (int c = 0; c < 3; ++c)
       lo[c] = fminf(lo[c], s_box[w][c]), hi[c] = fmaxf(hi[c], s_box[w][3 + c]);
-  const int ntot = e.nbody + e.nwake;
-  for (int p0 = 0; p0 < ntot; p0 += EF2_LOAD) {
+  for (int p0 = p_lo; p0 < p_hi; p0 += EF2_LOAD) {
     __syncthreads();
     // stage EF2_LOAD panels (EF2_SUB sub-tiles) with one barrier pair
     bool near_box = false;
     if (tid < EF2_LOAD) {
       float val[10] = {-1.0e6f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       float ffw = 0.f;
-      if (p0 + tid < ntot) {
+      if (p0 + tid < p_hi) {
         const FFRec &r = ff[p0 + tid];
         const float cx = (float)(r.c[0] - ref[0]), cy = (float)(r.c[1] - ref[1]),
                     cz = (float)(r.c[2] - ref[2]);
@@ -429,97 +428,110 @@ __global__ void __launch_bounds__(EF2_T) k_elem_far(FmmDev d, ElemDev e, const F
       for (int sb = 0; sb < 32 / EF2_TILE; ++sb)
         if ((bw >> (sb * EF2_TILE)) & ((1u << EF2_TILE) - 1u)) near_bits |= 1u << (w * (32 / EF2_TILE) + sb);
     }
-    const int nsub = min(EF2_SUB, (ntot - p0 + EF2_TILE - 1) / EF2_TILE);
+    const int nsub = min(EF2_SUB, (p_hi - p0 + EF2_TILE - 1) / EF2_TILE);
     for (int sb = 0; sb < nsub; ++sb) {
       const int q0 = p0 + sb * EF2_TILE;
-      double tv[EF2_PPT][3];
-      if (!((near_bits >> sb) & 1u)) {
-        float2 acc[EF2_PPT][3];
+      float2 acc[EF2_PPT][3];
 #pragma unroll
-        for (int i = 0; i < EF2_PPT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = make_float2(0.f, 0.f);
+      for (int i = 0; i < EF2_PPT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = make_float2(0.f, 0.f);
+      auto pair = [&](int pr, auto nearc) {
+        const float *pk = s_pk[sb * (EF2_TILE / 2) + pr];
+        const float4 A = *(const float4 *)&pk[0], B = *(const float4 *)&pk[4],
+                     C = *(const float4 *)&pk[8], D = *(const float4 *)&pk[12],
+                     E = *(const float4 *)&pk[16];
+        constexpr bool NEAR = decltype(nearc)::value;
+        const float2 ff2 = NEAR ? *(const float2 *)&s_ff[sb * EF2_TILE + 2 * pr]
+                                : make_float2(0.f, 0.f);
 #pragma unroll
-        for (int pr = 0; pr < EF2_TILE / 2; ++pr) {
-          const float *pk = s_pk[sb * (EF2_TILE / 2) + pr];
-          const float4 A = *(const float4 *)&pk[0], B = *(const float4 *)&pk[4],
-                       C = *(const float4 *)&pk[8], D = *(const float4 *)&pk[12],
-                       E = *(const float4 *)&pk[16];
-#pragma unroll
-          for (int i = 0; i < EF2_PPT; ++i)
-            ef2_term2(make_float2(px[i], px[i]), make_float2(py[i], py[i]),
-                      make_float2(pz[i], pz[i]), make_float2(A.x, A.y), make_float2(A.z, A.w),
-                      make_float2(B.x, B.y), make_float2(B.z, B.w), make_float2(C.x, C.y),
-                      make_float2(C.z, C.w), make_float2(D.x, D.y), make_float2(D.z, D.w),
-                      make_float2(E.x, E.y), make_float2(E.z, E.w), acc[i]);
+        for (int i = 0; i < EF2_PPT; ++i) {
+          unsigned m = ef2_term2<NEAR>(
+              make_float2(px[i], px[i]), make_float2(py[i], py[i]), make_float2(pz[i], pz[i]),
+              make_float2(A.x, A.y), make_float2(A.z, A.w), make_float2(B.x, B.y),
+              make_float2(B.z, B.w), make_float2(C.x, C.y), make_float2(C.z, C.w),
+              make_float2(D.x, D.y), make_float2(D.z, D.w), make_float2(E.x, E.y),
+              make_float2(E.z, E.w), ff2, acc[i]);
+          if (NEAR && act[i])
+            for (; m; m &= m - 1u)
+              s_q[atomicAdd(&s_qn, 1)] =
+                  ((uint32_t)(q0 - p_lo + 2 * pr + (m & 1u ? 0 : 1)) << 10) |
+                  (uint32_t)(tid + i * EF2_T);
         }
+      };
+      if (!((near_bits >> sb) & 1u)) {
 #pragma unroll
-        for (int i = 0; i < EF2_PPT; ++i)
-          for (int c = 0; c < 3; ++c) tv[i][c] = (double)acc[i][c].x + (double)acc[i][c].y;
+        for (int pr = 0; pr < EF2_TILE / 2; ++pr) pair(pr, std::false_type{});
       } else {
         // the queue must hold one sub-tile's worst case: flush first if not
         // (the near bits are the same in every thread, so are these barriers)
         __syncthreads();
-        if (s_qn > EF2_QCAP - EF2_NP * EF2_TILE) {
-          ef2_flush(s_q, s_qn, t0, count, list, cap, &s_base);
+        const int qn = s_qn;
+        if (qn > EF2_QCAP - EF2_NP * EF2_TILE) {
+          near_flush<EF2_T>(s_q, qn, t0, (uint32_t)p_lo, count, list, cap, &s_base);
           __syncthreads();
           if (tid == 0) s_qn = 0;
-          __syncthreads();
         }
-        float acc[EF2_PPT][3];
-#pragma unroll
-        for (int i = 0; i < EF2_PPT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = 0.f;
-#pragma unroll 4
-        for (int q = 0; q < EF2_TILE; ++q) {
-          const int ql = sb * EF2_TILE + q;
-          const float *pk = &s_pk[ql >> 1][ql & 1];
-          const float ffw = s_ff[ql];
-#pragma unroll
-          for (int i = 0; i < EF2_PPT; ++i) {
-            const float rx = px[i] + pk[0], ry = py[i] + pk[2], rz = pz[i] + pk[4];
-            const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-            if (r2 > ffw) {
-              ef2_term(rx, ry, rz, r2, pk[6], pk[8], pk[10], pk[12], pk[14], pk[16], pk[18],
-                       acc[i]);
-            } else if (act[i]) {
-              const int slot = atomicAdd(&s_qn, 1);
-              s_q[slot] = ((uint32_t)(q0 + q) << 10) | (uint32_t)(tid + i * EF2_T);
-            }
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < EF2_PPT; ++i)
-          for (int c = 0; c < 3; ++c) tv[i][c] = (double)acc[i][c];
+        __syncthreads();
+#pragma unroll 2
+        for (int pr = 0; pr < EF2_TILE / 2; ++pr) pair(pr, std::true_type{});
       }
 #pragma unroll
       for (int i = 0; i < EF2_PPT; ++i)
-        for (int c = 0; c < 3; ++c) v[i][c] += tv[i][c];
+        for (int c = 0; c < 3; ++c) v[i][c] += (double)acc[i][c].x + (double)acc[i][c].y;
     }
   }
   __syncthreads();
-  ef2_flush(s_q, s_qn, t0, count, list, cap, &s_base);
+  near_flush<EF2_T>(s_q, s_qn, t0, (uint32_t)p_lo, count, list, cap, &s_base);
 #pragma unroll
   for (int i = 0; i < EF2_PPT; ++i) {
     if (!act[i]) continue;
     const uint32_t t = t0 + tid + i * EF2_T;
-    for (int c = 0; c < 3; ++c) farv[(size_t)c * n + t] = v[i][c];
+    for (int c = 0; c < 3; ++c) {
+      double *o = farv + (size_t)c * n + t;
+      if (gridDim.y == 1) *o = v[i][c];
+      else atomicAdd(o, v[i][c]);
+    }
   }
 }
 
-// the queued near pairs, exact FP64 (one pair per thread)
+// The listed near pairs, exact FP64 (one pair per thread).  Where the list
+// overflowed its capacity (it grows before the next evaluation), every
+// (particle, panel) pair is tested again, with the far kernel's own test, and
+// the list is not used.
 #ifndef EN_MINB
 #define EN_MINB 8
 #endif
-__global__ void __launch_bounds__(128, EN_MINB) k_elem_near(FmmDev d, ElemDev e, const unsigned long long *count,
-                            const NearPair *list, unsigned long long cap, double *farv) {
-  const unsigned long long nq = min(*count, cap);
+template <bool F32>
+__global__ void __launch_bounds__(128, EN_MINB)
+    k_elem_near(FmmDev d, ElemDev e, const FFRec *ff, const unsigned long long *count,
+                const NearPair *list, unsigned long long cap, double *farv) {
   const size_t n = d.n;
+  const bool all = *count > cap;
+  const unsigned long long np = (unsigned long long)(e.nbody + e.nwake), nq = all ? n * np : *count;
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < nq;
        k += (unsigned long long)gridDim.x * blockDim.x) {
-    const NearPair np = list[k];
-    const double pos[3] = {d.P[np.t], d.P[n + np.t], d.P[2 * n + np.t]};
-    const PanelGeo *pg = (int)np.j < e.nbody ? e.body + np.j : e.wake + (np.j - e.nbody);
+    const NearPair pr = all ? NearPair{(uint32_t)(k / np), (uint32_t)(k % np)} : list[k];
+    const double pos[3] = {d.P[pr.t], d.P[n + pr.t], d.P[2 * n + pr.t]};
+    if (all) {
+      const FFRec &r = ff[pr.j];
+      bool far;
+      if constexpr (F32) {
+        const uint32_t r0 = pr.t / EF2_NP * EF2_NP;  // the far kernel's reference particle
+        float q[3];
+        for (int c = 0; c < 3; ++c) {
+          const double ref = d.P[(size_t)c * n + r0];
+          q[c] = (float)(pos[c] - ref) + -(float)(r.c[c] - ref);
+        }
+        far = fmaf(q[0], q[0], fmaf(q[1], q[1], q[2] * q[2])) > (float)r.ff2 * 1.0001f;
+      } else {
+        const double rx = pos[0] + -r.c[0], ry = pos[1] + -r.c[1], rz = pos[2] + -r.c[2];
+        far = fma(rx, rx, fma(ry, ry, rz * rz)) > r.ff2;
+      }
+      if (far) continue;
+    }
+    const PanelGeo *pg = (int)pr.j < e.nbody ? e.body + pr.j : e.wake + (pr.j - e.nbody);
     double u[3];
     vel_pan_near(e.rp, *pg, pos, u);
-    for (int c = 0; c < 3; ++c) atomicAdd(farv + (size_t)c * n + np.t, u[c]);
+    for (int c = 0; c < 3; ++c) atomicAdd(farv + (size_t)c * n + pr.t, u[c]);
   }
 }
 
@@ -577,6 +589,7 @@ __device__ __forceinline__ void line_vel_f(const double *vv, const float *q, con
 
 #define EL_T 128
 #define EL_TILE 64
+template <bool F32>
 __global__ void __launch_bounds__(EL_T) k_elem_fin(FmmDev d, ElemDev e, const double *farv,
                                                    double *vel, double *str, double *rot) {
   __shared__ double s_v[EL_TILE][6];
@@ -590,8 +603,14 @@ __global__ void __launch_bounds__(EL_T) k_elem_fin(FmmDev d, ElemDev e, const do
   const float rr2 = (float)(e.rp.r_rankine * e.rp.r_rankine), rc = (float)e.rp.r_cutoff;
   double w[3] = {0.0, 0.0, 0.0};
   if (act)
-    for (int c = 0; c < 3; ++c) w[c] = farv[(size_t)c * n + t];
-  for (int q0 = 0; q0 < e.nline; q0 += EL_TILE) {
+    for (int c = 0; c < 3; ++c) w[c] = farv ? farv[(size_t)c * n + t] : 0.0;
+  if (!F32 && act)
+    for (int q = 0; q < e.nline; ++q) {
+      double u[3];
+      vel_line(e.rp, e.lines[q], pos, u);
+      for (int c = 0; c < 3; ++c) w[c] += u[c];
+    }
+  for (int q0 = 0; F32 && q0 < e.nline; q0 += EL_TILE) {
     const int m = min(EL_TILE, e.nline - q0);
     __syncthreads();
     if (threadIdx.x < m) {
@@ -628,61 +647,69 @@ __global__ void __launch_bounds__(EL_T) k_elem_fin(FmmDev d, ElemDev e, const do
   }
 }
 
-// FP32C path: far kernel, (grow and redo if the near list overflowed), near
-// kernel, outputs
-static int elem_output_split(FmmDev &d, const ElemDev &e, const FFRec *ff, DevBuf &work,
-                             size_t &near_cap, double *vel, double *str, double *rot,
-                             cudaStream_t st, cudaEvent_t *kev, bool *kev_done) {
+// Panels per CTA of the far kernels: the particle blocks alone fill the
+// resident CTAs several times in a large evaluation; a small one shares the
+// panels out until they do, in whole loads and, the queue's packing, fewer than
+// 2^22 panels.
+static int elem_chunk(unsigned pblocks, int ntot, int load) {
+  const int want = (int)std::max<int64_t>(1, (148 * 12 + (int64_t)pblocks - 1) / pblocks);
+  const int loads = (ntot + load - 1) / load;
+  return std::min(std::max(1, (loads + want - 1) / want), (1 << 21) / load) * load;
+}
+
+int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
+                       size_t &near_cap, unsigned long long *near_seen, int precision,
+                       double *vel, double *str, double *rot, cudaStream_t st, cudaEvent_t *kev,
+                       bool *kev_done) {
+  if (kev_done) *kev_done = false;
+  const int ntot = e.nbody + e.nwake;
+  const bool f32 = precision == DUST_PREC_FP32C;
   const size_t n = d.n;
-  if (near_cap == 0) near_cap = std::max<size_t>(1 << 20, n * 96);
-  for (int attempt = 0; attempt < 3; ++attempt) {
+  double *farv = nullptr;
+  if (n > 0 && ntot > 0) {
+    DUST_TRY(devbuf_grow(ffbuf, sizeof(FFRec) * (size_t)ntot));
+    FFRec *ff = (FFRec *)ffbuf.p;
+    if (e.nbody) k_ffrec<<<nblk(e.nbody, 128), 128, 0, st>>>(e.body, e.nbody, e.rp.ff_dou, ff);
+    if (e.nwake)
+      k_ffrec<<<nblk(e.nwake, 128), 128, 0, st>>>(e.wake, e.nwake, e.rp.ff_dou, ff + e.nbody);
+    // near-pair list: a first size, grown when an earlier evaluation on the
+    // handle listed more (*near_seen, copied back without waiting for it)
+    if (near_cap == 0)
+      near_cap = std::max(std::max<size_t>(1 << 20, n * 96),
+                          std::min<size_t>(n * (size_t)ntot / 8, 1 << 26));
+    const unsigned long long seen = *(volatile unsigned long long *)near_seen;
+    if (seen > near_cap) near_cap = (size_t)(seen + seen / 4 + 1024);
     const size_t off_l = (n * 24 + 255) / 256 * 256 + 256;
     DUST_TRY(devbuf_grow(work, off_l + near_cap * sizeof(NearPair)));
-    double *farv = (double *)work.p;
+    farv = (double *)work.p;
     unsigned long long *count = (unsigned long long *)((char *)work.p + off_l - 256);
     NearPair *list = (NearPair *)((char *)work.p + off_l);
-    DUST_CUDA(cudaMemsetAsync(count, 0, 8, st));
+    const unsigned long long cap = near_cap;
+    const unsigned pb = nblk(n, f32 ? EF2_NP : EO_NP);
+    const int chunk = elem_chunk(pb, ntot, f32 ? EF2_LOAD : EO_LOAD);
+    const dim3 grid(pb, nblk(ntot, chunk));
+    DUST_CUDA(cudaMemsetAsync(farv, 0, off_l, st));
     if (kev) cudaEventRecord(kev[0], st);
-    k_elem_far<<<nblk(n, EF2_NP), EF2_T, 0, st>>>(d, e, ff, farv, count, list,
-                                                    (unsigned long long)near_cap);
+    if (f32)
+      k_elem_far<<<grid, EF2_T, 0, st>>>(d, e, ff, chunk, farv, count, list, cap);
+    else
+      k_elem_far64<<<grid, EO_T, 0, st>>>(d, e, ff, chunk, farv, count, list, cap);
     if (kev) {
       cudaEventRecord(kev[1], st);
       if (kev_done) *kev_done = true;
     }
-    unsigned long long h = 0;
-    DUST_CUDA(cudaMemcpyAsync(&h, count, 8, cudaMemcpyDeviceToHost, st));
-    DUST_CUDA(cudaStreamSynchronize(st));
-    if (h > near_cap) {
-      near_cap = (size_t)(h + h / 4 + 1024);
-      continue;
-    }
-    if (h > 0) {
-      const unsigned grid = (unsigned)std::min<unsigned long long>((h + 127) / 128, 148ull * 64);
-      k_elem_near<<<grid, 128, 0, st>>>(d, e, count, list, (unsigned long long)near_cap, farv);
-    }
-    k_elem_fin<<<nblk(n, EL_T), EL_T, 0, st>>>(d, e, farv, vel, str, rot);
-    DUST_CUDA(cudaGetLastError());
-    return DUST_OK;
-  }
-  return DUST_ERR_CAPACITY;
-}
-
-int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
-                       size_t &near_cap, int precision, double *vel, double *str, double *rot,
-                       cudaStream_t st, cudaEvent_t *kev, bool *kev_done) {
-  if (kev_done) *kev_done = false;
-  int ntot = e.nbody + e.nwake;
-  DUST_TRY(devbuf_grow(ffbuf, sizeof(FFRec) * (size_t)std::max(ntot, 1)));
-  FFRec *ff = (FFRec *)ffbuf.p;
-  if (e.nbody) k_ffrec<<<nblk(e.nbody, 128), 128, 0, st>>>(e.body, e.nbody, e.rp.ff_dou, ff);
-  if (e.nwake)
-    k_ffrec<<<nblk(e.nwake, 128), 128, 0, st>>>(e.wake, e.nwake, e.rp.ff_dou, ff + e.nbody);
-  if (d.n > 0) {
-    // the near-pair queue packs the panel index in 22 bits
-    if (precision == DUST_PREC_FP32C && ntot < (1 << 22))
-      return elem_output_split(d, e, ff, work, near_cap, vel, str, rot, st, kev, kev_done);
+    const unsigned gn = (unsigned)std::min<uint64_t>((uint64_t)n * ntot / 128 + 1, 148ull * 64);
+    if (f32)
+      k_elem_near<true><<<gn, 128, 0, st>>>(d, e, ff, count, list, cap, farv);
     else
-      k_elem_out<<<nblk(d.n, EO_NP), EO_T, 0, st>>>(d, e, ff, vel, str, rot);
+      k_elem_near<false><<<gn, 128, 0, st>>>(d, e, ff, count, list, cap, farv);
+    DUST_CUDA(cudaMemcpyAsync(near_seen, count, 8, cudaMemcpyDeviceToHost, st));
+  }
+  if (n > 0) {
+    if (f32)
+      k_elem_fin<true><<<nblk(n, EL_T), EL_T, 0, st>>>(d, e, farv, vel, str, rot);
+    else
+      k_elem_fin<false><<<nblk(n, EL_T), EL_T, 0, st>>>(d, e, farv, vel, str, rot);
   }
   DUST_CUDA(cudaGetLastError());
   return DUST_OK;

@@ -300,15 +300,44 @@ __device__ inline void vel_pan(const RegParams &rp, const PanelGeo &p, const dou
   }
 }
 
+// x^-1/2 and 1/x for x > 0: FP32 approximations refined by one second-order
+// step in FP64 (with the seed's relative error d < 2^-21, O(d^3) is below the
+// FP64 rounding); outside the FP32 range (and at zero) the library's.
+__device__ __forceinline__ bool near_f32_range(double x) {  // 2^-100 <= x < 2^100
+  return (unsigned)(__double2hiint(x) - ((1023 - 100) << 20)) < (200u << 20);
+}
+__device__ __forceinline__ double near_rsqrt(double x) {
+  if (!near_f32_range(x)) return 1.0 / sqrt(x);
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
+  const double y = (double)r, e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double near_rcp(double x) {
+  if (!near_f32_range(x)) return 1.0 / x;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
+  const double y = (double)r, e = fma(-x, y, 1.0);
+  return fma(y * e, 1.0 + e, y);
+}
+__device__ __forceinline__ double near_sqrt(double x, double irs) {
+  return x > 0.0 ? x * irs : 0.0;
+}
+
 // vel_pan for a point inside the panel's far-field radius, with the
 // per-vertex quantities shared between the edges: the distances to the
 // vertices and to the projected vertices are computed once per vertex (the
 // reference's loops recompute each at both of its edges), reciprocal
-// distances replace the divisions by them, the solid angle's atan2 takes its
-// two arguments unscaled (atan2(y/d, x/d) = atan2(y, x) for d > 0), and the
-// Rankine-core test compares squares.  Same branches and formulas as
-// vel_pan (vel_dou, vel_sou, pot_dou), equal up to rounding; points beyond
-// the far-field radii go to vel_pan.
+// distances and approximations refined to FP64 replace square roots and
+// quotients, and the Rankine-core test compares squares.  The solid angle
+// (pot_dou's sum of the polygon's angles less its flat value) is twice the
+// argument of the product of its triangles' complex numbers
+//   |a||b||c| + (a.b)|c| + (a.c)|b| + (b.c)|a| + i a.(b x c)
+// (van Oosterom and Strackee, IEEE Trans. Biomed. Eng. 30, 1983): one atan2
+// of products instead of one per vertex after normalisations, and no
+// cancellation of the flat value.  Same branches and values as vel_pan
+// (vel_dou, vel_sou, pot_dou) up to rounding; points beyond the far-field
+// radii go to vel_pan.
 template <int NV>
 __device__ inline void vel_pan_near_t(const RegParams &rp, const PanelGeo &p, const double *pos,
                                       double *v) {
@@ -328,8 +357,8 @@ __device__ inline void vel_pan_near_t(const RegParams &rp, const PanelGeo &p, co
   for (int i = 0; i < nv; ++i) {
     for (int d = 0; d < 3; ++d) dv[i][d] = pos[d] - p.ver[i][d];
     const double q = d3dot(dv[i], dv[i]);
-    R[i] = sqrt(q);
-    iR[i] = 1.0 / R[i];
+    iR[i] = near_rsqrt(q);
+    R[i] = near_sqrt(q, iR[i]);
   }
   double vd[3] = {0.0, 0.0, 0.0};
   if (dou_far) {
@@ -348,9 +377,9 @@ __device__ inline void vel_pan_near_t(const RegParams &rp, const PanelGeo &p, co
       const double rr = rp.r_rankine * L;
       double f;
       if (hi2 > rr * rr) {
-        f = ((L - ai) * iR[ip1] + ai * iR[i1]) / hi2;
+        f = ((L - ai) * iR[ip1] + ai * iR[i1]) * near_rcp(hi2);
       } else if (R[i1] > L * rp.r_cutoff && R[ip1] > L * rp.r_cutoff) {
-        f = ((L - ai) * iR[ip1] + ai * iR[i1]) / (rr * rr);
+        f = ((L - ai) * iR[ip1] + ai * iR[i1]) * near_rcp(rr * rr);
       } else {
         continue;
       }
@@ -369,14 +398,15 @@ __device__ inline void vel_pan_near_t(const RegParams &rp, const PanelGeo &p, co
 #pragma unroll
     for (int i = 0; i < nv; ++i) {
       const double a[3] = {pos[0] - p.verp[i][0], pos[1] - p.verp[i][1], pos[2] - p.verp[i][2]};
-      Rp[i] = sqrt(d3dot(a, a));
+      const double q = d3dot(a, a);
+      Rp[i] = near_sqrt(q, near_rsqrt(q));
     }
     double phix = 0.0, phiy = 0.0;
 #pragma unroll
     for (int i1 = 0; i1 < nv; ++i1) {
       const int ip1 = i1 + 1 == nv ? 0 : i1 + 1;
       const double L = p.edge_len[i1], s = Rp[i1] + Rp[ip1];
-      const double souLog = (s - L < 1e-12) ? 0.0 : log((s + L) / (s - L));
+      const double souLog = (s - L < 1e-12) ? 0.0 : log((s + L) * near_rcp(s - L));
       phix += p.sinTi[i1] * souLog;
       phiy -= p.cosTi[i1] * souLog;
     }
@@ -384,26 +414,20 @@ __device__ inline void vel_pan_near_t(const RegParams &rp, const PanelGeo &p, co
     if (dou_far) {
       pdou = d3dot(rv, p.nor) * p.area / (radius * radius * radius);
     } else {
-      double dou = 0.0;
+      double re = 1.0, im = 0.0;
 #pragma unroll
-    for (int i1 = 0; i1 < nv; ++i1) {
-        const int im1 = i1 == 0 ? nv - 1 : i1 - 1;
-        double ei[3], ap1[3], am1[3], cr[3];
-        for (int d = 0; d < 3; ++d) ei[d] = -dv[i1][d] * iR[i1];
-        const double ep = d3dot(ei, p.edge_vec[i1]), em = d3dot(ei, p.edge_vec[im1]);
-        for (int d = 0; d < 3; ++d) {
-          ap1[d] = p.edge_vec[i1][d] - ei[d] * ep;
-          am1[d] = -p.edge_vec[im1][d] + ei[d] * em;
-        }
-        d3cross(am1, ap1, cr);
-        dou += atan2(d3dot(ei, cr), d3dot(am1, ap1));
+      for (int t = 1; t + 1 < nv; ++t) {
+        const double *a = dv[0], *b = dv[t], *c = dv[t + 1];
+        double bc[3];
+        d3cross(b, c, bc);
+        const double y = d3dot(a, bc);
+        const double x = R[0] * R[t] * R[t + 1] + d3dot(a, b) * R[t + 1] + d3dot(a, c) * R[t] +
+                         d3dot(b, c) * R[0];
+        const double z = re * x - im * y;
+        im = re * y + im * x;
+        re = z;
       }
-      const double gb = (double)(nv - 2) * DUST_PI;
-      if (dou < -gb + 1.0e-5)
-        dou += gb;
-      else if (dou > gb - 1.0e-5)
-        dou -= gb;
-      pdou = dou;
+      pdou = 2.0 * atan2(im, re);
     }
     for (int d = 0; d < 3; ++d)
       vs[d] = -(p.tang[0][d] * phix + p.tang[1][d] * phiy + p.nor[d] * pdou);

@@ -194,6 +194,9 @@ extern "C" int dust_octree_create(const dust_fmm_params *prm, dust_octree **out)
   st = build_tables(o);
   if (st == DUST_OK) st = grow(o->small, 64 * 8);
   if (st == DUST_OK && cudaMemset(o->small.p, 0, 64 * 8) != cudaSuccess) st = DUST_ERR_CUDA;
+  if (st == DUST_OK && cudaMallocHost(&o->near_seen, sizeof(*o->near_seen)) != cudaSuccess)
+    st = DUST_ERR_CUDA;
+  if (st == DUST_OK) *o->near_seen = 0;
   if (st == DUST_OK) st = build_shift_tables(o);
   if (st == DUST_OK) st = m2l_batch_tables(o);
   if (st != DUST_OK) {
@@ -220,6 +223,7 @@ extern "C" int dust_octree_destroy(dust_octree *o) {
   devbuf_free(o->shift);
   devbuf_free(o->ffbuf);
   devbuf_free(o->elem_work);
+  if (o->near_seen) cudaFreeHost(o->near_seen);
   DevBuf *bufs[] = {&o->idxsum, &o->keys,   &o->keys_s, &o->vals,   &o->perm,
                     &o->cnt,    &o->cstart, &o->part,   &o->flags,  &o->ind,
                     &o->cidx,   &o->lidx,   &o->act_key, &o->act_lev, &o->leaf_ci,
@@ -1800,8 +1804,8 @@ int fmm_points_uvort_device(dust_octree *o, const ElemDev &lines, double *uv, cu
 int fmm_finish_device(dust_octree *o, int n, const ElemDev &e, double *vel, double *str,
                       double *rot, cudaStream_t st) {
   if (n > 0)
-    DUST_TRY(elem_output_device(o->dev, e, o->ffbuf, o->elem_work, o->near_cap, o->prm.precision,
-                                vel, str, rot, st, o->timing ? &o->ev[8] : nullptr, &o->kev_far));
+    DUST_TRY(elem_output_device(o->dev, e, o->ffbuf, o->elem_work, o->near_cap, o->near_seen,
+                                o->prm.precision, vel, str, rot, st, o->timing ? &o->ev[8] : nullptr, &o->kev_far));
   if (o->timing) cudaEventRecord(o->ev[5], st);
   DUST_CUDA(cudaGetLastError());
   return DUST_OK;

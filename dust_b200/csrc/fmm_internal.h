@@ -66,8 +66,9 @@ struct dust_octree {
   DevBuf act_key, act_lev, leaf_ci, mp, outs, cub_tmp, small;
   DevBuf h_in, h_out, h_pts, el_geo, el_raw;  // staging of host-API calls
   DevBuf ffbuf;                        // far-field panel records
-  DevBuf elem_work;                    // FP32C element sums: far sums, near-pair list
+  DevBuf elem_work;                    // element sums: far sums, near-pair list
   size_t near_cap = 0;                 // capacity of the near-pair list
+  unsigned long long *near_seen = nullptr;  // pairs the last evaluation listed (pinned host)
   DevBuf dtabs[DUST_MAXLEV + 1];       // dimensionless scalar M2L tables (FP64)
   DevBuf jsum;                         // M2L index table, then the classes' offsets
   DevBuf p2p_work;                     // near-field items and per-leaf split flags
@@ -134,8 +135,9 @@ int m2l_scale_sources(dust_octree *o, FmmDev &d, cudaStream_t st);
 
 // direct.cu
 int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
-                       size_t &near_cap, int precision, double *vel, double *str, double *rot,
-                       cudaStream_t st, cudaEvent_t *kev = nullptr, bool *kev_done = nullptr);
+                       size_t &near_cap, unsigned long long *near_seen, int precision,
+                       double *vel, double *str, double *rot, cudaStream_t st,
+                       cudaEvent_t *kev = nullptr, bool *kev_done = nullptr);
 // Morton order of n particles over the octree box (10 bits per axis): the
 // permutation in scratch (grown to morton_perm_bytes(n) if needed)
 size_t morton_perm_bytes(int n, cudaStream_t st);

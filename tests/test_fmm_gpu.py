@@ -355,3 +355,31 @@ def test_uvort_chunks_match_oracle(npts, n, nl, prec):
     uo = O.points_uvort(prm, pts, cen, dir_, mag, rv, ev)
     ug = octree.points_uvort(prm, pts, cen, dir_, mag, rv, ev)
     assert rel(ug, uo) < (TOL64 if prec == abi.DUST_PREC_FP64 else TOL32)
+
+
+@pytest.mark.parametrize("prec", [abi.DUST_PREC_FP64, abi.DUST_PREC_FP32C])
+@pytest.mark.parametrize("n,panels", [(1, (1, 1)), (257, (13, 5)), (3000, (40, 10))])
+def test_element_chunks_and_list_overflow(n, panels, prec):
+    """Element sums of few particles share the panels among CTAs; with all
+    1.2M pairs near (the last size) the pair list overflows in the first
+    evaluation and holds them in the second.  Both equal the oracle."""
+    rng = np.random.default_rng(n)
+    wing, te = synth.flat_wing(span=2.0, chord=1.0, n_span=panels[0], n_chord=panels[1])
+    body = abi.PanelSet(wing.ver, kind=wing.kind, mag=rng.standard_normal(wing.n))
+    if n == 3000:  # every pair inside the far-field radius
+        ratio = 1e4
+    else:
+        ratio = 10.0
+    cen = rng.uniform([-0.4, -1.4, 0.05], [1.4, 1.4, 0.6], (n, 3))
+    dir_ = rng.standard_normal((n, 3))
+    dir_ /= np.linalg.norm(dir_, axis=1)[:, None]
+    mag, rv = np.full(n, 1e-3), np.full(n, 0.05)
+    prm = FmmParams(box_length=4.0, origin=(-1.5, -2.0, -2.0), n_octree_levels=4,
+                    min_octree_part=5, multipole_degree=4, rankine_rad=0.1, precision=prec,
+                    far_field_ratio_doublet=ratio)
+    els = abi.elements_struct(body)
+    ov, _, _, _ = O.fmm_apply(prm, cen, dir_, mag, rv, els)
+    oc = octree.initialize_octree(prm)
+    for _ in range(2):
+        v, _, _ = oc.apply_multipole(cen, dir_, mag, rv, els)
+        assert rel(v, ov) < (TOL64 if prec == abi.DUST_PREC_FP64 else TOL32)
