@@ -73,11 +73,7 @@ __global__ void k_ffrec(const PanelGeo *pg, int n, double ff_dou, FFRec *out) {
 // box distance is formed with the per-pair test's own operation order, so
 // rounding, being monotone, cannot make the box call far a pair the per-pair
 // test calls near).  In the other sub-tiles each pair is tested and a near
-// pair queued.  The reciprocal square root of the far formula is the FP32
-// approximation refined by one second-order Newton-Raphson (Householder) step
-// in FP64: with y0 = x^-1/2 (1 + d) and e = 1 - x y0^2,
-// y = y0 (1 + e/2 + 3 e^2/8) has relative error O(d^3), below the FP64
-// rounding for |d| < 2^-21.
+// pair queued.
 #define EO_PPT 2
 #define EO_T 128
 #define EO_NP (EO_T * EO_PPT)
@@ -92,22 +88,6 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
-}
-
-// x^-1/2 for a normal FP32-range x > 0
-__device__ __forceinline__ double rsqrt_hh(double x) {
-  const double y = (double)rsqrt_approx((float)x);
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
-// x^-3/2 for a normal FP32-range x > 0: with the FP32 approximation y0 and
-// e = 1 - x y0^2, x^-3/2 = y0^3 (1 + 3e/2 + 15e^2/8 + O(e^3)); y0^2 is exact
-// in FP64.  One operation less than the cube of rsqrt_hh.
-__device__ __forceinline__ double rcube_hh(double x) {
-  const double y = (double)rsqrt_approx((float)x);
-  const double t = y * y, e = fma(-x, t, 1.0), y3 = t * y;
-  return fma(y3 * e, fma(1.875, e, 1.5), y3);
 }
 
 struct NearPair {
@@ -235,7 +215,7 @@ __global__ void __launch_bounds__(EO_T) k_elem_far64(FmmDev d, ElemDev e, const 
           const double r2 = fma(rx, rx, fma(ry, ry, rz * rz));
           const bool far = !near_sub || r2 > F.x;
           if (far) {
-            const double ir = rsqrt_hh(r2);
+            const double ir = rsqrt_r(r2);
             const double ir2 = ir * ir;
             const double k3 = ir2 * ir;
             const double rn = fma(rx, A.x, fma(ry, A.y, rz * B.x));
@@ -747,14 +727,13 @@ static int uvort_chunk(int pb, int n, int occ) {
   return best;
 }
 
-// FP64 uvort (plain mode): FP64-pipe and latency bound (18 FP64 operations and
-// two conversions a pair; 7,001 points x 50,021 particles 576 -> 502 us, 0.66
-// of the operations' rate; 2 points per thread and 6 CTAs per SM, 4 and 4:
-// 508 us).  Particles in the caller's order, UVD_PPT points
+// FP64 uvort (plain mode): FP64-pipe bound (18 FP64 operations a pair; 7,001
+// points x 50,021 particles 576 us at the start, 502 us with the chunks above,
+// 6 CTAs of 2 points per thread and x^-3/2 in one correction, 449 us without
+// the seed's conversions, 0.75 of the operations' rate).  Particles in the caller's order, UVD_PPT points
 // per thread (consecutive CTA slices of UV2_T points) against a shared tile
-// of (x, y, z, r_v^2, alpha, w = x x alpha) records; the reciprocal square
-// root as in k_elem_out (FP32 seed, one Householder step in FP64).  With
-// c = rho^-3 the tile's sum is
+// of (x, y, z, r_v^2, alpha, w = x x alpha) records.  With c = rho^-3 the
+// tile's sum is
 //   sum_q c_q (p - x_q) x alpha_q = p x (sum_q c_q alpha_q) - sum_q c_q w_q,
 // two 3-vector FMA accumulations per pair instead of a cross product and its
 // accumulation; in FP64 the difference of the two sums costs at most about
@@ -804,7 +783,7 @@ __global__ void __launch_bounds__(UV2_T, UVD_OCC) k_uvort(int npts, const double
       for (int i = 0; i < UVD_PPT; ++i) {
         const double dx = pos[i][0] - X.x, dy = pos[i][1] - X.y, dz = pos[i][2] - Y.x;
         const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, Y.y)));
-        const double c = rcube_hh(r2);
+        const double c = rcube_r(r2);
         A[i][0] = fma(c, Z.x, A[i][0]);
         A[i][1] = fma(c, Z.y, A[i][1]);
         A[i][2] = fma(c, P.x, A[i][2]);
@@ -893,7 +872,7 @@ __global__ void __launch_bounds__(UV2_T, UVDP_OCC) k_uvort_pres(int npts, const 
       for (int i = 0; i < UVD_PPT; ++i) {
         const double dx = pos[i][0] - X.x, dy = pos[i][1] - X.y, dz = pos[i][2] - Y.x;
         const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, Y.y)));
-        const double c = rcube_hh(r2);
+        const double c = rcube_r(r2);
         A[i][0] = fma(c, Z.x, A[i][0]);
         A[i][1] = fma(c, Z.y, A[i][1]);
         A[i][2] = fma(c, P.x, A[i][2]);

@@ -300,26 +300,40 @@ __device__ inline void vel_pan(const RegParams &rp, const PanelGeo &p, const dou
   }
 }
 
-// x^-1/2 and 1/x for x > 0: FP32 approximations refined by one second-order
-// step in FP64 (with the seed's relative error d < 2^-21, O(d^3) is below the
-// FP64 rounding); outside the FP32 range (and at zero) the library's.
-__device__ __forceinline__ bool near_f32_range(double x) {  // 2^-100 <= x < 2^100
-  return (unsigned)(__double2hiint(x) - ((1023 - 100) << 20)) < (200u << 20);
-}
-__device__ __forceinline__ double near_rsqrt(double x) {
-  if (!near_f32_range(x)) return 1.0 / sqrt(x);
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
-  const double y = (double)r, e = fma(-x * y, y, 1.0);
+// x^-1/2, x^-3/2 and 1/x for normal x > 0 from the approximation instructions
+// refined by one second-order step: with the seed's relative error d and
+// e = 1 - x y0^2 (1 - x y0), the result's error is O(d^3), below the FP64
+// rounding for |d| < 2^-18 (measured on sm_100: |d| < 2^-35, results within
+// 2 ulp).  The FP64 forms of the approximations need no conversion to FP32
+// and back, which the FP64 pair kernels spent more on the special-function
+// unit for than on the approximation itself.
+__device__ __forceinline__ double rsqrt_r(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
-__device__ __forceinline__ double near_rcp(double x) {
-  if (!near_f32_range(x)) return 1.0 / x;
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
-  const double y = (double)r, e = fma(-x, y, 1.0);
+__device__ __forceinline__ double rcube_r(double x) {
+  // x^-3/2 = y0^3 (1 + 3e/2 + 15e^2/8 + O(e^3))
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double t = y * y, e = fma(-x, t, 1.0), y3 = t * y;
+  return fma(y3 * e, fma(1.875, e, 1.5), y3);
+}
+__device__ __forceinline__ double rcp_r(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
   return fma(y * e, 1.0 + e, y);
 }
+// the same with zeros and infinities as the library's
+__device__ __forceinline__ bool near_range(double x) {  // 2^-1000 <= x < 2^1000
+  return (unsigned)(__double2hiint(x) - ((1023 - 1000) << 20)) < (2000u << 20);
+}
+__device__ __forceinline__ double near_rsqrt(double x) {
+  return near_range(x) ? rsqrt_r(x) : 1.0 / sqrt(x);
+}
+__device__ __forceinline__ double near_rcp(double x) { return near_range(x) ? rcp_r(x) : 1.0 / x; }
 __device__ __forceinline__ double near_sqrt(double x, double irs) {
   return x > 0.0 ? x * irs : 0.0;
 }

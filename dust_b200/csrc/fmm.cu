@@ -931,18 +931,6 @@ struct P2PAcc {
   double v[3], s[3], r[3], f[3];
 };
 
-// x^-1/2 for a normal FP32-range x > 0: the FP32 approximation refined by
-// one second-order Newton-Raphson (Householder) step in FP64.  With
-// y0 = x^-1/2 (1 + d) and e = 1 - x y0^2, y = y0 (1 + e/2 + 3 e^2/8) has
-// relative error O(d^3), below the FP64 rounding for |d| < 2^-21.
-__device__ __forceinline__ double p2p_rsqrt(double x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
-  const double y = (double)r;
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // One source q acting on target p: the reference's compute_vel,
 // compute_stretch, compute_rotu and compute_diffusion of source q
 // (mod_vortpart.f90:139-336), 4*pi factors applied by the caller.  s2 and
@@ -953,7 +941,7 @@ __device__ __forceinline__ void p2p_pair(const double *tp, const double *ta, dou
                                          double qaz, double s2, double is2, P2PAcc &A) {
   double dx = tp[0] - qx, dy = tp[1] - qy, dz = tp[2] - qz;
   double r2 = dx * dx + dy * dy + dz * dz;
-  double inv = p2p_rsqrt(r2 + s2);
+  double inv = rsqrt_r(r2 + s2);
   double inv2 = inv * inv;
   double c = -inv2 * inv;        // -1/rho^3
   double dd = -3.0 * c * inv2;   // 3/rho^5
@@ -979,7 +967,7 @@ __device__ __forceinline__ void p2p_pair(const double *tp, const double *ta, dou
   if (VD) {
     // (1/s^2) vol (aq - ap) eta, vol = 4/3 pi s^3, eta = 105/(8 pi)/s^3/(1+r^2/s^2)^4.5
     double t = r2 * is2 + 1.0;
-    double rt = p2p_rsqrt(t);
+    double rt = rsqrt_r(t);
     double rt2 = rt * rt, rt4 = rt2 * rt2;
     double w = 17.5 * is2 * (rt4 * rt4 * rt);
     A.f[0] += w * (qax - ta[0]);
