@@ -182,12 +182,20 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tf32_minus(int m, int n, in
 //  * warp 0 lane 0 produces (TMA, mbarrier expect-tx), warp 1 lane 0 issues
 //    tcgen05.mma (M = 128, N = 256, K = 8) and commits each stage back to
 //    its empty barrier; the accumulator lives in 256 TMEM columns;
+//  * an update of inner dimension 256 moves as many bytes of C as it has time
+//    to multiply, so it is bound by C's traffic: two CTAs per SM (2 stages and
+//    256 TMEM columns each), so that one's products run under the other's
+//    epilogue, and 8 warps that fetch C 16 columns ahead.  16,128 x 16,128 x
+//    256: 1,219 us with one CTA of 4 warps and 4 stages, 470 us now (2.1 GB of
+//    C: 317 us at the copy rate); the 16,384 LU's updates 31.8 -> 17.0 ms (one
+//    CTA of 8 warps and 4 stages: 21.9 ms); 12,000 x 1,920 x 12,000 the same;
 //  * every wait is bounded; on timeout the kernel flags the error, waits
 //    (bounded) for the copies and MMAs it issued, frees TMEM and returns.
 #define TP_BM 128
 #define TP_BN 256
 #define TP_BK 32
-#define TP_STAGES 4
+#define TP_STAGES 2    // and two CTAs per SM
+#define TP_T 256
 #define TP_A_BYTES (TP_BM * TP_BK * 4)  // 16 KiB
 #define TP_B_BYTES (TP_BN * TP_BK * 4)  // 32 KiB
 #define TP_STAGE_BYTES (TP_A_BYTES + TP_B_BYTES)
@@ -231,7 +239,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 // AK: A stored K-major (row-major M x K, i.e. the transpose is column-major)
 // and loaded like B; otherwise A is column-major and loaded MN-major.
 template <bool AK>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(TP_T, 2)
     k_gemm_tf32_tma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     int m, int n, int k, float *C, int ldc, int *err, float sign) {
   extern __shared__ __align__(1024) unsigned char smraw[];
@@ -332,6 +340,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             smem_u32(&s_done)));
   }
   __syncwarp();
+  // epilogue: warp w reads TMEM lanes 32 (w mod 4) .. of columns 128 (w / 4) ..;
+  // C comes 16 columns ahead of its use, the first ones before the products
+  // are complete
+  const int r = (warp & 3) * 32 + lane, gr = gm0 + r, cb = (warp >> 2) * (TP_BN / 2);
+  float cv[16], cn[16];
+  auto fetch = [&](int c0, float (&dst)[16]) {
+    const float *cp = C + (size_t)gr + (size_t)(gn0 + c0) * ldc;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      dst[j] = (gr < m && gn0 + c0 + j < n) ? __ldcg(cp + (size_t)j * ldc) : 0.f;
+  };
+  fetch(cb, cn);
   bool ok = mbar_wait(smem_u32(&s_done), 0u);
   const int all_ok = __syncthreads_and(ok && !*(volatile int *)&s_fail);
   if (!all_ok) {
@@ -345,8 +365,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   }
   asm volatile("tcgen05.fence::after_thread_sync;");
   if (all_ok && nk > 0) {
-    const int r = warp * 32 + lane, gr = gm0 + r;
-    for (int c0 = 0; c0 < TP_BN; c0 += 16) {
+#pragma unroll 2
+    for (int c0 = cb; c0 < cb + TP_BN / 2; c0 += 16) {
       if (gn0 + c0 >= n) break;  // warp-uniform
       uint32_t v[16];
       asm volatile(
@@ -355,17 +375,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
             "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
             "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
-      // the 16 loads of C are issued back to back, then the 16 stores
-      float cv[16];
-      float *cp = C + (size_t)gr + (size_t)(gn0 + c0) * ldc;
-      const int ncol = min(16, n - gn0 - c0);
+          : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0));
 #pragma unroll
-      for (int j = 0; j < 16; ++j) cv[j] = (gr < m && j < ncol) ? __ldcg(cp + (size_t)j * ldc) : 0.f;
+      for (int j = 0; j < 16; ++j) cv[j] = cn[j];
+      if (c0 + 16 < cb + TP_BN / 2) fetch(c0 + 16, cn);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      float *cp = C + (size_t)gr + (size_t)(gn0 + c0) * ldc;
 #pragma unroll
       for (int j = 0; j < 16; ++j)
-        if (gr < m && j < ncol) __stcg(cp + (size_t)j * ldc, cv[j] + sign * __uint_as_float(v[j]));
+        if (gr < m && gn0 + c0 + j < n)
+          __stcg(cp + (size_t)j * ldc, cv[j] + sign * __uint_as_float(v[j]));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -421,7 +440,7 @@ static int launch_tma(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap 
     attr_t = true;
   }
   dim3 grd((m + TP_BM - 1) / TP_BM, (n + TP_BN - 1) / TP_BN);
-  k_gemm_tf32_tma<AK><<<grd, TC_THREADS, smem_t, st>>>(ta, tb, m, n, k, C, ldc,
+  k_gemm_tf32_tma<AK><<<grd, TP_T, smem_t, st>>>(ta, tb, m, n, k, C, ldc,
                                                        (int *)g_tc_err.p, sign);
   DUST_CUDA(cudaGetLastError());
   return DUST_OK;
