@@ -15,9 +15,9 @@
 //
 //   for each outer panel of NP_NBO columns, for each block column k (NP_NB
 //   wide) in it:
-//     k_np_diag   one CTA: unpivoted LU of the diagonal block in shared
-//                 memory, its inverse triangles Linv (unit lower) and Uinv
-//                 (upper) by substitution, max |l| of the block;
+//     k_np_diag   one CTA: unpivoted LU of the diagonal block in registers,
+//                 its inverse triangles Linv (unit lower) and Uinv (upper) in
+//                 the same elimination, max |l| of the block;
 //     k_np_panel  L21 = A21 Uinv (row tiles, down to n) and U12 = Linv A12
 //                 (column tiles, inside the outer panel), 64 x 64
 //                 register-tiled products, max |l| of L21;
@@ -35,7 +35,9 @@
 // pivoted factorisation.  ipiv is the identity.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
+#include "elements.cuh"
 #include "lu.cuh"
 
 #define CUBLAS_CHECK(x)                                                   \
@@ -55,109 +57,178 @@ __device__ __forceinline__ void np_note_lmax(unsigned *bits, float v) {
   atomicMax(bits, __float_as_uint(v));
 }
 
-// Diagonal block.  Threads 0..63 hold one column each in registers (the
-// steps are unrolled, so every row index is a constant).  At step j the
-// owner of column j scales its rows below j by the reciprocal of the pivot
-// (as dgetf2 does) and publishes the multipliers in shared memory (two
-// buffers, so one barrier per step), and every later column subtracts its
-// row-j element times them.  The factored block then goes to shared memory
-// and the inverse triangles are solved one column per thread, Uinv by
-// threads 0..63 (back substitution) and Linv by threads 64..127 (forward
-// substitution), reading the factors as broadcasts; columns of the inverse
-// are zero above (Linv) or below (Uinv) the diagonal by the recurrences
-// themselves.  The block's LU, max |l| and the inverses go to global memory.
-#define NPD_T 128
+// reciprocal pivots: FP64 from the refined approximation (elements.cuh), whose
+// chain of dependent operations is a third of a division's
+__device__ __forceinline__ double np_rcp(double x) {
+  return near_range(fabs(x)) ? rcp_r(x) : 1.0 / x;
+}
+__device__ __forceinline__ float np_rcp(float x) { return 1.0f / x; }
+
+// Diagonal block: LU and both inverse triangles in one block elimination.
+// Thread (ty, tx) holds the 4 x 4 piece of rows 4 ty .. and columns 4 tx .. of
+// W in registers, W = A at first.  A step takes four pivots Q = 4 q .. 4 q + 3:
+// rows R = W(Q,:) and columns C = W(:,Q) come through shared memory (two
+// buffers, so one barrier a step), every thread factors the 4 x 4 pivot block
+// W(Q,Q) = L_d U_d and inverts its triangles itself, and with R' = L_d^-1 R and
+// f = C U_d^-1
+//   rows below Q:  f is L; W(r,c) -= f R'_c for every c outside Q (right of Q
+//                  the elimination, left of it the row operations of Linv),
+//                  W(r,Q) = -f L_d^-1;
+//   rows above Q:  W(r,Q) = f, Uinv's columns; W(r,c) -= f R'_c right of Q;
+//   rows Q:        R' is U right of Q and Linv's rows left of it;
+//                  W(Q,c) = -U_d^-1 R'_c right of Q, W(Q,Q) the two inverses.
+// L and U leave for global memory as the steps produce them; at the end W
+// holds Linv below the diagonal and Uinv on and above it.  Bound by a step's
+// chain (barrier, shared memory, reciprocals, products): four pivots a step
+// (one: 57 us in FP64), the pivot block factored by every thread (by its owner
+// ahead of the step: 41 us), a warp on two column stripes so that one warp
+// walks the columns-Q branch (on two row stripes: 39 us).  It replaces a
+// column per thread, unrolled, and two dependent substitutions, whose code did
+// not stay in the instruction caches: FP32 47 -> 20 us, FP64 54 -> 37 us per
+// block (one CTA).
+#define NPD_T 256
 template <typename T>
 __global__ void __launch_bounds__(NPD_T) k_np_diag(T *A, int lda, int k, int jb, T *Linv,
                                                    T *Uinv, unsigned *lmax_bits) {
-  extern __shared__ __align__(16) unsigned char np_sm[];
-  T *a = (T *)np_sm;                   // the block, [row][col], ld NP_LD
-  T *inv = a + NP_NB * NP_LD;          // Uinv, [row][col]
-  T *linv = inv + NP_NB * NP_LD;       // Linv, [row][col]
-  __shared__ T s_l[2][NP_NB];
-  __shared__ T s_rd[NP_NB];            // 1 / U(r, r)
-  const int tid = threadIdx.x;
-  for (int e = tid; e < NP_NB * NP_NB; e += NPD_T) {
-    const int i = e % NP_NB, c = e / NP_NB;
-    a[i * NP_LD + c] = (i < jb && c < jb) ? A[(size_t)(k + i) + (size_t)(k + c) * lda]
-                                          : (i == c ? (T)1 : (T)0);
-  }
-  __syncthreads();
+  __shared__ __align__(16) T s_row[2][4][NP_NB], s_col[2][4][NP_NB];
+  const int tid = threadIdx.x, tx = tid / 16, ty = tid % 16;
+  T *Ab = A + (size_t)k + (size_t)k * lda;
+  T w[4][4];
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int r = 4 * ty + u, c = 4 * tx + v;
+      w[u][v] = (r < jb && c < jb) ? Ab[(size_t)r + (size_t)c * lda] : (r == c ? (T)1 : (T)0);
+    }
   float lm = 0.f;
-  bool zero = false;
-  {
-    const int t = tid;  // column (threads >= 64 only pass the barriers)
-    T col[NP_NB];
+  // (pivots beyond jb meet the identity and change nothing)
+#pragma unroll 1
+  for (int q = 0; 4 * q < jb; ++q) {
+    const int b = q & 1;
+    if (ty == q) {
 #pragma unroll
-    for (int r = 0; r < NP_NB; ++r) col[r] = t < NP_NB ? a[r * NP_LD + t] : (T)0;
+      for (int u = 0; u < 4; ++u)
 #pragma unroll
-    for (int j = 0; j < NP_NB; ++j) {
-      if (j < jb) {
-        if (t == j) {
-          const T piv = col[j];
-          if (piv == (T)0) zero = true;
-          const T rinv = (T)1 / piv;
+        for (int v = 0; v < 4; ++v) s_row[b][u][4 * tx + v] = w[u][v];
+    }
+    if (tx == q) {
 #pragma unroll
-          for (int r = j + 1; r < NP_NB; ++r) {
-            col[r] *= rinv;
-            s_l[j & 1][r] = col[r];
-            if (r < jb) lm = fmaxf(lm, (float)fabs((double)col[r]));
-          }
-        }
-        __syncthreads();
-        if (t > j && t < NP_NB) {
-          const T u = col[j];
+      for (int u = 0; u < 4; ++u)
 #pragma unroll
-          for (int r = j + 1; r < NP_NB; ++r) col[r] = fma(-s_l[j & 1][r], u, col[r]);
-        }
-      }
+        for (int v = 0; v < 4; ++v) s_col[b][v][4 * ty + u] = w[u][v];
     }
     __syncthreads();
-    if (t < NP_NB)
+    T D[4][4], R[4][4], f[4][4], iu[4][4], il[4][4];
 #pragma unroll
-      for (int r = 0; r < NP_NB; ++r) a[r * NP_LD + t] = col[r];
-  }
-  if (zero) lm = INFINITY;
-  for (int o = 16; o > 0; o >>= 1) lm = fmaxf(lm, __shfl_xor_sync(0xffffffffu, lm, o));
-  if ((tid & 31) == 0) np_note_lmax(lmax_bits, lm);
-  __syncthreads();
-  if (tid < NP_NB) s_rd[tid] = (T)1 / a[tid * NP_LD + tid];
-  __syncthreads();
-  {
-    T x[NP_NB];
-    if (tid < NP_NB) {
-      // Uinv column c: U x = e_c, rows from the bottom
-      const int c = tid;
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int r = NP_NB - 1; r >= 0; --r) {
-        T acc = (r == c) ? (T)1 : (T)0;
+      for (int v = 0; v < 4; ++v) {
+        D[u][v] = s_row[b][u][4 * q + v];
+        R[u][v] = s_row[b][u][4 * tx + v];
+        f[u][v] = s_col[b][v][4 * ty + u];
+      }
+    // D = L_d U_d in place; iu = U_d^-1, il = L_d^-1 (strictly lower part)
 #pragma unroll
-        for (int p = r + 1; p < NP_NB; ++p) acc = fma(-a[r * NP_LD + p], x[p], acc);
-        x[r] = acc * s_rd[r];
+    for (int j = 0; j < 4; ++j) {
+      iu[j][j] = np_rcp(D[j][j]);
+#pragma unroll
+      for (int r = j + 1; r < 4; ++r) {
+        D[r][j] *= iu[j][j];
+#pragma unroll
+        for (int c = j + 1; c < 4; ++c) D[r][c] = fma(-D[r][j], D[j][c], D[r][c]);
+      }
+    }
+#pragma unroll
+    for (int c = 1; c < 4; ++c)
+#pragma unroll
+      for (int r = c - 1; r >= 0; --r) {
+        T x = D[r][c] * iu[c][c];
+#pragma unroll
+        for (int p = r + 1; p < c; ++p) x = fma(D[r][p], iu[p][c], x);
+        iu[r][c] = -x * iu[r][r];
       }
 #pragma unroll
-      for (int r = 0; r < NP_NB; ++r) inv[r * NP_LD + c] = x[r];
-    } else if (tid < 2 * NP_NB) {
-      // Linv column c: L x = e_c (unit diagonal), rows from the top
-      const int c = tid - NP_NB;
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
-      for (int r = 0; r < NP_NB; ++r) {
-        T acc = (r == c) ? (T)1 : (T)0;
+      for (int r = c + 1; r < 4; ++r) {
+        T x = D[r][c];
 #pragma unroll
-        for (int p = 0; p < r; ++p) acc = fma(-a[r * NP_LD + p], x[p], acc);
-        x[r] = acc;
+        for (int p = c + 1; p < r; ++p) x = fma(D[r][p], il[p][c], x);
+        il[r][c] = -x;
       }
+    // R' = L_d^-1 R and f = C U_d^-1
 #pragma unroll
-      for (int r = 0; r < NP_NB; ++r) linv[r * NP_LD + c] = x[r];
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int r = 1; r < 4; ++r)
+#pragma unroll
+        for (int p = 0; p < r; ++p) R[r][v] = fma(-D[r][p], R[p][v], R[r][v]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int c = 3; c >= 0; --c) {
+        T x = f[u][c] * iu[c][c];
+#pragma unroll
+        for (int p = 0; p < c; ++p) x = fma(f[u][p], iu[p][c], x);
+        f[u][c] = ty == q ? (u <= c ? iu[u][c] : (T)0) : x;
+      }
+    const bool right = tx > q, below = ty > q;
+    if (tx != q) {
+      if (ty == q) {
+        // U right of the pivots, Linv's rows left of them
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            if (right && 4 * tx + v < jb)
+              Ab[(size_t)(4 * q + u) + (size_t)(4 * tx + v) * lda] = R[u][v];
+            w[u][v] = right ? (T)0 : R[u][v];
+          }
+      }
+      if (below || right) {
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) w[u][v] = fma(-f[u][p], R[p][v], w[u][v]);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int r = 4 * ty + u, c = 4 * q + v;
+          T x = f[u][v];
+          if (below) {
+#pragma unroll
+            for (int p = v + 1; p < 4; ++p) x = fma(f[u][p], il[p][v], x);
+            x = -x;
+          }
+          if (ty == q && u > v) x = il[u][v];
+          w[u][v] = x;
+          if (r < jb && c < jb && (below || ty == q)) {
+            const T o = below ? f[u][v] : D[u][v];
+            Ab[(size_t)r + (size_t)c * lda] = o;
+            if (r > c) lm = fmaxf(lm, fabsf((float)o));
+            if (r == c && o == (T)0) lm = INFINITY;  // a zero pivot
+          }
+        }
     }
   }
-  __syncthreads();
-  for (int e = tid; e < jb * jb; e += NPD_T) {
-    const int r = e % jb, c = e / jb;
-    A[(size_t)(k + r) + (size_t)(k + c) * lda] = a[r * NP_LD + c];
-    Uinv[r + (size_t)c * NP_NB] = r <= c ? inv[r * NP_LD + c] : (T)0;
-    Linv[r + (size_t)c * NP_NB] = r > c ? linv[r * NP_LD + c] : (r == c ? (T)1 : (T)0);
-  }
+  for (int o = 16; o > 0; o >>= 1) lm = fmaxf(lm, __shfl_xor_sync(0xffffffffu, lm, o));
+  if ((tid & 31) == 0) np_note_lmax(lmax_bits, lm);
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int r = 4 * ty + u, c = 4 * tx + v;
+      if (r < jb && c < jb) {
+        Linv[r + (size_t)c * NP_NB] = r > c ? w[u][v] : (r == c ? (T)1 : (T)0);
+        Uinv[r + (size_t)c * NP_NB] = r <= c ? w[u][v] : (T)0;
+      }
+    }
 }
 
 // 64 x 64 tiles of the panel: blocks [0, nrb) take 64 rows of A21 (rows
@@ -180,10 +251,23 @@ __global__ void __launch_bounds__(NP_T) k_np_panel(T *A, int lda, int n, int k, 
   const int nr = rows ? min(NP_NB, n - r0) : jb;
   const int nc = rows ? jb : min(NP_NB, cend - c0);
   const T *W = rows ? Uinv : Linv;
-  for (int e = tid; e < NP_NB * NP_NB; e += NP_T) {
-    const int r = e % NP_NB, c = e / NP_NB;
-    x[r * NP_LD + c] = (r < nr && c < nc) ? A[(size_t)(r0 + r) + (size_t)(c0 + c) * lda] : (T)0;
-    w[r * NP_LD + c] = (r < jb && c < jb) ? W[r + (size_t)c * NP_NB] : (T)0;
+  {
+    // all of a thread's loads in flight together
+    constexpr int M = NP_NB * NP_NB / NP_T;
+    const int r = tid % NP_NB, cq = tid / NP_NB;
+    T xv[M], wv[M];
+#pragma unroll
+    for (int q = 0; q < M; ++q) {
+      const int c = cq + q * (NP_T / NP_NB);
+      xv[q] = (r < nr && c < nc) ? A[(size_t)(r0 + r) + (size_t)(c0 + c) * lda] : (T)0;
+      wv[q] = (r < jb && c < jb) ? W[r + (size_t)c * NP_NB] : (T)0;
+    }
+#pragma unroll
+    for (int q = 0; q < M; ++q) {
+      const int c = cq + q * (NP_T / NP_NB);
+      x[r * NP_LD + c] = xv[q];
+      w[r * NP_LD + c] = wv[q];
+    }
   }
   __syncthreads();
   // out = x w (rows) or w x (columns); thread (ty, tx) owns rows 4 ty .. and
@@ -267,10 +351,9 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
   unsigned *bits = (unsigned *)w.np.p;
   T *inv0 = (T *)((char *)w.np.p + 256);
   DUST_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned), st));
-  const int smd = 3 * NP_NB * NP_LD * (int)sizeof(T), smp = 2 * NP_NB * NP_LD * (int)sizeof(T);
+  const int smp = 2 * NP_NB * NP_LD * (int)sizeof(T);
   static bool attr = false;  // per element type
   if (!attr) {
-    DUST_CUDA(cudaFuncSetAttribute(k_np_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smd));
     DUST_CUDA(cudaFuncSetAttribute(k_np_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp));
     attr = true;
   }
@@ -294,7 +377,7 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
     for (int k = K; k < Ke; k += NP_NB) {
       const int jb = std::min(NP_NB, n - k), m2 = n - k - jb, wc = Ke - k - jb;
       T *Linv = inv0 + 2 * tri * (size_t)(k / NP_NB), *Uinv = Linv + tri;
-      k_np_diag<T><<<1, NPD_T, smd, st>>>(A, lda, k, jb, Linv, Uinv, bits);
+      k_np_diag<T><<<1, NPD_T, 0, st>>>(A, lda, k, jb, Linv, Uinv, bits);
       const int nrb = (m2 + NP_NB - 1) / NP_NB, ncb = (wc + NP_NB - 1) / NP_NB;
       if (nrb + ncb > 0)
         k_np_panel<T><<<nrb + ncb, NP_T, smp, st>>>(A, lda, n, k, jb, Linv, Uinv, nrb, k + jb,

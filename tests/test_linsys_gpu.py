@@ -206,3 +206,19 @@ def test_ellipsoid_dirichlet_parity():
     res, _ = ls.solve_linsys(abi.DUST_SOLVE_LU64)
     assert rel(res, ro) < 1e-10
     assert np.max(np.abs(Ag.sum(axis=1) - 4 * np.pi)) < 0.05 * 4 * np.pi
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 63, 64, 65, 127, 255, 256, 257, 511, 513])
+@pytest.mark.parametrize("nrhs", [1, 3, 65])
+@pytest.mark.parametrize("mode", [abi.DUST_SOLVE_LU64, abi.DUST_SOLVE_MIXED])
+def test_dense_unpivoted_remainders(n, nrhs, mode):
+    """Diagonally dominant systems (unpivoted LU) at the remainders of the
+    pivot blocks, diagonal blocks, outer panels and right-hand-side tiles.
+    The backward error of both modes is a small multiple of n eps."""
+    rng = np.random.default_rng(n + nrhs)
+    A = rng.standard_normal((n, n)) / n + 2.0 * np.eye(n)
+    B = rng.standard_normal((n, nrhs))
+    X, rep = linsys.dense_solve(A, B, mode, 1e-14)
+    assert rep["pivoted"] == 0
+    res = np.abs(B - A @ X).max() / (np.abs(A).sum(axis=1).max() * np.abs(X).max())
+    assert res < 1e-14
