@@ -192,6 +192,22 @@ static void launch_wake(dust_linsys *L, int r0, int r1, int ista, int iend, int 
       (double *)L->A.p, L->n, (double *)L->b.p, do_rhs);
 }
 
+int linsys_factor_static(dust_linsys *L) {
+  const size_t n = L->n, ns = L->nst;
+  DUST_TRY(lu_getrf_auto<double>(
+      L->cb, L->st, L->lu_s, L->nst, (double *)L->A.p, L->n, (int *)L->piv.p, (int *)L->info.p, 0,
+      nullptr, 1e-8,
+      [&]() -> int {
+        DUST_CUDA(cudaMemcpy2DAsync(L->A.p, n * 8, L->As.p, ns * 8, ns * 8, ns,
+                                    cudaMemcpyDeviceToDevice, L->st));
+        return DUST_OK;
+      },
+      &L->static_pivoted));
+  if (!L->static_pivoted)
+    DUST_TRY(lu_inv_build<double>(L->st, L->lu_s, L->nst, (const double *)L->A.p, L->n));
+  return DUST_OK;
+}
+
 extern "C" int dust_linsys_create(int rank, int nstatic, const dust_fmm_params *prm,
                                   const dust_panels *elems, const dust_wake_rows *wake,
                                   dust_linsys **out) {
@@ -236,16 +252,7 @@ extern "C" int dust_linsys_create(int rank, int nstatic, const dust_fmm_params *
       if ((st = devbuf_grow(As, (size_t)nstatic * nstatic * 8)) == DUST_OK) {
         cudaMemcpy2DAsync(As.p, (size_t)nstatic * 8, L->A.p, n * 8, (size_t)nstatic * 8, nstatic,
                           cudaMemcpyDeviceToDevice, L->st);
-        st = lu_getrf_auto<double>(
-            L->cb, L->st, L->lu, nstatic, (double *)L->A.p, rank, (int *)L->piv.p,
-            (int *)L->info.p, 0, nullptr, 1e-8,
-            [&]() -> int {
-              DUST_CUDA(cudaMemcpy2DAsync(L->A.p, n * 8, As.p, (size_t)nstatic * 8,
-                                          (size_t)nstatic * 8, nstatic, cudaMemcpyDeviceToDevice,
-                                          L->st));
-              return DUST_OK;
-            },
-            &L->static_pivoted);
+        st = linsys_factor_static(L);
         if (st == DUST_OK) {
           int info = 0;
           cudaMemcpy(&info, L->info.p, sizeof(int), cudaMemcpyDeviceToHost);
@@ -267,8 +274,9 @@ extern "C" int dust_linsys_destroy(dust_linsys *L) {
   if (!L) return DUST_OK;
   if (L->st) cudaStreamSynchronize(L->st);
   DevBuf *bufs[] = {&L->A,  &L->As, &L->b,    &L->bst,  &L->piv, &L->info, &L->geo,
-                    &L->raw, &L->impl, &L->work, &L->lu.sync, &L->lu.np, &L->lu.np_x, &L->A32, &L->gm, &L->ainv32, &L->mx, &L->kr,
-                    &L->mvb, &L->permv};
+                    &L->raw, &L->impl, &L->work, &L->A32, &L->gm, &L->ainv32, &L->mx, &L->kr,
+                    &L->mvb, &L->permv, &L->lu.sync, &L->lu.np, &L->lu.np_x, &L->lu.inv,
+                    &L->lu_s.sync, &L->lu_s.np, &L->lu_s.np_x, &L->lu_s.inv};
   for (DevBuf *b : bufs) devbuf_free(*b);
   if (L->cb) cublasDestroy(L->cb);
   if (L->st) cudaStreamDestroy(L->st);
@@ -324,16 +332,23 @@ int linsys_solve_lu64(dust_linsys *L, double *res_dev) {
   int *P = (int *)L->piv.p;
   cublasSetStream(L->cb, L->st);
   const double one = 1.0, mone = -1.0;
+  // the unpivoted static factors come with their inverse blocks
+  const bool blocks_s = nst == 0 || L->lu_s.inv_n == nst;
   if (nst > 0 && nmv > 0) {
-    lu_laswp<double>(L->st, A + 0, n, nst, n, 0, nst, P);
-    if (cublasDtrsm(L->cb, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
-                    CUBLAS_DIAG_UNIT, nst, nmv, &one, A, n, A + (size_t)nst * n,
-                    n) != CUBLAS_STATUS_SUCCESS)
-      return DUST_ERR_CUDA;
-    if (cublasDtrsm(L->cb, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
-                    CUBLAS_DIAG_NON_UNIT, nmv, nst, &one, A, n, A + nst,
-                    n) != CUBLAS_STATUS_SUCCESS)
-      return DUST_ERR_CUDA;
+    if (blocks_s) {
+      DUST_TRY(lu_trsm_blocks(L->cb, L->st, L->lu_s, nst, A, n, nmv, A + (size_t)nst * n,
+                              A + nst, n));
+    } else {
+      lu_laswp<double>(L->st, A + 0, n, nst, n, 0, nst, P);
+      if (cublasDtrsm(L->cb, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
+                      CUBLAS_DIAG_UNIT, nst, nmv, &one, A, n, A + (size_t)nst * n,
+                      n) != CUBLAS_STATUS_SUCCESS)
+        return DUST_ERR_CUDA;
+      if (cublasDtrsm(L->cb, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
+                      CUBLAS_DIAG_NON_UNIT, nmv, nst, &one, A, n, A + nst,
+                      n) != CUBLAS_STATUS_SUCCESS)
+        return DUST_ERR_CUDA;
+    }
     if (cublasDgemm(L->cb, CUBLAS_OP_N, CUBLAS_OP_N, nmv, nmv, nst, &mone, A + nst, n,
                     A + (size_t)nst * n, n, &one, A + nst + (size_t)nst * n,
                     n) != CUBLAS_STATUS_SUCCESS)
@@ -357,15 +372,21 @@ int linsys_solve_lu64(dust_linsys *L, double *res_dev) {
     int info = 0;
     DUST_CUDA(cudaMemcpy(&info, L->info.p, sizeof(int), cudaMemcpyDeviceToHost));
     if (info) return DUST_ERR_SINGULAR;
+    if (!L->last_pivoted)
+      DUST_TRY(lu_inv_build<double>(L->st, L->lu, nmv, Amm, n));
     if (nst > 0) {
       // dlaswp on A(nst+1:rank, 1:nst) with the moving pivots, then make
       // them global
-      lu_laswp<double>(L->st, A + nst, n, 0, nst, 0, nmv, P + nst);
+      if (L->last_pivoted) lu_laswp<double>(L->st, A + nst, n, 0, nst, 0, nmv, P + nst);
       linsys_shift_pivots(L->st, P + nst, nmv, nst);
     }
   }
   L->factored = true;
   DUST_CUDA(cudaMemcpyAsync(res_dev, L->b.p, (size_t)n * 8, cudaMemcpyDeviceToDevice, L->st));
+  if (blocks_s && (nmv == 0 || !L->last_pivoted))
+    return nst == 0 ? lu_solve_blocks<double>(L->st, L->lu.np_x, n, 1, A, n, res_dev, n, L->lu)
+                    : lu_solve_blocks<double>(L->st, L->lu.np_x, n, 1, A, n, res_dev, n, L->lu_s,
+                                              nmv > 0 ? &L->lu : nullptr);
   // the pivots' net row permutation, applied as one gather instead of n
   // dependent interchanges; a system without moving rows keeps its pivots,
   // so its permutation is built once

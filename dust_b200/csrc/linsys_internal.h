@@ -28,13 +28,18 @@ struct dust_linsys {
   bool ainv_ready = false;
   struct dust_precond *pc = nullptr;  // learned preconditioner (GMRES_NN)
   DevBuf kr;                          // GMRES Krylov basis and vectors
-  LuWork lu;
+  LuWork lu;    // of the moving block (each solve) or the Schur complement
+  LuWork lu_s;  // of the static block: its inverse blocks (lu_s.inv_n > 0) when
+                // the unpivoted factors were accepted
   const PanelGeo *el = nullptr, *wk = nullptr;
   int nwake = 0, n_impl = 0;
   bool assembled = false, factored = false, keep_static_copy = true;
 };
 
 int linsys_solve_lu64(dust_linsys *L, double *res_dev);
+// LU of the static block (F's first nst rows and columns, copy in As) with its
+// inverse blocks when unpivoted
+int linsys_factor_static(dust_linsys *L);
 int linsys_solve_iterative(dust_linsys *L, int mode, double *x_dev, dust_solve_report *rep);
 // Static/moving Schur solve in FP32/TF32 refined to FP64 (tol on the
 // normwise backward error ||b-Ax|| / (||A|| ||x||), max_iter refinements).

@@ -15,8 +15,10 @@
 struct LuWork {
   DevBuf sync;   // barrier counters, error flag, partials, candidate rows
   DevBuf np;     // unpivoted LU: max |l| word, inverse triangles of every
-                 // diagonal block (kept for lu_getrs_nopiv)
-  DevBuf np_x;   // lu_getrs_nopiv: the intermediate Y = L^-1 B
+                 // diagonal block (kept for lu_inv_build)
+  DevBuf inv;    // inverses of L's and U's larger diagonal blocks (lu_inv_build)
+  int inv_n = 0; // order of the system they belong to (0: none)
+  DevBuf np_x;   // lu_solve_blocks: the intermediate Y = L^-1 B
   int nsm = 0;
 };
 
@@ -52,12 +54,23 @@ template <typename T>
 int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, int lda,
                    int *ipiv, int gemm_update, int *perm, float *lmax);
 
-// Solves A X = B (X over B, nrhs columns, ldb) with the factors of the last
-// lu_getrf_nopiv on this LuWork (same A, n): forward and backward block
-// substitution with the kept inverse triangles, one launch per 64-row block.
+// Inverses of the 512 x 512 diagonal blocks of L and U from the kept 64 x 64
+// ones of the last lu_getrf_nopiv on this LuWork (same A, n), into w.inv.
 template <typename T>
-int lu_getrs_nopiv(cudaStream_t st, LuWork &w, int n, int nrhs, const T *A, int lda, T *B,
-                   int ldb);
+int lu_inv_build(cudaStream_t st, LuWork &w, int n, const T *A, int lda);
+
+// Solves A X = B (X over B, nrhs columns, ldb) with the unpivoted factors in A
+// and the inverse blocks of w1 (the leading w1.inv_n rows) and, when given, w2
+// (the rest).  `work` holds the intermediate n x nrhs.
+template <typename T>
+int lu_solve_blocks(cudaStream_t st, DevBuf &work, int n, int nrhs, const T *A, int lda, T *B,
+                    int ldb, const LuWork &w1, const LuWork *w2 = nullptr);
+
+// B := L^-1 B (n x m) and C := C U^-1 (m x n), ld lda each, with the unpivoted
+// factors in A and the inverse blocks of w, as products (DGEMM); `w.np_x` holds
+// the block in work.
+int lu_trsm_blocks(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, const double *A, int lda,
+                   int m, double *B, double *C, int ldbc);
 
 // lu_getrf through the unpivoted factorisation when its multipliers certify
 // it (max |l| < 1 - margin: partial pivoting would interchange no row), else

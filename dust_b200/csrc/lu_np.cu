@@ -344,7 +344,7 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
   *lmax = 0.f;
   if (n <= 0) return DUST_OK;
   // inverse triangles of every diagonal block are kept (Linv then Uinv per
-  // block) for lu_getrs_nopiv
+  // block) for lu_inv_build
   const size_t tri = (size_t)NP_NB * NP_NB;
   const int nblk_ = (n + NP_NB - 1) / NP_NB;
   DUST_TRY(devbuf_grow(w.np, 256 + 2 * tri * sizeof(T) * (size_t)nblk_));
@@ -406,216 +406,6 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
   return DUST_OK;
 }
 
-// Block substitution with the kept inverse triangles, one cooperative launch
-// per triangle (forward: blocks i ascending with Linv; backward: descending
-// with Uinv).  At step i every CTA computes Y_i = Inv_i B_i for a chunk of
-// NP_NB right-hand sides (B's block i is final: every earlier step ended at a
-// grid barrier) and then updates its share of the 64-row tiles not yet
-// solved, B_r -= A_(r,i) Y_i; CTA 0 stores Y_i into X.  The grid barrier
-// spins with an iteration limit and raises the error word instead of
-// hanging; every CTA then stops at the same step.
-#define NP_SPIN_LIMIT (1ll << 24)
-
-__device__ __forceinline__ bool np_grid_barrier(unsigned *bar, unsigned G, int *err) {
-  __syncthreads();
-  __shared__ int s_fail;
-  if (threadIdx.x == 0) {
-    s_fail = 0;
-    volatile unsigned *vgen = bar + 1;
-    const unsigned g0 = *vgen;
-    __threadfence();
-    const unsigned arrived = atomicAdd(bar, 1u);
-    if (arrived == G - 1u) {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      long long it = 0;
-      while (*vgen == g0) {
-        if (++it > NP_SPIN_LIMIT || *(volatile int *)err) {
-          atomicExch(err, 1);
-          s_fail = 1;
-          break;
-        }
-        if (it > 64) __nanosleep(32);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return s_fail == 0;
-}
-
-// out (64 x 64) of thread (ty, tx): rows 4 ty .., columns 4 tx .. of L R, both
-// [row][col] with ld NP_LD in shared memory
-template <typename T>
-__device__ __forceinline__ void np_mm64(const T *L, const T *R, int ty, int tx, T (&acc)[4][4]) {
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = (T)0;
-#pragma unroll 4
-  for (int p = 0; p < NP_NB; ++p) {
-    T lv[4], rv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) lv[u] = L[(4 * ty + u) * NP_LD + p];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) rv[v] = R[p * NP_LD + 4 * tx + v];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] = fma(lv[u], rv[v], acc[u][v]);
-  }
-}
-
-template <typename T, bool FWD>
-__global__ void __launch_bounds__(NP_T) k_np_subst(const T *A, int lda, int n, int nrhs,
-                                                   const T *Inv, T *B, int ldb, T *X, int ldx,
-                                                   unsigned *bar, int *err) {
-  extern __shared__ __align__(16) unsigned char np_sm[];
-  T *w = (T *)np_sm;               // Inv_i
-  T *b = w + NP_NB * NP_LD;        // B_i (a chunk of right-hand sides)
-  T *y = b + NP_NB * NP_LD;        // Y_i
-  T *l = y + NP_NB * NP_LD;        // A_(r,i) of the CTA's first tile
-  T *o = l + NP_NB * NP_LD;        // the update of a tile
-  const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
-  const unsigned G = gridDim.x;
-  const int nb = (n + NP_NB - 1) / NP_NB;
-  // the inverse triangle and the first coupling tile of a step depend only
-  // on the factors, so they are loaded before the grid barrier that ends the
-  // previous step; only B's block i waits for it
-  auto step_of = [&](int s) { return FWD ? s : nb - 1 - s; };
-  auto load_inv_tile = [&](int s, T *lt) {
-    const int i = step_of(s), k = i * NP_NB, jb = min(NP_NB, n - k);
-    const T *W = Inv + 2 * (size_t)NP_NB * NP_NB * i + (FWD ? 0 : (size_t)NP_NB * NP_NB);
-    const int nrest = FWD ? n - k - jb : k;
-    const int ntile = (nrest + NP_NB - 1) / NP_NB;
-    const int tile = blockIdx.x;
-    const int r0 = FWD ? k + jb + NP_NB * tile : NP_NB * tile;
-    const int nr = tile < ntile ? min(NP_NB, (FWD ? n : k) - r0) : 0;
-    for (int e = tid; e < NP_NB * NP_NB; e += NP_T) {
-      const int r = e % NP_NB, c = e / NP_NB;
-      w[r * NP_LD + c] = (r < jb && c < jb) ? W[r + (size_t)c * NP_NB] : (T)0;
-      lt[r * NP_LD + c] = (r < nr && c < jb) ? A[(size_t)(r0 + r) + (size_t)(k + c) * lda] : (T)0;
-    }
-  };
-  load_inv_tile(0, l);
-  for (int s = 0; s < nb; ++s) {
-    const int i = step_of(s);
-    const int k = i * NP_NB, jb = min(NP_NB, n - k);
-    const int nrest = FWD ? n - k - jb : k;
-    const int ntile = (nrest + NP_NB - 1) / NP_NB;
-    const bool busy = blockIdx.x == 0 || (int)blockIdx.x < ntile;
-    for (int c0 = 0; c0 < nrhs && busy; c0 += NP_NB) {
-      const int nc = min(NP_NB, nrhs - c0);
-      __syncthreads();
-      for (int e = tid; e < NP_NB * NP_NB; e += NP_T) {
-        const int r = e % NP_NB, c = e / NP_NB;
-        // B changes between steps on other SMs: read it past L1
-        b[r * NP_LD + c] =
-            (r < jb && c < nc) ? __ldcg(B + (size_t)(k + r) + (size_t)(c0 + c) * ldb) : (T)0;
-      }
-      __syncthreads();
-      T acc[4][4];
-      np_mm64(w, b, ty, tx, acc);
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) y[(4 * ty + u) * NP_LD + 4 * tx + v] = acc[u][v];
-      __syncthreads();
-      if (blockIdx.x == 0)
-        for (int e = tid; e < NP_NB * NP_NB; e += NP_T) {
-          const int r = e % NP_NB, c = e / NP_NB;
-          if (r < jb && c < nc) X[(size_t)(k + r) + (size_t)(c0 + c) * ldx] = y[r * NP_LD + c];
-        }
-      for (int tile = blockIdx.x; tile < ntile; tile += G) {
-        const int r0 = FWD ? k + jb + NP_NB * tile : NP_NB * tile;
-        const int nr = min(NP_NB, (FWD ? n : k) - r0);
-        T *lt = l;
-        if (tile != (int)blockIdx.x) {
-          // a further tile of this CTA: its coupling block is loaded here
-          lt = o;
-          __syncthreads();
-          for (int e = tid; e < NP_NB * NP_NB; e += NP_T) {
-            const int r = e % NP_NB, c = e / NP_NB;
-            lt[r * NP_LD + c] =
-                (r < nr && c < jb) ? A[(size_t)(r0 + r) + (size_t)(k + c) * lda] : (T)0;
-          }
-          __syncthreads();
-        }
-        np_mm64(lt, y, ty, tx, acc);
-        // through shared memory, then coalesced along the columns
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) o[(4 * ty + u) * NP_LD + 4 * tx + v] = acc[u][v];
-        __syncthreads();
-        for (int e = tid; e < NP_NB * NP_NB; e += NP_T) {
-          const int r = e % NP_NB, c = e / NP_NB;
-          if (r < nr && c < nc) {
-            T *bp = B + (size_t)(r0 + r) + (size_t)(c0 + c) * ldb;
-            *bp = __ldcg(bp) - o[r * NP_LD + c];
-          }
-        }
-      }
-    }
-    __syncthreads();
-    if (s + 1 < nb) load_inv_tile(s + 1, l);
-    if (!np_grid_barrier(bar, G, err)) return;
-  }
-}
-
-template <typename T>
-int lu_getrs_nopiv(cudaStream_t st, LuWork &w, int n, int nrhs, const T *A, int lda, T *B,
-                   int ldb) {
-  if (n <= 0 || nrhs <= 0) return DUST_OK;
-  const T *inv0 = (const T *)((const char *)w.np.p + 256);
-  const size_t xb = (size_t)n * nrhs * sizeof(T);
-  DUST_TRY(devbuf_grow(w.np_x, xb + 256));
-  T *X = (T *)((char *)w.np_x.p + 256);
-  unsigned *bar = (unsigned *)w.np_x.p;  // arrivals, generation, error word
-  int *err = (int *)(bar + 2);
-  const int sm = 5 * NP_NB * NP_LD * (int)sizeof(T);
-  static int G = 0;  // co-resident CTAs, per element type
-  if (G == 0) {
-    DUST_CUDA(cudaFuncSetAttribute(k_np_subst<T, true>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    DUST_CUDA(cudaFuncSetAttribute(k_np_subst<T, false>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    int dev = 0, nsm = 0, per = 0;
-    DUST_CUDA(cudaGetDevice(&dev));
-    DUST_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    DUST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_np_subst<T, true>, NP_T, sm));
-    G = std::max(1, nsm * std::max(per, 1));
-  }
-  const int nb = (n + NP_NB - 1) / NP_NB;
-  const int g = std::min(G, std::max(1, nb - 1));
-  DUST_CUDA(cudaMemsetAsync(bar, 0, 16, st));
-  // L Y = B: Y into X; U X = Y: X back into B
-  int ldn = n;
-  {
-    void *args[] = {(void *)&A, (void *)&lda, (void *)&n, (void *)&nrhs, (void *)&inv0,
-                    (void *)&B, (void *)&ldb, (void *)&X, (void *)&ldn, (void *)&bar, (void *)&err};
-    DUST_CUDA(cudaLaunchCooperativeKernel((void *)k_np_subst<T, true>, dim3(g), dim3(NP_T), args,
-                                          sm, st));
-  }
-  {
-    void *args[] = {(void *)&A, (void *)&lda, (void *)&n, (void *)&nrhs, (void *)&inv0,
-                    (void *)&X, (void *)&ldn, (void *)&B, (void *)&ldb, (void *)&bar, (void *)&err};
-    DUST_CUDA(cudaLaunchCooperativeKernel((void *)k_np_subst<T, false>, dim3(g), dim3(NP_T), args,
-                                          sm, st));
-  }
-  int herr = 0;
-  DUST_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  DUST_CUDA(cudaStreamSynchronize(st));
-  return herr ? DUST_ERR_TIMEOUT : DUST_OK;
-}
-
-template int lu_getrs_nopiv<double>(cudaStream_t, LuWork &, int, int, const double *, int,
-                                    double *, int);
-template int lu_getrs_nopiv<float>(cudaStream_t, LuWork &, int, int, const float *, int, float *,
-                                   int);
 template int lu_getrf_nopiv<double>(cublasHandle_t, cudaStream_t, LuWork &, int, double *, int,
                                     int *, int, int *, float *);
 template int lu_getrf_nopiv<float>(cublasHandle_t, cudaStream_t, LuWork &, int, float *, int,

@@ -408,15 +408,7 @@ extern "C" int dust_pressure_create(dust_linsys *ls, dust_pressure **out) {
                                        (double *)S->A.p, nsp, (double *)p->bsp.p, nsst);
     cudaMemcpy2DAsync(S->As.p, (size_t)nsst * 8, S->A.p, N * 8, (size_t)nsst * 8, nsst,
                       cudaMemcpyDeviceToDevice, S->st);
-    s = lu_getrf_auto<double>(
-        S->cb, S->st, S->lu, nsst, (double *)S->A.p, nsp, (int *)S->piv.p, (int *)S->info.p, 0,
-        nullptr, 1e-8,
-        [&]() -> int {
-          DUST_CUDA(cudaMemcpy2DAsync(S->A.p, N * 8, S->As.p, (size_t)nsst * 8,
-                                      (size_t)nsst * 8, nsst, cudaMemcpyDeviceToDevice, S->st));
-          return DUST_OK;
-        },
-        &S->static_pivoted);
+    s = linsys_factor_static(S);
     if (s == DUST_OK) {
       int info = 0;
       if (cudaMemcpy(&info, S->info.p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)

@@ -143,6 +143,7 @@ int linsys_solve_schur_mixed(dust_linsys *L, double *x, double tol, int max_iter
     DUST_TRY(build_s());
     DUST_TRY(lu_getrf_auto<float>(L->cb, st, L->lu, nmv, S, nmv, piv, info, 1,
                                   use_perm ? perm : nullptr, 0.0, build_s, &L->last_pivoted));
+    if (!L->last_pivoted) DUST_TRY(lu_inv_build<float>(st, L->lu, nmv, S, nmv));
     DUST_TRY(gemm_tf32_error(st));
     int hinfo = 0;
     DUST_CUDA(cudaMemcpyAsync(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -188,8 +189,11 @@ int linsys_solve_schur_mixed(dust_linsys *L, double *x, double tol, int max_iter
     if (nmv > 0) {
       DUST_CUDA(cudaMemcpyAsync(t32, r32 + nst, (size_t)nmv * 4, cudaMemcpyDeviceToDevice, st));
       if (nst > 0) DUST_TRY(gemv_n<float>(st, nmv, nst, -1.0f, Ads, nmv, d32, 1.0f, t32));
-      DUST_TRY(lu_getrs<float>(L->cb, st, nmv, 1, S, nmv, piv, t32, nmv,
-                               use_perm ? perm : nullptr));
+      if (!L->last_pivoted)
+        DUST_TRY(lu_solve_blocks<float>(st, L->lu.np_x, nmv, 1, S, nmv, t32, nmv, L->lu));
+      else
+        DUST_TRY(lu_getrs<float>(L->cb, st, nmv, 1, S, nmv, piv, t32, nmv,
+                                 use_perm ? perm : nullptr));
       DUST_CUDA(cudaMemcpyAsync(d32 + nst, t32, (size_t)nmv * 4, cudaMemcpyDeviceToDevice, st));
       if (nst > 0) DUST_TRY(gemv_n<float>(st, nst, nmv, -1.0f, Y, nst, t32, 1.0f, d32));
     }

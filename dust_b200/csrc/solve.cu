@@ -28,13 +28,18 @@ __global__ void k_add_f32(size_t n, const float *d, double *x) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (; i < n; i += (size_t)gridDim.x * blockDim.x) x[i] += (double)d[i];
 }
-// row sums |A| (for ||A||_inf), one thread per row, column-major
+// row sums |A| (for ||A||_inf), column-major, one thread per row and chunk of
+// RB_COLS columns (added atomically into rs): a thread per row alone kept too
+// few loads in flight (n = 16,384: 1.69 ms for 2.1 GB)
+#define RB_COLS 256
 __global__ void k_rowabs(int n, const double *A, double *rs) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  const int j0 = blockIdx.y * RB_COLS, j1 = min(n, j0 + RB_COLS);
   double s = 0.0;
-  for (int j = 0; j < n; ++j) s += fabs(A[(size_t)i + (size_t)j * n]);
-  rs[i] = s;
+#pragma unroll 8
+  for (int j = j0; j < j1; ++j) s += fabs(A[(size_t)i + (size_t)j * n]);
+  atomicAdd(rs + i, s);
 }
 // per column: max |r| and max |x|
 __global__ void k_colmax(int n, int nrhs, const double *R, const double *X, double *out) {
@@ -92,6 +97,7 @@ int mixed_solve_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, DevBuf &w
                                  return DUST_OK;
                                },
                                &piv);
+  if (s == DUST_OK && piv == 0) s = lu_inv_build<float>(st, lu, n, A32, n);
   if (rep) rep->pivoted = piv;
   cudaEventRecord(e1, st);
   if (s != DUST_OK) return s;
@@ -102,7 +108,8 @@ int mixed_solve_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, DevBuf &w
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (hinfo) return DUST_ERR_SINGULAR;
-  k_rowabs<<<nblk(n, 128), 128, 0, st>>>(n, A64, rs);
+  DUST_CUDA(cudaMemsetAsync(rs, 0, (size_t)n * 8, st));
+  k_rowabs<<<dim3(nblk(n, 128), nblk(n, RB_COLS)), 128, 0, st>>>(n, A64, rs);
   int imax = 0;
   double anorm = 0.0;
   cublasSetStream(cb, st);
@@ -137,7 +144,7 @@ int mixed_solve_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, DevBuf &w
     }
     k_to_f32<<<256, 256, 0, st>>>(nr, R, D32);
     if (piv == 0)
-      DUST_TRY(lu_getrs_nopiv<float>(st, lu, n, nrhs, A32, n, D32, n));
+      DUST_TRY(lu_solve_blocks<float>(st, lu.np_x, n, nrhs, A32, n, D32, n, lu));
     else
       DUST_TRY(lu_getrs<float>(cb, st, n, nrhs, A32, n, ipiv, D32, n));
     k_add_f32<<<256, 256, 0, st>>>(nr, D32, X);
@@ -184,6 +191,7 @@ static int dense_lu64_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, Dev
     else
       s = lu_getrf<double>(cb, st, lu, n, (double *)F.p, n, ipiv, info, 0);
   }
+  if (s == DUST_OK && pivd == 0) s = lu_inv_build<double>(st, lu, n, (const double *)F.p, n);
   if (r) r->pivoted = pivd;
   cudaEventRecord(e1, st);
   int hinfo = 0;
@@ -196,7 +204,7 @@ static int dense_lu64_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, Dev
     if (X != B && cudaMemcpyAsync(X, B, nr * 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       s = DUST_ERR_CUDA;
     if (s == DUST_OK)
-      s = pivd == 0 ? lu_getrs_nopiv<double>(st, lu, n, nrhs, (const double *)F.p, n, X, n)
+      s = pivd == 0 ? lu_solve_blocks<double>(st, lu.np_x, n, nrhs, (const double *)F.p, n, X, n, lu)
                     : lu_getrs<double>(cb, st, n, nrhs, (const double *)F.p, n, ipiv, X, n);
     cudaEventRecord(e2, st);
   }
@@ -303,6 +311,7 @@ extern "C" int dust_dense_solve(int n, int nrhs, const double *A, const double *
   devbuf_free(lu.sync);
   devbuf_free(lu.np);
   devbuf_free(lu.np_x);
+  devbuf_free(lu.inv);
   cublasDestroy(cb);
   cudaStreamDestroy(st);
   if (rep) *rep = r;

@@ -208,7 +208,7 @@ def test_ellipsoid_dirichlet_parity():
     assert np.max(np.abs(Ag.sum(axis=1) - 4 * np.pi)) < 0.05 * 4 * np.pi
 
 
-@pytest.mark.parametrize("n", [1, 3, 4, 5, 63, 64, 65, 127, 255, 256, 257, 511, 513])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 63, 64, 65, 127, 255, 257, 511, 513, 1090])
 @pytest.mark.parametrize("nrhs", [1, 3, 65])
 @pytest.mark.parametrize("mode", [abi.DUST_SOLVE_LU64, abi.DUST_SOLVE_MIXED])
 def test_dense_unpivoted_remainders(n, nrhs, mode):
@@ -222,3 +222,21 @@ def test_dense_unpivoted_remainders(n, nrhs, mode):
     assert rep["pivoted"] == 0
     res = np.abs(B - A @ X).max() / (np.abs(A).sum(axis=1).max() * np.abs(X).max())
     assert res < 1e-14
+
+
+@pytest.mark.parametrize("n_fus,n_span", [(520, 2), (1100, 17)])
+def test_linsys_block_solve_matches_oracle(n_fus, n_span):
+    """Static blocks beyond one inverse block (with a short last one) and a
+    moving block below and above one: the block Schur update and solve, or the
+    pivoted route where the factors ask for interchanges."""
+    case = synth.RotorFuselageCase(n_fus=n_fus, n_span=n_span)
+    els = case.system(3)
+    prm = case.fmm_params()
+    ls = linsys.initialize_linsys(prm, case.rank, case.nstatic, els)
+    none = (abi.empty_panels(), 0, np.zeros((1, 2), dtype=np.int32))
+    _, _, ro = O.linsys_run(prm, case.rank, case.nstatic, els, els, none, none)
+    for mode in (abi.DUST_SOLVE_LU64, abi.DUST_SOLVE_MIXED):
+        ls.assemble_linsys(els)
+        res, rep = ls.solve_linsys(mode)
+        assert rep["fell_back"] == 0
+        assert np.linalg.norm(res - ro) < 1e-10 * np.linalg.norm(ro)
