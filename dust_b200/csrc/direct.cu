@@ -638,7 +638,8 @@ static int elem_chunk(unsigned pblocks, int ntot, int load) {
 }
 
 int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
-                       size_t &near_cap, unsigned long long *near_seen, int precision,
+                       size_t &near_cap, unsigned long long near_seen,
+                       unsigned long long *count, int precision,
                        double *vel, double *str, double *rot, cudaStream_t st, cudaEvent_t *kev,
                        bool *kev_done) {
   if (kev_done) *kev_done = false;
@@ -652,23 +653,22 @@ int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
     if (e.nbody) k_ffrec<<<nblk(e.nbody, 128), 128, 0, st>>>(e.body, e.nbody, e.rp.ff_dou, ff);
     if (e.nwake)
       k_ffrec<<<nblk(e.nwake, 128), 128, 0, st>>>(e.wake, e.nwake, e.rp.ff_dou, ff + e.nbody);
-    // near-pair list: a first size, grown when an earlier evaluation on the
-    // handle listed more (*near_seen, copied back without waiting for it)
+    // near-pair list: a first size, grown when the previous evaluation on the
+    // handle listed more (near_seen)
     if (near_cap == 0)
       near_cap = std::max(std::max<size_t>(1 << 20, n * 96),
                           std::min<size_t>(n * (size_t)ntot / 8, 1 << 26));
-    const unsigned long long seen = *(volatile unsigned long long *)near_seen;
-    if (seen > near_cap) near_cap = (size_t)(seen + seen / 4 + 1024);
-    const size_t off_l = (n * 24 + 255) / 256 * 256 + 256;
+    if (near_seen > near_cap) near_cap = (size_t)(near_seen + near_seen / 4 + 1024);
+    const size_t off_l = (n * 24 + 255) / 256 * 256;
     DUST_TRY(devbuf_grow(work, off_l + near_cap * sizeof(NearPair)));
     farv = (double *)work.p;
-    unsigned long long *count = (unsigned long long *)((char *)work.p + off_l - 256);
     NearPair *list = (NearPair *)((char *)work.p + off_l);
     const unsigned long long cap = near_cap;
     const unsigned pb = nblk(n, f32 ? EF2_NP : EO_NP);
     const int chunk = elem_chunk(pb, ntot, f32 ? EF2_LOAD : EO_LOAD);
     const dim3 grid(pb, nblk(ntot, chunk));
-    DUST_CUDA(cudaMemsetAsync(farv, 0, off_l, st));
+    DUST_CUDA(cudaMemsetAsync(farv, 0, n * 24, st));
+    DUST_CUDA(cudaMemsetAsync(count, 0, 8, st));
     if (kev) cudaEventRecord(kev[0], st);
     if (f32)
       k_elem_far<<<grid, EF2_T, 0, st>>>(d, e, ff, chunk, farv, count, list, cap);
@@ -683,7 +683,6 @@ int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
       k_elem_near<true><<<gn, 128, 0, st>>>(d, e, ff, count, list, cap, farv);
     else
       k_elem_near<false><<<gn, 128, 0, st>>>(d, e, ff, count, list, cap, farv);
-    DUST_CUDA(cudaMemcpyAsync(near_seen, count, 8, cudaMemcpyDeviceToHost, st));
   }
   if (n > 0) {
     if (f32)

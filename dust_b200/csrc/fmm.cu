@@ -194,9 +194,6 @@ extern "C" int dust_octree_create(const dust_fmm_params *prm, dust_octree **out)
   st = build_tables(o);
   if (st == DUST_OK) st = grow(o->small, 64 * 8);
   if (st == DUST_OK && cudaMemset(o->small.p, 0, 64 * 8) != cudaSuccess) st = DUST_ERR_CUDA;
-  if (st == DUST_OK && cudaMallocHost(&o->near_seen, sizeof(*o->near_seen)) != cudaSuccess)
-    st = DUST_ERR_CUDA;
-  if (st == DUST_OK) *o->near_seen = 0;
   if (st == DUST_OK) st = build_shift_tables(o);
   if (st == DUST_OK) st = m2l_batch_tables(o);
   if (st != DUST_OK) {
@@ -223,7 +220,6 @@ extern "C" int dust_octree_destroy(dust_octree *o) {
   devbuf_free(o->shift);
   devbuf_free(o->ffbuf);
   devbuf_free(o->elem_work);
-  if (o->near_seen) cudaFreeHost(o->near_seen);
   DevBuf *bufs[] = {&o->idxsum, &o->keys,   &o->keys_s, &o->vals,   &o->perm,
                     &o->cnt,    &o->cstart, &o->part,   &o->flags,  &o->ind,
                     &o->cidx,   &o->lidx,   &o->act_key, &o->act_lev, &o->leaf_ci,
@@ -1525,6 +1521,7 @@ int fmm_prepare_device(dust_octree *o, int n, const double *cen, const double *d
   int herr, hperr;
   memcpy(&herr, &hsmall[40], sizeof(int));
   memcpy(&hperr, &hsmall[41], sizeof(int));
+  o->near_seen = (unsigned long long)hsmall[52];  // of the evaluation before
   if (hsmall[50]) {  // of the previous evaluation: a bounded wait of its M2L gave up
     DUST_CUDA(cudaMemsetAsync(small + 48, 0, 4 * sizeof(int64_t), st));
     dust_set_last_error("a wait in the previous M2L gave up", __FILE__, __LINE__);
@@ -1793,7 +1790,8 @@ int fmm_finish_device(dust_octree *o, int n, const ElemDev &e, double *vel, doub
                       double *rot, cudaStream_t st) {
   if (n > 0)
     DUST_TRY(elem_output_device(o->dev, e, o->ffbuf, o->elem_work, o->near_cap, o->near_seen,
-                                o->prm.precision, vel, str, rot, st, o->timing ? &o->ev[8] : nullptr, &o->kev_far));
+                                (unsigned long long *)o->small.p + 52, o->prm.precision, vel, str,
+                                rot, st, o->timing ? &o->ev[8] : nullptr, &o->kev_far));
   if (o->timing) cudaEventRecord(o->ev[5], st);
   DUST_CUDA(cudaGetLastError());
   return DUST_OK;

@@ -68,7 +68,7 @@ struct dust_octree {
   DevBuf ffbuf;                        // far-field panel records
   DevBuf elem_work;                    // element sums: far sums, near-pair list
   size_t near_cap = 0;                 // capacity of the near-pair list
-  unsigned long long *near_seen = nullptr;  // pairs the last evaluation listed (pinned host)
+  unsigned long long near_seen = 0;    // pairs that an evaluation before listed
   DevBuf dtabs[DUST_MAXLEV + 1];       // dimensionless scalar M2L tables (FP64)
   DevBuf jsum;                         // M2L index table, then the classes' offsets
   DevBuf p2p_work;                     // near-field items and per-leaf split flags
@@ -135,7 +135,8 @@ int m2l_scale_sources(dust_octree *o, FmmDev &d, cudaStream_t st);
 
 // direct.cu
 int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
-                       size_t &near_cap, unsigned long long *near_seen, int precision,
+                       size_t &near_cap, unsigned long long near_seen,
+                       unsigned long long *count, int precision,
                        double *vel, double *str, double *rot, cudaStream_t st,
                        cudaEvent_t *kev = nullptr, bool *kev_done = nullptr);
 // Morton order of n particles over the octree box (10 bits per axis): the
