@@ -146,19 +146,60 @@ __global__ void k_pc_agg(int n, int K, const int *nbr, const float *w, const flo
   m[e] = s;
 }
 
-// z = Ws h + Wn m + b, h' = relu(z); a CTA of 64 threads per node row
-__global__ void k_pc_layer(int n, const float *P, int l, const float *h, const float *m, float *z,
-                           float *hn) {
-  __shared__ float sh[PC_H], sm[PC_H];
-  const int i = blockIdx.x, f = threadIdx.x;
-  sh[f] = h[(size_t)i * PC_H + f];
-  sm[f] = m[(size_t)i * PC_H + f];
+// z = Ws h + Wn m + b, h' = relu(z).  A CTA takes PC_LN nodes: the two weight
+// matrices go to shared memory once, transposed, so that the threads of a node
+// (one per feature) read consecutive words; each thread sums 8 nodes' outputs
+// in the order of k.  (A CTA of 64 threads per node, every thread walking its
+// own weight row in global memory: 210 us for 6,954 nodes; 13 us now.)
+#define PC_LN 32
+__global__ void __launch_bounds__(256) k_pc_layer(int n, const float *P, int l, const float *h,
+                                                  const float *m, float *z, float *hn) {
+  extern __shared__ __align__(16) float sl[];
+  float(*ws)[PC_H] = (float(*)[PC_H])sl, (*wn)[PC_H] = ws + PC_H;  // [k][f]
+  float(*sh)[PC_H] = wn + PC_H, (*sm)[PC_H] = sh + PC_LN;           // [node][k]
+  const int i0 = blockIdx.x * PC_LN, nn = min(PC_LN, n - i0), f = threadIdx.x % PC_H,
+            g = threadIdx.x / PC_H;
+  const float *Ws = P + pc_off_ws(l), *Wn = P + pc_off_wn(l);
+  // (rotated by the row, so that neither the rows read nor the columns written
+  // meet in one bank: word (k, f) lies at column (f + k) mod 64)
+  for (int e = threadIdx.x; e < PC_H * PC_H; e += 256) {
+    const int r = e / PC_H, k = e % PC_H;
+    ws[k][(r + k) % PC_H] = Ws[e];
+    wn[k][(r + k) % PC_H] = Wn[e];
+  }
+  for (int e = threadIdx.x; e < PC_LN * PC_H; e += 256) {
+    sh[e / PC_H][e % PC_H] = e / PC_H < nn ? h[(size_t)i0 * PC_H + e] : 0.f;
+    sm[e / PC_H][e % PC_H] = e / PC_H < nn ? m[(size_t)i0 * PC_H + e] : 0.f;
+  }
   __syncthreads();
-  const float *Ws = P + pc_off_ws(l) + f * PC_H, *Wn = P + pc_off_wn(l) + f * PC_H;
-  float s = P[pc_off_bl(l) + f];
-  for (int k = 0; k < PC_H; ++k) s = fmaf(Ws[k], sh[k], fmaf(Wn[k], sm[k], s));
-  z[(size_t)i * PC_H + f] = s;
-  hn[(size_t)i * PC_H + f] = fmaxf(s, 0.f);
+  float s[PC_LN / 4];
+#pragma unroll
+  for (int q = 0; q < PC_LN / 4; ++q) s[q] = P[pc_off_bl(l) + f];
+#pragma unroll 1
+  for (int k = 0; k < PC_H; k += 4) {
+    float a[4], b[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      a[x] = ws[k + x][(f + k + x) % PC_H];
+      b[x] = wn[k + x][(f + k + x) % PC_H];
+    }
+#pragma unroll
+    for (int q = 0; q < PC_LN / 4; ++q) {
+      const float4 H = *(const float4 *)&sh[g + 4 * q][k], M = *(const float4 *)&sm[g + 4 * q][k];
+      s[q] = fmaf(a[0], H.x, fmaf(b[0], M.x, s[q]));
+      s[q] = fmaf(a[1], H.y, fmaf(b[1], M.y, s[q]));
+      s[q] = fmaf(a[2], H.z, fmaf(b[2], M.z, s[q]));
+      s[q] = fmaf(a[3], H.w, fmaf(b[3], M.w, s[q]));
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < PC_LN / 4; ++q) {
+    const int i = g + 4 * q;
+    if (i < nn) {
+      z[(size_t)(i0 + i) * PC_H + f] = s[q];
+      hn[(size_t)(i0 + i) * PC_H + f] = fmaxf(s[q], 0.f);
+    }
+  }
 }
 
 // o_ij = sum_f u_f h_i,f h_j,f + c . e_ij; warp per edge
@@ -200,25 +241,51 @@ __global__ void k_pc_resid(int n, int K, int C, const int *nbr, const float *o, 
 
 // ------------------------------------------------------------ backward
 // do_ij = scale * sum_c R_ic Y_jc; dc += do_ij e_ij; du_f += do_ij h_i,f h_j,f;
-// dh_i += do_ij u h_j, dh_j += do_ij u h_i (warp per edge)
-__global__ void k_pc_out_bwd(int n, int K, int C, float scale, const float *P, const int *nbr,
-                             const float *ef, const float *h, const float *R, const float *Y,
-                             float *G, float *dh) {
-  const size_t wid = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (wid >= (size_t)n * K) return;
-  const int i = (int)(wid / K), j = nbr[wid];
-  float d = 0.f;
-  for (int c = lane; c < C; c += 32) d += R[(size_t)i * C + c] * Y[(size_t)j * C + c];
-  for (int q = 16; q > 0; q >>= 1) d += __shfl_xor_sync(0xffffffffu, d, q);
-  d *= scale;
-  if (lane < PC_EF) atomicAdd(G + pc_off_c() + lane, d * ef[wid * PC_EF + lane]);
+// dh_i += do_ij u h_j, dh_j += do_ij u h_i.  A warp takes a node's edges: du, dc
+// and dh_i stay in registers over them, and du and dc leave once per CTA.  (A
+// warp per edge added every edge's du and dc to the same 68 words: 262 us for
+// 62,586 edges; 12 us now.)
+__global__ void __launch_bounds__(256) k_pc_out_bwd(int n, int K, int C, float scale,
+                                                    const float *P, const int *nbr,
+                                                    const float *ef, const float *h,
+                                                    const float *R, const float *Y, float *G,
+                                                    float *dh) {
+  __shared__ float su[8][PC_H], sc[8][PC_EF];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 8 + warp;
   const float *u = P + pc_off_u();
-  for (int f = lane; f < PC_H; f += 32) {
-    const float hi = h[(size_t)i * PC_H + f], hj = h[(size_t)j * PC_H + f];
-    atomicAdd(G + pc_off_u() + f, d * hi * hj);
-    atomicAdd(dh + (size_t)i * PC_H + f, d * u[f] * hj);
-    atomicAdd(dh + (size_t)j * PC_H + f, d * u[f] * hi);
+  const float u0 = u[lane], u1 = u[lane + 32];
+  float du0 = 0.f, du1 = 0.f, dc = 0.f;
+  if (i < n) {
+    const float h0 = h[(size_t)i * PC_H + lane], h1 = h[(size_t)i * PC_H + lane + 32];
+    float a0 = 0.f, a1 = 0.f;
+    for (int q = 0; q < K; ++q) {
+      const size_t e = (size_t)i * K + q;
+      const int j = nbr[e];
+      float d = 0.f;
+      for (int c = lane; c < C; c += 32) d += R[(size_t)i * C + c] * Y[(size_t)j * C + c];
+      for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+      d *= scale;
+      if (lane < PC_EF) dc += d * ef[e * PC_EF + lane];
+      const float g0 = h[(size_t)j * PC_H + lane], g1 = h[(size_t)j * PC_H + lane + 32];
+      du0 += d * h0 * g0;
+      du1 += d * h1 * g1;
+      a0 += d * u0 * g0;
+      a1 += d * u1 * g1;
+      atomicAdd(dh + (size_t)j * PC_H + lane, d * u0 * h0);
+      atomicAdd(dh + (size_t)j * PC_H + lane + 32, d * u1 * h1);
+    }
+    atomicAdd(dh + (size_t)i * PC_H + lane, a0);
+    atomicAdd(dh + (size_t)i * PC_H + lane + 32, a1);
+  }
+  su[warp][lane] = du0;
+  su[warp][lane + 32] = du1;
+  if (lane < PC_EF) sc[warp][lane] = dc;
+  __syncthreads();
+  if (threadIdx.x < PC_H + PC_EF) {
+    const int t = threadIdx.x;
+    float s = 0.f;
+    for (int w = 0; w < 8; ++w) s += t < PC_H ? su[w][t] : sc[w][t - PC_H];
+    atomicAdd(G + (t < PC_H ? pc_off_u() + t : pc_off_c() + t - PC_H), s);
   }
 }
 
@@ -258,27 +325,44 @@ __global__ void k_pc_agg_bwd(int n, int K, const int *nbr, const float *w, const
 }
 
 // G[off + f*cols + k] += sum_i dz_i,f a_i,k and G[boff + f] += sum_i dz_i,f
-// (boff < 0: none); CTA per chunk of nodes, partial sums in shared memory
+// (boff < 0: none); CTA per chunk of nodes.  Both operands of a chunk are
+// staged in shared memory (every thread read them from global memory for each
+// of its products before: 41 us a call at 6,954 nodes, 12 us now).
 #define PC_WG_CHUNK 64
-__global__ void k_pc_wgrad(int n, const float *dz, const float *a, int cols, float *G, int off,
-                           int boff) {
-  extern __shared__ float sacc[];  // PC_H x cols
+__global__ void __launch_bounds__(256) k_pc_wgrad(int n, const float *dz, const float *a, int cols,
+                                                  float *G, int off, int boff) {
+  __shared__ __align__(16) float sd[PC_WG_CHUNK][PC_H], sa[PC_WG_CHUNK][PC_H];
   const int tid = threadIdx.x;
-  const int i0 = blockIdx.x * PC_WG_CHUNK, i1 = min(n, i0 + PC_WG_CHUNK);
-  for (int e = tid; e < PC_H * cols; e += blockDim.x) {
-    const int f = e / cols, k = e % cols;
-    float s = 0.f;
-    for (int i = i0; i < i1; ++i) s = fmaf(dz[(size_t)i * PC_H + f], a[(size_t)i * cols + k], s);
-    sacc[e] = s;
+  const int i0 = blockIdx.x * PC_WG_CHUNK, ni = min(n - i0, PC_WG_CHUNK);
+  for (int e = tid; e < PC_WG_CHUNK * PC_H; e += 256) {
+    const int i = e / PC_H, k = e % PC_H;
+    sd[i][k] = i < ni ? dz[(size_t)(i0 + i) * PC_H + k] : 0.f;
+    sa[i][k] = i < ni && k < cols ? a[(size_t)(i0 + i) * cols + k] : 0.f;
   }
   __syncthreads();
-  for (int e = tid; e < PC_H * cols; e += blockDim.x) atomicAdd(G + off + e, sacc[e]);
-  if (boff >= 0)
-    for (int f = tid; f < PC_H; f += blockDim.x) {
-      float s = 0.f;
-      for (int i = i0; i < i1; ++i) s += dz[(size_t)i * PC_H + f];
-      atomicAdd(G + boff + f, s);
+  // thread (fy, kx): features 4 fy .., columns 4 kx ..
+  const int fy = tid / 16, kx = tid % 16;
+  if (4 * kx < cols) {
+    float s[4][4] = {};
+    for (int i = 0; i < ni; ++i) {
+      const float4 D = *(const float4 *)&sd[i][4 * fy], A = *(const float4 *)&sa[i][4 * kx];
+      const float d[4] = {D.x, D.y, D.z, D.w}, x[4] = {A.x, A.y, A.z, A.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) s[u][v] = fmaf(d[u], x[v], s[u][v]);
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        if (4 * kx + v < cols) atomicAdd(G + off + (4 * fy + u) * cols + 4 * kx + v, s[u][v]);
+  }
+  if (boff >= 0 && tid < PC_H) {
+    float s = 0.f;
+    for (int i = 0; i < ni; ++i) s += sd[i][tid];
+    atomicAdd(G + boff + tid, s);
+  }
 }
 
 __global__ void k_pc_adam(int np, float *P, const float *G, float *m, float *v, float lr, float b1,
@@ -302,8 +386,9 @@ static int pc_forward(dust_precond *p, const float *x, const float *ef, const fl
   for (int l = 0; l < PC_L; ++l) {
     k_pc_agg<<<nblk(nh, 256), 256, 0, st>>>(n, K, (const int *)p->nbr.p, w, h + l * nh,
                                              m + l * nh);
-    k_pc_layer<<<n, PC_H, 0, st>>>(n, P, l, h + l * nh, m + l * nh, z + (l + 1) * nh,
-                                   h + (l + 1) * nh);
+    const int smem = (2 * PC_H + 2 * PC_LN) * PC_H * 4;  // 48 KB: needs no opt-in
+    k_pc_layer<<<nblk(n, PC_LN), 256, smem, st>>>(n, P, l, h + l * nh, m + l * nh,
+                                                  z + (l + 1) * nh, h + (l + 1) * nh);
   }
   k_pc_out<<<nblk((size_t)n * K * 32, 256), 256, 0, st>>>(n, K, P, (const int *)p->nbr.p, ef,
                                                            h + PC_L * nh, (float *)p->o.p);
@@ -331,21 +416,21 @@ static int pc_loss_grad(dust_precond *p, int si, float *loss_host) {
   k_pc_resid<<<nblk((size_t)n * C, 256), 256, 0, st>>>(n, K, C, nbr, (const float *)p->o.p, Y, T,
                                                         R, ls);
   const float scale = 2.f / ((float)n * C);
-  k_pc_out_bwd<<<nblk((size_t)n * K * 32, 256), 256, 0, st>>>(
+  k_pc_out_bwd<<<nblk(n, 8), 256, 0, st>>>(
       n, K, C, scale, (const float *)p->par.p, nbr, ef, h + PC_L * nh, R, Y, G, dh);
   const unsigned nch = nblk(n, PC_WG_CHUNK);
   for (int l = PC_L - 1; l >= 0; --l) {
     // dh holds dL/dh(l+1): mask by z(l+1)
     k_pc_relu_bwd<<<nblk(nh, 256), 256, 0, st>>>(nh, z + (l + 1) * nh, dh);
-    k_pc_wgrad<<<nch, 256, PC_H * PC_H * 4, st>>>(n, dh, h + l * nh, PC_H, G, pc_off_ws(l),
+    k_pc_wgrad<<<nch, 256, 0, st>>>(n, dh, h + l * nh, PC_H, G, pc_off_ws(l),
                                                    pc_off_bl(l));
-    k_pc_wgrad<<<nch, 256, PC_H * PC_H * 4, st>>>(n, dh, m + l * nh, PC_H, G, pc_off_wn(l), -1);
+    k_pc_wgrad<<<nch, 256, 0, st>>>(n, dh, m + l * nh, PC_H, G, pc_off_wn(l), -1);
     k_pc_layer_bwd<<<n, PC_H, 0, st>>>(n, (const float *)p->par.p, l, dh, dhp, dm);
     k_pc_agg_bwd<<<nblk(nh, 256), 256, 0, st>>>(n, K, nbr, w, dm, dhp);
     std::swap(dh, dhp);
   }
   k_pc_relu_bwd<<<nblk(nh, 256), 256, 0, st>>>(nh, z, dh);
-  k_pc_wgrad<<<nch, 256, PC_H * PC_FIN * 4, st>>>(n, dh, x, PC_FIN, G, pc_off_w0(), pc_off_b0());
+  k_pc_wgrad<<<nch, 256, 0, st>>>(n, dh, x, PC_FIN, G, pc_off_w0(), pc_off_b0());
   DUST_CUDA(cudaGetLastError());
   if (loss_host) {
     float l = 0.f;

@@ -99,3 +99,23 @@ def test_gmres_without_network_falls_back_to_lu():
     xg, rep = ls.solve_linsys(abi.DUST_SOLVE_GMRES_NN)
     assert rep["fell_back"] == 1 and rep["mode_used"] == abi.DUST_SOLVE_LU64
     assert rel(xg, xl) < 1e-12
+
+
+@pytest.mark.parametrize("n_fus,n_span,n_chord,k", [(32, 2, 1, 4), (33, 1, 1, 5), (130, 3, 2, 8)])
+def test_gnn_gradient_small_and_ragged(n_fus, n_span, n_chord, k):
+    """Node counts around the kernels' groups of 32 nodes, and other degrees."""
+    els, nst = _system(0.3, n_fus=n_fus, n_span=n_span, n_chord=n_chord)
+    ls = linsys.initialize_linsys(PRM, els.n, nst, els)
+    x = _solve_lu(ls, els)
+    ls.assemble_linsys(els)
+    pc = precond.Precond(els.ver.mean(axis=1), k=k, seed=1)
+    pc.add_sample(ls, x, seed=5)
+    p = (np.random.default_rng(2).standard_normal(pc.num_params()) * 0.15).astype(np.float32)
+    pc.set_params(p)
+    loss, g = pc.loss_grad(0)
+    xs, ef, w, nbr, Y, T = pc.get_sample(0)
+    lo, go = G.loss_grad(p.astype(np.float64), xs.astype(np.float64), ef.astype(np.float64),
+                         w.astype(np.float64), nbr.astype(np.int64), Y.astype(np.float64),
+                         T.astype(np.float64))
+    assert abs(loss - lo) <= 1e-4 * abs(lo)
+    assert rel(g.astype(np.float64), go) < 2e-3
