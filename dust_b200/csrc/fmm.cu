@@ -406,112 +406,89 @@ __global__ void k_level_counts(TreeGeom G, const uint32_t *__restrict__ cidx,
   if (threadIdx.x == 0) out[0] = lidx[G.lev_off[G.ll + 1]];
 }
 
-__device__ inline double ipow_d(double x, int e) {
-  double r = 1.0;
-  for (int q = 0; q < e; ++q) r *= x;
-  return r;
+// Coefficient m of a cell's multipole (rows m >= nm: the padding of the scaled
+// copy) into A and, for the cells that are M2L sources, scaled by 1/(n! h^|n|),
+// into ahat as [cell][component][rs].
+__device__ __forceinline__ void put_multipole(const FmmDev &d, uint32_t ci, int l, int m,
+                                              const double *v) {
+  if (m < d.nm) {
+    double *a = d.A + (size_t)ci * 3 * d.nm + 3 * m;
+    for (int c = 0; c < 3; ++c) a[c] = v[c];
+  }
+  if (d.ahat && ci >= d.ahat_c0) {
+    double f = 0.0;
+    if (m < d.nm) {
+      int i, j, k;
+      mono_exp(m, i, j, k);
+      const double hi = 1.0 / d.G.csize[l];
+      f = d.inv_fact[m];
+      for (int q = 0; q < i + j + k; ++q) f *= hi;
+    }
+    double *o = d.ahat + (size_t)(ci - d.ahat_c0) * 3 * d.ahat_rs + m;
+    for (int c = 0; c < 3; ++c) o[c * d.ahat_rs] = f * v[c];
+  }
 }
 
-// P2M (leaf_M_multipole, mod_multipole.f90:224-251): one warp per leaf.
+// P2M (leaf_M_multipole, mod_multipole.f90:224-251): one warp per leaf, the
+// leaf's particles in chunks of 32: lane t forms the powers of particle t's
+// offsets into the warp's shared memory (rows of 33 words: the lanes of a
+// product read different rows), then the lanes take the output coefficients m
+// and sum the chunk's products in particle order.  (Powers formed per
+// coefficient and particle: 31 us for 3,000 particles, 381 us for 1,100,000,
+// and 4 and 170 us for the scaled copy; 10 and 208 us together.)
 #define P2M_W 4
+#define P2M_LD 33
 __global__ void __launch_bounds__(P2M_W * 32) k_p2m(FmmDev d) {
-  // one warp per leaf: the leaf's particles in chunks of 32 in the warp's
-  // shared memory, lanes over the output coefficients m (32 at a time); each
-  // coefficient sums its particles in the same order as a serial loop
-  __shared__ double sh[P2M_W][6][32];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  extern __shared__ __align__(16) double p2m_sm[];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, np = d.p + 1;
   const uint32_t leaf = blockIdx.x * P2M_W + w;
   if (leaf >= d.n_leaves) return;  // warp-uniform
-  uint32_t ci = d.leaf_ci[leaf];
-  int l = d.act_lev[ci];
-  uint32_t key = d.act_key[ci];
-  int ci_, cj, ck;
-  cart_of_key(d.G, l, key, ci_, cj, ck);
-  double c[3];
-  cell_center(d.G, l, ci_, cj, ck, c);
-  uint32_t lo = cell_lo(d.G, d.cstart, l, key), hi = cell_hi(d.G, d.cstart, l, key);
+  const uint32_t ci = d.leaf_ci[leaf];
+  const int l = d.act_lev[ci];
+  const uint32_t key = d.act_key[ci];
+  const uint32_t lo = cell_lo(d.G, d.cstart, l, key), hi = cell_hi(d.G, d.cstart, l, key);
   if (hi == lo) return;  // empty leaf: a = 0 (block zeroed before the pass)
+  int i, j, k;
+  cart_of_key(d.G, l, key, i, j, k);
+  double c[3];
+  cell_center(d.G, l, i, j, k, c);
   const size_t n = d.n;
-  double(*sp)[32] = sh[w];
-  for (int m0 = 0; m0 < d.nm; m0 += 32) {
+  double *pw = p2m_sm + (size_t)w * (3 * np + 3) * P2M_LD;  // [axis][power][t], alpha[3][t]
+  double *al = pw + 3 * np * P2M_LD;
+  const int rs = d.ahat ? d.ahat_rs : d.nm;
+  for (int m0 = 0; m0 < rs; m0 += 32) {
     const int m = m0 + lane;
     int mi = 0, mj = 0, mk = 0;
     if (m < d.nm) mono_exp(m, mi, mj, mk);
-    double ax = 0, ay = 0, az = 0;
+    const double *px = pw + mi * P2M_LD, *py = pw + (np + mj) * P2M_LD,
+                 *pz = pw + (2 * np + mk) * P2M_LD;
+    double v[3] = {0.0, 0.0, 0.0};
     for (uint32_t s0 = lo; s0 < hi; s0 += 32) {
       const int cnt = min((int)(hi - s0), 32);
-      __syncwarp();
-      if (lane < cnt) {
-        const uint32_t s = s0 + lane;
-        sp[0][lane] = d.P[s] - c[0];
-        sp[1][lane] = d.P[n + s] - c[1];
-        sp[2][lane] = d.P[2 * n + s] - c[2];
-        sp[3][lane] = d.P[3 * n + s];
-        sp[4][lane] = d.P[4 * n + s];
-        sp[5][lane] = d.P[5 * n + s];
+      if (m0 == 0 || hi - lo > 32) {  // (one chunk: its powers stay for every m0)
+        __syncwarp();
+        if (lane < cnt) {
+          const uint32_t s = s0 + lane;
+          for (int x = 0; x < 3; ++x) {
+            const double dx = d.P[x * n + s] - c[x];
+            double q = 1.0;
+            for (int e = 0; e < np; ++e, q *= dx) pw[(x * np + e) * P2M_LD + lane] = q;
+            al[x * P2M_LD + lane] = d.P[(3 + x) * n + s];
+          }
+        }
+        __syncwarp();
       }
-      __syncwarp();
       if (m < d.nm)
+#pragma unroll 4
         for (int t = 0; t < cnt; ++t) {
-          double pr = ipow_d(sp[0][t], mi) * ipow_d(sp[1][t], mj) * ipow_d(sp[2][t], mk);
-          ax += pr * sp[3][t];
-          ay += pr * sp[4][t];
-          az += pr * sp[5][t];
+          const double pr = px[t] * py[t] * pz[t];
+          v[0] += pr * al[t];
+          v[1] += pr * al[P2M_LD + t];
+          v[2] += pr * al[2 * P2M_LD + t];
         }
     }
-    if (m < d.nm) {
-      double *a = d.A + (size_t)ci * 3 * d.nm;
-      a[3 * m] = ax;
-      a[3 * m + 1] = ay;
-      a[3 * m + 2] = az;
-    }
+    if (m < rs) put_multipole(d, ci, l, m, v);
   }
-}
-
-__device__ inline double binom_d(int n, int k) {
-  double r = 1.0;
-  for (int q = 1; q <= k; ++q) r = r * (double)(n - k + q) / (double)q;
-  return r;
-}
-
-// M2M (mod_multipole.f90:256-278) into the active branch cells of level l.
-__global__ void k_m2m(FmmDev d, int l, uint32_t act_lo) {
-  uint32_t ci = act_lo + blockIdx.x;
-  uint32_t key = d.act_key[ci];
-  if (!(d.flags[d.G.lev_off[l] + key] & FL_BRANCH)) return;
-  int m = threadIdx.x;
-  if (m >= d.nm) return;
-  int i, j, k;
-  cart_of_key(d.G, l, key, i, j, k);
-  double cp[3];
-  cell_center(d.G, l, i, j, k, cp);
-  int mi, mj, mk;
-  mono_exp(m, mi, mj, mk);
-  double acc[3] = {0, 0, 0};
-  for (int ch = 0; ch < 8; ++ch) {
-    uint32_t ckey = 8u * key + (uint32_t)ch;
-    uint32_t cc = d.cidx[d.G.lev_off[l + 1] + ckey];
-    int ii, jj, kk;
-    cart_of_key(d.G, l + 1, ckey, ii, jj, kk);
-    double cc3[3];
-    cell_center(d.G, l + 1, ii, jj, kk, cc3);
-    double dx = cc3[0] - cp[0], dy = cc3[1] - cp[1], dz = cc3[2] - cp[2];
-    const double *a = d.A + (size_t)cc * 3 * d.nm;
-    for (int ks = 0; ks <= mk; ++ks)
-      for (int js = 0; js <= mj; ++js)
-        for (int is = 0; is <= mi; ++is) {
-          int s = mono_idx(is, js, ks);
-          double w = binom_d(mi, is) * binom_d(mj, js) * binom_d(mk, ks) *
-                     (ipow_d(dx, mi - is) * ipow_d(dy, mj - js) * ipow_d(dz, mk - ks));
-          acc[0] += w * a[3 * s];
-          acc[1] += w * a[3 * s + 1];
-          acc[2] += w * a[3 * s + 2];
-        }
-  }
-  double *ap = d.A + (size_t)ci * 3 * d.nm;
-  ap[3 * m] = acc[0];
-  ap[3 * m + 1] = acc[1];
-  ap[3 * m + 2] = acc[2];
 }
 
 // ------------------------------------------------ M2M / L2L from tables
@@ -521,34 +498,58 @@ __global__ void k_m2m(FmmDev d, int l, uint32_t act_lo) {
 //   a_par(m) += sum_{s <= m} C(m,s) d^(m-s) a_child(s)
 // and of L2L_multipole (:360-384)
 //   b_child(m) += sum_{s >= m, |s| <= p} C(s,m) d^(s-m) b_par(s)
-// are per level the same up to the sign (-1)^(sum of the exponents along the
-// axes where d < 0).  The host lists, per output m, the terms (s, exponent,
-// unsigned weight); the kernels apply the octant's sign.
+// are per level the same up to the sign chi_q(ch) = (-1)^(popcount of q and the
+// octant bits that are clear), q the parities of the exponents m - s along the
+// axes.  The signs are a Walsh-Hadamard transform over the 8 children, so a
+// weight acts once per parent instead of once per child:
+//   M2M  a_par(m)   = sum_s w(m,s) H_q(m,s)(s),  H_q(s) = sum_ch chi_q(ch) a_ch(s)
+//   L2L  b_ch(m)   += sum_q chi_q(ch) T_q(m),    T_q(m) = sum_{s of parity q} w(m,s) b_par(s)
+// The host lists, per output m, the terms (w, position of the source value).
 struct ShiftTerm {
   double w;
-  uint16_t s;
-  uint8_t ex, ey, ez, pad[3];
+  int at;  // M2M: q (3 nm) + 3 s; L2L: 3 s
+  int q;
 };
 
-__device__ __forceinline__ double shift_w(const ShiftTerm &t, uint32_t oct) {
-  const int par = ((oct & 1u) ? 0 : t.ex) + ((oct & 2u) ? 0 : t.ey) + ((oct & 4u) ? 0 : t.ez);
-  return (par & 1) ? -t.w : t.w;
+// y_q = sum_ch chi_q(ch) x_ch, in place (index bits are octant / parity bits)
+__device__ __forceinline__ void wht_up(double (&x)[8]) {
+#pragma unroll
+  for (int b = 1; b < 8; b *= 2)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (!(i & b)) {
+        const double u = x[i], v = x[i | b];
+        x[i] = u + v;
+        x[i | b] = v - u;
+      }
+}
+// y_ch = sum_q chi_q(ch) x_q, in place
+__device__ __forceinline__ void wht_down(double (&x)[8]) {
+#pragma unroll
+  for (int b = 1; b < 8; b *= 2)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (!(i & b)) {
+        const double u = x[i], v = x[i | b];
+        x[i] = u - v;
+        x[i | b] = u + v;
+      }
 }
 
 #define SH_T 128
 #define SH_W (SH_T / 32)
-// M2M into the active branch cells of level l: one warp per parent, lanes
-// over the output coefficient m; terms and offsets staged in shared memory,
-// and each warp stages its parent's 8 children's coefficients (missing
-// children as zeros) before the term loops
+// M2M into the active branch cells of level l: one warp per parent; terms and
+// offsets staged in shared memory, the children's transforms H in the warp's
+// own, lanes over the output coefficient m.  (Every weight applied to each
+// child: 22 us a level at least and 472 us for 1,100,000 particles; 6 and 122 us.)
 __global__ void __launch_bounds__(SH_T) k_m2m_t(FmmDev d, int l, uint32_t act_lo, uint32_t na,
                                                 const ShiftTerm *terms, const int *off, int nterm) {
   extern __shared__ __align__(16) unsigned char shm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w3 = 3 * d.nm;
-  double *sa = (double *)shm + (size_t)warp * 8 * w3;  // [8][3 nm]
-  ShiftTerm *st = (ShiftTerm *)((double *)shm + (size_t)SH_W * 8 * w3);
-  int *so = (int *)(st + nterm);
+  ShiftTerm *st = (ShiftTerm *)shm;
+  double *H = (double *)(st + nterm) + (size_t)warp * 8 * w3;  // [q][3 nm]
+  int *so = (int *)((double *)(st + nterm) + (size_t)SH_W * 8 * w3);
   for (int e = threadIdx.x; e < nterm; e += SH_T) st[e] = terms[e];
   for (int e = threadIdx.x; e <= d.nm; e += SH_T) so[e] = off[e];
   __syncthreads();
@@ -556,78 +557,60 @@ __global__ void __launch_bounds__(SH_T) k_m2m_t(FmmDev d, int l, uint32_t act_lo
     const uint32_t ci = act_lo + c;
     const uint32_t key = d.act_key[ci];
     if (!(d.flags[d.G.lev_off[l] + key] & FL_BRANCH)) continue;
+    uint32_t cc[8];
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch) cc[ch] = d.cidx[d.G.lev_off[l + 1] + 8u * key + (uint32_t)ch];
     __syncwarp();
-    for (int ch = 0; ch < 8; ++ch) {
-      const uint32_t cc = d.cidx[d.G.lev_off[l + 1] + 8u * key + (uint32_t)ch];
-      const double *a = d.A + (size_t)cc * w3;
-      for (int e = lane; e < w3; e += 32) sa[ch * w3 + e] = a[e];
+    for (int e = lane; e < w3; e += 32) {
+      double x[8];
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) x[ch] = d.A[(size_t)cc[ch] * w3 + e];
+      wht_up(x);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) H[q * w3 + e] = x[q];
     }
     __syncwarp();
-    for (int m = lane; m < d.nm; m += 32) {
+    const int rs = d.ahat ? d.ahat_rs : d.nm;
+    for (int m = lane; m < rs; m += 32) {
       double acc[3] = {0, 0, 0};
-      for (int ch = 0; ch < 8; ++ch) {
-        const double *a = sa + ch * w3;
-        for (int t = so[m]; t < so[m + 1]; ++t) {
-          const double w = shift_w(st[t], (uint32_t)ch);
-          const int s3 = 3 * st[t].s;
-          acc[0] += w * a[s3];
-          acc[1] += w * a[s3 + 1];
-          acc[2] += w * a[s3 + 2];
+      if (m < d.nm) {
+        const int t1 = so[m + 1];
+#pragma unroll 4
+        for (int t = so[m]; t < t1; ++t) {
+          const ShiftTerm tm = st[t];
+          const double *h = H + tm.at;
+          acc[0] = fma(tm.w, h[0], acc[0]);
+          acc[1] = fma(tm.w, h[1], acc[1]);
+          acc[2] = fma(tm.w, h[2], acc[2]);
         }
       }
-      double *ap = d.A + (size_t)ci * w3;
-      ap[3 * m] = acc[0];
-      ap[3 * m + 1] = acc[1];
-      ap[3 * m + 2] = acc[2];
+      put_multipole(d, ci, l, m, acc);
     }
   }
 }
 
-// L2L into the active cells of level l (>= 2) from their parents: one warp
-// per parent (an active branch cell of level l - 1), lanes over the output
-// coefficient m.  The 8 children's weights differ only in sign (the octant's
-// parity of the exponents), so each term's products are formed once and
-// added to all 8 children's sums; the parent's b and g are staged in shared
-// memory; only active children are written.  b terms (|s| <= p) and, with
-// stretching, g terms (|s| <= p+1).
-__device__ __forceinline__ void l2l_terms(const ShiftTerm *tt, int t0, int t1, const double *src,
-                                          double (*acc)[3]) {
-#pragma unroll
-  for (int ch = 0; ch < 8; ++ch) acc[ch][0] = acc[ch][1] = acc[ch][2] = 0.0;
-  for (int t = t0; t < t1; ++t) {
-    const ShiftTerm tm = tt[t];
-    const int s3 = 3 * tm.s;
-    const double v0 = tm.w * src[s3], v1 = tm.w * src[s3 + 1], v2 = tm.w * src[s3 + 2];
-    const unsigned px = tm.ex & 1u, py = tm.ey & 1u, pz = tm.ez & 1u;
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      // sign of shift_w for octant ch
-      const unsigned neg = ((ch & 1) ? 0u : px) ^ ((ch & 2) ? 0u : py) ^ ((ch & 4) ? 0u : pz);
-      if (neg) {
-        acc[ch][0] -= v0, acc[ch][1] -= v1, acc[ch][2] -= v2;
-      } else {
-        acc[ch][0] += v0, acc[ch][1] += v1, acc[ch][2] += v2;
-      }
-    }
-  }
-}
-
+// L2L into the active cells of level l (>= 2) from their parents: one warp per
+// parent (an active branch cell of level l - 1) and expansion (b with |s| <= p,
+// and, with stretching, g with |s| <= p+1), lanes over the output coefficient
+// m: the parity sums T_q from the terms (sorted by q), their transform to the
+// 8 children, added to the children that are active.  (Every term added to
+// each child's sum: 27 us a level at least and 626 us for 1,100,000 particles; 9
+// and 328 us.)
 __global__ void __launch_bounds__(SH_T) k_l2l_t(FmmDev d, int l, uint32_t act_lo, uint32_t na,
                                                 const ShiftTerm *tb, const int *ob, int ntb,
                                                 const ShiftTerm *tg, const int *og, int ntg) {
   extern __shared__ __align__(16) unsigned char shm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wb = 3 * d.nm, wg = ntg > 0 ? 3 * d.nm1 : 0;
-  double *sbp = (double *)shm + (size_t)warp * (wb + wg);  // parent's b, then g
-  double *sgp = sbp + wb;
-  ShiftTerm *sb = (ShiftTerm *)((double *)shm + (size_t)SH_W * (wb + wg));
-  ShiftTerm *sg = sb + ntb;
-  int *sob = (int *)(sg + ntg);
-  int *sog = sob + d.nm + 1;
-  for (int e = threadIdx.x; e < ntb; e += SH_T) sb[e] = tb[e];
-  for (int e = threadIdx.x; e < ntg; e += SH_T) sg[e] = tg[e];
-  for (int e = threadIdx.x; e <= d.nm; e += SH_T) sob[e] = ob[e];
-  for (int e = threadIdx.x; e <= d.nm1 && ntg > 0; e += SH_T) sog[e] = og[e];
+  const bool isg = blockIdx.y == 1;
+  const int nm = isg ? d.nm1 : d.nm, nt = isg ? ntg : ntb, w3 = 3 * nm;
+  const ShiftTerm *tt = isg ? tg : tb;
+  const int *oo = isg ? og : ob;
+  double *E = isg ? d.Gx : d.B;
+  ShiftTerm *st = (ShiftTerm *)shm;
+  double *sp = (double *)(st + nt) + (size_t)warp * w3;  // parent's expansion
+  int *so = (int *)((double *)(st + nt) + (size_t)SH_W * w3);
+  for (int e = threadIdx.x; e < nt; e += SH_T) st[e] = tt[e];
+  for (int e = threadIdx.x; e <= 8 * nm; e += SH_T) so[e] = oo[e];
   __syncthreads();
   // act_lo / na: the active cells of level l - 1 (the candidate parents)
   for (uint32_t c = blockIdx.x * SH_W + warp; c < na; c += gridDim.x * SH_W) {
@@ -644,33 +627,42 @@ __global__ void __launch_bounds__(SH_T) k_l2l_t(FmmDev d, int l, uint32_t act_lo
     }
     if (!live) continue;
     __syncwarp();
-    const double *bp = d.B + (size_t)pc * wb;
-    for (int e = lane; e < wb; e += 32) sbp[e] = bp[e];
-    if (wg > 0) {
-      const double *gp = d.Gx + (size_t)pc * wg;
-      for (int e = lane; e < wg; e += 32) sgp[e] = gp[e];
-    }
+    for (int e = lane; e < w3; e += 32) sp[e] = E[(size_t)pc * w3 + e];
     __syncwarp();
-    double acc[8][3];
-    for (int m = lane; m < d.nm; m += 32) {
-      l2l_terms(sb, sob[m], sob[m + 1], sbp, acc);
+    for (int m = lane; m < nm; m += 32) {
+      // (the children's values are fetched while the sums are formed)
+      double T[3][8], old[8][3];
 #pragma unroll
       for (int ch = 0; ch < 8; ++ch)
         if ((live >> ch) & 1u) {
-          double *b = d.B + (size_t)cc[ch] * wb + 3 * m;
-          b[0] += acc[ch][0], b[1] += acc[ch][1], b[2] += acc[ch][2];
+          const double *b = E + (size_t)cc[ch] * w3 + 3 * m;
+          old[ch][0] = b[0], old[ch][1] = b[1], old[ch][2] = b[2];
         }
-    }
-    if (wg > 0) {
-      for (int m = lane; m < d.nm1; m += 32) {
-        l2l_terms(sg, sog[m], sog[m + 1], sgp, acc);
 #pragma unroll
-        for (int ch = 0; ch < 8; ++ch)
-          if ((live >> ch) & 1u) {
-            double *g = d.Gx + (size_t)cc[ch] * wg + 3 * m;
-            g[0] += acc[ch][0], g[1] += acc[ch][1], g[2] += acc[ch][2];
-          }
+      for (int q = 0; q < 8; ++q) {
+        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+        const int t1 = so[8 * m + q + 1];
+#pragma unroll 2
+        for (int t = so[8 * m + q]; t < t1; ++t) {
+          const ShiftTerm tm = st[t];
+          const double *v = sp + tm.at;
+          a0 = fma(tm.w, v[0], a0);
+          a1 = fma(tm.w, v[1], a1);
+          a2 = fma(tm.w, v[2], a2);
+        }
+        T[0][q] = a0, T[1][q] = a1, T[2][q] = a2;
       }
+      wht_down(T[0]);
+      wht_down(T[1]);
+      wht_down(T[2]);
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch)
+        if ((live >> ch) & 1u) {
+          double *b = E + (size_t)cc[ch] * w3 + 3 * m;
+          b[0] = old[ch][0] + T[0][ch];
+          b[1] = old[ch][1] + T[1][ch];
+          b[2] = old[ch][2] + T[2][ch];
+        }
     }
   }
 }
@@ -681,15 +673,18 @@ static double binom_h(int n, int k) {
   return r;
 }
 
-// term lists of one shift: up = false: s <= m (M2M, deg <= p); up = true:
-// s >= m with |s| <= q (L2L of a degree-q expansion)
+// term lists of one shift: up = false: s <= m (M2M, deg <= p), offsets per m;
+// up = true: s >= m with |s| <= q (L2L of a degree-q expansion), sorted by
+// parity class, offsets per (m, class)
 static void shift_terms(int nout, int q, bool up, double delta, std::vector<ShiftTerm> &t,
                         std::vector<int> &off) {
   t.clear();
   off.assign(1, 0);
+  const int w3 = 3 * n_mon(q);
   for (int m = 0; m < nout; ++m) {
     int mi, mj, mk;
     mono_exp(m, mi, mj, mk);
+    std::vector<ShiftTerm> cls[8];
     for (int s = 0; s < n_mon(q); ++s) {
       int si, sj, sk;
       mono_exp(s, si, sj, sk);
@@ -711,15 +706,15 @@ static void shift_terms(int nout, int q, bool up, double delta, std::vector<Shif
       double dp = 1.0;
       for (int e = 0; e < ex + ey + ez; ++e) dp *= delta;
       ShiftTerm x;
-      memset(&x, 0, sizeof(x));
       x.w = w * dp;
-      x.s = (uint16_t)s;
-      x.ex = (uint8_t)ex;
-      x.ey = (uint8_t)ey;
-      x.ez = (uint8_t)ez;
-      t.push_back(x);
+      x.q = (ex & 1) | (ey & 1) << 1 | (ez & 1) << 2;
+      x.at = 3 * s + (up ? 0 : x.q * w3);
+      cls[up ? x.q : 0].push_back(x);
     }
-    off.push_back((int)t.size());
+    for (int c = 0; c < (up ? 8 : 1); ++c) {
+      t.insert(t.end(), cls[c].begin(), cls[c].end());
+      off.push_back((int)t.size());
+    }
   }
 }
 
@@ -864,61 +859,6 @@ __global__ void k_m2l(FmmDev d, int l, uint32_t act_lo) {
       double *b = d.B + (size_t)ci * 3 * nm;
       for (int e = 0; e < 3; ++e) b[3 * mo + e] += sc * acc[e];
     }
-  }
-}
-
-// L2L (mod_multipole.f90:360-384) into the active cells of level l from
-// their parents: b truncated at degree p, g at degree p+1.
-__global__ void k_l2l(FmmDev d, int l, uint32_t act_lo) {
-  uint32_t ci = act_lo + blockIdx.x;
-  uint32_t key = d.act_key[ci];
-  uint32_t pkey = key >> 3;
-  uint32_t pc = d.cidx[d.G.lev_off[l - 1] + pkey];
-  int i, j, k, pi_, pj, pk;
-  cart_of_key(d.G, l, key, i, j, k);
-  cart_of_key(d.G, l - 1, pkey, pi_, pj, pk);
-  double c[3], cp[3];
-  cell_center(d.G, l, i, j, k, c);
-  cell_center(d.G, l - 1, pi_, pj, pk, cp);
-  double dx = c[0] - cp[0], dy = c[1] - cp[1], dz = c[2] - cp[2];
-  int m = threadIdx.x;
-  int p = d.p;
-  if (m < d.nm) {
-    int mi, mj, mk;
-    mono_exp(m, mi, mj, mk);
-    const double *bp = d.B + (size_t)pc * 3 * d.nm;
-    double acc[3] = {0, 0, 0};
-    for (int ks = mk; ks <= p; ++ks)
-      for (int js = mj; js <= p - ks; ++js)
-        for (int is = mi; is <= p - ks - js; ++is) {
-          int s = mono_idx(is, js, ks);
-          double w = binom_d(is, mi) * binom_d(js, mj) * binom_d(ks, mk) *
-                     (ipow_d(dx, is - mi) * ipow_d(dy, js - mj) * ipow_d(dz, ks - mk));
-          acc[0] += w * bp[3 * s];
-          acc[1] += w * bp[3 * s + 1];
-          acc[2] += w * bp[3 * s + 2];
-        }
-    double *b = d.B + (size_t)ci * 3 * d.nm;
-    for (int e = 0; e < 3; ++e) b[3 * m + e] += acc[e];
-  }
-  if (d.use_vs && m < d.nm1) {
-    int mi, mj, mk;
-    mono_exp(m, mi, mj, mk);
-    const double *gp = d.Gx + (size_t)pc * 3 * d.nm1;
-    double acc[3] = {0, 0, 0};
-    int q = p + 1;
-    for (int ks = mk; ks <= q; ++ks)
-      for (int js = mj; js <= q - ks; ++js)
-        for (int is = mi; is <= q - ks - js; ++is) {
-          int s = mono_idx(is, js, ks);
-          double w = binom_d(is, mi) * binom_d(js, mj) * binom_d(ks, mk) *
-                     (ipow_d(dx, is - mi) * ipow_d(dy, js - mj) * ipow_d(dz, ks - mk));
-          acc[0] += w * gp[3 * s];
-          acc[1] += w * gp[3 * s + 1];
-          acc[2] += w * gp[3 * s + 2];
-        }
-    double *g = d.Gx + (size_t)ci * 3 * d.nm1;
-    for (int e = 0; e < 3; ++e) g[3 * m + e] += acc[e];
   }
 }
 
@@ -1571,8 +1511,10 @@ int fmm_prepare_device(dust_octree *o, int n, const double *cen, const double *d
   DUST_CUDA(cudaMemsetAsync(d.counters, 0, 4 * sizeof(int64_t), st));
   o->dev = d;
   DUST_TRY(m2l_prepare(o, d, st));
+  o->dev = d;
   if (o->n_leaves > 0) {
-    k_p2m<<<(unsigned)((o->n_leaves + P2M_W - 1) / P2M_W), P2M_W * 32, 0, st>>>(d);
+    const size_t shm = (size_t)P2M_W * (3 * (o->p + 1) + 3) * P2M_LD * 8;
+    k_p2m<<<(unsigned)((o->n_leaves + P2M_W - 1) / P2M_W), P2M_W * 32, shm, st>>>(d);
   }
   for (int l = ll - 1; l >= 1; --l) {
     int64_t na = o->act_off[l + 1] - o->act_off[l];
@@ -1588,7 +1530,6 @@ int fmm_prepare_device(dust_octree *o, int n, const double *cen, const double *d
                                                   (const int *)o->shift_o[l][0], nt);
     }
   }
-  DUST_TRY(m2l_scale_sources(o, d, st));
   if (o->timing) cudaEventRecord(o->ev[2], st);
   // downward pass: M2L of every level (level 1 per target, levels >= 2 in
   // one batched launch), then L2L level by level adds the parents' final
@@ -1605,13 +1546,14 @@ int fmm_prepare_device(dust_octree *o, int n, const double *cen, const double *d
     int64_t na = o->act_off[l + 1] - o->act_off[l];
     if (na <= 0) continue;
     const int ntb = o->shift_n[l][1], ntg = d.use_vs ? o->shift_n[l][2] : 0;
-    const size_t shm = (size_t)SH_W * 3 * (o->nm + (ntg > 0 ? o->nm1 : 0)) * 8 +
-                       (size_t)(ntb + ntg) * sizeof(ShiftTerm) + (size_t)(o->nm + o->nm1 + 2) * 4;
+    const int nmx = ntg > 0 ? o->nm1 : o->nm;
+    const size_t shm = (size_t)SH_W * 3 * nmx * 8 + (size_t)std::max(ntb, ntg) * sizeof(ShiftTerm) +
+                       (size_t)(8 * nmx + 1) * 4;
     if (shm > 48 * 1024)
       DUST_CUDA(cudaFuncSetAttribute(k_l2l_t, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)shm));
     const int64_t npar = o->act_off[l] - o->act_off[l - 1];
-    k_l2l_t<<<shift_grid(npar), SH_T, shm, st>>>(
+    k_l2l_t<<<dim3(shift_grid(npar), ntg > 0 ? 2 : 1), SH_T, shm, st>>>(
         d, l, (uint32_t)o->act_off[l - 1], (uint32_t)npar, (const ShiftTerm *)o->shift_t[l][1],
         (const int *)o->shift_o[l][1], ntb, (const ShiftTerm *)o->shift_t[l][2],
         (const int *)o->shift_o[l][2], ntg);

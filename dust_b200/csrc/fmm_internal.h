@@ -35,6 +35,9 @@ struct FmmDev {
   const uint32_t *leaf_ci;
   uint32_t n_leaves;
   double *A, *B, *Gx;  // multipole a, local b (deg p), local g (deg p+1)
+  double *ahat;        // scaled multipoles of the M2L sources, cells ahat_c0 .., rows of
+  uint32_t ahat_c0;    // ahat_rs (m2l.cu)
+  int ahat_rs;
   double *out;         // sorted-order vel(3), stretch(3), rotu(3), SoA
   int64_t *counters;   // [0] M2L pairs, [1] P2P pairs
   double inv_fact[224];
@@ -130,7 +133,6 @@ bool uvort_args_ok(const dust_fmm_params *prm, int n_pts, const double *pts, int
 int m2l_batch_tables(dust_octree *o);
 int m2l_prepare(dust_octree *o, FmmDev &d, cudaStream_t st);
 int m2l_all_levels(dust_octree *o, FmmDev &d, cudaStream_t st);
-int m2l_scale_sources(dust_octree *o, FmmDev &d, cudaStream_t st);
 
 
 // direct.cu

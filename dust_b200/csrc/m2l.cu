@@ -293,25 +293,6 @@ __global__ void __launch_bounds__((M2L_MAXW + 1) * 32)
   }
 }
 
-// ahat'(n) = a(n) / (n! h^|n|) for every active cell of levels >= 2, as
-// [cell][component][rs] with zeros beyond nm
-__global__ void k_scale_a(FmmDev d, uint32_t c0, uint32_t nact, int rs, double *out) {
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (size_t)(nact - c0) * 3 * rs) return;
-  const uint32_t ci = c0 + (uint32_t)(e / (3 * rs));
-  const int r = (int)(e % (3 * rs)), c = r / rs, nn = r - c * rs;
-  double v = 0.0;
-  if (nn < d.nm) {
-    int ni, nj, nk;
-    mono_exp(nn, ni, nj, nk);
-    const double hi = 1.0 / d.G.csize[d.act_lev[ci]];
-    double hp = 1.0;
-    for (int q = 0; q < ni + nj + nk; ++q) hp *= hi;
-    v = d.A[(size_t)ci * 3 * d.nm + 3 * nn + c] * d.inv_fact[nn] * hp;
-  }
-  out[e] = v;
-}
-
 // class keys of the active cells of levels >= 2: (level << 3 | key & 7) for
 // non-empty cells and for empty leaves that hold evaluation points, 0xff for
 // the other empty ones (dropped)
@@ -432,21 +413,13 @@ int m2l_prepare(dust_octree *o, FmmDev &d, cudaStream_t st) {
   DUST_CUDA(cudaStreamSynchronize(st));
   memcpy(o->m2l_cnt, h, sizeof(int) * 8 * (DUST_MAXLEV + 1));
   o->m2l_list = v_out;
-  // pre-scaled source coefficients of all active cells of levels >= 2
+  // scaled source coefficients of the active cells of levels >= 2, written by
+  // the upward pass beside the multipoles (put_multipole)
   DUST_TRY(devbuf_grow(o->ahat, (size_t)m * 3 * m2l_rs(4 * m2l_ks(o->p)) * 8 + 256));
   o->ahat_c0 = c0;
-  return DUST_OK;
-}
-
-// fills the pre-scaled coefficients once the upward pass is complete
-int m2l_scale_sources(dust_octree *o, FmmDev &d, cudaStream_t st) {
-  if (!o->m2l_list) return DUST_OK;
-  uint32_t c0 = o->ahat_c0, nact = (uint32_t)o->n_active;
-  const int rs = m2l_rs(4 * m2l_ks(o->p));
-  const size_t tot = (size_t)(nact - c0) * 3 * rs;
-  if (tot == 0) return DUST_OK;
-  k_scale_a<<<nblk(tot, 256), 256, 0, st>>>(d, c0, nact, rs, (double *)o->ahat.p);
-  DUST_CUDA(cudaGetLastError());
+  d.ahat = (double *)o->ahat.p;
+  d.ahat_c0 = c0;
+  d.ahat_rs = m2l_rs(4 * m2l_ks(o->p));
   return DUST_OK;
 }
 
