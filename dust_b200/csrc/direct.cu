@@ -567,6 +567,10 @@ __device__ __forceinline__ void line_vel_f(const double *vv, const float *q, con
   u[2] = f * cz;
 }
 
+// FP32: a thread per particle, the lines staged.  FP64: a warp per 32 particles
+// was bound by the latency of one line after the other (36 us for 3,000
+// particles, 232 us for 60,000), so four warps share the lines of the same 32
+// particles: 8 and 94 us.
 #define EL_T 128
 #define EL_TILE 64
 template <bool F32>
@@ -574,7 +578,8 @@ __global__ void __launch_bounds__(EL_T) k_elem_fin(FmmDev d, ElemDev e, const do
                                                    double *vel, double *str, double *rot) {
   __shared__ double s_v[EL_TILE][6];
   __shared__ float s_l[EL_TILE][6];
-  const uint32_t t0 = blockIdx.x * EL_T, t = t0 + threadIdx.x;
+  const int grp = threadIdx.x >> 5;  // FP64: a warp takes every fourth line
+  const uint32_t t = F32 ? blockIdx.x * EL_T + threadIdx.x : blockIdx.x * 32 + (threadIdx.x & 31);
   const size_t n = d.n;
   const bool act = t < n;
   double pos[3] = {0.0, 0.0, 0.0};
@@ -584,12 +589,20 @@ __global__ void __launch_bounds__(EL_T) k_elem_fin(FmmDev d, ElemDev e, const do
   double w[3] = {0.0, 0.0, 0.0};
   if (act)
     for (int c = 0; c < 3; ++c) w[c] = farv ? farv[(size_t)c * n + t] : 0.0;
-  if (!F32 && act)
-    for (int q = 0; q < e.nline; ++q) {
-      double u[3];
-      vel_line(e.rp, e.lines[q], pos, u);
-      for (int c = 0; c < 3; ++c) w[c] += u[c];
-    }
+  if (!F32 && e.nline > 0) {
+    double l[3] = {0.0, 0.0, 0.0};
+    if (act)
+      for (int q = grp; q < e.nline; q += EL_T / 32) {
+        double u[3];
+        vel_line_near(e.rp, e.lines[q], pos, u);
+        for (int c = 0; c < 3; ++c) l[c] += u[c];
+      }
+    double(*s_g)[3] = (double(*)[3])s_v;  // [128][3] of the 64 x 6 words
+    for (int c = 0; c < 3; ++c) s_g[threadIdx.x][c] = l[c];
+    __syncthreads();
+    for (int g = 0; g < EL_T / 32; ++g)
+      for (int c = 0; c < 3; ++c) w[c] += s_g[32 * g + (threadIdx.x & 31)][c];
+  }
   for (int q0 = 0; F32 && q0 < e.nline; q0 += EL_TILE) {
     const int m = min(EL_TILE, e.nline - q0);
     __syncthreads();
@@ -620,10 +633,14 @@ __global__ void __launch_bounds__(EL_T) k_elem_fin(FmmDev d, ElemDev e, const do
   if (!act) return;
   const double k4pi = 1.0 / (4.0 * DUST_PI);
   const uint32_t ip = d.perm[t];
+  // (FP64: an output each for the first three warps)
   for (int c = 0; c < 3; ++c) {
-    vel[3 * (size_t)ip + c] = d.out[(size_t)c * n + t] + w[c] * k4pi + d.u_inf[c];
-    if (str) str[3 * (size_t)ip + c] = (d.use_vs || d.use_vd) ? d.out[(size_t)(3 + c) * n + t] : 0.0;
-    if (rot) rot[3 * (size_t)ip + c] = (d.use_vs && d.use_df) ? d.out[(size_t)(6 + c) * n + t] : 0.0;
+    if (F32 || grp == 0)
+      vel[3 * (size_t)ip + c] = d.out[(size_t)c * n + t] + w[c] * k4pi + d.u_inf[c];
+    if (str && (F32 || grp == 1))
+      str[3 * (size_t)ip + c] = (d.use_vs || d.use_vd) ? d.out[(size_t)(3 + c) * n + t] : 0.0;
+    if (rot && (F32 || grp == 2))
+      rot[3 * (size_t)ip + c] = (d.use_vs && d.use_df) ? d.out[(size_t)(6 + c) * n + t] : 0.0;
   }
 }
 
@@ -688,7 +705,7 @@ int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
     if (f32)
       k_elem_fin<true><<<nblk(n, EL_T), EL_T, 0, st>>>(d, e, farv, vel, str, rot);
     else
-      k_elem_fin<false><<<nblk(n, EL_T), EL_T, 0, st>>>(d, e, farv, vel, str, rot);
+      k_elem_fin<false><<<nblk(n, 32), EL_T, 0, st>>>(d, e, farv, vel, str, rot);
   }
   DUST_CUDA(cudaGetLastError());
   return DUST_OK;

@@ -46,6 +46,8 @@ __host__ __device__ inline void d3cross(const double *a, const double *b, double
 }
 
 // calc_geo_data_surfpan / calc_geo_data_vortlatt from the vertices.
+// (every index is known at compile time, so that the device keeps the panel in
+// registers)
 __host__ __device__ inline void panel_build(const double *ver12, int nv, int kind,
                                             double mag, const double *ub,
                                             const double *uvort, const double *u_inf,
@@ -56,7 +58,8 @@ __host__ __device__ inline void panel_build(const double *ver12, int nv, int kin
     for (int d = 0; d < 3; ++d) p.ver[v][d] = ver12[3 * v + d];
   for (int d = 0; d < 3; ++d) {
     double s = 0.0;
-    for (int v = 0; v < nv; ++v) s += p.ver[v][d];
+    for (int v = 0; v < 4; ++v)
+      if (v < nv) s += p.ver[v][d];
     p.cen[d] = s / (double)nv;
   }
   double a[3], b[3], nor[3];
@@ -78,15 +81,16 @@ __host__ __device__ inline void panel_build(const double *ver12, int nv, int kin
   }
   for (int d = 0; d < 3; ++d) p.nor[d] = nor[d] / nn;
   double tanl[3];
-  for (int d = 0; d < 3; ++d) tanl[d] = 0.5 * (p.ver[nv - 1][d] + p.ver[0][d]) - p.cen[d];
+  for (int d = 0; d < 3; ++d)
+    tanl[d] = 0.5 * ((nv == 4 ? p.ver[3][d] : p.ver[2][d]) + p.ver[0][d]) - p.cen[d];
   double tn = sqrt(d3dot(tanl, tanl));
   for (int d = 0; d < 3; ++d) p.tang[0][d] = tanl[d] / tn;
   d3cross(p.nor, p.tang[0], p.tang[1]);
   p.max_edge = 0.0;
   for (int v = 0; v < 4; ++v) {
     if (v < nv) {
-      int vn = (v + 1) % nv;
-      for (int d = 0; d < 3; ++d) p.edge_vec[v][d] = p.ver[vn][d] - p.ver[v][d];
+      for (int d = 0; d < 3; ++d)
+        p.edge_vec[v][d] = (v + 1 < nv ? p.ver[(v + 1) & 3][d] : p.ver[0][d]) - p.ver[v][d];
       p.edge_len[v] = sqrt(d3dot(p.edge_vec[v], p.edge_vec[v]));
       if (v == 0 || p.edge_len[v] > p.max_edge) p.max_edge = p.edge_len[v];
       for (int d = 0; d < 3; ++d) p.edge_uni[v][d] = p.edge_vec[v][d] / p.edge_len[v];
@@ -336,6 +340,27 @@ __device__ __forceinline__ double near_rsqrt(double x) {
 __device__ __forceinline__ double near_rcp(double x) { return near_range(x) ? rcp_r(x) : 1.0 / x; }
 __device__ __forceinline__ double near_sqrt(double x, double irs) {
   return x > 0.0 ? x * irs : 0.0;
+}
+
+// vel_line with reciprocal distances instead of square roots and quotients,
+// the core test on squares
+__device__ inline void vel_line_near(const RegParams &rp, const LineGeo &l, const double *pos,
+                                     double *v) {
+  const double av[3] = {pos[0] - l.ver[0][0], pos[1] - l.ver[0][1], pos[2] - l.ver[0][2]};
+  const double bv[3] = {pos[0] - l.ver[1][0], pos[1] - l.ver[1][1], pos[2] - l.ver[1][2]};
+  const double ai = d3dot(av, l.edge_uni), L = l.edge_len, rr = rp.r_rankine * L;
+  const double qa = d3dot(av, av), qb = d3dot(bv, bv);
+  const double ia = near_rsqrt(qa), ib = near_rsqrt(qb);
+  double hv[3], cr[3];
+  for (int d = 0; d < 3; ++d) hv[d] = av[d] - ai * l.edge_uni[d];
+  const double hi2 = d3dot(hv, hv);
+  d3cross(l.edge_uni, hv, cr);
+  double f = 0.0;
+  if (hi2 > rr * rr)
+    f = ((L - ai) * ib + ai * ia) * near_rcp(hi2);
+  else if (near_sqrt(qa, ia) > L * rp.r_cutoff && near_sqrt(qb, ib) > L * rp.r_cutoff)
+    f = ((L - ai) * ib + ai * ia) * near_rcp(rr * rr);
+  for (int d = 0; d < 3; ++d) v[d] = f * cr[d] * l.mag;
 }
 
 // vel_pan for a point inside the panel's far-field radius, with the

@@ -383,3 +383,23 @@ def test_element_chunks_and_list_overflow(n, panels, prec):
     for _ in range(2):
         v, _, _ = oc.apply_multipole(cen, dir_, mag, rv, els)
         assert rel(v, ov) < (TOL64 if prec == abi.DUST_PREC_FP64 else TOL32)
+
+
+@pytest.mark.parametrize("p,vs,n_box", [(0, False, (3, 2, 2)), (4, True, (5, 1, 1)),
+                                        (8, True, (2, 2, 2)), (8, False, (2, 3, 1))])
+def test_fmm_level1_pairs_match_oracle(p, vs, n_box):
+    """Level-1 interactions: one to seven groups of outputs, sources shared
+    among as many warps as remain."""
+    rng = np.random.default_rng(p)
+    n = 400
+    cen = rng.uniform(0.02, 0.98, (n, 3)) * np.array(n_box)
+    dir_ = rng.standard_normal((n, 3))
+    dir_ /= np.linalg.norm(dir_, axis=1)[:, None]
+    mag, rv = rng.uniform(0.5e-3, 1.5e-3, n), np.full(n, 0.02)
+    prm = FmmParams(box_length=1.0, n_box=n_box, origin=(0, 0, 0), n_octree_levels=2,
+                    min_octree_part=2, multipole_degree=p, rankine_rad=0.02, vortstretch=vs)
+    ov, os_, orr, _ = O.fmm_apply(prm, cen, dir_, mag, rv)
+    v, s, r = octree.initialize_octree(prm).apply_multipole(cen, dir_, mag, rv)
+    assert rel(v, ov) < TOL64 and rel(s, os_) < TOL64
+    if vs:
+        assert rel(r, orr) < TOL64

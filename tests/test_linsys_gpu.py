@@ -240,3 +240,19 @@ def test_linsys_block_solve_matches_oracle(n_fus, n_span):
         res, rep = ls.solve_linsys(mode)
         assert rep["fell_back"] == 0
         assert np.linalg.norm(res - ro) < 1e-10 * np.linalg.norm(ro)
+
+
+@pytest.mark.parametrize("n_span,n_chord", [(1, 3), (16, 1), (31, 2), (33, 1), (50, 1)])
+@pytest.mark.parametrize("nst_frac", [1.0, 0.4])
+def test_linsys_wake_rows_ragged(n_span, n_chord, nst_frac):
+    """Wake panels around a warp's 32, implicit ones ending inside a group;
+    row counts around a CTA's eight."""
+    prm = FmmParams(u_inf=(1.0, 0.0, 0.0), rankine_rad=0.1)
+    wing, wk, n_impl, ind = wing_case(n_span, n_chord)
+    nst = int(wing.n * nst_frac)
+    Ao, bo, _ = O.linsys_run(prm, wing.n, nst, wing, wing, (wk, n_impl, ind), (wk, n_impl, ind))
+    ls = linsys.initialize_linsys(prm, wing.n, nst, wing, wk, n_impl, ind)
+    ls.assemble_linsys(wing, wk, n_impl, ind)
+    Ag, bg = ls.get_system()
+    assert rel(Ag, Ao) < 1e-10
+    assert rel(bg, bo) < 1e-10
