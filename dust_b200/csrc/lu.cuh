@@ -12,6 +12,30 @@
 #include "dust_common.cuh"
 #include "fmm_internal.h"
 
+// The second stream of the unpivoted factorisation, made at its first use and
+// owned by the work area (one factorisation at a time).
+struct LuSide {
+  cudaStream_t st = nullptr;
+  cudaEvent_t go = nullptr, done = nullptr;
+  int make() {
+    if (done) return DUST_OK;
+    int lo = 0, hi = 0;
+    DUST_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    if (!st) DUST_CUDA(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, hi));
+    if (!go) DUST_CUDA(cudaEventCreateWithFlags(&go, cudaEventDisableTiming));
+    DUST_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    return DUST_OK;
+  }
+  LuSide() = default;
+  LuSide(const LuSide &) = delete;
+  LuSide &operator=(const LuSide &) = delete;
+  ~LuSide() {
+    if (st) cudaStreamDestroy(st);
+    if (go) cudaEventDestroy(go);
+    if (done) cudaEventDestroy(done);
+  }
+};
+
 struct LuWork {
   DevBuf sync;   // barrier counters, error flag, partials, candidate rows
   DevBuf np;     // unpivoted LU: max |l| word, inverse triangles of every
@@ -19,6 +43,7 @@ struct LuWork {
   DevBuf inv;    // inverses of L's and U's larger diagonal blocks (lu_inv_build)
   int inv_n = 0; // order of the system they belong to (0: none)
   DevBuf np_x;   // lu_solve_blocks: the intermediate Y = L^-1 B
+  LuSide side;   // lu_getrf_nopiv: the next panel's stream
   int nsm = 0;
 };
 

@@ -19,13 +19,19 @@
 //                 its inverse triangles Linv (unit lower) and Uinv (upper) in
 //                 the same elimination, max |l| of the block;
 //     k_np_panel  L21 = A21 Uinv (row tiles, down to n) and U12 = Linv A12
-//                 (column tiles, inside the outer panel), 64 x 64
-//                 register-tiled products, max |l| of L21;
-//     update      of the outer panel's own columns;
-//   then the outer panel's U12 right of it (forward substitution over its
-//   blocks with Linv) and the trailing update A22 -= L21 U12 of inner
-//   dimension NP_NBO (tcgen05 TF32 GEMM for FP32, DGEMM for FP64), which
-//   streams the trailing matrix a quarter as often as NP_NB-wide steps.
+//                 (column tiles, inside the outer panel), max |l| of L21;
+//     k_np_inner  update of the outer panel's own columns;
+//   then k_np_cols, the outer panel's U12 right of it, and the trailing update
+//   A22 -= L21 U12 of inner dimension NP_NBO (tcgen05 TF32 GEMM for FP32, DGEMM
+//   for FP64), which streams the trailing matrix a quarter as often as
+//   NP_NB-wide steps.
+//
+// A panel is a chain of small kernels with one CTA at its core (four times 24 us
+// and more), the update fills the chip: the next panel's columns are
+// updated first and the panel factored on a second stream of high priority
+// under the update of the other columns.  Systems of up to two panels have
+// nothing to overlap and stay on the caller's stream.  n = 3,001 in
+// FP64: 4.54 -> 3.52 ms with the solve; n = 16,384 in FP32: 47.2 -> 42.0 ms.
 //
 // The largest |l| is kept as float bits (monotone for non-negative values)
 // with atomicMax.  The caller accepts the factors when it is below
@@ -34,6 +40,7 @@
 // diagonal); otherwise, and on a zero diagonal, it restores A and runs the
 // pivoted factorisation.  ipiv is the identity.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <type_traits>
 
@@ -51,7 +58,6 @@
 #define NP_NB 64
 #define NP_NBO 256  // outer panel width (a multiple of NP_NB)
 #define NP_T 256
-#define NP_LD (NP_NB + 1)
 
 __device__ __forceinline__ void np_note_lmax(unsigned *bits, float v) {
   atomicMax(bits, __float_as_uint(v));
@@ -62,73 +68,84 @@ __device__ __forceinline__ void np_note_lmax(unsigned *bits, float v) {
 __device__ __forceinline__ double np_rcp(double x) {
   return near_range(fabs(x)) ? rcp_r(x) : 1.0 / x;
 }
-__device__ __forceinline__ float np_rcp(float x) { return 1.0f / x; }
 
-// Diagonal block: LU and both inverse triangles in one block elimination.
-// Thread (ty, tx) holds the 4 x 4 piece of rows 4 ty .. and columns 4 tx .. of
-// W in registers, W = A at first.  A step takes four pivots Q = 4 q .. 4 q + 3:
-// rows R = W(Q,:) and columns C = W(:,Q) come through shared memory (two
-// buffers, so one barrier a step), every thread factors the 4 x 4 pivot block
-// W(Q,Q) = L_d U_d and inverts its triangles itself, and with R' = L_d^-1 R and
-// f = C U_d^-1
+// Diagonal block: LU and both inverse triangles in one block elimination, in
+// FP64 for either element type.  Warp i holds rows 8 i .. 8 i + 7 of W as eight
+// 8 x 8 accumulators of the FP64 tensor instruction, W = A at first.  A step
+// takes four pivots Q = 4 q .. 4 q + 3.  The warp that holds their rows R = W(Q,:)
+// factors W(Q,Q) = L_d U_d, inverts both triangles and leaves R' = L_d^-1 R in
+// shared memory; after the step's one barrier every warp forms f = W(:,Q) U_d^-1
+// of its rows, and with one instruction per tile
 //   rows below Q:  f is L; W(r,c) -= f R'_c for every c outside Q (right of Q
 //                  the elimination, left of it the row operations of Linv),
 //                  W(r,Q) = -f L_d^-1;
 //   rows above Q:  W(r,Q) = f, Uinv's columns; W(r,c) -= f R'_c right of Q;
 //   rows Q:        R' is U right of Q and Linv's rows left of it;
 //                  W(Q,c) = -U_d^-1 R'_c right of Q, W(Q,Q) the two inverses.
-// L and U leave for global memory as the steps produce them; at the end W
-// holds Linv below the diagonal and Uinv on and above it.  Bound by a step's
-// chain (barrier, shared memory, reciprocals, products): four pivots a step
-// (one: 57 us in FP64), the pivot block factored by every thread (by its owner
-// ahead of the step: 41 us), a warp on two column stripes so that one warp
-// walks the columns-Q branch (on two row stripes: 39 us).  It replaces a
-// column per thread, unrolled, and two dependent substitutions, whose code did
-// not stay in the instruction caches: FP32 47 -> 20 us, FP64 54 -> 37 us per
-// block (one CTA).
+// At the end W holds Linv below the diagonal and Uinv on and above it.  Bound by
+// the chain of a step: one warp's rows through shared memory, four dependent
+// reciprocals, R', barrier, f, the products.  (Rows and columns Q through shared
+// memory to a 4 x 4 piece per thread, every thread factoring the pivot block:
+// 160 FP64 instructions a warp and step instead of about 50, 37 us in FP64 and
+// 20 us in FP32 per block; 24 us in either now, 28 us beside an update.)
 #define NPD_T 256
+__device__ __forceinline__ void np_ld4(const double *s, double &a, double &b, double &c,
+                                       double &d) {
+  const double2 x = *(const double2 *)s, y = *(const double2 *)(s + 2);
+  a = x.x, b = x.y, c = y.x, d = y.y;
+}
+__device__ __forceinline__ void np_ld4(const float *s, float &a, float &b, float &c, float &d) {
+  const float4 x = *(const float4 *)s;
+  a = x.x, b = x.y, c = x.z, d = x.w;
+}
+__device__ __forceinline__ void np_st4(double *s, double a, double b, double c, double d) {
+  *(double2 *)s = make_double2(a, b);
+  *(double2 *)(s + 2) = make_double2(c, d);
+}
+__device__ __forceinline__ void np_st4(float *s, float a, float b, float c, float d) {
+  *(float4 *)s = make_float4(a, b, c, d);
+}
+
+__device__ __forceinline__ void np_dmma(double &c0, double &c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c0), "+d"(c1)
+      : "d"(a), "d"(b));
+}
+#define NPD_LD (NP_NB + 4)  // the four rows of a B operand in different banks
+
 template <typename T>
 __global__ void __launch_bounds__(NPD_T) k_np_diag(T *A, int lda, int k, int jb, T *Linv,
                                                    T *Uinv, unsigned *lmax_bits) {
-  __shared__ __align__(16) T s_row[2][4][NP_NB], s_col[2][4][NP_NB];
-  const int tid = threadIdx.x, tx = tid / 16, ty = tid % 16;
+  __shared__ __align__(16) double s_rp[NP_NB][NPD_LD];  // R' of every step, L_d below its diagonal
+  __shared__ __align__(16) double s_raw[4][NP_NB];
+  __shared__ __align__(16) double s_iu[2][4][4], s_il[2][4][4];
+  const int i = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   T *Ab = A + (size_t)k + (size_t)k * lda;
-  T w[4][4];
+  double w[8][2];
 #pragma unroll
-  for (int v = 0; v < 4; ++v)
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int r = 8 * i + g, c = 8 * j + 2 * t + e;
+      w[j][e] = (r < jb && c < jb) ? (double)Ab[(size_t)r + (size_t)c * lda] : (r == c ? 1.0 : 0.0);
+    }
+  if (threadIdx.x < 8) s_il[threadIdx.x & 1][0][threadIdx.x >> 1] = threadIdx.x < 2 ? 1.0 : 0.0;
+  float lm = 0.f;
+  // the pivot rows of step q, by the warp that holds them
+  auto pivots = [&](int q) {
+    if ((lane >> 4) == (q & 1)) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *(double2 *)&s_raw[g & 3][8 * j + 2 * t] = make_double2(w[j][0], w[j][1]);
+    }
+    __syncwarp();
+    double D[4][4], x[2][4], iu[4][4], il[4][4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int r = 4 * ty + u, c = 4 * tx + v;
-      w[u][v] = (r < jb && c < jb) ? Ab[(size_t)r + (size_t)c * lda] : (r == c ? (T)1 : (T)0);
+      np_ld4(&s_raw[u][4 * q], D[u][0], D[u][1], D[u][2], D[u][3]);
+      x[0][u] = s_raw[u][lane];
+      x[1][u] = s_raw[u][lane + 32];
     }
-  float lm = 0.f;
-  // (pivots beyond jb meet the identity and change nothing)
-#pragma unroll 1
-  for (int q = 0; 4 * q < jb; ++q) {
-    const int b = q & 1;
-    if (ty == q) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) s_row[b][u][4 * tx + v] = w[u][v];
-    }
-    if (tx == q) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) s_col[b][v][4 * ty + u] = w[u][v];
-    }
-    __syncthreads();
-    T D[4][4], R[4][4], f[4][4], iu[4][4], il[4][4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        D[u][v] = s_row[b][u][4 * q + v];
-        R[u][v] = s_row[b][u][4 * tx + v];
-        f[u][v] = s_col[b][v][4 * ty + u];
-      }
-    // D = L_d U_d in place; iu = U_d^-1, il = L_d^-1 (strictly lower part)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       iu[j][j] = np_rcp(D[j][j]);
@@ -137,179 +154,321 @@ __global__ void __launch_bounds__(NPD_T) k_np_diag(T *A, int lda, int k, int jb,
         D[r][j] *= iu[j][j];
 #pragma unroll
         for (int c = j + 1; c < 4; ++c) D[r][c] = fma(-D[r][j], D[j][c], D[r][c]);
+        x[0][r] = fma(-D[r][j], x[0][j], x[0][r]);
+        x[1][r] = fma(-D[r][j], x[1][j], x[1][r]);
       }
     }
 #pragma unroll
     for (int c = 1; c < 4; ++c)
 #pragma unroll
       for (int r = c - 1; r >= 0; --r) {
-        T x = D[r][c] * iu[c][c];
+        double y = D[r][c] * iu[c][c];
 #pragma unroll
-        for (int p = r + 1; p < c; ++p) x = fma(D[r][p], iu[p][c], x);
-        iu[r][c] = -x * iu[r][r];
+        for (int p = r + 1; p < c; ++p) y = fma(D[r][p], iu[p][c], y);
+        iu[r][c] = -y * iu[r][r];
+        iu[c][r] = 0.0;
       }
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 4; ++c) {
+      il[c][c] = 1.0;
 #pragma unroll
       for (int r = c + 1; r < 4; ++r) {
-        T x = D[r][c];
+        double y = D[r][c];
 #pragma unroll
-        for (int p = c + 1; p < r; ++p) x = fma(D[r][p], il[p][c], x);
-        il[r][c] = -x;
+        for (int p = c + 1; p < r; ++p) y = fma(D[r][p], il[p][c], y);
+        il[r][c] = -y;
+        il[c][r] = 0.0;
       }
-    // R' = L_d^-1 R and f = C U_d^-1
+    }
 #pragma unroll
-    for (int v = 0; v < 4; ++v)
+    for (int u = 0; u < 4; ++u) {
+      s_rp[4 * q + u][lane] = x[0][u];
+      s_rp[4 * q + u][lane + 32] = x[1][u];
+    }
+    if (lane == 0) {
 #pragma unroll
-      for (int r = 1; r < 4; ++r)
-#pragma unroll
-        for (int p = 0; p < r; ++p) R[r][v] = fma(-D[r][p], R[p][v], R[r][v]);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int c = 3; c >= 0; --c) {
-        T x = f[u][c] * iu[c][c];
-#pragma unroll
-        for (int p = 0; p < c; ++p) x = fma(f[u][p], iu[p][c], x);
-        f[u][c] = ty == q ? (u <= c ? iu[u][c] : (T)0) : x;
+      for (int u = 0; u < 4; ++u) {
+        np_st4(s_iu[q & 1][u], iu[u][0], iu[u][1], iu[u][2], iu[u][3]);
+        if (u > 0) np_st4(s_il[q & 1][u], il[u][0], il[u][1], il[u][2], il[u][3]);
       }
-    const bool right = tx > q, below = ty > q;
-    if (tx != q) {
-      if (ty == q) {
-        // U right of the pivots, Linv's rows left of them
+    }
+    __syncwarp();
+    if (lane == 0) {  // L_d, read at the end only
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+      for (int u = 1; u < 4; ++u)
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            if (right && 4 * tx + v < jb)
-              Ab[(size_t)(4 * q + u) + (size_t)(4 * tx + v) * lda] = R[u][v];
-            w[u][v] = right ? (T)0 : R[u][v];
-          }
+        for (int v = 0; v < u; ++v) s_rp[4 * q + u][4 * q + v] = D[u][v];
+    }
+  };
+  const int nq = (jb + 3) / 4;  // (pivots beyond jb meet the identity and change nothing)
+  if (i == 0) pivots(0);
+#pragma unroll 1
+  for (int q = 0; q < nq; ++q) {
+    __syncthreads();
+    const int iq = q >> 1, h = q & 1;
+    const double(*siu)[4] = s_iu[h], (*sil)[4] = s_il[h];
+    // the rows' values in columns Q, from the accumulators' layout
+    double v0 = w[0][0], v1 = w[0][1];
+#pragma unroll
+    for (int j = 1; j < 8; ++j)
+      if (j == iq) v0 = w[j][0], v1 = w[j][1];
+    const int from = (lane & ~3) + 2 * h;
+    const double c0 = __shfl_sync(~0u, v0, from), c1 = __shfl_sync(~0u, v1, from),
+                 c2 = __shfl_sync(~0u, v0, from + 1), c3 = __shfl_sync(~0u, v1, from + 1);
+    const double f = fma(c0, siu[0][t], c1 * siu[1][t]) + fma(c2, siu[2][t], c3 * siu[3][t]);
+    const bool rq = i == iq && (lane >> 4) == h;        // a pivot row
+    const bool lower = i > iq || (i == iq && h == 0);   // the warp has rows below Q
+    const double a = -(rq ? siu[g & 3][t] : f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (j < iq && !lower) continue;  // left of Q, no rows below it
+      double b = s_rp[4 * q + t][8 * j + g], d0 = w[j][0], d1 = w[j][1];
+      if (j == iq) {
+        if ((g >> 2) == h)
+          b = lower ? sil[t][g & 3] : (t == (g & 3) ? -1.0 : 0.0);
+        else if (h == 1 && !lower)
+          b = 0.0;
+        if ((t >> 1) == h) d0 = d1 = 0.0;
       }
-      if (below || right) {
+      if (rq && j >= iq) d0 = d1 = 0.0;
+      np_dmma(d0, d1, a, b);
+      w[j][0] = d0;
+      w[j][1] = d1;
+    }
+    if (q + 1 < nq && i == (q + 1) >> 1) pivots(q + 1);
+    // (what the next pivots do not wait for)
+    if (lower && !rq) {
+      const int r = 8 * i + g, c = 4 * q + t;
+      if (r < jb && c < jb) Ab[(size_t)r + (size_t)c * lda] = (T)f;
+      lm = fmaxf(lm, fabsf((float)f));
+    }
+    if (rq) {
+      // Linv's rows left of Q and the inverses of the pivot block
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) w[u][v] = fma(-f[u][p], R[p][v], w[u][v]);
-      }
-    } else {
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int r = 4 * ty + u, c = 4 * q + v;
-          T x = f[u][v];
-          if (below) {
-#pragma unroll
-            for (int p = v + 1; p < 4; ++p) x = fma(f[u][p], il[p][v], x);
-            x = -x;
-          }
-          if (ty == q && u > v) x = il[u][v];
-          w[u][v] = x;
-          if (r < jb && c < jb && (below || ty == q)) {
-            const T o = below ? f[u][v] : D[u][v];
-            Ab[(size_t)r + (size_t)c * lda] = o;
-            if (r > c) lm = fmaxf(lm, fabsf((float)o));
-            if (r == c && o == (T)0) lm = INFINITY;  // a zero pivot
-          }
+      for (int j = 0; j < 8; ++j)
+        if (j < iq || (j == iq && h == 1 && t < 2)) {
+          w[j][0] = s_rp[4 * q + (g & 3)][8 * j + 2 * t];
+          w[j][1] = s_rp[4 * q + (g & 3)][8 * j + 2 * t + 1];
+        } else if (j == iq && (t >> 1) == h) {
+          const int r = g & 3, c = (2 * t) & 3;
+          w[j][0] = r > c ? sil[r][c] : siu[r][c];
+          w[j][1] = r > c + 1 ? sil[r][c + 1] : siu[r][c + 1];
         }
     }
   }
+  __syncthreads();
+  for (int e = threadIdx.x; e < NP_NB * NP_NB; e += NPD_T) {
+    const int r = e % NP_NB, c = e / NP_NB;
+    if (r >= jb || c >= jb || c < (r & ~3)) continue;
+    const T o = (T)s_rp[r][c];
+    Ab[(size_t)r + (size_t)c * lda] = o;
+    if (r > c) lm = fmaxf(lm, fabsf((float)o));
+    if (r == c && o == (T)0) lm = INFINITY;  // a zero pivot
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int r = 8 * i + g, c = 8 * j + 2 * t + e;
+      if (r < jb && c < jb) {
+        Linv[r + (size_t)c * NP_NB] = r > c ? (T)w[j][e] : (r == c ? (T)1 : (T)0);
+        Uinv[r + (size_t)c * NP_NB] = r <= c ? (T)w[j][e] : (T)0;
+      }
+    }
   for (int o = 16; o > 0; o >>= 1) lm = fmaxf(lm, __shfl_xor_sync(0xffffffffu, lm, o));
-  if ((tid & 31) == 0) np_note_lmax(lmax_bits, lm);
+  if (lane == 0) np_note_lmax(lmax_bits, lm);
+}
+
+// 64 x 64 x 64 products of the panel kernels: acc = or -= L X with both operands
+// in shared memory by columns, L[p][r] (ld 64) and X[c][p] (ld 65); thread
+// (ty, tx) owns rows 4 ty .. and columns tx, tx + 16, ..: a warp's reads of L are
+// vectors at two places, those of X 16 columns of one row, without conflicts
+// (columns 4 tx ..: four-way).
+#define NP_XLD (NP_NB + 1)
+template <bool MINUS, typename T>
+__device__ __forceinline__ void np_tile(T (&acc)[4][4], const T *L, const T *X, int ty, int tx) {
+#pragma unroll 4
+  for (int p = 0; p < NP_NB; ++p) {
+    T l[4], x[4];
+    np_ld4(L + p * NP_NB + 4 * ty, l[0], l[1], l[2], l[3]);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) x[v] = X[(tx + 16 * v) * NP_XLD + p];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[u][v] = fma(MINUS ? -l[u] : l[u], x[v], acc[u][v]);
+  }
+}
+// a tile (nr x nc of it, zeros beyond) to a thread's registers, all loads in
+// flight together, and from there to shared memory with rows of ld words
+template <typename T>
+__device__ __forceinline__ void np_fetch(T (&v)[16], const T *G, int ld, int nr, int nc) {
+  const int r = threadIdx.x % NP_NB, c0 = threadIdx.x / NP_NB;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int c = c0 + 4 * q;
+    v[q] = (r < nr && c < nc) ? G[r + (size_t)c * ld] : (T)0;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void np_put(T *S, const T (&v)[16], int ld) {
+  const int r = threadIdx.x % NP_NB, c0 = threadIdx.x / NP_NB;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) S[(c0 + 4 * q) * ld + r] = v[q];
+}
+// the result through shared memory (X[c][p]'s place) back to A, coalesced
+template <typename T>
+__device__ __forceinline__ void np_keep(T *X, const T (&acc)[4][4], int ty, int tx) {
 #pragma unroll
   for (int v = 0; v < 4; ++v)
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int r = 4 * ty + u, c = 4 * tx + v;
-      if (r < jb && c < jb) {
-        Linv[r + (size_t)c * NP_NB] = r > c ? w[u][v] : (r == c ? (T)1 : (T)0);
-        Uinv[r + (size_t)c * NP_NB] = r <= c ? w[u][v] : (T)0;
-      }
-    }
+    for (int u = 0; u < 4; ++u) X[(tx + 16 * v) * NP_XLD + 4 * ty + u] = acc[u][v];
 }
+template <typename T>
+__device__ __forceinline__ void np_write(T *G, int ld, const T *X, int nr, int nc) {
+  const int r = threadIdx.x % NP_NB, c0 = threadIdx.x / NP_NB;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int c = c0 + 4 * q;
+    if (r < nr && c < nc) G[r + (size_t)c * ld] = X[c * NP_XLD + r];
+  }
+}
+#define NP_TILE(T) ((NP_NB * NP_NB + NP_NB * NP_XLD) * (int)sizeof(T))
 
 // 64 x 64 tiles of the panel: blocks [0, nrb) take 64 rows of A21 (rows
 // below the block, to n) and write A21 Uinv over them; blocks [nrb, nrb + ncb)
 // take 64 columns of A12 (rows of the block, columns [cbeg, cend)) and write
-// Linv A12.  Each thread computes a 4 x 4 piece of the tile from the two
-// shared operands (the tile and the inverse triangle).
+// Linv A12.
 template <typename T>
 __global__ void __launch_bounds__(NP_T) k_np_panel(T *A, int lda, int n, int k, int jb,
                                                    const T *Linv, const T *Uinv, int nrb,
                                                    int cbeg, int cend, unsigned *lmax_bits) {
   extern __shared__ __align__(16) unsigned char np_sm[];
-  T *x = (T *)np_sm;            // 64 x 64 operand tile, [row][col], ld NP_LD
-  T *w = x + NP_NB * NP_LD;     // 64 x 64 inverse, [row][col], ld NP_LD
-  const int tid = threadIdx.x;
+  T *L = (T *)np_sm, *X = L + NP_NB * NP_NB;
   const bool rows = (int)blockIdx.x < nrb;
   const int b = rows ? blockIdx.x : blockIdx.x - nrb;
   const int r0 = rows ? k + jb + NP_NB * b : k;      // first row of the tile in A
   const int c0 = rows ? k : cbeg + NP_NB * b;        // first column of the tile in A
   const int nr = rows ? min(NP_NB, n - r0) : jb;
   const int nc = rows ? jb : min(NP_NB, cend - c0);
-  const T *W = rows ? Uinv : Linv;
+  T *At = A + (size_t)r0 + (size_t)c0 * lda;
   {
-    // all of a thread's loads in flight together
-    constexpr int M = NP_NB * NP_NB / NP_T;
-    const int r = tid % NP_NB, cq = tid / NP_NB;
-    T xv[M], wv[M];
-#pragma unroll
-    for (int q = 0; q < M; ++q) {
-      const int c = cq + q * (NP_T / NP_NB);
-      xv[q] = (r < nr && c < nc) ? A[(size_t)(r0 + r) + (size_t)(c0 + c) * lda] : (T)0;
-      wv[q] = (r < jb && c < jb) ? W[r + (size_t)c * NP_NB] : (T)0;
-    }
-#pragma unroll
-    for (int q = 0; q < M; ++q) {
-      const int c = cq + q * (NP_T / NP_NB);
-      x[r * NP_LD + c] = xv[q];
-      w[r * NP_LD + c] = wv[q];
-    }
+    T av[16], wv[16];
+    np_fetch(av, At, lda, nr, nc);
+    np_fetch(wv, rows ? Uinv : Linv, NP_NB, jb, jb);
+    np_put(L, rows ? av : wv, NP_NB);
+    np_put(X, rows ? wv : av, NP_XLD);
   }
   __syncthreads();
-  // out = x w (rows) or w x (columns); thread (ty, tx) owns rows 4 ty .. and
-  // columns 4 tx ..
-  const int ty = tid / 16, tx = tid % 16;
-  T acc[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = (T)0;
-  const T *L = rows ? x : w, *R = rows ? w : x;
-#pragma unroll 4
-  for (int p = 0; p < NP_NB; ++p) {
-    T lv[4], rv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) lv[u] = L[(4 * ty + u) * NP_LD + p];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) rv[v] = R[p * NP_LD + 4 * tx + v];
+  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+  T acc[4][4] = {};
+  np_tile<false>(acc, L, X, ty, tx);
+  __syncthreads();
+  np_keep(X, acc, ty, tx);
+  __syncthreads();
+  np_write(At, lda, X, nr, nc);
+  if (rows) {
+    float lm = 0.f;  // (rows and columns beyond the tile are zero)
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] = fma(lv[u], rv[v], acc[u][v]);
-  }
-  // through shared memory back to A, coalesced along the columns
-  __syncthreads();
-  float lm = 0.f;
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int r = 4 * ty + u, c = 4 * tx + v;
-      x[r * NP_LD + c] = acc[u][v];
-      if (rows && r < nr && c < nc) lm = fmaxf(lm, (float)fabs((double)acc[u][v]));
-    }
-  __syncthreads();
-  for (int e = tid; e < NP_NB * NP_NB; e += NP_T) {
-    const int r = e % NP_NB, c = e / NP_NB;
-    if (r < nr && c < nc) A[(size_t)(r0 + r) + (size_t)(c0 + c) * lda] = x[r * NP_LD + c];
-  }
-  if (rows) {
+      for (int v = 0; v < 4; ++v) lm = fmaxf(lm, (float)fabs((double)acc[u][v]));
     for (int o = 16; o > 0; o >>= 1) lm = fmaxf(lm, __shfl_xor_sync(0xffffffffu, lm, o));
-    if ((tid & 31) == 0) np_note_lmax(lmax_bits, lm);
+    if ((threadIdx.x & 31) == 0) np_note_lmax(lmax_bits, lm);
+  }
+}
+
+// The outer panel's own update after block k: A(r, c) -= L21 U12 for the 64 x 64
+// tile blockIdx of the rows below the block and the panel's columns [c0, cend).
+template <typename T>
+__global__ void __launch_bounds__(NP_T) k_np_inner(T *A, int lda, int n, int k, int cend) {
+  extern __shared__ __align__(16) unsigned char np_sm[];
+  T *L = (T *)np_sm, *X = L + NP_NB * NP_NB;
+  const int r0 = k + NP_NB + NP_NB * blockIdx.x, c0 = k + NP_NB + NP_NB * blockIdx.y;
+  const int nr = min(NP_NB, n - r0), nc = min(NP_NB, cend - c0);
+  T *At = A + (size_t)r0 + (size_t)c0 * lda;
+  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+  T acc[4][4];
+  {
+    T av[16], wv[16];
+    np_fetch(av, A + (size_t)r0 + (size_t)k * lda, lda, nr, NP_NB);
+    np_fetch(wv, A + (size_t)k + (size_t)c0 * lda, lda, NP_NB, nc);
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int r = 4 * ty + u, c = tx + 16 * v;
+        acc[u][v] = (r < nr && c < nc) ? At[r + (size_t)c * lda] : (T)0;
+      }
+    np_put(L, av, NP_NB);
+    np_put(X, wv, NP_XLD);
+  }
+  __syncthreads();
+  np_tile<true>(acc, L, X, ty, tx);
+  __syncthreads();
+  np_keep(X, acc, ty, tx);
+  __syncthreads();
+  np_write(At, lda, X, nr, nc);
+}
+
+// U12 of an outer panel (columns K .. Ke, whole blocks) for 64 columns of the
+// trailing matrix per CTA: forward substitution over the panel's blocks,
+//   X_b = Linv_b (A_b - sum_{j < b} L_bj X_j),
+// with the X_j staying in shared memory and each operand fetched under the
+// product before it.  (A launch and a pass over the rows for each block and each
+// update between them, before.)
+template <typename T>
+__global__ void __launch_bounds__(NP_T) k_np_cols(T *A, int lda, int n, int K, int Ke,
+                                                  const T *inv0) {
+  extern __shared__ __align__(16) unsigned char np_sm[];
+  T *L = (T *)np_sm, *X = L + NP_NB * NP_NB;  // X: NP_NBO / NP_NB tiles
+  const int c0 = Ke + NP_NB * blockIdx.x, nc = min(NP_NB, n - c0), nb = (Ke - K) / NP_NB;
+  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+  const size_t tri = (size_t)NP_NB * NP_NB;
+  T op[16];
+  np_fetch(op, inv0 + 2 * tri * (size_t)(K / NP_NB), NP_NB, NP_NB, NP_NB);
+  for (int b = 0; b < nb; ++b) {
+    T *Ab = A + (size_t)(K + NP_NB * b) + (size_t)c0 * lda;
+    T *Xb = X + (size_t)b * NP_NB * NP_XLD;
+    T acc[4][4];
+    {
+      T av[16];
+      np_fetch(av, Ab, lda, NP_NB, nc);
+      np_put(Xb, av, NP_XLD);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[u][v] = Xb[(tx + 16 * v) * NP_XLD + 4 * ty + u];
+    for (int j = 0; j <= b; ++j) {
+      // op: L_bj, at the end Linv_b; the next one: L_b,j+1, Linv_b or L_b+1,0
+      __syncthreads();
+      np_put(L, op, NP_NB);
+      if (j == b) np_keep(Xb, acc, ty, tx);
+      __syncthreads();
+      const int jn = j < b ? j + 1 : 0, bn = j < b ? b : b + 1;
+      if (bn < nb) {
+        if (jn < bn)
+          np_fetch(op, A + (size_t)(K + NP_NB * bn) + (size_t)(K + NP_NB * jn) * lda, lda, NP_NB,
+                   NP_NB);
+        else
+          np_fetch(op, inv0 + 2 * tri * (size_t)(K / NP_NB + bn), NP_NB, NP_NB, NP_NB);
+      }
+      if (j < b) {
+        np_tile<true>(acc, L, X + (size_t)j * NP_NB * NP_XLD, ty, tx);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) acc[u][v] = (T)0;
+        np_tile<false>(acc, L, Xb, ty, tx);
+      }
+    }
+    __syncthreads();
+    np_keep(Xb, acc, ty, tx);
+    __syncthreads();
+    np_write(Ab, lda, Xb, NP_NB, nc);
   }
 }
 
@@ -351,12 +510,16 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
   unsigned *bits = (unsigned *)w.np.p;
   T *inv0 = (T *)((char *)w.np.p + 256);
   DUST_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned), st));
-  const int smp = 2 * NP_NB * NP_LD * (int)sizeof(T);
-  static bool attr = false;  // per element type
+  const int smp = NP_TILE(T);
+  const int smc = (NP_NB * NP_NB + NP_NBO * NP_XLD) * (int)sizeof(T);
+  static std::atomic<bool> attr{false};  // per element type
   if (!attr) {
     DUST_CUDA(cudaFuncSetAttribute(k_np_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp));
+    DUST_CUDA(cudaFuncSetAttribute(k_np_inner<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp));
+    DUST_CUDA(cudaFuncSetAttribute(k_np_cols<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smc));
     attr = true;
   }
+  if (n > 2 * NP_NBO) DUST_TRY(w.side.make());
   CUBLAS_CHECK(cublasSetStream(cb, st));
   // C -= A B (m x nn, inner kk) on the tensor cores (FP32) or DGEMM
   auto update = [&](int m, int nn, int kk, const T *Am, const T *Bm, T *Cm) -> int {
@@ -368,32 +531,40 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
     return DUST_OK;
   };
   auto at = [&](int r, int c) { return A + r + (size_t)c * lda; };
-  // two levels: outer panels of NP_NBO columns factored in NP_NB steps that
-  // update only the panel's own columns; then the panel's U12 (its unit lower
-  // block's forward substitution, with the kept inverse triangles) and one
-  // trailing update of inner dimension NP_NBO
-  for (int K = 0; K < n; K += NP_NBO) {
+  // two levels: an outer panel of NP_NBO columns is factored in NP_NB steps that
+  // update only the panel's own columns
+  auto panel = [&](int K, cudaStream_t s) {
     const int Ke = std::min(K + NP_NBO, n);
     for (int k = K; k < Ke; k += NP_NB) {
       const int jb = std::min(NP_NB, n - k), m2 = n - k - jb, wc = Ke - k - jb;
       T *Linv = inv0 + 2 * tri * (size_t)(k / NP_NB), *Uinv = Linv + tri;
-      k_np_diag<T><<<1, NPD_T, 0, st>>>(A, lda, k, jb, Linv, Uinv, bits);
+      k_np_diag<T><<<1, NPD_T, 0, s>>>(A, lda, k, jb, Linv, Uinv, bits);
       const int nrb = (m2 + NP_NB - 1) / NP_NB, ncb = (wc + NP_NB - 1) / NP_NB;
       if (nrb + ncb > 0)
-        k_np_panel<T><<<nrb + ncb, NP_T, smp, st>>>(A, lda, n, k, jb, Linv, Uinv, nrb, k + jb,
-                                                     Ke, bits);
-      DUST_TRY(update(m2, wc, jb, at(k + jb, k), at(k, k + jb), at(k + jb, k + jb)));
+        k_np_panel<T><<<nrb + ncb, NP_T, smp, s>>>(A, lda, n, k, jb, Linv, Uinv, nrb, k + jb, Ke,
+                                                    bits);
+      if (nrb > 0 && ncb > 0) k_np_inner<T><<<dim3(nrb, ncb), NP_T, smp, s>>>(A, lda, n, k, Ke);
     }
-    if (Ke < n) {
-      const int ncb = (n - Ke + NP_NB - 1) / NP_NB;
-      for (int k = K; k < Ke; k += NP_NB) {
-        const T *Linv = inv0 + 2 * tri * (size_t)(k / NP_NB);
-        k_np_panel<T><<<ncb, NP_T, smp, st>>>(A, lda, n, k, NP_NB, Linv, Linv, 0, Ke, n, bits);
-        DUST_TRY(update(Ke - k - NP_NB, n - Ke, NP_NB, at(k + NP_NB, k), at(k, Ke),
-                        at(k + NP_NB, Ke)));
-      }
-      DUST_TRY(update(n - Ke, n - Ke, Ke - K, at(Ke, K), at(K, Ke), at(Ke, Ke)));
+  };
+  // Then the panel's U12 right of it and the trailing update, the next panel's
+  // columns first: that panel, a chain of small kernels, is factored on a second
+  // stream under the update of the rest.
+  panel(0, st);
+  for (int K = 0; K + NP_NBO < n; K += NP_NBO) {
+    const int Ke = K + NP_NBO, Kn = std::min(Ke + NP_NBO, n);
+    k_np_cols<T><<<(n - Ke + NP_NB - 1) / NP_NB, NP_T, smc, st>>>(A, lda, n, K, Ke, inv0);
+    DUST_TRY(update(n - Ke, Kn - Ke, NP_NBO, at(Ke, K), at(K, Ke), at(Ke, Ke)));
+    if (Kn == n) {
+      panel(Ke, st);
+      break;
     }
+    DUST_CUDA(cudaEventRecord(w.side.go, st));
+    DUST_CUDA(cudaStreamWaitEvent(w.side.st, w.side.go, 0));
+    panel(Ke, w.side.st);
+    DUST_CUDA(cudaEventRecord(w.side.done, w.side.st));
+    const int s = update(n - Ke, n - Kn, NP_NBO, at(Ke, K), at(K, Kn), at(Ke, Kn));
+    DUST_CUDA(cudaStreamWaitEvent(st, w.side.done, 0));  // joined whatever s is
+    DUST_TRY(s);
   }
   if (ipiv) k_np_ipiv<<<(n + 255) / 256, 256, 0, st>>>(n, ipiv);
   if (perm) k_np_iota<<<(n + 255) / 256, 256, 0, st>>>(n, perm);
