@@ -25,22 +25,53 @@
 static inline int ti_blocks(int n) { return (n + TI_B - 1) / TI_B; }
 
 // ------------------------------------------------------------ 64 x 64 products
-// acc (4 x 4 per thread, rows 4 ty .., columns 4 tx ..) += A(:, k0 .. k1) B(k0 ..
+// acc (4 x TN per thread, rows 4 ty .., columns TN tx ..) += A(:, k0 .. k1) B(k0 ..
 // k1, :) of column-major operands; mr / nc valid rows and columns.  The next
-// slice is loaded into registers while this one is multiplied.
+// slice is loaded into registers while this one is multiplied.  Bound by shared
+// memory if it is read word by word (eight reads, half of them in two-way
+// conflicts, for 16 products: a quarter of the FP32 rate), so operands are read
+// and B's slice is stored as vectors of four: NNN.
 template <typename T, int TN>
 struct TiSmem {
-  T a[TI_K][TI_T + 4];
-  T b[TI_K][16 * TN + 4];
+  alignas(16) T a[TI_K][TI_T + 4];
+  alignas(16) T b[TI_K][16 * TN + 4];
 };
+__device__ __forceinline__ void ti_ld(const float *s, float (&v)[4]) {
+  const float4 x = *(const float4 *)s;
+  v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+}
+__device__ __forceinline__ void ti_ld(const double *s, double (&v)[4]) {
+  const double2 x = *(const double2 *)s, y = *(const double2 *)(s + 2);
+  v[0] = x.x, v[1] = x.y, v[2] = y.x, v[3] = y.y;
+}
+__device__ __forceinline__ void ti_ld(const float *s, float (&v)[2]) {
+  const float2 x = *(const float2 *)s;
+  v[0] = x.x, v[1] = x.y;
+}
+__device__ __forceinline__ void ti_ld(const double *s, double (&v)[2]) {
+  const double2 x = *(const double2 *)s;
+  v[0] = x.x, v[1] = x.y;
+}
+template <typename T>
+__device__ __forceinline__ void ti_ld(const T *s, T (&v)[1]) {
+  v[0] = *s;
+}
+__device__ __forceinline__ void ti_st(float *s, const float *v) {
+  *(float4 *)s = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void ti_st(double *s, const double *v) {
+  *(double2 *)s = make_double2(v[0], v[1]);
+  *(double2 *)(s + 2) = make_double2(v[2], v[3]);
+}
 
 template <typename T, int TN>
 __device__ __forceinline__ void ti_mm(TiSmem<T, TN> &s, const T *A, int lda, int mr, const T *B,
                                       int ldb, int nc, int k0, int k1, T (&acc)[4][TN]) {
-  constexpr int NA = TI_K * TI_T / TI_NT, NBV = TI_K * 16 * TN / TI_NT;
+  // B: a thread takes four columns of one k (TN = 1: half of the threads)
+  constexpr int NA = TI_K * TI_T / TI_NT, NG = (4 * TN + 7) / 8;
   const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
-  const int ar = tid % TI_T, ak = tid / TI_T, bk = tid % TI_K, bc = tid / TI_K;
-  T av[NA], bv[NBV];
+  const int ar = tid % TI_T, ak = tid / TI_T, bk = tid % TI_K, bc = 4 * (tid / TI_K);
+  T av[NA], bv[NG][4];
   auto fetch = [&](int k) {
 #pragma unroll
     for (int q = 0; q < NA; ++q) {
@@ -48,10 +79,14 @@ __device__ __forceinline__ void ti_mm(TiSmem<T, TN> &s, const T *A, int lda, int
       av[q] = (ar < mr && kk < k1) ? A[(size_t)ar + (size_t)kk * lda] : (T)0;
     }
 #pragma unroll
-    for (int q = 0; q < NBV; ++q) {
-      const int c = bc + q * (TI_NT / TI_K);
-      bv[q] = (c < nc && k + bk < k1) ? B[(size_t)(k + bk) + (size_t)c * ldb] : (T)0;
-    }
+    for (int q = 0; q < NG; ++q)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int c = bc + 32 * q + v;
+        bv[q][v] = (c < nc && c < 16 * TN && k + bk < k1)
+                       ? B[(size_t)(k + bk) + (size_t)c * ldb]
+                       : (T)0;
+      }
   };
   fetch(k0);
   for (int k = k0; k < k1; k += TI_K) {
@@ -59,16 +94,15 @@ __device__ __forceinline__ void ti_mm(TiSmem<T, TN> &s, const T *A, int lda, int
 #pragma unroll
     for (int q = 0; q < NA; ++q) s.a[ak + q * (TI_NT / TI_T)][ar] = av[q];
 #pragma unroll
-    for (int q = 0; q < NBV; ++q) s.b[bk][bc + q * (TI_NT / TI_K)] = bv[q];
+    for (int q = 0; q < NG; ++q)
+      if (bc + 32 * q < 16 * TN) ti_st(&s.b[bk][bc + 32 * q], bv[q]);
     __syncthreads();
     if (k + TI_K < k1) fetch(k + TI_K);
 #pragma unroll 8
     for (int p = 0; p < TI_K; ++p) {
       T x[4], y[TN];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) x[u] = s.a[p][4 * ty + u];
-#pragma unroll
-      for (int v = 0; v < TN; ++v) y[v] = s.b[p][TN * tx + v];
+      ti_ld(&s.a[p][4 * ty], x);
+      ti_ld(&s.b[p][TN * tx], y);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -201,10 +235,22 @@ __global__ void __launch_bounds__(TI_NT) k_ti_gemm(int m, int nr, int k, T alpha
   int k0 = blockIdx.z * kshare, k1 = min(k, k0 + kshare);
   if (TRI == 1) k1 = min(k1, r0 + TI_T);
   if (TRI == 2) k0 = max(k0, r0);
-  T acc[4][TN] = {};
+  const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16, Z = gridDim.z;
+  T acc[4][TN] = {}, old[4][TN];
+  // C's values, all loads in flight together and, without shares, under the
+  // product (added one after the other they took longer than the product)
+  auto fetch_c = [&]() {
+#pragma unroll
+    for (int v = 0; v < TN; ++v)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int r = r0 + 4 * ty + u, c = c0 + TN * tx + v;
+        old[u][v] = (r < m && c < nr) ? C[(size_t)r + (size_t)c * ldc] : (T)0;
+      }
+  };
+  if (Z == 1) fetch_c();
   if (k0 < k1)
     ti_mm<T, TN>(sm, A + r0, lda, m - r0, B + (size_t)c0 * ldb, ldb, nr - c0, k0, k1, acc);
-  const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16, Z = gridDim.z;
   if (Z > 1) {
     const int tile = blockIdx.x + gridDim.x * blockIdx.y;
     T *mine = P.part + ((size_t)tile * Z + blockIdx.z) * 4096 + tid;
@@ -213,11 +259,13 @@ __global__ void __launch_bounds__(TI_NT) k_ti_gemm(int m, int nr, int k, T alpha
 #pragma unroll
       for (int v = 0; v < TN; ++v) __stcg(mine + TI_NT * (TN * u + v), acc[u][v]);
     if (!ti_last(P.arrived + tile, Z)) return;
+    fetch_c();
     const T *all = P.part + (size_t)tile * Z * 4096 + tid;
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
       for (int v = 0; v < TN; ++v) acc[u][v] = __ldcg(all + TI_NT * (TN * u + v));
+#pragma unroll 2
     for (int z = 1; z < Z; ++z)
 #pragma unroll
       for (int u = 0; u < 4; ++u)
@@ -230,7 +278,7 @@ __global__ void __launch_bounds__(TI_NT) k_ti_gemm(int m, int nr, int k, T alpha
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int r = r0 + 4 * ty + u, c = c0 + TN * tx + v;
-      if (r < m && c < nr) C[(size_t)r + (size_t)c * ldc] += alpha * acc[u][v];
+      if (r < m && c < nr) C[(size_t)r + (size_t)c * ldc] = old[u][v] + alpha * acc[u][v];
     }
 }
 
