@@ -411,43 +411,59 @@ __global__ void __launch_bounds__(NP_T) k_np_inner(T *A, int lda, int n, int k, 
   np_write(At, lda, X, nr, nc);
 }
 
-// U12 of an outer panel (columns K .. Ke, whole blocks) for 64 columns of the
+// U12 of an outer panel (columns K .. Ke, whole blocks) for NC columns of the
 // trailing matrix per CTA: forward substitution over the panel's blocks,
 //   X_b = Linv_b (A_b - sum_{j < b} L_bj X_j),
-// with the X_j staying in shared memory and each operand fetched under the
-// product before it.  (A launch and a pass over the rows for each block and each
-// update between them, before.)
-template <typename T>
+// products by the FP64 tensor instruction (a warp: 8 rows, all NC columns), the
+// X_j staying in shared memory, the next operand and the next block's values
+// fetched under a product.  It stands between a panel and everything after it,
+// so NC is small: 16, or 32 from two waves of SMs on.  (A launch per block and
+// per update between them: 10 and 8 us each, seven in all; 64 columns and 4 x 4
+// per thread: 56 us in FP64, 40 us in FP32.  17 us for 2,700 columns, 40 for
+// 12,000; 64 columns there: 74, 16: 44.)
+#define NPC_LD (NP_NB + 4)  // words: the reads of a half warp in different banks
+template <typename T, int NC>
 __global__ void __launch_bounds__(NP_T) k_np_cols(T *A, int lda, int n, int K, int Ke,
                                                   const T *inv0) {
   extern __shared__ __align__(16) unsigned char np_sm[];
-  T *L = (T *)np_sm, *X = L + NP_NB * NP_NB;  // X: NP_NBO / NP_NB tiles
-  const int c0 = Ke + NP_NB * blockIdx.x, nc = min(NP_NB, n - c0), nb = (Ke - K) / NP_NB;
-  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+  double *L = (double *)np_sm, *X = L + NP_NB * NPC_LD;  // X: a tile per block, by columns
+  const int i = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int c0 = Ke + NC * blockIdx.x, nb = (Ke - K) / NP_NB, r = 8 * i + g;
   const size_t tri = (size_t)NP_NB * NP_NB;
-  T op[16];
+  T op[16], nx[NC / 8][2];
+  auto block = [&](int b) {
+#pragma unroll
+    for (int j = 0; j < NC / 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + 8 * j + 2 * t + e;
+        nx[j][e] = c < n ? A[(size_t)(K + NP_NB * b + r) + (size_t)c * lda] : (T)0;
+      }
+  };
   np_fetch(op, inv0 + 2 * tri * (size_t)(K / NP_NB), NP_NB, NP_NB, NP_NB);
+  block(0);
   for (int b = 0; b < nb; ++b) {
-    T *Ab = A + (size_t)(K + NP_NB * b) + (size_t)c0 * lda;
-    T *Xb = X + (size_t)b * NP_NB * NP_XLD;
-    T acc[4][4];
-    {
-      T av[16];
-      np_fetch(av, Ab, lda, NP_NB, nc);
-      np_put(Xb, av, NP_XLD);
-    }
-    __syncthreads();
+    double *Xb = X + (size_t)b * NC * NPC_LD;
+    double acc[NC / 8][2];
 #pragma unroll
-    for (int v = 0; v < 4; ++v)
+    for (int j = 0; j < NC / 8; ++j) acc[j][0] = (double)nx[j][0], acc[j][1] = (double)nx[j][1];
+    if (b + 1 < nb) block(b + 1);
+    for (int jb = 0; jb <= b; ++jb) {
+      // op: L_b,jb, at the end Linv_b; the next one: L_b,jb+1, Linv_b or L_b+1,0
+      __syncthreads();
+      {
+        const int lr = threadIdx.x % NP_NB, lc = threadIdx.x / NP_NB;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) acc[u][v] = Xb[(tx + 16 * v) * NP_XLD + 4 * ty + u];
-    for (int j = 0; j <= b; ++j) {
-      // op: L_bj, at the end Linv_b; the next one: L_b,j+1, Linv_b or L_b+1,0
+        for (int q = 0; q < 16; ++q) L[(lc + 4 * q) * NPC_LD + lr] = (double)op[q];
+      }
+      if (jb == b) {
+#pragma unroll
+        for (int j = 0; j < NC / 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) Xb[(8 * j + 2 * t + e) * NPC_LD + r] = acc[j][e];
+      }
       __syncthreads();
-      np_put(L, op, NP_NB);
-      if (j == b) np_keep(Xb, acc, ty, tx);
-      __syncthreads();
-      const int jn = j < b ? j + 1 : 0, bn = j < b ? b : b + 1;
+      const int jn = jb < b ? jb + 1 : 0, bn = jb < b ? b : b + 1;
       if (bn < nb) {
         if (jn < bn)
           np_fetch(op, A + (size_t)(K + NP_NB * bn) + (size_t)(K + NP_NB * jn) * lda, lda, NP_NB,
@@ -455,21 +471,40 @@ __global__ void __launch_bounds__(NP_T) k_np_cols(T *A, int lda, int n, int K, i
         else
           np_fetch(op, inv0 + 2 * tri * (size_t)(K / NP_NB + bn), NP_NB, NP_NB, NP_NB);
       }
-      if (j < b) {
-        np_tile<true>(acc, L, X + (size_t)j * NP_NB * NP_XLD, ty, tx);
-      } else {
+      const double sign = jb < b ? -1.0 : 1.0, *Xj = X + (size_t)jb * NC * NPC_LD;
+      if (jb == b) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int j = 0; j < NC / 8; ++j) acc[j][0] = acc[j][1] = 0.0;
+      }
+#pragma unroll 4
+      for (int p = 0; p < NP_NB; p += 4) {
+        const double a = sign * L[(p + t) * NPC_LD + r];
 #pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u][v] = (T)0;
-        np_tile<false>(acc, L, Xb, ty, tx);
+        for (int j = 0; j < NC / 8; ++j)
+          np_dmma(acc[j][0], acc[j][1], a, Xj[(8 * j + g) * NPC_LD + p + t]);
       }
     }
     __syncthreads();
-    np_keep(Xb, acc, ty, tx);
-    __syncthreads();
-    np_write(Ab, lda, Xb, NP_NB, nc);
+#pragma unroll
+    for (int j = 0; j < NC / 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = 8 * j + 2 * t + e;
+        Xb[c * NPC_LD + r] = acc[j][e];
+        if (c0 + c < n)
+          A[(size_t)(K + NP_NB * b + r) + (size_t)(c0 + c) * lda] = (T)acc[j][e];
+      }
   }
+}
+template <typename T, int NC>
+static void np_cols(cudaStream_t st, T *A, int lda, int n, int K, int Ke, const T *inv0) {
+  const int smem = (NP_NB + NP_NBO / NP_NB * NC) * NPC_LD * 8;
+  static std::atomic<bool> attr{false};  // per instance
+  if (!attr) {
+    cudaFuncSetAttribute(k_np_cols<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    attr = true;
+  }
+  k_np_cols<T, NC><<<(n - Ke + NC - 1) / NC, NP_T, smem, st>>>(A, lda, n, K, Ke, inv0);
 }
 
 __global__ void k_np_ipiv(int n, int *ipiv) {
@@ -511,12 +546,10 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
   T *inv0 = (T *)((char *)w.np.p + 256);
   DUST_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned), st));
   const int smp = NP_TILE(T);
-  const int smc = (NP_NB * NP_NB + NP_NBO * NP_XLD) * (int)sizeof(T);
   static std::atomic<bool> attr{false};  // per element type
   if (!attr) {
     DUST_CUDA(cudaFuncSetAttribute(k_np_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp));
     DUST_CUDA(cudaFuncSetAttribute(k_np_inner<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smp));
-    DUST_CUDA(cudaFuncSetAttribute(k_np_cols<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smc));
     attr = true;
   }
   if (n > 2 * NP_NBO) DUST_TRY(w.side.make());
@@ -552,7 +585,10 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
   panel(0, st);
   for (int K = 0; K + NP_NBO < n; K += NP_NBO) {
     const int Ke = K + NP_NBO, Kn = std::min(Ke + NP_NBO, n);
-    k_np_cols<T><<<(n - Ke + NP_NB - 1) / NP_NB, NP_T, smc, st>>>(A, lda, n, K, Ke, inv0);
+    if (n - Ke >= 148 * 64)
+      np_cols<T, 32>(st, A, lda, n, K, Ke, inv0);
+    else
+      np_cols<T, 16>(st, A, lda, n, K, Ke, inv0);
     DUST_TRY(update(n - Ke, Kn - Ke, NP_NBO, at(Ke, K), at(K, Ke), at(Ke, Ke)));
     if (Kn == n) {
       panel(Ke, st);
