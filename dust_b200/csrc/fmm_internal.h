@@ -65,7 +65,7 @@ struct dust_octree {
   int kdlen[DUST_MAXLEV + 1][3];
   DevBuf idxsum;
   // per-call buffers (grown on demand, kept across calls)
-  DevBuf keys, keys_s, vals, perm, cnt, cstart, part, flags, ind, cidx, lidx;
+  DevBuf keys, keys_s, vals, perm, cnt, cstart, part, flags, cidx, lidx;
   DevBuf act_key, act_lev, leaf_ci, mp, outs, cub_tmp, small;
   DevBuf h_in, h_out, h_pts, el_geo, el_raw;  // staging of host-API calls
   DevBuf ffbuf;                        // far-field panel records

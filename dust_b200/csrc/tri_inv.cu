@@ -30,7 +30,7 @@ static inline int ti_blocks(int n) { return (n + TI_B - 1) / TI_B; }
 // slice is loaded into registers while this one is multiplied.  Bound by shared
 // memory if it is read word by word (eight reads, half of them in two-way
 // conflicts, for 16 products: a quarter of the FP32 rate), so operands are read
-// and B's slice is stored as vectors of four: NNN.
+// and B's slice is stored as vectors of four.
 template <typename T, int TN>
 struct TiSmem {
   alignas(16) T a[TI_K][TI_T + 4];
