@@ -866,96 +866,110 @@ __global__ void __launch_bounds__(M1_T) k_m2l_1(FmmDev d, uint32_t act_lo) {
 }
 
 // ------------------------------------------------------------- L2P + P2P
-struct P2PAcc {
-  double v[3], s[3], r[3], f[3];
+// One source q (strength a) acting on target p (strength ta): the reference's
+// compute_vel, compute_stretch, compute_rotu and compute_diffusion of source q
+// (mod_vortpart.f90:139-336), 4*pi factors applied by the caller.  With d = p - q,
+// rho^2 = d^2 + s^2, s the source's r_v, the pair's terms are
+//   velocity      -d x a / rho^3
+//   stretching    x / rho^3 - 3 (d.x) d / rho^5, x = ta x a
+//   rotational    a (3 s^2/rho^2 - 1) / rho^3 + 3 (d.a) d / rho^5
+//   diffusion     17.5 s^-2 (s/rho)^9 (a - ta)
+// (d^2 = rho^2 - s^2, 1 + d^2/s^2 = rho^2/s^2): one reciprocal root serves all
+// four (v: without the sign): 63 FP64 operations a pair where term by term took
+// 78 (110,000 particles: 1.22 -> 0.92 ms).  q[7] = 17.5 / s.
+// (ta x taken out of the sum too, 56 operations: three times the FP32 error
+// of the stretching, whose terms cancel in x where strengths are parallel.)
+template <typename V>
+struct P2PSums {
+  V v[3], s[3], r[3], f[3];
 };
-
-// One source q acting on target p: the reference's compute_vel,
-// compute_stretch, compute_rotu and compute_diffusion of source q
-// (mod_vortpart.f90:139-336), 4*pi factors applied by the caller.  s2 and
-// is2 are the source's r_v^2 and 1 / r_v^2.
 template <bool VS, bool DF, bool VD>
-__device__ __forceinline__ void p2p_pair(const double *tp, const double *ta, double qx,
-                                         double qy, double qz, double qax, double qay,
-                                         double qaz, double s2, double is2, P2PAcc &A) {
-  double dx = tp[0] - qx, dy = tp[1] - qy, dz = tp[2] - qz;
-  double r2 = dx * dx + dy * dy + dz * dz;
-  double inv = rsqrt_r(r2 + s2);
-  double inv2 = inv * inv;
-  double c = -inv2 * inv;        // -1/rho^3
-  double dd = -3.0 * c * inv2;   // 3/rho^5
-  double cx = dy * qaz - dz * qay, cy = dz * qax - dx * qaz, cz = dx * qay - dy * qax;
-  A.v[0] += c * cx;
-  A.v[1] += c * cy;
-  A.v[2] += c * cz;
+__device__ __forceinline__ void p2p_pair(const double *tp, const double *ta, const double (&q)[8],
+                                         bool self, P2PSums<double> &A) {
+  const double d[3] = {tp[0] - q[0], tp[1] - q[1], tp[2] - q[2]};
+  const double *a = q + 3, s2 = q[6];
+  const double r = rsqrt_r(fma(d[0], d[0], fma(d[1], d[1], fma(d[2], d[2], s2))));
+  const double inv = self ? 0.0 : r, i2 = inv * inv, i3 = i2 * inv, rt2 = s2 * i2;
+  const double c[3] = {d[1] * a[2] - d[2] * a[1], d[2] * a[0] - d[0] * a[2],
+                       d[0] * a[1] - d[1] * a[0]};
+#pragma unroll
+  for (int e = 0; e < 3; ++e) A.v[e] = fma(i3, c[e], A.v[e]);
   if (VS) {
-    double vx = ta[1] * qaz - ta[2] * qay, vy = ta[2] * qax - ta[0] * qaz,
-           vz = ta[0] * qay - ta[1] * qax;
-    double dv = dx * vx + dy * vy + dz * vz;
-    A.s[0] -= c * vx + dd * dx * dv;
-    A.s[1] -= c * vy + dd * dy * dv;
-    A.s[2] -= c * vz + dd * dz * dv;
+    const double k3 = 3.0 * i3, i5 = k3 * i2;
+    const double x[3] = {ta[1] * a[2] - ta[2] * a[1], ta[2] * a[0] - ta[0] * a[2],
+                         ta[0] * a[1] - ta[1] * a[0]};
+    const double t = i5 * -fma(d[0], x[0], fma(d[1], x[1], d[2] * x[2]));
+#pragma unroll
+    for (int e = 0; e < 3; ++e) A.s[e] = fma(i3, x[e], fma(t, d[e], A.s[e]));
     if (DF) {
-      // dist x (dist x aq) = dist (dist.aq) - aq r^2
-      double da = dx * qax + dy * qay + dz * qaz;
-      A.r[0] += -2.0 * c * qax + dd * (dx * da - qax * r2);
-      A.r[1] += -2.0 * c * qay + dd * (dy * da - qay * r2);
-      A.r[2] += -2.0 * c * qaz + dd * (dz * da - qaz * r2);
+      const double u = i5 * fma(d[0], a[0], fma(d[1], a[1], d[2] * a[2]));
+      const double g = fma(k3, rt2, -i3);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) A.r[e] = fma(g, a[e], fma(u, d[e], A.r[e]));
     }
   }
   if (VD) {
-    // (1/s^2) vol (aq - ap) eta, vol = 4/3 pi s^3, eta = 105/(8 pi)/s^3/(1+r^2/s^2)^4.5
-    double t = r2 * is2 + 1.0;
-    double rt = rsqrt_r(t);
-    double rt2 = rt * rt, rt4 = rt2 * rt2;
-    double w = 17.5 * is2 * (rt4 * rt4 * rt);
-    A.f[0] += w * (qax - ta[0]);
-    A.f[1] += w * (qay - ta[1]);
-    A.f[2] += w * (qaz - ta[2]);
+    const double rt4 = rt2 * rt2, w = (q[7] * inv) * (rt4 * rt4);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) A.f[e] = fma(w, a[e] - ta[e], A.f[e]);
   }
 }
-
-struct P2PAccF {
-  float v[3], s[3], r[3], f[3];
-};
-
-// FP32 form of p2p_pair on coordinates relative to the leaf centre
+// FP32 form of two sources at a time in packed operations, on coordinates
+// relative to the leaf centre.  Each output gets one addition a pair, and the
+// diffusion its own reciprocal root (from 1 / s^2 = q[7]; its ninth power of
+// s / rho would carry the other's error): the sums' errors against 64 bits are
+// those of the term-by-term form (0.97 to 0.99 of them over 16 sets of 37 to 2,500
+// particles; 1,100,000 particles: 4.59 -> 3.7 ms).
 template <bool VS, bool DF, bool VD>
-__device__ __forceinline__ void p2p_pair_f(const float *tp, const float *ta, float qx, float qy,
-                                           float qz, float qax, float qay, float qaz, float s2,
-                                           float is2, P2PAccF &A) {
-  float dx = tp[0] - qx, dy = tp[1] - qy, dz = tp[2] - qz;
-  float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  float inv = rsqrtf(r2 + s2);
-  float inv2 = inv * inv;
-  float c = -inv2 * inv;
-  float dd = -3.0f * c * inv2;
-  float cx = dy * qaz - dz * qay, cy = dz * qax - dx * qaz, cz = dx * qay - dy * qax;
-  A.v[0] = fmaf(c, cx, A.v[0]);
-  A.v[1] = fmaf(c, cy, A.v[1]);
-  A.v[2] = fmaf(c, cz, A.v[2]);
+__device__ __forceinline__ void p2p_pair2_f(const float *tp, const float *ta, const float2 (&q)[8],
+                                            bool self0, bool self1, P2PSums<float2> &A) {
+  auto two = [](float x) { return make_float2(x, x); };
+  auto neg = [](float2 x) { return make_float2(-x.x, -x.y); };
+  float2 d[3], m[3];  // d and -d
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    m[e] = __fadd2_rn(q[e], two(-tp[e]));
+    d[e] = neg(m[e]);
+  }
+  const float2 *a = q + 3, s2 = q[6];
+  const float2 r2 = __ffma2_rn(m[0], m[0], __ffma2_rn(m[1], m[1], __fmul2_rn(m[2], m[2])));
+  const float2 rho2 = __fadd2_rn(r2, s2);
+  const float2 inv = make_float2(self0 ? 0.f : rsqrtf(rho2.x), self1 ? 0.f : rsqrtf(rho2.y));
+  const float2 i2 = __fmul2_rn(inv, inv), i3 = __fmul2_rn(i2, inv);
+  const float2 c[3] = {__ffma2_rn(d[1], a[2], __fmul2_rn(m[2], a[1])),
+                       __ffma2_rn(d[2], a[0], __fmul2_rn(m[0], a[2])),
+                       __ffma2_rn(d[0], a[1], __fmul2_rn(m[1], a[0]))};
+#pragma unroll
+  for (int e = 0; e < 3; ++e) A.v[e] = __ffma2_rn(i3, c[e], A.v[e]);
   if (VS) {
-    float vx = ta[1] * qaz - ta[2] * qay, vy = ta[2] * qax - ta[0] * qaz,
-          vz = ta[0] * qay - ta[1] * qax;
-    float dv = dx * vx + dy * vy + dz * vz;
-    A.s[0] -= c * vx + dd * dx * dv;
-    A.s[1] -= c * vy + dd * dy * dv;
-    A.s[2] -= c * vz + dd * dz * dv;
+    const float2 i5 = __fmul2_rn(__fmul2_rn(i3, two(3.0f)), i2);
+    const float2 x[3] = {
+        __ffma2_rn(two(ta[1]), a[2], __fmul2_rn(two(-ta[2]), a[1])),
+        __ffma2_rn(two(ta[2]), a[0], __fmul2_rn(two(-ta[0]), a[2])),
+        __ffma2_rn(two(ta[0]), a[1], __fmul2_rn(two(-ta[1]), a[0]))};
+    const float2 t = __fmul2_rn(
+        i5, __ffma2_rn(m[0], x[0], __ffma2_rn(m[1], x[1], __fmul2_rn(m[2], x[2]))));
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+      A.s[e] = __fadd2_rn(A.s[e], __ffma2_rn(i3, x[e], __fmul2_rn(t, d[e])));
     if (DF) {
-      float da = dx * qax + dy * qay + dz * qaz;
-      A.r[0] += -2.0f * c * qax + dd * (dx * da - qax * r2);
-      A.r[1] += -2.0f * c * qay + dd * (dy * da - qay * r2);
-      A.r[2] += -2.0f * c * qaz + dd * (dz * da - qaz * r2);
+      const float2 u = __ffma2_rn(d[0], a[0], __ffma2_rn(d[1], a[1], __fmul2_rn(d[2], a[2])));
+      const float2 k = __fadd2_rn(i3, i3);
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+        A.r[e] = __fadd2_rn(
+            A.r[e], __ffma2_rn(k, a[e],
+                               __fmul2_rn(i5, __ffma2_rn(d[e], u, __fmul2_rn(neg(r2), a[e])))));
     }
   }
   if (VD) {
-    float t = fmaf(r2, is2, 1.0f);
-    float rt = rsqrtf(t);
-    float rt2 = rt * rt, rt4 = rt2 * rt2;
-    float w = 17.5f * is2 * (rt4 * rt4 * rt);
-    A.f[0] += w * (qax - ta[0]);
-    A.f[1] += w * (qay - ta[1]);
-    A.f[2] += w * (qaz - ta[2]);
+    const float2 t = __ffma2_rn(r2, q[7], two(1.0f));
+    const float2 rt = make_float2(self0 ? 0.f : rsqrtf(t.x), self1 ? 0.f : rsqrtf(t.y));
+    const float2 rt2 = __fmul2_rn(rt, rt), rt4 = __fmul2_rn(rt2, rt2),
+                 w = __fmul2_rn(q[7], __fmul2_rn(__fmul2_rn(rt4, rt4), rt));
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+      A.f[e] = __ffma2_rn(w, __fadd2_rn(a[e], two(-ta[e])), A.f[e]);
   }
 }
 
@@ -988,7 +1002,8 @@ __device__ __forceinline__ void p2p_pair_f(const float *tp, const float *ta, flo
 // the outputs atomically, the first one of a target also its L2P.
 #define P2W_TILE 32
 #define P2W_MAXR (26 * DUST_MAXLEV + 4)
-#define P2W_NV 8  // staged per source: x y z, alpha x y z, r_v^2, 1 / r_v^2
+#define P2W_NV 8  // staged per source: x y z, alpha x y z, s^2 and, with
+                  // s = r_v, 17.5 / s (FP64) or 1 / s^2 (FP32)
 #define P2W_LQ 4  // levels whose near-field loads are issued together
 #define P2W_XB (148 * 16)  // CTAs for the items: the resident ones
 #define P2W_CAP (1u << 18) // items (4 MB)
@@ -1079,7 +1094,7 @@ __device__ __forceinline__ void p2p_share(const FmmDev &d, uint32_t leaf, int tb
                                           uint32_t s_lo, uint32_t s_hi, bool split) {
   using R = typename std::conditional<F32, float, double>::type;
   __shared__ __align__(16) R s_src[P2W_NV][P2W_TILE];
-  __shared__ uint32_t s_sid[P2W_TILE];
+  __shared__ __align__(8) uint32_t s_sid[P2W_TILE];
   __shared__ uint32_t rlo[P2W_MAXR];
   __shared__ uint32_t rcum[P2W_MAXR + 1];
   __shared__ double s_acc[12][32];
@@ -1196,14 +1211,25 @@ __device__ __forceinline__ void p2p_share(const FmmDev &d, uint32_t leaf, int tb
     }
     // FP64 sums: in registers (FP64 pairs) or in shared memory (FP32C,
     // which keeps its registers for the FP32 partial sums)
-    P2PAcc A;
-    P2PAccF B;
-    for (int e = 0; e < 3; ++e) {
-      A.v[e] = A.s[e] = A.r[e] = A.f[e] = 0.0;
-      B.v[e] = B.s[e] = B.r[e] = B.f[e] = 0.0f;
-    }
+    P2PSums<double> A;
+    P2PSums<float2> B;
+    auto clear_f = [&]() {
+      for (int e = 0; e < 3; ++e)
+        B.v[e] = B.s[e] = B.r[e] = B.f[e] = make_float2(0.f, 0.f);
+    };
+    for (int e = 0; e < 3; ++e) A.v[e] = A.s[e] = A.r[e] = A.f[e] = 0.0;
+    clear_f();
     if (F32)
       for (int e = 0; e < 12; ++e) acc[32 * e] = 0.0;
+    // adds the four outputs of a pair's sums to acc
+    auto put = [&](const double *v, const double *ss, const double *r, const double *f) {
+      for (int e = 0; e < 3; ++e) {
+        acc[32 * e] -= v[e];
+        if (VS) acc[32 * (3 + e)] += ss[e];
+        if (VS && DF) acc[32 * (6 + e)] += r[e];
+        if (VD) acc[32 * (9 + e)] += (F32 ? 17.5 : 1.0) * f[e];
+      }
+    };
     int since = 0;
     // the sources of the next tile are loaded into registers while the
     // current tile is evaluated; each lane's range index only moves forward
@@ -1224,60 +1250,62 @@ __device__ __forceinline__ void p2p_share(const FmmDev &d, uint32_t leaf, int tb
     fetch(s_lo + lane);
     for (uint32_t s0 = s_lo; s0 < s_hi; s0 += P2W_TILE) {
       __syncwarp();
+      // (beyond the last source: no strength, kv = 0)
+      R st8[8] = {(R)0, (R)0, (R)0, (R)0, (R)0, (R)0, (R)1, (R)0};
       if (pv) {
-        s_sid[lane] = psid;
-        for (int q = 0; q < 3; ++q)
-          fs[q * P2W_TILE + lane] = F32 ? (R)(pf[q] - cc[q]) : (R)pf[q];
-        for (int q = 3; q < 6; ++q) fs[q * P2W_TILE + lane] = (R)pf[q];
-        const double rv = pf[6];
-        if constexpr (F32) {
-          const float s2 = (float)rv * (float)rv;
-          fs[6 * P2W_TILE + lane] = s2;
-          fs[7 * P2W_TILE + lane] = VD ? __frcp_rn(s2) : 0.f;
-        } else {
-          const double s2 = rv * rv;
-          fs[6 * P2W_TILE + lane] = s2;
-          fs[7 * P2W_TILE + lane] = VD ? __drcp_rn(s2) : 0.0;
-        }
+        for (int q = 0; q < 3; ++q) st8[q] = F32 ? (R)(pf[q] - cc[q]) : (R)pf[q];
+        for (int q = 3; q < 6; ++q) st8[q] = (R)pf[q];
+        const R rv = (R)pf[6];
+        st8[6] = rv * rv;
+        if (VD) st8[7] = F32 ? (R)1 / st8[6] : (R)17.5 / rv;
       }
+      s_sid[lane] = psid;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) fs[q * P2W_TILE + lane] = st8[q];
       __syncwarp();
       fetch(s0 + P2W_TILE + lane);
       const int m = (int)min((uint32_t)P2W_TILE, s_hi - s0);
       if (act)
-        for (int u = grp; u < m; u += G) {
-          if (s_sid[u] == ti) continue;
-          if constexpr (F32)
-            p2p_pair_f<VS, DF, VD>(tp, ta, fs[u], fs[P2W_TILE + u], fs[2 * P2W_TILE + u],
-                                   fs[3 * P2W_TILE + u], fs[4 * P2W_TILE + u],
-                                   fs[5 * P2W_TILE + u], fs[6 * P2W_TILE + u],
-                                   fs[7 * P2W_TILE + u], B);
-          else
-            p2p_pair<VS, DF, VD>(tp, ta, fs[u], fs[P2W_TILE + u], fs[2 * P2W_TILE + u],
-                                 fs[3 * P2W_TILE + u], fs[4 * P2W_TILE + u],
-                                 fs[5 * P2W_TILE + u], fs[6 * P2W_TILE + u],
-                                 fs[7 * P2W_TILE + u], A);
+#pragma unroll 1
+        for (int u = 2 * grp; u < m; u += 2 * G) {
+          const uint2 id = *(const uint2 *)&s_sid[u];
+          if constexpr (F32) {
+            float2 q[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) q[e] = *(const float2 *)&fs[e * P2W_TILE + u];
+            p2p_pair2_f<VS, DF, VD>(tp, ta, q, id.x == ti, id.y == ti, B);
+          } else {
+            double q0[8], q1[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const double2 x = *(const double2 *)&fs[e * P2W_TILE + u];
+              q0[e] = x.x;
+              q1[e] = x.y;
+            }
+            p2p_pair<VS, DF, VD>(tp, ta, q0, id.x == ti, A);
+            p2p_pair<VS, DF, VD>(tp, ta, q1, id.y == ti, A);
+          }
         }
       if (F32 && (++since == 4 || s0 + P2W_TILE >= s_hi)) {
         // FP32 partial sums of up to 128 sources folded into FP64
         since = 0;
+        double v[3], ss[3], r[3], f[3];
         for (int e = 0; e < 3; ++e) {
-          acc[32 * e] += (double)B.v[e];
-          acc[32 * (3 + e)] += (double)B.s[e];
-          acc[32 * (6 + e)] += (double)B.r[e];
-          acc[32 * (9 + e)] += (double)B.f[e];
-          B.v[e] = B.s[e] = B.r[e] = B.f[e] = 0.0f;
+          v[e] = (double)B.v[e].x + (double)B.v[e].y;
+          ss[e] = (double)B.s[e].x + (double)B.s[e].y;
+          r[e] = (double)B.r[e].x + (double)B.r[e].y;
+          f[e] = (double)B.f[e].x + (double)B.f[e].y;
         }
+        put(v, ss, r, f);
+        clear_f();
       }
     }
     // combine the groups of each target (group 0's lane sums the others'
     // shared-memory sums)
-    if (!F32)
-      for (int e = 0; e < 3; ++e) {
-        acc[32 * e] = A.v[e];
-        acc[32 * (3 + e)] = A.s[e];
-        acc[32 * (6 + e)] = A.r[e];
-        acc[32 * (9 + e)] = A.f[e];
-      }
+    if (!F32) {
+      for (int e = 0; e < 12; ++e) acc[32 * e] = 0.0;
+      put(A.v, A.s, A.r, A.f);
+    }
     __syncwarp();
     double Q[12];
     for (int e = 0; e < 12; ++e) {
