@@ -185,10 +185,12 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tf32_minus(int m, int n, in
 //  * an update of inner dimension 256 moves as many bytes of C as it has time
 //    to multiply, so it is bound by C's traffic: two CTAs per SM (2 stages and
 //    256 TMEM columns each), so that one's products run under the other's
-//    epilogue, and 8 warps that fetch C 16 columns ahead.  16,128 x 16,128 x
-//    256: 1,219 us with one CTA of 4 warps and 4 stages, 470 us now (2.1 GB of
-//    C: 317 us at the copy rate); the 16,384 LU's updates 31.8 -> 17.0 ms (one
-//    CTA of 8 warps and 4 stages: 21.9 ms); 12,000 x 1,920 x 12,000 the same;
+//    epilogue, and 8 warps whose additions go to the L2 (one reduction per
+//    element, no read of C and no wait for it; like every FP32 atomic addition
+//    they flush subnormals).  16,128 x 16,128 x 256: 1,219 us with one CTA of 4
+//    warps and 4 stages, 470 us with two and C read 16 columns ahead of its
+//    use (2.1 GB of C: 317 us at the copy rate); the 16,384 LU's updates 31.8,
+//    14.8 and, with the reductions, 12.6 ms;
 //  * every wait is bounded; on timeout the kernel flags the error, waits
 //    (bounded) for the copies and MMAs it issued, frees TMEM and returns.
 #define TP_BM 128
@@ -340,18 +342,8 @@ __global__ void __launch_bounds__(TP_T, 2)
             smem_u32(&s_done)));
   }
   __syncwarp();
-  // epilogue: warp w reads TMEM lanes 32 (w mod 4) .. of columns 128 (w / 4) ..;
-  // C comes 16 columns ahead of its use, the first ones before the products
-  // are complete
+  // epilogue: warp w reads TMEM lanes 32 (w mod 4) .. of columns 128 (w / 4) ..
   const int r = (warp & 3) * 32 + lane, gr = gm0 + r, cb = (warp >> 2) * (TP_BN / 2);
-  float cv[16], cn[16];
-  auto fetch = [&](int c0, float (&dst)[16]) {
-    const float *cp = C + (size_t)gr + (size_t)(gn0 + c0) * ldc;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      dst[j] = (gr < m && gn0 + c0 + j < n) ? __ldcg(cp + (size_t)j * ldc) : 0.f;
-  };
-  fetch(cb, cn);
   bool ok = mbar_wait(smem_u32(&s_done), 0u);
   const int all_ok = __syncthreads_and(ok && !*(volatile int *)&s_fail);
   if (!all_ok) {
@@ -376,15 +368,12 @@ __global__ void __launch_bounds__(TP_T, 2)
             "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
             "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
           : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0));
-#pragma unroll
-      for (int j = 0; j < 16; ++j) cv[j] = cn[j];
-      if (c0 + 16 < cb + TP_BN / 2) fetch(c0 + 16, cn);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       float *cp = C + (size_t)gr + (size_t)(gn0 + c0) * ldc;
 #pragma unroll
       for (int j = 0; j < 16; ++j)
         if (gr < m && gn0 + c0 + j < n)
-          __stcg(cp + (size_t)j * ldc, cv[j] + sign * __uint_as_float(v[j]));
+          atomicAdd(cp + (size_t)j * ldc, sign * __uint_as_float(v[j]));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
