@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(AIC_RX *AIC_CY)
 
 // static columns of static rows: b(ie) += sum_j bst(ie,j) nor_j.(-wind - uvort_j);
 // blockIdx.y takes a chunk of RS_COLS columns (partial sums added atomically)
-#define RS_COLS 256
+#define RS_COLS 64
 __global__ void k_rhs_static(const PanelGeo *el, const double *bst, int nst, double *b) {
   __shared__ double s_sig[RS_COLS];
   const int j0 = blockIdx.y * RS_COLS, j1 = min(nst, j0 + RS_COLS);
@@ -108,8 +108,18 @@ __global__ void k_rhs_static(const PanelGeo *el, const double *bst, int nst, dou
   __syncthreads();
   const int ie = blockIdx.x * blockDim.x + threadIdx.x;
   if (ie >= nst) return;
+  // 16 columns' loads in flight (as the compiler unrolls it, and chunks of 256:
+  // 27 us for 800 panels, 65 us for 6,000; 5 and 45 us)
   double s = 0.0;
-  for (int j = j0; j < j1; ++j) s += bst[(size_t)ie + (size_t)j * nst] * s_sig[j - j0];
+  int j = j0;
+  for (; j + 16 <= j1; j += 16) {
+    double v[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = bst[(size_t)ie + (size_t)(j + q) * nst];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) s += v[q] * s_sig[j + q - j0];
+  }
+  for (; j < j1; ++j) s += bst[(size_t)ie + (size_t)j * nst] * s_sig[j - j0];
   atomicAdd(b + ie, s);
 }
 
