@@ -568,7 +568,7 @@ __device__ __forceinline__ void line_vel_f(const double *vv, const float *q, con
 }
 
 // FP32: a thread per particle, the lines staged.  FP64: a warp per 32 particles
-// was bound by the latency of one line after the other (36 us for 3,000
+// was bound by the latency of one line after the other (36 us for 12,800
 // particles, 232 us for 60,000), so four warps share the lines of the same 32
 // particles: 8 and 94 us.
 #define EL_T 128

@@ -33,7 +33,7 @@ struct PanRaw {
 };
 
 // (CTAs of one warp: a warp's stores of a member meet 32 rows, so the panels of
-// a small set are shared out over the SMs; 9.5 us for 800 panels in CTAs of 128,
+// a small set are shared out over the SMs; 9.5 us for 400 panels in CTAs of 128,
 // 6.5 us)
 __global__ void k_panel_build(PanRaw r, double u0, double u1, double u2, PanelGeo *out) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(EP_T) k_elements_vel(int n, const double *pts,
 // 32 panels, staged for the CTA's points in shared memory (rows of an odd
 // number of words: the lanes read one member of 32 panels at a time), and adds
 // its part atomically into vel (zeroed first); the first part also the lines
-// and u_inf.  (A thread per point with 32 panels one after the other: 147 us
-// for 42 points and 800 panels; one panel a CTA: 42 us, most of it atomic adds
+// and u_inf.  (A thread per point with 32 panels one after the other, 147 us
+// in the 400-panel wing's step; one panel a CTA: 42 us, most of it atomic adds
 // to the same words; 9 us.)
 #define EPC_T 256
 #define EPC_LD ((int)(sizeof(PanelGeo) / 8) | 1)
