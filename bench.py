@@ -1071,14 +1071,15 @@ FLOP_P2P_PAIR = 95
 # count to 2M (profiles/k_elem_far_300k.txt)
 TRAFFIC_ELEM_FAR_PER_PARTICLE = 381.5
 # DRAM bytes per launch per particle of the 300k-particle full step (ncu,
-# profiles/k_uvort_300k.txt, k_m2l_batch_f32_300k.txt, k_p2p_w_f32_300k.txt),
+# profiles/k_uvort_300k.txt, k_m2l_batch_300k.txt, k_p2p_w_f32_300k.txt),
 # scaled by the particle count to the benchmark's size
 TRAFFIC_UVORT_PER_PARTICLE = 19.88e6 / 3.0e5
-TRAFFIC_M2L_F32_PER_PARTICLE = (138.53e6 + 53.36e6) / 3.0e5
-TRAFFIC_P2P_F32_PER_PARTICLE = (119.11e6 + 21.72e6) / 3.0e5
-# FMA-pipe activity of the FP32C kernels in the same captures
-# (sm__pipe_fma_cycles_active, profiles/*_300k.txt)
-FMA_PIPE_NCU = {"k_m2l_batch": 0.376, "k_p2p_w": 0.305, "k_uvort_pres_sorted": 0.807,
+TRAFFIC_M2L_PER_PARTICLE = 204.5e6 / 3.0e5
+TRAFFIC_P2P_F32_PER_PARTICLE = 145.3e6 / 3.0e5
+# FMA-pipe activity of the FP32C kernels, and FP64 tensor-pipe activity of the
+# M2L, in the same captures (profiles/*_300k.txt)
+DMMA_PIPE_NCU = {"k_m2l_batch": 0.687}
+FMA_PIPE_NCU = {"k_p2p_w": 0.245, "k_uvort_pres_sorted": 0.807,
                 "k_elem_far": 0.67}
 
 
@@ -1119,26 +1120,27 @@ def roofline(ph, case, params, best):
                    "pairs": p["n_elem_pairs"], "ms": p["k_elem_far_ms"]})
     elif p.get("fmm_elements"):
         a = FLOP_ELEM_PAIR * p["n_elem_pairs"] / (p["fmm_elements"] * 1e-3) / 1e12
-        ks.append({"kernel": "k_elem_out (elements, end vortices, outputs)",
+        ks.append({"kernel": "k_elem_far64 + k_elem_near + k_elem_fin (elements, end vortices, outputs)",
                    "bound": "fp64" if f64 else "fp32", "achieved": round(a, 2),
                    "peak": round(simt, 1), "unit": "TFLOP/s", "frac": round(a / simt, 3),
                    "traffic": None, "peak_source": simt_name, "flop_per_pair": FLOP_ELEM_PAIR,
                    "pairs": p["n_elem_pairs"], "ms": p["fmm_elements"]})
     if p.get("k_m2l_batch_ms"):
+        # bytes counted in the mode's words (the kernel itself is FP64 on the
+        # tensor pipe in every mode, whose peak is the FP64 SIMT one)
         t = p["k_m2l_batch_ms"] * 1e-3
         gbs = BYTES_M2L_PAIR_WORDS * w * p["n_m2l_pairs"] / t / 1e9
         fl = FLOP_M2L_PAIR * p["n_m2l_pairs"] / t / 1e12
         ks.append({"kernel": "k_m2l_batch", "bound": "hbm", "achieved": round(gbs, 1),
                    "peak": round(hbm, 1), "unit": "GB/s", "frac": round(gbs / hbm, 3),
-                   "traffic": None if f64 else int(TRAFFIC_M2L_F32_PER_PARTICLE * n),
+                   "traffic": int(TRAFFIC_M2L_PER_PARTICLE * n),
                    "peak_source": "HBM copy %s" % hbm_src,
                    "bytes_per_pair": BYTES_M2L_PAIR_WORDS * w, "pairs": p["n_m2l_pairs"],
                    "ms": p["k_m2l_batch_ms"],
-                   "flops": {"achieved": round(fl, 2), "peak": round(simt, 1),
-                             "unit": "TFLOP/s", "frac": round(fl / simt, 3),
-                             "flop_per_pair": FLOP_M2L_PAIR, "peak_source": simt_name,
-                             "fma_pipe_active_ncu": None if f64 else
-                             FMA_PIPE_NCU["k_m2l_batch"]}})
+                   "flops": {"achieved": round(fl, 2), "peak": round(fp64_peak, 1),
+                             "unit": "TFLOP/s", "frac": round(fl / fp64_peak, 3),
+                             "flop_per_pair": FLOP_M2L_PAIR, "peak_source": name_of(True),
+                             "dmma_pipe_active_ncu": DMMA_PIPE_NCU["k_m2l_batch"]}})
     if p.get("fmm_p2p"):
         a = FLOP_P2P_PAIR * p["n_p2p_pairs"] / (p["fmm_p2p"] * 1e-3) / 1e12
         ks.append({"kernel": "k_p2p_w (L2P + P2P)", "bound": "fp64" if f64 else "fp32",
