@@ -28,6 +28,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "stream_scratch.cuh"
 #include "dust_common.cuh"
 #include "elements.cuh"
 #include "fmm_internal.h"
@@ -1379,14 +1380,12 @@ extern "C" int dust_points_uvort_device_noalloc(const dust_fmm_params *prm, int 
 // dust_points_uvort_device and the pressure equation's particle term in one
 // pass, FP64 (k_uvort_pres) or FP32C on Morton-sorted particles
 // (k_uvort_pres_sorted); the end vortices go to uvort as before.
-// end-vortex records and the FP32C pass's sorted particles (one host thread)
-static DevBuf g_uvp_raw, g_uvp_geo, g_uvp_sort;
-
-// the fused pass on device arrays, end vortices already built into e
+// the fused pass on device arrays, end vortices already built into e; `sort`
+// holds the FP32C pass's sorted particles
 static int uvort_pressure_run(const dust_fmm_params *prm, int n_pts, const double *pts, int n,
                               const double *cen, const double *dir, const double *mag,
                               const double *r_vortex, const double *vel, const ElemDev &e,
-                              double *uvort, double *pterm, cudaStream_t st) {
+                              DevBuf &sort, double *uvort, double *pterm, cudaStream_t st) {
   DUST_CUDA(cudaMemsetAsync(uvort, 0, (size_t)n_pts * 24, st));
   DUST_CUDA(cudaMemsetAsync(pterm, 0, (size_t)n_pts * 8, st));
   if (n > 0 && prm->precision == DUST_PREC_FP32C) {
@@ -1398,8 +1397,8 @@ static int uvort_pressure_run(const dust_fmm_params *prm, int n_pts, const doubl
                                               st));
     const size_t off_f = round256(16 * N), off_x = off_f + round256(28 * N),
                  off_t = off_x + round256(24 * N);
-    DUST_TRY(devbuf_grow(g_uvp_sort, off_t + round256(tb)));
-    char *b = (char *)g_uvp_sort.p;
+    DUST_TRY(devbuf_grow(sort, off_t + round256(tb)));
+    char *b = (char *)sort.p;
     uint32_t *k_in = (uint32_t *)b, *v_in = k_in + N, *k_out = v_in + N, *v_out = k_out + N;
     float *F = (float *)(b + off_f);
     double *X = (double *)(b + off_x);
@@ -1449,11 +1448,13 @@ extern "C" int dust_points_uvort_pressure_device(const dust_fmm_params *prm, int
     return DUST_ERR_BAD_ARG;
   if (n_pts == 0) return DUST_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  StreamScratch::Use s(StreamScratch::get(), st);
+  DUST_TRY(s.status);
   ElemDev e;
   DUST_TRY(elem_build_device(nullptr, nullptr, end_vort, prm->u_inf, reg_params(prm), false,
-                             g_uvp_raw, g_uvp_geo, e, st));
-  return uvort_pressure_run(prm, n_pts, pts, n, cen, dir, mag, r_vortex, vel, e, uvort, pterm,
-                            st);
+                             s->raw, s->geo, e, st));
+  return uvort_pressure_run(prm, n_pts, pts, n, cen, dir, mag, r_vortex, vel, e, s->work, uvort,
+                            pterm, st);
 }
 
 // Host arrays: inputs copied to a staging buffer kept across calls (one host
@@ -1471,9 +1472,11 @@ extern "C" int dust_points_uvort_pressure(const dust_fmm_params *prm, int n_pts,
     return DUST_ERR_BAD_ARG;
   if (n_pts == 0) return DUST_OK;
   cudaStream_t st = 0;
+  StreamScratch::Use s(StreamScratch::get(), st);  // (and the staging array, under its lock)
+  DUST_TRY(s.status);
   ElemDev e;
   DUST_TRY(elem_build_device(nullptr, nullptr, end_vort, prm->u_inf, reg_params(prm), true,
-                             g_uvp_raw, g_uvp_geo, e, st));
+                             s->raw, s->geo, e, st));
   const size_t P = (size_t)n_pts, N = (size_t)n;
   const size_t o_u = round256(24 * P), o_t = o_u + round256(24 * P), o_c = o_t + round256(8 * P);
   const size_t o_d = o_c + round256(24 * N), o_m = o_d + round256(24 * N),
@@ -1492,7 +1495,7 @@ extern "C" int dust_points_uvort_pressure(const dust_fmm_params *prm, int n_pts,
     DUST_CUDA(cudaMemcpyAsync(dr, r_vortex, 8 * N, cudaMemcpyHostToDevice, st));
     DUST_CUDA(cudaMemcpyAsync(dv, vel, 24 * N, cudaMemcpyHostToDevice, st));
   }
-  DUST_TRY(uvort_pressure_run(prm, n_pts, dp, n, dc, dd, dm, dr, dv, e, du, dt, st));
+  DUST_TRY(uvort_pressure_run(prm, n_pts, dp, n, dc, dd, dm, dr, dv, e, s->work, du, dt, st));
   DUST_CUDA(cudaMemcpyAsync(uvort, du, 24 * P, cudaMemcpyDeviceToHost, st));
   DUST_CUDA(cudaMemcpyAsync(pterm, dt, 8 * P, cudaMemcpyDeviceToHost, st));
   DUST_CUDA(cudaStreamSynchronize(st));

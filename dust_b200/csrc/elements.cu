@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "stream_scratch.cuh"
 #include "dust_common.cuh"
 #include "elements.cuh"
 #include "fmm_internal.h"
@@ -342,12 +343,12 @@ extern "C" int dust_elements_vel(const dust_fmm_params *prm, int n_pts, const do
   return DUST_OK;
 }
 
-static DevBuf g_uv_scratch;  // sort scratch of the uvort entry points (one host thread)
-
 int points_uvort_device(const dust_fmm_params *prm, int n_pts, const double *pts, int n,
                         const double *cen, const double *dir, const double *mag,
                         const double *rv, const ElemDev &lines, double *uv, cudaStream_t st) {
-  return points_uvort_run(prm, n_pts, pts, n, cen, dir, mag, rv, lines, g_uv_scratch, uv, st);
+  StreamScratch::Use s(StreamScratch::get(), st);
+  DUST_TRY(s.status);
+  return points_uvort_run(prm, n_pts, pts, n, cen, dir, mag, rv, lines, s->work, uv, st);
 }
 
 bool uvort_args_ok(const dust_fmm_params *prm, int n_pts, const double *pts, int n,
@@ -369,8 +370,10 @@ extern "C" int dust_points_uvort(const dust_fmm_params *prm, int n_pts, const do
   if (!uvort_args_ok(prm, n_pts, pts, n, cen, dir, mag, r_vortex, end_vort, uvort))
     return DUST_ERR_BAD_ARG;
   if (n_pts == 0) return DUST_OK;
-  static Scratch s;  // kept across calls (one host thread)
   cudaStream_t st = 0;
+  StreamScratch::Use sort(StreamScratch::get(), st);  // (and the arrays below, under its lock)
+  DUST_TRY(sort.status);
+  static Scratch s;  // kept across calls
   ElemDev e;
   DUST_TRY(elem_build_device(nullptr, nullptr, end_vort, prm->u_inf, reg_params(prm), true,
                              s.raw, s.geo, e, st));
@@ -386,7 +389,7 @@ extern "C" int dust_points_uvort(const dust_fmm_params *prm, int n_pts, const do
     DUST_CUDA(cudaMemcpyAsync(dm, mag, (size_t)n * 8, cudaMemcpyHostToDevice, st));
     DUST_CUDA(cudaMemcpyAsync(dr, r_vortex, (size_t)n * 8, cudaMemcpyHostToDevice, st));
   }
-  DUST_TRY(points_uvort_device(prm, n_pts, dp, n, dc, dd, dm, dr, e, du, st));
+  DUST_TRY(points_uvort_run(prm, n_pts, dp, n, dc, dd, dm, dr, e, sort->work, du, st));
   DUST_CUDA(cudaMemcpyAsync(uvort, du, (size_t)n_pts * 24, cudaMemcpyDeviceToHost, st));
   DUST_CUDA(cudaStreamSynchronize(st));
   return DUST_OK;
@@ -460,11 +463,12 @@ extern "C" int dust_points_uvort_device(const dust_fmm_params *prm, int n_pts, c
     return DUST_ERR_BAD_ARG;
   if (n_pts == 0) return DUST_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  static thread_local Scratch s;
+  StreamScratch::Use s(StreamScratch::get(), st);
+  DUST_TRY(s.status);
   ElemDev e;
   DUST_TRY(elem_build_device(nullptr, nullptr, end_vort, prm->u_inf, reg_params(prm), false,
-                             s.raw, s.geo, e, st));
-  DUST_TRY(points_uvort_device(prm, n_pts, pts, n, cen, dir, mag, r_vortex, e, uvort, st));
+                             s->raw, s->geo, e, st));
+  DUST_TRY(points_uvort_run(prm, n_pts, pts, n, cen, dir, mag, r_vortex, e, s->work, uvort, st));
   return DUST_OK;
 }
 

@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "stream_scratch.cuh"
 #include "dust_common.cuh"
 #include "fmm_internal.h"
 
@@ -257,8 +258,6 @@ extern "C" int dust_particles_update_device(const dust_update_params *u, int n, 
   return DUST_OK;
 }
 
-static DevBuf g_pa_rec;  // element records of the penetration-avoidance entry point
-
 extern "C" int dust_particles_update_pa_device(const dust_update_params *u,
                                                const dust_pa_params *pa,
                                                const dust_panels *elems, int n, double *cen,
@@ -271,8 +270,10 @@ extern "C" int dust_particles_update_pa_device(const dust_update_params *u,
     return DUST_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   const int nel = elems->n;
-  DUST_TRY(devbuf_grow(g_pa_rec, sizeof(PaRec) * (size_t)std::max(nel, 1)));
-  PaRec *rec = (PaRec *)g_pa_rec.p;
+  StreamScratch::Use s(StreamScratch::get(), st);  // the element records
+  DUST_TRY(s.status);
+  DUST_TRY(devbuf_grow(s->work, sizeof(PaRec) * (size_t)std::max(nel, 1)));
+  PaRec *rec = (PaRec *)s->work.p;
   if (nel > 0)
     k_pa_records<<<nblk((size_t)nel, 128), 128, 0, st>>>(nel, elems->n_ver, elems->kind,
                                                          elems->ver, elems->ub, rec);

@@ -403,3 +403,52 @@ def test_fmm_level1_pairs_match_oracle(p, vs, n_box):
     assert rel(v, ov) < TOL64 and rel(s, os_) < TOL64
     if vs:
         assert rel(r, orr) < TOL64
+
+
+@pytest.mark.parametrize("prec", [abi.DUST_PREC_FP64, abi.DUST_PREC_FP32C])
+def test_uvort_calls_on_several_streams(prec):
+    """The entry points without a handle share their scratch among calls: six
+    streams' calls queued at once (more than there are sets of buffers), with
+    other inputs each, give what each gives alone."""
+    import ctypes as C
+    import torch
+    from dust_b200._lib import check, lib
+    ptr = lambda t: C.cast(C.c_void_p(t.data_ptr()), C.POINTER(C.c_double))
+    gpu = lambda a: torch.as_tensor(a, dtype=torch.float64, device="cuda").contiguous()
+    prm = prm_ring(precision=prec).struct()
+    npts, n, sets = 700, 40_000, []
+    for k in range(6):
+        rng = np.random.default_rng(100 + k)
+        cen, dir_, mag = synth.ring_particles(n, 0, seed=k)
+        v0 = rng.uniform(1.6, 2.0, (9, 3))
+        sets.append(dict(pts=gpu(rng.uniform(-1.5, 1.5, (npts, 3))), cen=gpu(cen), dir=gpu(dir_),
+                         mag=gpu(mag), rv=gpu(np.full(n, 0.05)),
+                         vel=gpu(rng.standard_normal((n, 3))),
+                         lver=gpu(np.stack([v0, v0 + 0.3], axis=1)),
+                         lmag=gpu(rng.standard_normal(9)), stream=torch.cuda.Stream(),
+                         uv=torch.empty((npts, 3), dtype=torch.float64, device="cuda"),
+                         up=torch.empty((npts, 3), dtype=torch.float64, device="cuda"),
+                         pt=torch.empty(npts, dtype=torch.float64, device="cuda")))
+    torch.cuda.synchronize()
+
+    def call(s):
+        ev = abi.Lines(9, ptr(s["lver"]), ptr(s["lmag"]))
+        st = C.c_void_p(s["stream"].cuda_stream)
+        args = (C.byref(prm), npts, ptr(s["pts"]), n, ptr(s["cen"]), ptr(s["dir"]), ptr(s["mag"]),
+                ptr(s["rv"]))
+        check(lib().dust_points_uvort_device(*args, C.byref(ev), ptr(s["uv"]), st), "uvort")
+        check(lib().dust_points_uvort_pressure_device(*args, ptr(s["vel"]), C.byref(ev),
+                                                      ptr(s["up"]), ptr(s["pt"]), st), "pressure")
+
+    alone = []
+    for s in sets:
+        call(s)
+        torch.cuda.synchronize()
+        alone.append([s[k].clone() for k in ("uv", "up", "pt")])
+    for _ in range(5):
+        for s in sets:
+            call(s)
+    torch.cuda.synchronize()
+    for s, a in zip(sets, alone):
+        for k, x in zip(("uv", "up", "pt"), a):
+            assert rel(s[k].cpu().numpy(), x.cpu().numpy()) < 1e-12
