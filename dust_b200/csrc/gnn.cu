@@ -289,27 +289,86 @@ __global__ void __launch_bounds__(256) k_pc_out_bwd(int n, int K, int C, float s
   }
 }
 
-// dz = dh * (z > 0), in place
-__global__ void k_pc_relu_bwd(size_t cnt, const float *z, float *d) {
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < cnt && !(z[e] > 0.f)) d[e] = 0.f;
-}
-
-// dh_prev_i = Ws^T dz_i, dm_i = Wn^T dz_i (CTA of 64 per node)
-__global__ void k_pc_layer_bwd(int n, const float *P, int l, const float *dz, float *dhp,
-                               float *dm) {
-  __shared__ float sd[PC_H];
-  const int i = blockIdx.x, f = threadIdx.x;
-  sd[f] = dz[(size_t)i * PC_H + f];
-  __syncthreads();
+// One layer backward: dz = dh where z > 0, dh_prev_i = Ws^T dz_i, dm_i = Wn^T dz_i,
+// and the gradients of Ws (sum_i dz_i,f h_i,k), Wn (with m) and b.  A CTA takes
+// PC_BN nodes and stages their dz, h and m and the two weight matrices: the four
+// products need each of them twice, and a launch each (mask 2.5, both weight
+// gradients 24 and the products 11 us at 6,954 nodes; NETNEW us together).  Node
+// groups of 64 keep the additions into the 8,256 gradient words few.
+#define PC_BN 64
+#define PC_BSM ((3 * PC_BN + 2 * PC_H) * PC_H * (int)sizeof(float))
+__global__ void __launch_bounds__(256) k_pc_layer_bwd(int n, const float *P, int l,
+                                                      const float *dh, const float *z,
+                                                      const float *h, const float *m, float *G,
+                                                      float *dhp, float *dm) {
+  extern __shared__ __align__(16) float sl[];
+  float(*sd)[PC_H] = (float(*)[PC_H])sl, (*sh)[PC_H] = sd + PC_BN, (*sm)[PC_H] = sh + PC_BN,
+  (*ws)[PC_H] = sm + PC_BN, (*wn)[PC_H] = ws + PC_H;
+  const int tid = threadIdx.x, i0 = blockIdx.x * PC_BN, nn = min(PC_BN, n - i0);
+  const size_t at = (size_t)i0 * PC_H;
   const float *Ws = P + pc_off_ws(l), *Wn = P + pc_off_wn(l);
-  float a = 0.f, b = 0.f;
-  for (int k = 0; k < PC_H; ++k) {
-    a = fmaf(Ws[k * PC_H + f], sd[k], a);
-    b = fmaf(Wn[k * PC_H + f], sd[k], b);
+  for (int e = tid; e < PC_H * PC_H; e += 256) {
+    ws[e / PC_H][e % PC_H] = Ws[e];
+    wn[e / PC_H][e % PC_H] = Wn[e];
   }
-  dhp[(size_t)i * PC_H + f] = a;
-  dm[(size_t)i * PC_H + f] = b;
+  for (int e = tid; e < PC_BN * PC_H; e += 256) {
+    const bool in = e / PC_H < nn;
+    sd[e / PC_H][e % PC_H] = in && z[at + e] > 0.f ? dh[at + e] : 0.f;
+    sh[e / PC_H][e % PC_H] = in ? h[at + e] : 0.f;
+    sm[e / PC_H][e % PC_H] = in ? m[at + e] : 0.f;
+  }
+  __syncthreads();
+  {
+    // thread (f, g): feature f of the nodes g, g + 4, ..
+    const int f = tid % PC_H, g = tid / PC_H;
+    float a[PC_BN / 4] = {}, b[PC_BN / 4] = {};
+#pragma unroll 1
+    for (int k = 0; k < PC_H; k += 4) {
+      float u[4], v[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) u[x] = ws[k + x][f], v[x] = wn[k + x][f];
+#pragma unroll
+      for (int q = 0; q < PC_BN / 4; ++q) {
+        const float4 D = *(const float4 *)&sd[g + 4 * q][k];
+        a[q] = fmaf(u[3], D.w, fmaf(u[2], D.z, fmaf(u[1], D.y, fmaf(u[0], D.x, a[q]))));
+        b[q] = fmaf(v[3], D.w, fmaf(v[2], D.z, fmaf(v[1], D.y, fmaf(v[0], D.x, b[q]))));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < PC_BN / 4; ++q)
+      if (g + 4 * q < nn) {
+        dhp[at + (size_t)(g + 4 * q) * PC_H + f] = a[q];
+        dm[at + (size_t)(g + 4 * q) * PC_H + f] = b[q];
+      }
+  }
+  // thread (fy, kx): features 4 fy .., columns 4 kx ..
+  const int fy = tid / 16, kx = tid % 16;
+  float s[4][4] = {}, t[4][4] = {};
+  for (int i = 0; i < nn; ++i) {
+    const float4 D = *(const float4 *)&sd[i][4 * fy], A = *(const float4 *)&sh[i][4 * kx],
+                 M = *(const float4 *)&sm[i][4 * kx];
+    const float d[4] = {D.x, D.y, D.z, D.w}, x[4] = {A.x, A.y, A.z, A.w},
+                y[4] = {M.x, M.y, M.z, M.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        s[u][v] = fmaf(d[u], x[v], s[u][v]);
+        t[u][v] = fmaf(d[u], y[v], t[u][v]);
+      }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      atomicAdd(G + pc_off_ws(l) + (4 * fy + u) * PC_H + 4 * kx + v, s[u][v]);
+      atomicAdd(G + pc_off_wn(l) + (4 * fy + u) * PC_H + 4 * kx + v, t[u][v]);
+    }
+  if (tid < PC_H) {
+    float r = 0.f;
+    for (int i = 0; i < nn; ++i) r += sd[i][tid];
+    atomicAdd(G + pc_off_bl(l) + tid, r);
+  }
 }
 
 // dh_prev_j += w_ij dm_i (scatter over the edges)
@@ -324,44 +383,30 @@ __global__ void k_pc_agg_bwd(int n, int K, const int *nbr, const float *w, const
     atomicAdd(dhp + (size_t)nbr[(size_t)i * K + q] * PC_H + f, w[(size_t)i * K + q] * g);
 }
 
-// G[off + f*cols + k] += sum_i dz_i,f a_i,k and G[boff + f] += sum_i dz_i,f
-// (boff < 0: none); CTA per chunk of nodes.  Both operands of a chunk are
-// staged in shared memory (every thread read them from global memory for each
-// of its products before: 41 us a call at 6,954 nodes, 12 us now).
+// The input layer's gradients: with dz = dh where z > 0, G[W0 + f PC_FIN + k] +=
+// sum_i dz_i,f x_i,k and G[b0 + f] += sum_i dz_i,f; CTA per chunk of nodes, both
+// operands staged in shared memory.
 #define PC_WG_CHUNK 64
-__global__ void __launch_bounds__(256) k_pc_wgrad(int n, const float *dz, const float *a, int cols,
-                                                  float *G, int off, int boff) {
-  __shared__ __align__(16) float sd[PC_WG_CHUNK][PC_H], sa[PC_WG_CHUNK][PC_H];
-  const int tid = threadIdx.x;
-  const int i0 = blockIdx.x * PC_WG_CHUNK, ni = min(n - i0, PC_WG_CHUNK);
-  for (int e = tid; e < PC_WG_CHUNK * PC_H; e += 256) {
-    const int i = e / PC_H, k = e % PC_H;
-    sd[i][k] = i < ni ? dz[(size_t)(i0 + i) * PC_H + k] : 0.f;
-    sa[i][k] = i < ni && k < cols ? a[(size_t)(i0 + i) * cols + k] : 0.f;
-  }
+__global__ void __launch_bounds__(256) k_pc_in_bwd(int n, const float *dh, const float *z,
+                                                   const float *x, float *G) {
+  __shared__ float sd[PC_WG_CHUNK][PC_H], sx[PC_WG_CHUNK][PC_FIN];
+  const int tid = threadIdx.x, i0 = blockIdx.x * PC_WG_CHUNK, ni = min(n - i0, PC_WG_CHUNK);
+  const size_t at = (size_t)i0 * PC_H;
+  for (int e = tid; e < ni * PC_H; e += 256)
+    sd[e / PC_H][e % PC_H] = z[at + e] > 0.f ? dh[at + e] : 0.f;
+  for (int e = tid; e < ni * PC_FIN; e += 256)
+    sx[e / PC_FIN][e % PC_FIN] = x[(size_t)i0 * PC_FIN + e];
   __syncthreads();
-  // thread (fy, kx): features 4 fy .., columns 4 kx ..
-  const int fy = tid / 16, kx = tid % 16;
-  if (4 * kx < cols) {
-    float s[4][4] = {};
-    for (int i = 0; i < ni; ++i) {
-      const float4 D = *(const float4 *)&sd[i][4 * fy], A = *(const float4 *)&sa[i][4 * kx];
-      const float d[4] = {D.x, D.y, D.z, D.w}, x[4] = {A.x, A.y, A.z, A.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) s[u][v] = fmaf(d[u], x[v], s[u][v]);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-        if (4 * kx + v < cols) atomicAdd(G + off + (4 * fy + u) * cols + 4 * kx + v, s[u][v]);
+  for (int o = tid; o < PC_H * PC_FIN; o += 256) {
+    const int f = o / PC_FIN, k = o % PC_FIN;
+    float s = 0.f;
+    for (int i = 0; i < ni; ++i) s = fmaf(sd[i][f], sx[i][k], s);
+    atomicAdd(G + pc_off_w0() + o, s);
   }
-  if (boff >= 0 && tid < PC_H) {
+  if (tid < PC_H) {
     float s = 0.f;
     for (int i = 0; i < ni; ++i) s += sd[i][tid];
-    atomicAdd(G + boff + tid, s);
+    atomicAdd(G + pc_off_b0() + tid, s);
   }
 }
 
@@ -418,19 +463,17 @@ static int pc_loss_grad(dust_precond *p, int si, float *loss_host) {
   const float scale = 2.f / ((float)n * C);
   k_pc_out_bwd<<<nblk(n, 8), 256, 0, st>>>(
       n, K, C, scale, (const float *)p->par.p, nbr, ef, h + PC_L * nh, R, Y, G, dh);
-  const unsigned nch = nblk(n, PC_WG_CHUNK);
+  DUST_CUDA(cudaFuncSetAttribute(k_pc_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 PC_BSM));
   for (int l = PC_L - 1; l >= 0; --l) {
-    // dh holds dL/dh(l+1): mask by z(l+1)
-    k_pc_relu_bwd<<<nblk(nh, 256), 256, 0, st>>>(nh, z + (l + 1) * nh, dh);
-    k_pc_wgrad<<<nch, 256, 0, st>>>(n, dh, h + l * nh, PC_H, G, pc_off_ws(l),
-                                                   pc_off_bl(l));
-    k_pc_wgrad<<<nch, 256, 0, st>>>(n, dh, m + l * nh, PC_H, G, pc_off_wn(l), -1);
-    k_pc_layer_bwd<<<n, PC_H, 0, st>>>(n, (const float *)p->par.p, l, dh, dhp, dm);
+    // dh holds dL/dh(l+1)
+    k_pc_layer_bwd<<<nblk(n, PC_BN), 256, PC_BSM, st>>>(n, (const float *)p->par.p, l, dh,
+                                                        z + (l + 1) * nh, h + l * nh, m + l * nh,
+                                                        G, dhp, dm);
     k_pc_agg_bwd<<<nblk(nh, 256), 256, 0, st>>>(n, K, nbr, w, dm, dhp);
     std::swap(dh, dhp);
   }
-  k_pc_relu_bwd<<<nblk(nh, 256), 256, 0, st>>>(nh, z, dh);
-  k_pc_wgrad<<<nch, 256, 0, st>>>(n, dh, x, PC_FIN, G, pc_off_w0(), pc_off_b0());
+  k_pc_in_bwd<<<nblk(n, PC_WG_CHUNK), 256, 0, st>>>(n, dh, z, x, G);
   DUST_CUDA(cudaGetLastError());
   if (loss_host) {
     float l = 0.f;
