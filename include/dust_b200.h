@@ -17,7 +17,10 @@
  * owns one CUDA stream.  The handle-less host-array calls (dust_points_uvort,
  * dust_points_uvort_pressure, dust_particles_update, ...) keep their device
  * staging buffers across calls, so they too are called from one host thread
- * at a time.
+ * at a time.  The handle-less device-array calls (dust_points_uvort_device,
+ * dust_points_uvort_pressure_device, dust_particles_update_pa_device) may
+ * overlap, on several streams and from several threads: each takes its scratch
+ * from a few sets kept by the library.
  */
 #ifndef DUST_B200_H
 #define DUST_B200_H
