@@ -1069,7 +1069,7 @@ FLOP_P2P_PAIR = 95
 # DRAM bytes per launch measured by ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum) on the 300k-particle case and scaled by the particle
 # count to 2M (profiles/k_elem_far_300k.txt)
-TRAFFIC_ELEM_FAR_PER_PARTICLE = 381.5
+TRAFFIC_ELEM_FAR_PER_PARTICLE = 479.3
 # DRAM bytes per launch per particle of the 300k-particle full step (ncu,
 # profiles/k_uvort_300k.txt, k_m2l_batch_300k.txt, k_p2p_w_f32_300k.txt),
 # scaled by the particle count to the benchmark's size
@@ -1079,8 +1079,8 @@ TRAFFIC_P2P_F32_PER_PARTICLE = 145.3e6 / 3.0e5
 # FMA-pipe activity of the FP32C kernels, and FP64 tensor-pipe activity of the
 # M2L, in the same captures (profiles/*_300k.txt)
 DMMA_PIPE_NCU = {"k_m2l_batch": 0.687}
-FMA_PIPE_NCU = {"k_p2p_w": 0.245, "k_uvort_pres_sorted": 0.807,
-                "k_elem_far": 0.67}
+FMA_PIPE_NCU = {"k_p2p_w": 0.245, "k_uvort_pres_sorted": 0.820,
+                "k_elem_far": 0.680}
 
 
 def roofline(ph, case, params, best):
