@@ -745,7 +745,7 @@ static int uvort_chunk(int pb, int n, int occ) {
 }
 
 // FP64 uvort (plain mode): FP64-pipe bound (18 FP64 operations a pair; 7,001
-// points x 50,021 particles 576 us at the start, 502 us with the chunks above,
+// points x 50,021 particles 576 us before, 502 us with the chunks above,
 // 6 CTAs of 2 points per thread and x^-3/2 in one correction, 449 us without
 // the seed's conversions, 0.75 of the operations' rate).  Particles in the caller's order, UVD_PPT points
 // per thread (consecutive CTA slices of UV2_T points) against a shared tile
