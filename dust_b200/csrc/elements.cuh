@@ -368,18 +368,21 @@ __device__ inline void vel_line_near(const RegParams &rp, const LineGeo &l, cons
 // vertices and to the projected vertices are computed once per vertex (the
 // reference's loops recompute each at both of its edges), reciprocal
 // distances and approximations refined to FP64 replace square roots and
-// quotients, and the Rankine-core test compares squares.  The solid angle
-// (pot_dou's sum of the polygon's angles less its flat value) is twice the
-// argument of the product of its triangles' complex numbers
-//   |a||b||c| + (a.b)|c| + (a.c)|b| + (b.c)|a| + i a.(b x c)
-// (van Oosterom and Strackee, IEEE Trans. Biomed. Eng. 30, 1983): one atan2
-// of products instead of one per vertex after normalisations, and no
-// cancellation of the flat value.  Same branches and values as vel_pan
-// (vel_dou, vel_sou, pot_dou) up to rounding; points beyond the far-field
-// radii and points at a vertex go to vel_pan.  The kernels that call it lose a
-// fifth of their issue slots to instruction fetches, so one copy of the
-// logarithm serves the edges and one range test the distances: 7.4 -> 6.7 ms for
-// the 134M near pairs of 2M particles.
+// quotients, and the Rankine-core test compares squares.  The solid angle is
+// pot_dou's: the sum of the angles at the polygon's vertices, less its flat
+// value where the sum passes it.  Each angle is the argument of a complex
+// number, so one atan2 of their product gives the sum up to whole turns, and
+// the turns are counted as the product is formed: two arguments of one sign add
+// up to more than pi in size where the product's imaginary part has the other
+// sign (zeros by their sign bits, as atan2 takes them).  (The product of the two
+// triangles' half angles, which needs no count, is the solid angle to the
+// triangles' surface: 2 pi off pot_dou inside the warp of a quad that is not
+// plane, and it cancels near their diagonal, 4e-10 at a height of 1e-6.)  Same
+// branches and values as vel_pan (vel_dou, vel_sou, pot_dou) up to rounding;
+// points beyond the far-field radii and points at a vertex go to vel_pan.  The
+// kernels that call it lose a fifth of their issue slots to instruction fetches,
+// so one copy of the logarithm serves the edges and one range test the
+// distances.
 template <int NV>
 __device__ inline void vel_pan_near_t(const RegParams &rp, const PanelGeo &p, const double *pos,
                                       double *v) {
@@ -475,19 +478,32 @@ __device__ inline void vel_pan_near_t(const RegParams &rp, const PanelGeo &p, co
       pdou = d3dot(rv, p.nor) * p.area / (radius * radius * radius);
     } else {
       double re = 1.0, im = 0.0;
+      int turns = 0;
 #pragma unroll
-      for (int t = 1; t + 1 < nv; ++t) {
-        const double *a = dv[0], *b = dv[t], *c = dv[t + 1];
-        double bc[3];
-        d3cross(b, c, bc);
-        const double y = d3dot(a, bc);
-        const double x = R[0] * R[t] * R[t + 1] + d3dot(a, b) * R[t + 1] + d3dot(a, c) * R[t] +
-                         d3dot(b, c) * R[0];
-        const double z = re * x - im * y;
-        im = re * y + im * x;
+      for (int i1 = 0; i1 < nv; ++i1) {
+        const int im1 = i1 == 0 ? nv - 1 : i1 - 1;
+        double ei[3], ap1[3], am1[3], cr[3];
+        for (int d = 0; d < 3; ++d) ei[d] = -dv[i1][d] * iR[i1];
+        const double ep = d3dot(ei, p.edge_vec[i1]), em = d3dot(ei, p.edge_vec[im1]);
+        for (int d = 0; d < 3; ++d) {
+          ap1[d] = p.edge_vec[i1][d] - ei[d] * ep;
+          am1[d] = -p.edge_vec[im1][d] + ei[d] * em;
+        }
+        d3cross(am1, ap1, cr);
+        const double y = d3dot(ei, cr);
+        double x = d3dot(am1, ap1);
+        if (x == 0.0 && y == 0.0) x = copysign(1.0, x);
+        const double z = re * x - im * y, w = re * y + im * x;
+        if (signbit(im) == signbit(y) && signbit(w) != signbit(y)) turns += signbit(y) ? -1 : 1;
         re = z;
+        im = w;
       }
-      pdou = 2.0 * atan2(im, re);
+      pdou = atan2(im, re) + 2.0 * DUST_PI * turns;
+      const double gb = (double)(nv - 2) * DUST_PI;
+      if (pdou < -gb + 1.0e-5)
+        pdou += gb;
+      else if (pdou > gb - 1.0e-5)
+        pdou -= gb;
     }
     for (int d = 0; d < 3; ++d)
       vs[d] = -(p.tang[0][d] * phix + p.tang[1][d] * phiy + p.nor[d] * pdou);

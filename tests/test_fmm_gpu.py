@@ -452,3 +452,41 @@ def test_uvort_calls_on_several_streams(prec):
     for s, a in zip(sets, alone):
         for k, x in zip(("uv", "up", "pt"), a):
             assert rel(s[k].cpu().numpy(), x.cpu().numpy()) < 1e-12
+
+
+@pytest.mark.parametrize("prec", [abi.DUST_PREC_FP64, abi.DUST_PREC_FP32C])
+@pytest.mark.parametrize("warp", [0.0, 0.05, 0.3])
+def test_element_sums_close_to_panels(warp, prec):
+    """Particles just above surface panels, over the diagonals and inside the
+    warp of quads whose vertices do not lie in a plane.  The vertices' angles
+    that the reference sums are well away from their branches here (1e-6 and
+    more off every plane of three vertices, 0.2 edges from the edges), so near
+    pairs, FP64 in both precisions, equal the oracle to their rounding: 1e-11
+    of the largest velocity."""
+    rng = np.random.default_rng(7)
+    ver, cen = [], []
+    for k in range(12):
+        q = np.array([[0, 0, 0], [1, 0.1, 0], [1.2, 1.1, 0], [0.1, 0.9, 0]], float)
+        q += 0.1 * rng.standard_normal((4, 3)) * [1, 1, 0]
+        q[:, 2] = warp * np.array([1, -1, 1, -1]) * rng.uniform(0.5, 1.0, 4)
+        for z in (3e-1, 1e-1, 1e-2, 1e-3, 1e-4, 1e-6, -1e-2, -1e-6):
+            for d in (0, 1):  # above or below a diagonal's point
+                p = q[d] + rng.uniform(0.3, 0.7) * (q[d + 2] - q[d])
+                cen.append(p + [0, 0, z] + [4.0 * k, 0, 0])
+        for _ in range(8):  # about the centre, through the warp
+            cen.append(q.mean(axis=0) + [4.0 * k, 0, 0] +
+                       rng.uniform(-1, 1, 3) * [0.1, 0.1, max(warp, 0.01)])
+        ver.append(q + [4.0 * k, 0, 0])
+    body = abi.PanelSet(np.array(ver), kind=np.full(12, abi.DUST_ELEM_SURFPAN),
+                        mag=rng.standard_normal(12))
+    cen = np.array(cen)
+    n = len(cen)
+    dir_, mag, rv = np.tile([1.0, 0, 0], (n, 1)), np.zeros(n), np.full(n, 0.05)
+    prm = FmmParams(box_length=52.0, origin=(-2.0, -26.0, -26.0), n_octree_levels=4,
+                    min_octree_part=5, multipole_degree=2, rankine_rad=0.01, precision=prec,
+                    u_inf=(0.3, 0.2, 1.0))
+    els = abi.elements_struct(body)
+    ov, _, _, _ = O.fmm_apply(prm, cen, dir_, mag, rv, els)
+    v, _, _ = octree.initialize_octree(prm).apply_multipole(cen, dir_, mag, rv, els)
+    far = 1e-6 if prec == abi.DUST_PREC_FP32C else 0.0  # the other panels' FP32 far field
+    assert np.abs(v - ov).max() < (1e-11 + far) * np.abs(ov).max()
