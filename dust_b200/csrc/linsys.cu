@@ -375,7 +375,8 @@ int linsys_solve_lu64(dust_linsys *L, double *res_dev) {
   int *P = (int *)L->piv.p;
   cublasSetStream(L->cb, L->st);
   const double one = 1.0, mone = -1.0;
-  // the unpivoted static factors come with their inverse blocks
+  // the unpivoted static factors come with their inverse blocks, where those are
+  // accepted
   const bool blocks_s = nst == 0 || L->lu_s.inv_n == nst;
   if (nst > 0 && nmv > 0) {
     if (blocks_s) {
@@ -412,11 +413,13 @@ int linsys_solve_lu64(dust_linsys *L, double *res_dev) {
           return DUST_OK;
         },
         &L->last_pivoted));
-    int info = 0;
-    DUST_CUDA(cudaMemcpy(&info, L->info.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (info) return DUST_ERR_SINGULAR;
-    if (!L->last_pivoted)
+    if (!L->last_pivoted) {  // (without a zero pivot)
       DUST_TRY(lu_inv_build<double>(L->st, L->lu, nmv, Amm, n));
+    } else {
+      int info = 0;
+      DUST_CUDA(cudaMemcpy(&info, L->info.p, sizeof(int), cudaMemcpyDeviceToHost));
+      if (info) return DUST_ERR_SINGULAR;
+    }
     if (nst > 0) {
       // dlaswp on A(nst+1:rank, 1:nst) with the moving pivots, then make
       // them global
@@ -426,7 +429,7 @@ int linsys_solve_lu64(dust_linsys *L, double *res_dev) {
   }
   L->factored = true;
   DUST_CUDA(cudaMemcpyAsync(res_dev, L->b.p, (size_t)n * 8, cudaMemcpyDeviceToDevice, L->st));
-  if (blocks_s && (nmv == 0 || !L->last_pivoted))
+  if (blocks_s && (nmv == 0 || (!L->last_pivoted && L->lu.inv_n == nmv)))
     return nst == 0 ? lu_solve_blocks<double>(L->st, L->lu.np_x, n, 1, A, n, res_dev, n, L->lu)
                     : lu_solve_blocks<double>(L->st, L->lu.np_x, n, 1, A, n, res_dev, n, L->lu_s,
                                               nmv > 0 ? &L->lu : nullptr);

@@ -41,7 +41,7 @@ struct LuWork {
   DevBuf np;     // unpivoted LU: max |l| word, inverse triangles of every
                  // diagonal block (kept for lu_inv_build)
   DevBuf inv;    // inverses of L's and U's larger diagonal blocks (lu_inv_build)
-  int inv_n = 0; // order of the system they belong to (0: none)
+  int inv_n = 0; // order of the system they belong to (0: none, or not accepted)
   DevBuf np_x;   // lu_solve_blocks: the intermediate Y = L^-1 B
   LuSide side;   // lu_getrf_nopiv: the next panel's stream
   int nsm = 0;
@@ -80,7 +80,9 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
                    int *ipiv, int gemm_update, int *perm, float *lmax);
 
 // Inverses of the 512 x 512 diagonal blocks of L and U from the kept 64 x 64
-// ones of the last lu_getrf_nopiv on this LuWork (same A, n), into w.inv.
+// ones of the last lu_getrf_nopiv on this LuWork (same A, n), into w.inv.  Sets
+// w.inv_n = n where the blocks' condition lets products with them stand for a
+// substitution, else 0: then lu_getrs solves (waits for the stream).
 template <typename T>
 int lu_inv_build(cudaStream_t st, LuWork &w, int n, const T *A, int lda);
 

@@ -143,7 +143,7 @@ int mixed_solve_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, DevBuf &w
       if (it == max_iter) break;
     }
     k_to_f32<<<256, 256, 0, st>>>(nr, R, D32);
-    if (piv == 0)
+    if (piv == 0 && lu.inv_n == n)
       DUST_TRY(lu_solve_blocks<float>(st, lu.np_x, n, nrhs, A32, n, D32, n, lu));
     else
       DUST_TRY(lu_getrs<float>(cb, st, n, nrhs, A32, n, ipiv, D32, n));
@@ -195,7 +195,7 @@ static int dense_lu64_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, Dev
   if (r) r->pivoted = pivd;
   cudaEventRecord(e1, st);
   int hinfo = 0;
-  if (s == DUST_OK) {
+  if (s == DUST_OK && pivd) {  // (unpivoted factors have no zero pivot)
     cudaMemcpyAsync(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) s = DUST_ERR_CUDA;
     else if (hinfo) s = DUST_ERR_SINGULAR;
@@ -204,8 +204,9 @@ static int dense_lu64_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, Dev
     if (X != B && cudaMemcpyAsync(X, B, nr * 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       s = DUST_ERR_CUDA;
     if (s == DUST_OK)
-      s = pivd == 0 ? lu_solve_blocks<double>(st, lu.np_x, n, nrhs, (const double *)F.p, n, X, n, lu)
-                    : lu_getrs<double>(cb, st, n, nrhs, (const double *)F.p, n, ipiv, X, n);
+      s = pivd == 0 && lu.inv_n == n
+              ? lu_solve_blocks<double>(st, lu.np_x, n, nrhs, (const double *)F.p, n, X, n, lu)
+              : lu_getrs<double>(cb, st, n, nrhs, (const double *)F.p, n, ipiv, X, n);
     cudaEventRecord(e2, st);
   }
   if (s == DUST_OK && cudaStreamSynchronize(st) == cudaSuccess && r) {

@@ -17,10 +17,21 @@
 
 #include "lu.cuh"
 
+// A product with the inverse of a triangular block T leaves a residual of up to
+// cond(T) = || |T^-1| |T| ||_inf times a substitution's.  Certified factors
+// (multipliers below 1) do not bound it: multipliers of -0.1 alone make it grow like
+// 1.1^512.  So lu_inv_build measures it, and above TI_COND the inverses are not
+// used (w.inv_n = 0): the caller substitutes.  Panels' systems have 1.4 to 6
+// (ellipsoids, rotor and fuselage, their Schur complements), where both ways have
+// the same backward errors; at 700 a solve by blocks has ten times the
+// substitution's, at 2e4 a hundred times.  An FP32 solve is refined, and a
+// sweep gains digits as long as cond(T) 6e-8 is small.
 #define TI_B 512
 #define TI_T 64   // tile edge of the products
 #define TI_K 32   // inner dimension staged at once
 #define TI_NT 256
+template <typename T>
+constexpr float TI_COND = sizeof(T) == 8 ? 64.f : 1e4f;
 
 static inline int ti_blocks(int n) { return (n + TI_B - 1) / TI_B; }
 
@@ -177,6 +188,49 @@ __global__ void __launch_bounds__(TI_NT) k_ti_merge(int n, int s, int phase, con
           phase == 0 ? acc[u][v] : -acc[u][v];
 }
 
+// cond(T) of every block (blockIdx.y) of L (blockIdx.z = 0) and U (1): a CTA
+// takes 32 rows (lanes), its 8 warps the columns, 16 loads in flight per thread.
+// Phase 0 writes w = |T| 1, phase 1 the largest (|T^-1| w)_r (float bits, infinity
+// where it is no number).
+template <typename T>
+__global__ void __launch_bounds__(TI_NT) k_ti_cond(int n, int phase, const T *A, int lda, T *inv,
+                                                   double *w, unsigned *bits) {
+  __shared__ double s_s[TI_NT / 32][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, r = 32 * blockIdx.x + lane;
+  const int k = TI_B * blockIdx.y, m = min(TI_B, n - k), up = blockIdx.z;
+  w += (size_t)(2 * blockIdx.y + up) * TI_B;
+  const T *M = phase == 0 ? A + (size_t)k + (size_t)k * lda
+                          : ti_linv(inv, blockIdx.y) + (up ? (size_t)TI_B * TI_B : 0);
+  const size_t ld = phase == 0 ? lda : TI_B;
+  double s = 0.0;
+  for (int c0 = g; c0 < m; c0 += 16 * (TI_NT / 32)) {
+    double v[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const int c = c0 + q * (TI_NT / 32);
+      // (L's diagonal: 1)
+      const bool in = r < m && c < m && (up ? c >= r : c < r);
+      v[q] = in ? fabs((double)M[r + c * ld]) : (c == r ? 1.0 : 0.0);
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const int c = c0 + q * (TI_NT / 32);
+      if (c < m) s += phase == 0 ? v[q] : v[q] * w[c];
+    }
+  }
+  s_s[g][lane] = s;
+  __syncthreads();
+  if (g > 0) return;
+  for (int q = 1; q < TI_NT / 32; ++q) s += s_s[q][lane];
+  if (phase == 0) {
+    if (r < m) w[r] = s;
+    return;
+  }
+  float f = s <= 3.0e38 ? (float)s : INFINITY;
+  for (int o = 16; o > 0; o >>= 1) f = fmaxf(f, __shfl_xor_sync(~0u, f, o));
+  if (lane == 0) atomicMax(bits, __float_as_uint(f));
+}
+
 template <typename T>
 int lu_inv_build(cudaStream_t st, LuWork &w, int n, const T *A, int lda) {
   w.inv_n = 0;
@@ -187,13 +241,21 @@ int lu_inv_build(cudaStream_t st, LuWork &w, int n, const T *A, int lda) {
   DUST_TRY(devbuf_grow(w.inv, (per + per / 4) * sizeof(T)));
   T *inv = (T *)w.inv.p, *tmp = inv + per;
   const T *np = (const T *)((const char *)w.np.p + 256);
+  unsigned *bits = (unsigned *)w.np.p + 1;
+  DUST_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned), st));
   k_ti_init<T><<<(unsigned)((per + 255) / 256), 256, 0, st>>>(n, np, inv);
   for (int s = 64; s < TI_B && s < n; s *= 2)
     for (int ph = 0; ph < 2; ++ph)
       k_ti_merge<T><<<dim3((s / TI_T) * (s / TI_T), nb * (TI_B / (2 * s)), 2), TI_NT, 0, st>>>(
           n, s, ph, A, lda, inv, tmp);
+  for (int ph = 0; ph < 2; ++ph)  // (tmp: the merges are done with it)
+    k_ti_cond<T><<<dim3((std::min(TI_B, n) + 31) / 32, nb, 2), TI_NT, 0, st>>>(
+        n, ph, A, lda, inv, (double *)tmp, bits);
   DUST_CUDA(cudaGetLastError());
-  w.inv_n = n;
+  float cond = INFINITY;
+  DUST_CUDA(cudaMemcpyAsync(&cond, bits, sizeof(float), cudaMemcpyDeviceToHost, st));
+  DUST_CUDA(cudaStreamSynchronize(st));
+  if (cond <= TI_COND<T>) w.inv_n = n;
   return DUST_OK;
 }
 

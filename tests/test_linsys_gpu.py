@@ -256,3 +256,57 @@ def test_linsys_wake_rows_ragged(n_span, n_chord, nst_frac):
     Ag, bg = ls.get_system()
     assert rel(Ag, Ao) < 1e-10
     assert rel(bg, bo) < 1e-10
+
+
+def growing_system(n, nrhs, seed):
+    """Multipliers of -0.1 in blocks of 200 rows: partial pivoting interchanges
+    nothing, and the inverses of the blocks grow to 1.1^199 = 1.7e8."""
+    rng = np.random.default_rng(seed)
+    blk = np.arange(n) // 200
+    L = np.tril(np.where(blk[:, None] == blk[None, :], -0.1, 0.0), -1) + np.eye(n)
+    A = L @ (np.triu(rng.standard_normal((n, n)) / n, 1) + np.diag(rng.uniform(1.0, 3.0, n)))
+    return A, A @ rng.standard_normal((n, nrhs))
+
+
+@pytest.mark.parametrize("n,nrhs", [(200, 1), (200, 3), (600, 1), (600, 40), (1100, 65), (1700, 1)])
+def test_dense_growing_inverse(n, nrhs):
+    """Products with inverses of large diagonal blocks lose eight digits here and
+    substitution none.  Blocks of 64 (1.1^63 = 405), which the factorisation
+    itself uses, leave 405 (1 + 0.1 64) eps = 7e-13 at most."""
+    A, B = growing_system(n, nrhs, n)
+    X, rep = linsys.dense_solve(A, B, abi.DUST_SOLVE_LU64)
+    assert rep["pivoted"] == 0
+    assert np.abs(B - A @ X).max() < 1e-12 * np.abs(A).sum(axis=1).max() * np.abs(X).max()
+
+
+@pytest.mark.parametrize("n,nrhs", [(65, 1), (513, 3), (1090, 65)])
+def test_dense_mixed_sweeps(n, nrhs):
+    """Each sweep of the mixed solve gains the FP32 factors' digits (three at
+    least, with TF32 updates): 1e-12 takes five sweeps at most, which a fault in
+    the FP32 block solves would exceed."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) / n + 2.0 * np.eye(n)
+    X, rep = linsys.dense_solve(A, rng.standard_normal((n, nrhs)), abi.DUST_SOLVE_MIXED, 1e-12)
+    assert rep["iterations"] <= 5 and rep["pivoted"] == 0
+
+
+@pytest.mark.parametrize("nst_frac", [1.0, 0.5, 0.0])
+@pytest.mark.parametrize("mode", [abi.DUST_SOLVE_LU64, abi.DUST_SOLVE_MIXED])
+def test_linsys_stacked_plates(nst_frac, mode):
+    """Plates of falling size behind one another: multipliers below 0.9, but the
+    condition of L's blocks (1e3) asks for substitution in the static block, the
+    moving one or both.  Backward error of n eps, 120 x 2.2e-16, times four."""
+    n = 120
+    size = 0.93 ** np.arange(n)
+    ver = np.zeros((n, 4, 3))
+    ver[:, :, :2] = 0.5 * np.array([[-1, -1], [1, -1], [1, 1], [-1, 1]]) * size[:, None, None]
+    ver[:, :, 2] = -size[:, None]
+    els = abi.PanelSet(ver, kind=np.full(n, abi.DUST_ELEM_SURFPAN), mag=np.zeros(n))
+    prm = FmmParams(u_inf=(1.0, 0.0, 0.2), rankine_rad=0.1)
+    ls = linsys.initialize_linsys(prm, n, int(n * nst_frac), els)
+    none = (abi.empty_panels(), 0, np.zeros((1, 2), dtype=np.int32))
+    A, b, _ = O.linsys_run(prm, n, 0, els, els, none, none)
+    for _ in range(2):
+        ls.assemble_linsys(els)
+        x, rep = ls.solve_linsys(mode)
+        assert np.abs(b - A @ x).max() < 1e-13 * np.abs(A).sum(axis=1).max() * np.abs(x).max()
