@@ -1257,7 +1257,12 @@ __device__ __forceinline__ void p2p_share(const FmmDev &d, uint32_t leaf, int tb
         for (int q = 3; q < 6; ++q) st8[q] = (R)pf[q];
         const R rv = (R)pf[6];
         st8[6] = rv * rv;
-        if (VD) st8[7] = F32 ? (R)1 / st8[6] : (R)17.5 / rv;
+        if (VD) {
+          // (a core of zero diffuses nothing, and the particle itself is among the
+          // sources, with inv = 0)
+          const R k = F32 ? (R)1 / st8[6] : (R)17.5 / fabs(rv);
+          st8[7] = isinf(k) ? (R)0 : k;
+        }
       }
       s_sid[lane] = psid;
 #pragma unroll

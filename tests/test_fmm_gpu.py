@@ -490,3 +490,19 @@ def test_element_sums_close_to_panels(warp, prec):
     v, _, _ = octree.initialize_octree(prm).apply_multipole(cen, dir_, mag, rv, els)
     far = 1e-6 if prec == abi.DUST_PREC_FP32C else 0.0  # the other panels' FP32 far field
     assert np.abs(v - ov).max() < (1e-11 + far) * np.abs(ov).max()
+
+
+@pytest.mark.parametrize("prec", [abi.DUST_PREC_FP64, abi.DUST_PREC_FP32C])
+def test_near_field_core_of_zero_or_negative(prec):
+    """A particle without a core has no pair with itself, and the core enters
+    by its square."""
+    prm = prm_ring(precision=prec)
+    one = np.array([[0.1, 0.2, 0.3]])
+    for out in octree.initialize_octree(prm).apply_multipole(one, np.array([[0, 0, 1.0]]),
+                                                             np.ones(1), np.zeros(1)):
+        assert np.array_equal(out, np.zeros((1, 3)))
+    cen, dir_, mag, rv = ring(900, seed=4)
+    oc = octree.initialize_octree(prm)
+    a, b = oc.apply_multipole(cen, dir_, mag, rv), oc.apply_multipole(cen, dir_, mag, -rv)
+    for x, y in zip(a, b):
+        assert rel(x, y) < 1e-13
