@@ -32,6 +32,7 @@
 #include "dust_common.cuh"
 #include "elements.cuh"
 #include "fmm_internal.h"
+#include "near_list.h"
 
 static inline unsigned nblk(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(EF2_T, 8) k_elem_far(FmmDev d, ElemDev e, cons
 }
 
 // The listed near pairs, exact FP64 (one pair per thread).  Where the list
-// overflowed its capacity (it grows before the next evaluation), every
+// overflowed its capacity (near_list.h), every
 // (particle, panel) pair is tested again, with the far kernel's own test, and
 // the list is not used.
 #ifndef EN_MINB
@@ -655,8 +656,37 @@ static int elem_chunk(unsigned pblocks, int ntot, int load) {
   return std::min(std::max(1, (loads + want - 1) / want), (1 << 21) / load) * load;
 }
 
-int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
-                       size_t &near_cap, unsigned long long near_seen,
+// The list for this evaluation: *cap pairs (0, without memory for any: every
+// pair is then tested again).  The old list is kept until a larger one is there.
+#define NEAR_SMALL ((size_t)256 << 20)  // a size that needs no look at the free memory
+static int near_list(DevBuf &list, size_t n, size_t panels, unsigned long long seen, size_t limit,
+                     size_t *cap) {
+  const size_t most = limit ? limit : SIZE_MAX, have = list.cap / sizeof(NearPair);
+  if (!list.p || (seen > have && have < most)) {
+    auto size = [&](size_t lim) {
+      return list.p ? near_list_next(have, seen, lim) : near_list_first(n, panels, lim);
+    };
+    size_t want = size(most);
+    if (!limit && want * sizeof(NearPair) > NEAR_SMALL) {  // at most a quarter of what is free
+      size_t avail = 0, total = 0;
+      DUST_CUDA(cudaMemGetInfo(&avail, &total));
+      want = size((avail + list.cap) / 4 / sizeof(NearPair));
+    }
+    void *p = nullptr;
+    if (want > have && cudaMalloc(&p, want * sizeof(NearPair)) == cudaSuccess) {
+      devbuf_free(list);
+      list.p = p;
+      list.cap = want * sizeof(NearPair);
+    } else {
+      cudaGetLastError();
+    }
+  }
+  *cap = std::min(most, list.cap / sizeof(NearPair));
+  return DUST_OK;
+}
+
+int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &near_buf,
+                       size_t near_limit, unsigned long long near_seen,
                        unsigned long long *count, int precision,
                        double *vel, double *str, double *rot, cudaStream_t st, cudaEvent_t *kev,
                        bool *kev_done) {
@@ -671,17 +701,10 @@ int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
     if (e.nbody) k_ffrec<<<nblk(e.nbody, 128), 128, 0, st>>>(e.body, e.nbody, e.rp.ff_dou, ff);
     if (e.nwake)
       k_ffrec<<<nblk(e.nwake, 128), 128, 0, st>>>(e.wake, e.nwake, e.rp.ff_dou, ff + e.nbody);
-    // near-pair list: a first size, grown when the previous evaluation on the
-    // handle listed more (near_seen)
-    if (near_cap == 0)
-      near_cap = std::max(std::max<size_t>(1 << 20, n * 96),
-                          std::min<size_t>(n * (size_t)ntot / 8, 1 << 26));
-    if (near_seen > near_cap) near_cap = (size_t)(near_seen + near_seen / 4 + 1024);
-    const size_t off_l = (n * 24 + 255) / 256 * 256;
-    DUST_TRY(devbuf_grow(work, off_l + near_cap * sizeof(NearPair)));
-    farv = (double *)work.p;
-    NearPair *list = (NearPair *)((char *)work.p + off_l);
-    const unsigned long long cap = near_cap;
+    size_t cap = 0;
+    DUST_TRY(near_list(near_buf, n, (size_t)ntot, near_seen, near_limit, &cap));
+    farv = d.out + 9 * n;  // the panels' sums
+    NearPair *list = (NearPair *)near_buf.p;
     const unsigned pb = nblk(n, f32 ? EF2_NP : EO_NP);
     const int chunk = elem_chunk(pb, ntot, f32 ? EF2_LOAD : EO_LOAD);
     const dim3 grid(pb, nblk(ntot, chunk));

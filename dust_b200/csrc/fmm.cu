@@ -222,7 +222,7 @@ extern "C" int dust_octree_destroy(dust_octree *o) {
   devbuf_free(o->p2p_work);
   devbuf_free(o->shift);
   devbuf_free(o->ffbuf);
-  devbuf_free(o->elem_work);
+  devbuf_free(o->near_buf);
   DevBuf *bufs[] = {&o->idxsum, &o->keys,   &o->keys_s, &o->vals,   &o->perm,
                     &o->cnt,    &o->cstart, &o->part,   &o->flags,
                     &o->cidx,   &o->lidx,   &o->act_key, &o->act_lev, &o->leaf_ci,
@@ -240,6 +240,12 @@ extern "C" int dust_octree_get_stats(const dust_octree *o, dust_fmm_stats *st) {
   *st = o->stats;
   return DUST_OK;
 }
+extern "C" int dust_octree_set_near_limit(dust_octree *o, long long pairs) {
+  if (!o || pairs < 0) return DUST_ERR_BAD_ARG;
+  o->near_limit = (size_t)pairs;
+  return DUST_OK;
+}
+
 extern "C" int dust_octree_set_timing(dust_octree *o, int on) {
   if (!o) return DUST_ERR_BAD_ARG;
   o->timing = on != 0;
@@ -1446,7 +1452,7 @@ int fmm_prepare_device(dust_octree *o, int n, const double *cen, const double *d
   DUST_TRY(grow(o->cidx, (size_t)(ntot + 1) * 4));
   DUST_TRY(grow(o->lidx, (size_t)(ntot + 1) * 4));
   DUST_TRY(grow(o->srcix, (size_t)(ntot + 1) * 4));
-  DUST_TRY(grow(o->outs, N * 9 * 8));
+  DUST_TRY(grow(o->outs, N * 12 * 8));
   uint32_t *keys = (uint32_t *)o->keys.p, *keys_s = (uint32_t *)o->keys_s.p;
   uint32_t *vals = (uint32_t *)o->vals.p, *perm = (uint32_t *)o->perm.p;
   uint32_t *cnt = (uint32_t *)o->cnt.p, *cstart = (uint32_t *)o->cstart.p;
@@ -1767,7 +1773,7 @@ int fmm_points_uvort_device(dust_octree *o, const ElemDev &lines, double *uv, cu
 int fmm_finish_device(dust_octree *o, int n, const ElemDev &e, double *vel, double *str,
                       double *rot, cudaStream_t st) {
   if (n > 0)
-    DUST_TRY(elem_output_device(o->dev, e, o->ffbuf, o->elem_work, o->near_cap, o->near_seen,
+    DUST_TRY(elem_output_device(o->dev, e, o->ffbuf, o->near_buf, o->near_limit, o->near_seen,
                                 (unsigned long long *)o->small.p + 52, o->prm.precision, vel, str,
                                 rot, st, o->timing ? &o->ev[8] : nullptr, &o->kev_far));
   if (o->timing) cudaEventRecord(o->ev[5], st);

@@ -38,7 +38,8 @@ struct FmmDev {
   double *ahat;        // scaled multipoles of the M2L sources, cells ahat_c0 .., rows of
   uint32_t ahat_c0;    // ahat_rs (m2l.cu)
   int ahat_rs;
-  double *out;         // sorted-order vel(3), stretch(3), rotu(3), SoA
+  double *out;         // sorted-order vel(3), stretch(3), rotu(3), SoA; then the
+                       // element sums' velocities (3)
   int64_t *counters;   // [0] M2L pairs, [1] P2P pairs
   double inv_fact[224];
 };
@@ -69,8 +70,8 @@ struct dust_octree {
   DevBuf act_key, act_lev, leaf_ci, mp, outs, cub_tmp, small;
   DevBuf h_in, h_out, h_pts, el_geo, el_raw;  // staging of host-API calls
   DevBuf ffbuf;                        // far-field panel records
-  DevBuf elem_work;                    // element sums: far sums, near-pair list
-  size_t near_cap = 0;                 // capacity of the near-pair list
+  DevBuf near_buf;                     // element sums: near-pair list
+  size_t near_limit = 0;               // its largest size in pairs (0: by the free memory)
   unsigned long long near_seen = 0;    // pairs that an evaluation before listed
   DevBuf dtabs[DUST_MAXLEV + 1];       // dimensionless scalar M2L tables (FP64)
   DevBuf jsum;                         // M2L index table, then the classes' offsets
@@ -136,8 +137,8 @@ int m2l_all_levels(dust_octree *o, FmmDev &d, cudaStream_t st);
 
 
 // direct.cu
-int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &work,
-                       size_t &near_cap, unsigned long long near_seen,
+int elem_output_device(FmmDev &d, const ElemDev &e, DevBuf &ffbuf, DevBuf &near_buf,
+                       size_t near_limit, unsigned long long near_seen,
                        unsigned long long *count, int precision,
                        double *vel, double *str, double *rot, cudaStream_t st,
                        cudaEvent_t *kev = nullptr, bool *kev_done = nullptr);

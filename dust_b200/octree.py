@@ -40,6 +40,12 @@ class Octree:
     def set_timing(self, on=True):
         check(lib().dust_octree_set_timing(self._h, int(bool(on))), "dust_octree_set_timing")
 
+    def set_near_limit(self, pairs):
+        """Largest near-pair list the handle keeps (8 bytes a pair); 0: a
+        quarter of the free device memory."""
+        check(lib().dust_octree_set_near_limit(self._h, C.c_longlong(int(pairs))),
+              "dust_octree_set_near_limit")
+
     def stats(self):
         s = abi.FmmStats()
         check(lib().dust_octree_get_stats(self._h, C.byref(s)), "dust_octree_get_stats")

@@ -218,6 +218,12 @@ DUST_API int dust_fmm_finish_device(dust_octree *oct, const dust_elements *elems
 DUST_API int dust_octree_get_stats(const dust_octree *oct, dust_fmm_stats *st);
 DUST_API int dust_octree_set_timing(dust_octree *oct, int on);
 
+/* Largest list of near (particle, panel) pairs that the handle keeps for the
+ * element sums, 8 bytes a pair; 0 (the default): a quarter of the free device
+ * memory.  Where the pairs do not fit, every pair is tested again: the same
+ * sums in more time. */
+DUST_API int dust_octree_set_near_limit(dust_octree *oct, long long pairs);
+
 /* Direct O(N^2) evaluation of the same particle kernels over all pairs
  * (the reference's P2P formulas of src/aeroel/mod_vortpart.f90:139-336
  * applied to every particle pair); used as the FMM truth.  Targets are the

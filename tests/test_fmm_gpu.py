@@ -506,3 +506,26 @@ def test_near_field_core_of_zero_or_negative(prec):
     a, b = oc.apply_multipole(cen, dir_, mag, rv), oc.apply_multipole(cen, dir_, mag, -rv)
     for x, y in zip(a, b):
         assert rel(x, y) < 1e-13
+
+
+@pytest.mark.parametrize("prec", [abi.DUST_PREC_FP64, abi.DUST_PREC_FP32C])
+def test_near_pairs_beyond_the_list_limit(prec):
+    """12,000 near pairs on a list held to 1,000: every evaluation tests the
+    pairs again and equals the oracle, and with the limit lifted they are listed."""
+    rng = np.random.default_rng(3)
+    wing, te = synth.flat_wing(span=2.0, chord=1.0, n_span=8, n_chord=5)
+    body = abi.PanelSet(wing.ver, kind=wing.kind, mag=rng.standard_normal(wing.n))
+    n = 300
+    cen = rng.uniform([-0.4, -1.4, 0.05], [1.4, 1.4, 0.6], (n, 3))
+    dir_ = np.tile([0.0, 1.0, 0.0], (n, 1))
+    mag, rv = np.full(n, 1e-3), np.full(n, 0.05)
+    prm = FmmParams(box_length=4.0, origin=(-1.5, -2.0, -2.0), n_octree_levels=4,
+                    min_octree_part=5, multipole_degree=4, rankine_rad=0.1, precision=prec,
+                    far_field_ratio_doublet=1e4)
+    els = abi.elements_struct(body)
+    ov, _, _, _ = O.fmm_apply(prm, cen, dir_, mag, rv, els)
+    oc = octree.initialize_octree(prm)
+    for limit in (1000, 1000, 1000, 1, 1, 0, 0, 500):
+        oc.set_near_limit(limit)
+        v, _, _ = oc.apply_multipole(cen, dir_, mag, rv, els)
+        assert rel(v, ov) < (TOL64 if prec == abi.DUST_PREC_FP64 else TOL32)
