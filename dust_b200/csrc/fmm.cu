@@ -37,6 +37,7 @@
 #include "dust_common.cuh"
 #include "elements.cuh"
 #include "fmm_internal.h"
+#include "p2p_items.h"
 
 static int build_shift_tables(dust_octree *o);
 
@@ -1070,23 +1071,21 @@ __global__ void __launch_bounds__(256) k_p2p_split(FmmDev d, P2PItems w) {
   S = __reduce_add_sync(0xffffffffu, S) + nt;
   if (lane == 0 && nt > 0 && d.counters)
     atomicAdd((unsigned long long *)d.counters + 1, (unsigned long long)nt * (S - 1));
-  // sources per item of a full block of 32 targets and of the last block
-  const uint32_t nb = nt / 32, rem = nt % 32;
-  const uint32_t seg_r = rem ? (uint32_t)w.it * (32u / rem) : 1u;
-  const uint32_t ni_b = (S + w.it - 1) / w.it, ni_r = rem ? (S + seg_r - 1) / seg_r : 0u;
-  const uint32_t ni = nb * ni_b + ni_r;
-  bool split = ni > 1;
-  unsigned long long at = 0;
-  if (split) {
-    if (lane == 0) at = atomicAdd(w.count, (unsigned long long)ni);
-    at = __shfl_sync(0xffffffffu, at, 0);
-    if (at + ni > w.cap) split = false;
-    for (uint32_t e = lane; e < ni; e += 32) {
-      const uint32_t b = min(e / ni_b, nb), s = e - b * ni_b, seg = b < nb ? (uint32_t)w.it : seg_r;
-      // (an item past the list's end is never read: the count is clamped)
-      if (at + e < w.cap)
-        w.item[at + e] = split ? make_uint4(leaf, 32 * b, s * seg, min(S, (s + 1) * seg))
-                               : make_uint4(leaf, 0, 0, 0);
+  bool split = false;
+  if (nt > 0) {
+    const P2PCut c = p2p_cut(nt, S, (uint32_t)w.it, w.cap);
+    if (c.ni > 1 && c.ni <= w.cap) {  // (else whole, and nothing of the list taken)
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(w.count, (unsigned long long)c.ni);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      split = at + c.ni <= w.cap;
+      for (uint32_t e = lane; e < c.ni; e += 32) {
+        uint32_t tb, s0, s1;
+        p2p_item(c, S, e, tb, s0, s1);
+        // (an item past the list's end is never read: the count is clamped)
+        if (at + e < w.cap)
+          w.item[at + e] = split ? make_uint4(leaf, tb, s0, s1) : make_uint4(leaf, 0, 0, 0);
+      }
     }
     if (split)
       for (uint32_t t = lane; t < nt; t += 32)
