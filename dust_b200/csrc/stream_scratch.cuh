@@ -6,7 +6,9 @@
 // own stream's, an unused one, one whose last use has finished, or else the
 // least recently used one, for which its stream waits.  The pool is locked while
 // a call is queued, so host threads may call at the same time.  Buffers grow and
-// are kept; there are never more than SLOTS sets of them.
+// are kept; there are never more than SLOTS sets of them.  A captured call holds
+// its buffers' addresses without an event: the caller keeps the graph's launches
+// apart from other calls.
 #pragma once
 
 #include <mutex>
@@ -64,6 +66,10 @@ class StreamScratch {
       if (!s && c.dev == dev && c.st == st) s = &c;
     for (Slot &c : slot_)
       if (!s && c.dev < 0) s = &c;
+    // (a query is among the calls that spoil another stream's capture of this
+    // thread, or of any in the global mode, unless this thread's mode is relaxed)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    DUST_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     for (Slot &c : slot_)
       if (!s && !u.capturing_ && c.dev == dev) {
         if (cudaEventQuery(c.done) == cudaSuccess)
@@ -71,6 +77,7 @@ class StreamScratch {
         else
           cudaGetLastError();  // not ready
       }
+    DUST_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     for (int same = 1; same >= 0 && !s; --same)
       for (Slot &c : slot_)
         if ((!same || c.dev == dev) && (!s || c.turn < s->turn)) s = &c;

@@ -20,7 +20,10 @@
  * at a time.  The handle-less device-array calls (dust_points_uvort_device,
  * dust_points_uvort_pressure_device, dust_particles_update_pa_device) may
  * overlap, on several streams and from several threads: each takes its scratch
- * from a few sets kept by the library.
+ * from a few sets kept by the library.  A call captured into a graph keeps the
+ * addresses of the set it was given, so the graph's launches must not overlap
+ * with other calls of these, nor follow a call that made the set grow
+ * (dust_points_uvort_device_noalloc has scratch of a fixed address).
  */
 #ifndef DUST_B200_H
 #define DUST_B200_H

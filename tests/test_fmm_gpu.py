@@ -529,3 +529,42 @@ def test_near_pairs_beyond_the_list_limit(prec):
         oc.set_near_limit(limit)
         v, _, _ = oc.apply_multipole(cen, dir_, mag, rv, els)
         assert rel(v, ov) < (TOL64 if prec == abi.DUST_PREC_FP64 else TOL32)
+
+
+def test_uvort_calls_leave_a_capture_alone():
+    """Calls on more streams than there are sets of scratch, while another
+    stream is being captured: the capture goes on and ends well."""
+    import ctypes as C
+    import torch
+    from dust_b200._lib import check, lib
+    ptr = lambda t: C.cast(C.c_void_p(t.data_ptr()), C.POINTER(C.c_double))
+    gpu = lambda a: torch.as_tensor(a, dtype=torch.float64, device="cuda").contiguous()
+    prm = prm_ring().struct()
+    cen, dir_, mag = synth.ring_particles(5000, 0, seed=1)
+    a = [gpu(x) for x in (cen[:100], cen, dir_, mag, np.full(5000, 0.05))]
+    uv = torch.empty((6, 100, 3), dtype=torch.float64, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(6)]
+    x, cap = torch.zeros(4, device="cuda"), torch.cuda.Stream()
+
+    def calls():
+        for k, s in enumerate(streams):
+            ev = abi.Lines(0, C.POINTER(C.c_double)(), C.POINTER(C.c_double)())
+            check(lib().dust_points_uvort_device(
+                C.byref(prm), 100, ptr(a[0]), 5000, ptr(a[1]), ptr(a[2]), ptr(a[3]), ptr(a[4]),
+                C.byref(ev), ptr(uv[k]), C.c_void_p(s.cuda_stream)), "uvort")
+
+    calls()
+    torch.cuda.synchronize()
+    want = uv.clone()
+    uv.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(cap):
+        g.capture_begin(capture_error_mode="global")
+        x.add_(1.0)
+        calls()
+        g.capture_end()
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.cpu().tolist() == [1.0] * 4
+    assert rel(uv.cpu().numpy(), want.cpu().numpy()) < 1e-12
