@@ -51,6 +51,8 @@ def parse():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--particles", type=int, default=2_000_000)
     ap.add_argument("--degree", type=int, default=4)
+    ap.add_argument("--details", default=os.path.join(ROOT, "bench_details.json"),
+                    help="file for the whole record of the default workload")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--quick", action="store_true", help="small case (smoke)")
@@ -597,10 +599,54 @@ def main():
             "gpu_launches": launches,
             "workloads": subs,
         }
-        print(json.dumps(line), flush=True)
+        print(json.dumps(short_line(line, write_details(line, args.details))), flush=True)
     if ws > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
+
+
+LINE_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+             "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config", "mode",
+             "uvort", "plain_fp64_ms", "speedup_vs_plain_fp64", "load_error_vs_fp64",
+             "steps_advected", "load_error_max_over_steps", "fp64_sensitivity_floor",
+             "headline_rule", "clocks", "cpu_baseline", "e2e", "gpu_launches")
+
+
+def short_line(line, details):
+    """The printed line: the whole record's keys with one figure per mode and
+    workload.  The record itself (loads and errors of every step, all phases, the
+    workloads' tables) is some 30 KB, of which a reader who keeps the end of the
+    output loses the value; it goes to ``details``."""
+    pick = lambda d, keys: {k: d[k] for k in keys if k in d}
+    out = pick(line, LINE_KEYS)
+    out["modes"] = {k: pick(v, ("ms", "load_error_vs_fp64", "load_error_max_over_steps"))
+                    for k, v in line["modes"].items()}
+    out["phases_ms"] = line["phases_ms"].get(line["mode"])
+    rf = line["roofline"]
+    keys = ("kernel", "bound", "limited_by", "achieved", "peak", "unit", "frac", "traffic", "ms")
+    out["roofline"] = dict(pick(rf, keys + ("peak_source",)),
+                           others=[pick(o, keys) for o in rf["others"]])
+    w = line.get("workloads")
+    if w:
+        res = lambda n, *keys: {k: pick(v, keys) for k, v in w[n]["results"].items()}
+        out["workloads"] = {
+            "fmm": res("fmm", "ms"), "dense": res("dense", "ms", "backward_error"),
+            "learned": res("learned", "ms_mean", "iterations_mean"),
+            "wing": pick(w["wing"], ("ms_per_step_mean", "ms_per_step_last20",
+                                     "solution_rel_error_vs_oracle_max_over_steps"))}
+    out["details"] = details
+    return out
+
+
+def write_details(line, path):
+    """Writes the whole record; its path, or None where that fails."""
+    try:
+        with open(path, "w") as f:
+            json.dump(line, f, indent=1)
+        return os.path.relpath(path, ROOT)
+    except OSError as e:
+        print("details not written: %s" % e, file=sys.stderr)
+        return None
 
 
 def _peaks():
