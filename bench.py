@@ -754,7 +754,8 @@ def run_fmm_workload(reps, warm, degrees=(4, 6, 8), n_truth=32768, flush=None):
             p2p_peak = pk["fp64"] if prec == 0 else pk["fp32"]
             p2p_ach = FLOP_P2P_PAIR * sx["n_p2p_pairs"] / (sx["ms_p2p"] * 1e-3) / 1e12
             r["roofline"] = {
-                "m2l": {"bound": "hbm", "achieved": round(byts / (m2l_ms * 1e-3) / 1e9, 1),
+                "m2l": {"bound": "hbm", "limited_by": "fp64 tensor pipe",
+                        "achieved": round(byts / (m2l_ms * 1e-3) / 1e9, 1),
                         "peak": pk["hbm_gbs"], "unit": "GB/s",
                         "frac": round(byts / (m2l_ms * 1e-3) / 1e9 / pk["hbm_gbs"], 3),
                         "tflops": round(flo / (m2l_ms * 1e-3) / 1e12, 2),
@@ -1172,12 +1173,15 @@ def roofline(ph, case, params, best):
                    "traffic": None, "peak_source": simt_name, "flop_per_pair": FLOP_ELEM_PAIR,
                    "pairs": p["n_elem_pairs"], "ms": p["fmm_elements"]})
     if p.get("k_m2l_batch_ms"):
-        # bytes counted in the mode's words (the kernel itself is FP64 on the
-        # tensor pipe in every mode, whose peak is the FP64 SIMT one)
+        # bytes counted by the algorithm in the mode's words, which is a convention:
+        # the kernel reads FP64 in every mode, and what limits it is the FP64 tensor
+        # pipe (the flops entry; its peak is the FP64 SIMT one)
         t = p["k_m2l_batch_ms"] * 1e-3
         gbs = BYTES_M2L_PAIR_WORDS * w * p["n_m2l_pairs"] / t / 1e9
         fl = FLOP_M2L_PAIR * p["n_m2l_pairs"] / t / 1e12
-        ks.append({"kernel": "k_m2l_batch", "bound": "hbm", "achieved": round(gbs, 1),
+        ks.append({"kernel": "k_m2l_batch", "bound": "hbm",
+                   "limited_by": "fp64 tensor pipe, %.3f of its peak" % (fl / fp64_peak),
+                   "achieved": round(gbs, 1),
                    "peak": round(hbm, 1), "unit": "GB/s", "frac": round(gbs / hbm, 3),
                    "traffic": int(TRAFFIC_M2L_PER_PARTICLE * n),
                    "peak_source": "HBM copy %s" % hbm_src,
