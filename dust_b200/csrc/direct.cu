@@ -261,9 +261,9 @@ __global__ void __launch_bounds__(EO_T) k_elem_far64(FmmDev d, ElemDev e, const 
 // order.  Keeping the heavy FP64 formulas out of the far kernels keeps their
 // register count, and so their occupancy, at the level of the far-field
 // arithmetic, and spreads the near pairs over all threads: the FP64 form
-// evaluated them inside k_elem_out's divergent branches by a thread per two
+// evaluated them inside the far kernel's divergent branches by a thread per two
 // particles (12,800 particles x 440 panels 887 us, 60,000 x 3,270 8.3 ms; now
-// 76 us and 1.0 ms with k_elem_fin).
+// 50 us and 0.9 ms with k_elem_fin).
 //
 // Most tiles lie beyond the far-field radius of every particle of the CTA:
 // the loader threads test each panel against the bounding box of the CTA's
@@ -479,9 +479,7 @@ __global__ void __launch_bounds__(EF2_T, 8) k_elem_far(FmmDev d, ElemDev e, cons
 // overflowed its capacity (near_list.h), every
 // (particle, panel) pair is tested again, with the far kernel's own test, and
 // the list is not used.
-#ifndef EN_MINB
 #define EN_MINB 8
-#endif
 template <bool F32>
 __global__ void __launch_bounds__(128, EN_MINB)
     k_elem_near(FmmDev d, ElemDev e, const FFRec *ff, const unsigned long long *count,
@@ -853,7 +851,7 @@ __global__ void __launch_bounds__(UV2_T, UVD_OCC) k_uvort(int npts, const double
 // (assemble_pressure_sys, src/linsys/mod_pressure_equation.f90:170-186):
 // both sums run over the same (point, particle) pairs and share the
 // difference, rho^2 and rho^-3, so the pressure term adds four FMAs per pair
-// to k_uvort's nineteen FP64 operations instead of a second pass over the
+// to k_uvort's eighteen FP64 operations instead of a second pass over the
 // particles.  pt[i] = sum_q (x_q - p_i) . (dir_q x vel_q) mag_q rho^-3.
 __global__ void __launch_bounds__(UV2_T, UVDP_OCC) k_uvort_pres(int npts, const double *pts, int n,
                                                       const double *cen, const double *dir,
@@ -973,9 +971,7 @@ __global__ void k_uv_gather(int n, const uint32_t *perm, const double *cen, cons
 }
 
 // UV2_PPT points per thread (consecutive CTA slices of UV2_T points)
-#ifndef UV2_PPT
 #define UV2_PPT 4
-#endif
 __global__ void __launch_bounds__(UV2_T, UV2_OCC) k_uvort_sorted(int npts, const double *pts, int n,
                                                         const double *X, const float *F,
                                                         int chunk, double *uv) {

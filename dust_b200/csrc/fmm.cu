@@ -10,19 +10,19 @@
 //    particle range (the reference's pointer lists, mod_octree.f90:746-773
 //    and 911-961, in the same order);
 //  * the reference's leaf rule (npart >= min_octree_part at fixed depth,
-//    siblings of leaves become leaves, :896-962) runs as one dense kernel
-//    per level over Morton-ordered flag arrays; active cells and leaves are
-//    compacted with device scans;
+//    siblings of leaves become leaves, :896-962) runs over Morton-ordered flag
+//    arrays, three levels a launch; active cells and leaves are compacted with
+//    one device scan;
 //  * multipole data live in compact per-active-cell SoA blocks;
 //  * M2L evaluates the degree-(p+1) velocity local expansion g once and
 //    derives the reference's gradient coefficients from it exactly,
 //    c(r,:,m) = (m_r+1) g(:, m+e_r); the velocity coefficients b (degree p)
 //    and g are translated with the reference's own truncations in L2L;
-//  * L2P is fused into the leaf-pair P2P kernel: one CTA per leaf, the
-//    near-field source ranges concatenated into one virtual index space
-//    streamed through shared memory in 128-particle tiles, thread groups
-//    splitting the sources of small leaves, group partials reduced through
-//    shared memory.
+//  * L2P is fused into the leaf-pair P2P kernel: one warp per leaf, or per item
+//    of a leaf with a large near field; the near-field source ranges are
+//    concatenated into one virtual index space streamed through shared memory in
+//    32-particle tiles, lane groups split the sources of small leaves, and their
+//    partial sums meet in shared memory.
 #include <cub/cub.cuh>
 #include <thrust/iterator/transform_iterator.h>
 #include <thrust/iterator/transform_output_iterator.h>
@@ -994,7 +994,7 @@ __device__ __forceinline__ void p2p_pair2_f(const float *tp, const float *ta, co
 // concatenated ranges by a search over the range prefix sums (walked forward
 // tile by tile).
 //   FP64: pairs by p2p_pair on absolute coordinates, summed in FP64.
-//   FP32C (F32): pairs by p2p_pair_f on coordinates relative to the leaf
+//   FP32C (F32): pairs by p2p_pair2_f on coordinates relative to the leaf
 //   centre (differences formed in FP64, rounded once), FP32 partial sums of
 //   up to 128 sources folded into FP64.
 // L2P (mod_octree.f90:1171-1212) is FP64 in both.

@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(256) k_pc_out_bwd(int n, int K, int C, float s
 // and the gradients of Ws (sum_i dz_i,f h_i,k), Wn (with m) and b.  A CTA takes
 // PC_BN nodes and stages their dz, h and m and the two weight matrices: the four
 // products need each of them twice, and a launch each (mask 2.5, both weight
-// gradients 24 and the products 11 us at 6,954 nodes; NETNEW us together).  Node
+// gradients 24 and the products 11 us at 6,954 nodes; 30 us together).  Node
 // groups of 64 keep the additions into the 8,256 gradient words few.
 #define PC_BN 64
 #define PC_BSM ((3 * PC_BN + 2 * PC_H) * PC_H * (int)sizeof(float))

@@ -108,8 +108,8 @@ __global__ void k_rhs_static(const PanelGeo *el, const double *bst, int nst, dou
   __syncthreads();
   const int ie = blockIdx.x * blockDim.x + threadIdx.x;
   if (ie >= nst) return;
-  // 16 columns' loads in flight (as the compiler unrolls it, and chunks of 256:
-    // 27 us for 400 panels, 65 us for 6,000; 5 and 45 us)
+  // 16 columns' loads in flight (in chunks of 256, unrolled by the compiler: 27 us
+  // for 400 panels and 65 us for 6,000; 5 and 45 us)
   double s = 0.0;
   int j = j0;
   for (; j + 16 <= j1; j += 16) {
