@@ -377,7 +377,7 @@ int linsys_solve_lu64(dust_linsys *L, double *res_dev) {
   const double one = 1.0, mone = -1.0;
   // the unpivoted static factors come with their inverse blocks, where those are
   // accepted
-  const bool blocks_s = nst == 0 || L->lu_s.inv_n == nst;
+  const bool blocks_s = nst == 0 || (L->lu_s.inv_n == nst && L->lu_s.inv_ok);
   if (nst > 0 && nmv > 0) {
     if (blocks_s) {
       DUST_TRY(lu_trsm_blocks(L->cb, L->st, L->lu_s, nst, A, n, nmv, A + (size_t)nst * n,
@@ -429,7 +429,7 @@ int linsys_solve_lu64(dust_linsys *L, double *res_dev) {
   }
   L->factored = true;
   DUST_CUDA(cudaMemcpyAsync(res_dev, L->b.p, (size_t)n * 8, cudaMemcpyDeviceToDevice, L->st));
-  if (blocks_s && (nmv == 0 || (!L->last_pivoted && L->lu.inv_n == nmv)))
+  if (blocks_s && (nmv == 0 || (!L->last_pivoted && L->lu.inv_ok)))
     return nst == 0 ? lu_solve_blocks<double>(L->st, L->lu.np_x, n, 1, A, n, res_dev, n, L->lu)
                     : lu_solve_blocks<double>(L->st, L->lu.np_x, n, 1, A, n, res_dev, n, L->lu_s,
                                               nmv > 0 ? &L->lu : nullptr);

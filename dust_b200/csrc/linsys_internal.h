@@ -29,7 +29,7 @@ struct dust_linsys {
   struct dust_precond *pc = nullptr;  // learned preconditioner (GMRES_NN)
   DevBuf kr;                          // GMRES Krylov basis and vectors
   LuWork lu;    // of the moving block (each solve) or the Schur complement
-  LuWork lu_s;  // of the static block: its inverse blocks (lu_s.inv_n > 0) when
+  LuWork lu_s;  // of the static block: its inverse blocks (lu_s.inv_ok) when
                 // the unpivoted factors were accepted
   const PanelGeo *el = nullptr, *wk = nullptr;
   int nwake = 0, n_impl = 0;

@@ -41,7 +41,8 @@ struct LuWork {
   DevBuf np;     // unpivoted LU: max |l| word, inverse triangles of every
                  // diagonal block (kept for lu_inv_build)
   DevBuf inv;    // inverses of L's and U's larger diagonal blocks (lu_inv_build)
-  int inv_n = 0; // order of the system they belong to (0: none, or not accepted)
+  int inv_n = 0; // order of the system they belong to (0: none)
+  bool inv_ok = false;  // their condition lets solves use them
   DevBuf np_x;   // lu_solve_blocks: the intermediate Y = L^-1 B
   LuSide side;   // lu_getrf_nopiv: the next panel's stream
   int nsm = 0;
@@ -80,15 +81,16 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
                    int *ipiv, int gemm_update, int *perm, float *lmax);
 
 // Inverses of the 512 x 512 diagonal blocks of L and U from the kept 64 x 64
-// ones of the last lu_getrf_nopiv on this LuWork (same A, n), into w.inv.  Sets
-// w.inv_n = n where the blocks' condition lets products with them stand for a
-// substitution, else 0: then lu_getrs solves (waits for the stream).
+// ones of the last lu_getrf_nopiv on this LuWork (same A, n), into w.inv.
+// w.inv_ok says whether their condition lets products with them stand for a
+// substitution (waits for the stream).
 template <typename T>
 int lu_inv_build(cudaStream_t st, LuWork &w, int n, const T *A, int lda);
 
 // Solves A X = B (X over B, nrhs columns, ldb) with the unpivoted factors in A
 // and the inverse blocks of w1 (the leading w1.inv_n rows) and, when given, w2
-// (the rest).  `work` holds the intermediate n x nrhs.
+// (the rest): the large ones where accepted, else the kept 64 x 64 ones.  `work`
+// holds the intermediate n x nrhs.
 template <typename T>
 int lu_solve_blocks(cudaStream_t st, DevBuf &work, int n, int nrhs, const T *A, int lda, T *B,
                     int ldb, const LuWork &w1, const LuWork *w2 = nullptr);

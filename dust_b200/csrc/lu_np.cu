@@ -537,6 +537,7 @@ int lu_getrf_nopiv(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, T *A, i
                    int *ipiv, int gemm_update, int *perm, float *lmax) {
   *lmax = 0.f;
   w.inv_n = 0;
+  w.inv_ok = false;
   if (n <= 0) return DUST_OK;
   // inverse triangles of every diagonal block are kept (Linv then Uinv per
   // block) for lu_inv_build

@@ -189,7 +189,7 @@ int linsys_solve_schur_mixed(dust_linsys *L, double *x, double tol, int max_iter
     if (nmv > 0) {
       DUST_CUDA(cudaMemcpyAsync(t32, r32 + nst, (size_t)nmv * 4, cudaMemcpyDeviceToDevice, st));
       if (nst > 0) DUST_TRY(gemv_n<float>(st, nmv, nst, -1.0f, Ads, nmv, d32, 1.0f, t32));
-      if (!L->last_pivoted && L->lu.inv_n == nmv)
+      if (!L->last_pivoted)
         DUST_TRY(lu_solve_blocks<float>(st, L->lu.np_x, nmv, 1, S, nmv, t32, nmv, L->lu));
       else
         DUST_TRY(lu_getrs<float>(L->cb, st, nmv, 1, S, nmv, piv, t32, nmv,

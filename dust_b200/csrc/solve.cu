@@ -143,7 +143,7 @@ int mixed_solve_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, DevBuf &w
       if (it == max_iter) break;
     }
     k_to_f32<<<256, 256, 0, st>>>(nr, R, D32);
-    if (piv == 0 && lu.inv_n == n)
+    if (piv == 0)
       DUST_TRY(lu_solve_blocks<float>(st, lu.np_x, n, nrhs, A32, n, D32, n, lu));
     else
       DUST_TRY(lu_getrs<float>(cb, st, n, nrhs, A32, n, ipiv, D32, n));
@@ -204,9 +204,8 @@ static int dense_lu64_device(cublasHandle_t cb, cudaStream_t st, LuWork &lu, Dev
     if (X != B && cudaMemcpyAsync(X, B, nr * 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       s = DUST_ERR_CUDA;
     if (s == DUST_OK)
-      s = pivd == 0 && lu.inv_n == n
-              ? lu_solve_blocks<double>(st, lu.np_x, n, nrhs, (const double *)F.p, n, X, n, lu)
-              : lu_getrs<double>(cb, st, n, nrhs, (const double *)F.p, n, ipiv, X, n);
+      s = pivd == 0 ? lu_solve_blocks<double>(st, lu.np_x, n, nrhs, (const double *)F.p, n, X, n, lu)
+                    : lu_getrs<double>(cb, st, n, nrhs, (const double *)F.p, n, ipiv, X, n);
     cudaEventRecord(e2, st);
   }
   if (s == DUST_OK && cudaStreamSynchronize(st) == cudaSuccess && r) {

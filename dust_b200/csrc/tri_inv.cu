@@ -20,12 +20,14 @@
 // A product with the inverse of a triangular block T leaves a residual of up to
 // cond(T) = || |T^-1| |T| ||_inf times a substitution's.  Certified factors
 // (multipliers below 1) do not bound it: multipliers of -0.1 alone make it grow like
-// 1.1^512.  So lu_inv_build measures it, and above TI_COND the inverses are not
-// used (w.inv_n = 0): the caller substitutes.  Panels' systems have 1.4 to 6
-// (ellipsoids, rotor and fuselage, their Schur complements), where both ways have
-// the same backward errors; at 700 a solve by blocks has ten times the
-// substitution's, at 2e4 a hundred times.  An FP32 solve is refined, and a
-// sweep gains digits as long as cond(T) 6e-8 is small.
+// 1.1^512.  So lu_inv_build measures it, and above TI_COND a solve takes the
+// 64 x 64 inverses that the factorisation itself used (or the caller
+// substitutes).  Panels' systems have 1.1 to 6 (ellipsoids, rotor and fuselage,
+// their Schur complements), where both ways have the same backward errors; at 700
+// a solve by the large blocks has ten times the substitution's, at 2e4 a hundred
+// times.  An FP32 solve is refined, and a sweep gains digits as long as
+// cond(T) 6e-8 is small.  (A system above the limit, n = 3,001 with 16 right-hand
+// sides: 4.1 ms with the small blocks, 8.4 with the library's substitution.)
 #define TI_B 512
 #define TI_T 64   // tile edge of the products
 #define TI_K 32   // inner dimension staged at once
@@ -234,6 +236,7 @@ __global__ void __launch_bounds__(TI_NT) k_ti_cond(int n, int phase, const T *A,
 template <typename T>
 int lu_inv_build(cudaStream_t st, LuWork &w, int n, const T *A, int lda) {
   w.inv_n = 0;
+  w.inv_ok = false;
   if (n <= 0) return DUST_OK;
   const int nb = ti_blocks(n);
   const size_t per = (size_t)2 * TI_B * TI_B * nb;
@@ -255,7 +258,8 @@ int lu_inv_build(cudaStream_t st, LuWork &w, int n, const T *A, int lda) {
   float cond = INFINITY;
   DUST_CUDA(cudaMemcpyAsync(&cond, bits, sizeof(float), cudaMemcpyDeviceToHost, st));
   DUST_CUDA(cudaStreamSynchronize(st));
-  if (cond <= TI_COND<T>) w.inv_n = n;
+  w.inv_n = n;
+  w.inv_ok = cond <= TI_COND<T>;
   return DUST_OK;
 }
 
@@ -421,13 +425,15 @@ int lu_solve_blocks(cudaStream_t st, DevBuf &work, int n, int nrhs, const T *A, 
                     int ldb, const LuWork &w1, const LuWork *w2) {
   if (n <= 0 || nrhs <= 0) return DUST_OK;
   struct Blk {
-    int k, s;
-    const T *linv;
+    int k, s, ld;          // first row, rows, stride of the inverses
+    const T *linv, *uinv;
   };
   std::vector<Blk> bl;
   auto add = [&](const LuWork &w, int base) {
-    for (int k = 0; k < w.inv_n; k += TI_B)
-      bl.push_back({base + k, std::min(TI_B, w.inv_n - k), ti_linv((const T *)w.inv.p, k / TI_B)});
+    const int ld = w.inv_ok ? TI_B : 64;
+    const T *inv = w.inv_ok ? (const T *)w.inv.p : (const T *)((const char *)w.np.p + 256);
+    for (int k = 0; k < w.inv_n; k += ld, inv += 2 * ld * ld)
+      bl.push_back({base + k, std::min(ld, w.inv_n - k), ld, inv, inv + ld * ld});
     return base + w.inv_n;
   };
   int end = add(w1, 0);
@@ -447,7 +453,7 @@ int lu_solve_blocks(cudaStream_t st, DevBuf &work, int n, int nrhs, const T *A, 
   // L Y = B: Y into X, the rest of B updated; then U X = Y into B
   DUST_CUDA(cudaMemsetAsync(X, 0, (size_t)n * nrhs * sizeof(T), st));
   for (const Blk &b : bl) {
-    ti_mul<T, 1>(st, P, b.s, nrhs, b.s, (T)1, b.linv, TI_B, B + b.k, ldb, X + b.k, n);
+    ti_mul<T, 1>(st, P, b.s, nrhs, b.s, (T)1, b.linv, b.ld, B + b.k, ldb, X + b.k, n);
     const int r = b.k + b.s;
     ti_mul<T, 0>(st, P, n - r, nrhs, b.s, (T)-1, A + (size_t)r + (size_t)b.k * lda, lda, X + b.k, n,
                  B + r, ldb);
@@ -455,8 +461,7 @@ int lu_solve_blocks(cudaStream_t st, DevBuf &work, int n, int nrhs, const T *A, 
   DUST_CUDA(cudaMemset2DAsync(B, (size_t)ldb * sizeof(T), 0, (size_t)n * sizeof(T), nrhs, st));
   for (size_t q = bl.size(); q-- > 0;) {
     const Blk &b = bl[q];
-    ti_mul<T, 2>(st, P, b.s, nrhs, b.s, (T)1, b.linv + (size_t)TI_B * TI_B, TI_B, X + b.k, n,
-                 B + b.k, ldb);
+    ti_mul<T, 2>(st, P, b.s, nrhs, b.s, (T)1, b.uinv, b.ld, X + b.k, n, B + b.k, ldb);
     ti_mul<T, 0>(st, P, b.k, nrhs, b.s, (T)-1, A + (size_t)b.k * lda, lda, B + b.k, ldb, X, n);
   }
   DUST_CUDA(cudaGetLastError());
@@ -466,7 +471,8 @@ int lu_solve_blocks(cudaStream_t st, DevBuf &work, int n, int nrhs, const T *A, 
 int lu_trsm_blocks(cublasHandle_t cb, cudaStream_t st, LuWork &w, int n, const double *A, int lda,
                    int m, double *B, double *C, int ldbc) {
   if (n <= 0 || m <= 0) return DUST_OK;
-  if (w.inv_n != n || cublasSetStream(cb, st) != CUBLAS_STATUS_SUCCESS) return DUST_ERR_BAD_ARG;
+  if (w.inv_n != n || !w.inv_ok || cublasSetStream(cb, st) != CUBLAS_STATUS_SUCCESS)
+    return DUST_ERR_BAD_ARG;
   DUST_TRY(devbuf_grow(w.np_x, (size_t)TI_B * m * 8));
   double *X = (double *)w.np_x.p;
   const double one = 1.0, mone = -1.0, zero = 0.0;
